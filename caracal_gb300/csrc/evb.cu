@@ -17,10 +17,11 @@ struct cr_evb {
 // e, g <- EVB energy and gradient of nbeads beads; e2, g2 are scratch of the
 // same sizes for the second force field.
 int evb_launch(const cr_evb* evb, const double* d_q, int nbeads, double* d_e, double* d_g, double* d_e2,
-               double* d_g2, int precision, cudaStream_t s) {
-  int rc = qmdff_launch(evb->ff1, d_q, nbeads, d_e, d_g, precision, s);
+               double* d_g2, int precision, cudaStream_t s, cr::BeadRows rows) {
+  const int ne = nbeads / rows.P * rows.U;
+  int rc = qmdff_launch(evb->ff1, d_q, ne, d_e, d_g, precision, s, nullptr, rows);
   if (rc) return rc;
-  rc = qmdff_launch(evb->ff2, d_q, nbeads, d_e2, d_g2, precision, s);
+  rc = qmdff_launch(evb->ff2, d_q, ne, d_e2, d_g2, precision, s, nullptr, rows);
   if (rc) return rc;
   if (nbeads <= 0) return CR_OK;
   const int threads = 128;

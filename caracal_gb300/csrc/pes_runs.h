@@ -8,6 +8,8 @@
 
 #include <cuda_runtime.h>
 
+#include "bead_rows.cuh"
+
 namespace cr {
 
 struct StepParams;
@@ -19,8 +21,8 @@ struct PesRuns {
                      cudaStream_t st, int istep, int nsteps);
   // dynamic shared-memory limit of that kernel (set outside a stream capture)
   cudaError_t (*set_smem)(bool mixed, int tpb, size_t smem);
-  // egrad_kernel<surface, mixed>: V and dV/dq of nbeads beads
-  cudaError_t (*egrad)(bool mixed, int nbeads, const double* q, double* V, double* g, cudaStream_t st);
+  // egrad_kernel<surface, mixed>: V and dV/dq of nbeads evaluations at the rows of `rows`
+  cudaError_t (*egrad)(bool mixed, int nbeads, BeadRows rows, const double* q, double* V, double* g, cudaStream_t st);
 };
 
 // The table of CR_PES_H3 / CH4H / CH4OH / OH3 / GEH4OH / BRH2; NULL for any other surface.

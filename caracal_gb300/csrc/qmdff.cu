@@ -123,17 +123,21 @@ namespace cr {
 // occupancy differently from the mixed form; the autotuner below picks.
 template <bool MIXED, int MINB, int MODE = qmdff::kFree>
 __global__ void __launch_bounds__(kQmdffWarps * 32, MINB)
-    qmdff_egrad_kernel(qmdff::Dev D, int nbeads, const double* q, double* e, double* g) {
+    qmdff_egrad_kernel(qmdff::Dev D, int nbeads, BeadRows rows, const double* q, double* e, double* g) {
   extern __shared__ double qsm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n3 = 3 * D.n;
   double* ws = qsm + (size_t)warp * (qmdff::warp_smem_bytes(D.n) / sizeof(double));
   for (int b = blockIdx.x * kQmdffWarps + warp; b < nbeads; b += gridDim.x * kQmdffWarps) {
-    const double* qb = q + (size_t)b * n3;
+    const size_t r = rows.row(b), r2 = rows.twin(b);
+    const double* qb = q + r * n3;
     for (int a = lane; a < n3; a += 32) ws[a] = qb[a];
     __syncwarp();
-    const double v = qmdff::warp_egrad<MIXED, MODE>(D, ws, g + (size_t)b * n3, 1.0, lane, b);
-    if (lane == 0) e[b] = v;
+    const double v = qmdff::warp_egrad<MIXED, MODE>(D, ws, g + r * n3, g + r2 * n3, 1.0, lane, r, r2);
+    if (lane == 0) {
+      e[r] = v;
+      if (r2 != r) e[r2] = v;
+    }
     __syncwarp();
   }
 }
@@ -236,7 +240,7 @@ int qmdff_vjp_launch(const cr_qmdff* ff, const double* d_q, const double* d_v, i
 
 namespace {
 
-using QmdffKernel = void (*)(cr::qmdff::Dev, int, const double*, double*, double*);
+using QmdffKernel = void (*)(cr::qmdff::Dev, int, cr::BeadRows, const double*, double*, double*);
 constexpr int kVariants = 3;
 // [precision][variant]: blocks per SM 2 / 3 / 4 (FP64), 4 / 5 / 6 (mixed)
 const QmdffKernel kKernels[2][kVariants] = {
@@ -251,24 +255,24 @@ const QmdffKernel kNptKernels[2] = {cr::qmdff_egrad_kernel<false, 3, cr::qmdff::
                                     cr::qmdff_egrad_kernel<true, 5, cr::qmdff::kNpt>};
 constexpr int kTuneMinBeads = 2048;  // smaller batches keep the default
 
-int launch_dev(const cr::qmdff::Dev& D, int prec, int v, const double* d_q, int nbeads, double* d_e, double* d_g,
+int launch_dev(const cr::qmdff::Dev& D, int prec, int v, cr::BeadRows rows, const double* d_q, int nbeads, double* d_e, double* d_g,
                cudaStream_t s) {
   const size_t smem = (size_t)kQmdffWarps * cr::qmdff::warp_smem_bytes(D.n);
   int grid = (nbeads + kQmdffWarps - 1) / kQmdffWarps;
   if (grid > 1 << 20) grid = 1 << 20;
   const QmdffKernel k = D.periodic ? kBoxKernels[prec] : kKernels[prec][v];
-  k<<<grid, kQmdffWarps * 32, smem, s>>>(D, nbeads, d_q, d_e, d_g);
+  k<<<grid, kQmdffWarps * 32, smem, s>>>(D, nbeads, rows, d_q, d_e, d_g);
   CR_TRY_CUDA(cudaGetLastError());
   return CR_OK;
 }
 
-int launch_variant(const cr_qmdff* ff, int prec, int v, const double* d_q, int nbeads, double* d_e, double* d_g,
+int launch_variant(const cr_qmdff* ff, int prec, int v, cr::BeadRows rows, const double* d_q, int nbeads, double* d_e, double* d_g,
                    cudaStream_t s) {
-  return launch_dev(ff->dev, prec, v, d_q, nbeads, d_e, d_g, s);
+  return launch_dev(ff->dev, prec, v, rows, d_q, nbeads, d_e, d_g, s);
 }
 
 // The NpT instantiation with the launch's boxes and virial array.
-int launch_npt(const cr_qmdff* ff, int prec, const QmdffNpt& npt, const double* d_q, int nbeads, double* d_e,
+int launch_npt(const cr_qmdff* ff, int prec, const QmdffNpt& npt, cr::BeadRows rows, const double* d_q, int nbeads, double* d_e,
                double* d_g, cudaStream_t s) {
   cr::qmdff::Dev D = ff->dev;
   D.tbox = npt.tbox;
@@ -280,7 +284,7 @@ int launch_npt(const cr_qmdff* ff, int prec, const QmdffNpt& npt, const double* 
   if (nbeads <= 0) return CR_OK;
   int grid = (nbeads + kQmdffWarps - 1) / kQmdffWarps;
   if (grid > 1 << 20) grid = 1 << 20;
-  kNptKernels[prec]<<<grid, kQmdffWarps * 32, smem, s>>>(D, nbeads, d_q, d_e, d_g);
+  kNptKernels[prec]<<<grid, kQmdffWarps * 32, smem, s>>>(D, nbeads, rows, d_q, d_e, d_g);
   CR_TRY_CUDA(cudaGetLastError());
   return CR_OK;
 }
@@ -306,7 +310,7 @@ int qmdff_launch_kinds(const cr_qmdff* ff, unsigned mask, bool ezero, const doub
       if (!((mask >> k) & 1u)) D.sched[p].nb[k] = 0;
   if (!ezero) D.e_zero = 0.0;
   const int v = ff->variant[prec] >= 0 ? ff->variant[prec] : kDefaultVariant;
-  return launch_dev(D, prec, v, d_q, nbeads, d_e, d_g, s);
+  return launch_dev(D, prec, v, cr::all_rows(), d_q, nbeads, d_e, d_g, s);
 }
 
 // Host-array call of a kind subset: e, g overwritten, or accumulated into.
@@ -356,11 +360,11 @@ int qmdff_host_kinds(cr_qmdff* ff, unsigned mask, bool ezero, bool accumulate, c
 // once on the caller's data (each writes the same outputs) and keeps the
 // fastest for this force field and form.
 int qmdff_launch(const cr_qmdff* ff_c, const double* d_q, int nbeads, double* d_e, double* d_g, int precision,
-                 cudaStream_t s, const QmdffNpt* npt) {
+                 cudaStream_t s, const QmdffNpt* npt, cr::BeadRows rows) {
   cr_qmdff* ff = const_cast<cr_qmdff*>(ff_c);
   if (precision != CR_PREC_MIXED && precision != CR_PREC_FP64) return cr_set_error(CR_ERR_ARG, "unknown precision");
   const int prec = precision == CR_PREC_MIXED ? 1 : 0;
-  if (npt) return launch_npt(ff, prec, *npt, d_q, nbeads, d_e, d_g, s);
+  if (npt) return launch_npt(ff, prec, *npt, rows, d_q, nbeads, d_e, d_g, s);
   const size_t smem = (size_t)kQmdffWarps * cr::qmdff::warp_smem_bytes(ff->n);
   // the attribute is set even for nbeads = 0, so a caller can prepare the
   // kernels before a stream capture
@@ -381,7 +385,7 @@ int qmdff_launch(const cr_qmdff* ff_c, const double* d_q, int nbeads, double* d_
       float best = 0.f;
       // one untimed launch first: the first launch of a kernel pays for
       // module load and cold caches, which would count against variant 0
-      int rc0 = launch_variant(ff, prec, 0, d_q, nbeads, d_e, d_g, s);
+      int rc0 = launch_variant(ff, prec, 0, rows, d_q, nbeads, d_e, d_g, s);
       if (rc0) {
         cudaEventDestroy(a);
         cudaEventDestroy(b);
@@ -389,7 +393,7 @@ int qmdff_launch(const cr_qmdff* ff_c, const double* d_q, int nbeads, double* d_
       }
       for (int v = 0; v < kVariants; ++v) {
         cudaEventRecord(a, s);
-        int rc = launch_variant(ff, prec, v, d_q, nbeads, d_e, d_g, s);
+        int rc = launch_variant(ff, prec, v, rows, d_q, nbeads, d_e, d_g, s);
         if (rc) {
           cudaEventDestroy(a);
           cudaEventDestroy(b);
@@ -412,7 +416,7 @@ int qmdff_launch(const cr_qmdff* ff_c, const double* d_q, int nbeads, double* d_
     }
     choice = kDefaultVariant;
   }
-  return launch_variant(ff, prec, choice, d_q, nbeads, d_e, d_g, s);
+  return launch_variant(ff, prec, choice, rows, d_q, nbeads, d_e, d_g, s);
 }
 
 extern "C" {

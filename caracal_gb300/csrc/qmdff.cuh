@@ -1326,11 +1326,12 @@ __host__ __device__ inline size_t warp_smem_bytes(int n) { return (size_t)3 * n 
 
 // Energy (with E_zero) and gradient (times gscale) of one bead by one warp.
 // ws: the warp's shared memory with the bead's FP64 coordinates in its first
-// 3n doubles; gout: the gradient destination.  Returns the energy on every lane.
+// 3n doubles; gout, gout2: the gradient destinations (gout2 = gout: one).  Returns the energy on every lane.
 template <bool MIXED, int MODE = kFree>
-__device__ inline double warp_egrad(const Dev& D, double* ws, double* gout, double gscale, int lane, int bead = 0) {
+__device__ inline double warp_egrad(const Dev& D, double* ws, double* gout, double* gout2, double gscale, int lane, size_t bead = 0,
+                                   size_t twin = 0) {
   // MODE (kFree, kBox, kNpt): with kNpt the bead's trajectory box from D.tbox
-  // and the virial trace into D.vir
+  // and the virial trace into D.vir (rows bead and twin)
   using F = typename std::conditional<MIXED, float, double>::type;
   const int n3 = 3 * D.n;
   double* xs = ws;
@@ -1341,7 +1342,7 @@ __device__ inline double warp_egrad(const Dev& D, double* ws, double* gout, doub
   PBox tb;
   const PBox* pb = nullptr;
   if constexpr (MODE == kNpt) {  // this trajectory's box
-    tb = make_box(D.tbox + 3 * (size_t)(bead / D.tbox_beads));
+    tb = make_box(D.tbox + 3 * (size_t)(bead / (size_t)D.tbox_beads));
     pb = &tb;
   } else if constexpr (MODE == kBox) {
     tb = D.box;
@@ -1374,7 +1375,11 @@ __device__ inline double warp_egrad(const Dev& D, double* ws, double* gout, doub
   if constexpr (MIXED) pair_batches_mixed<MODE>(D, X, G, es, ec, wv, lane);
   else kind_batches<MIXED, 3, 2, MODE>(D, X, G, es, ec, wv, lane);
   kind_batches<MIXED, 4, 3, MODE>(D, X, G, es, ec, wv, lane);
-  for (int a = lane; a < n3; a += 32) gout[a] = gscale * G.get(a);
+  for (int a = lane; a < n3; a += 32) {
+    const double v = gscale * G.get(a);
+    gout[a] = v;
+    if (gout2 != gout) gout2[a] = v;
+  }
   double e = (double)es + (double)ec;
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
@@ -1382,7 +1387,10 @@ __device__ inline double warp_egrad(const Dev& D, double* ws, double* gout, doub
     double w = (double)wv;
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-    if (lane == 0) D.vir[bead] = w;
+    if (lane == 0) {
+      D.vir[bead] = w;
+      if (twin != bead) D.vir[twin] = w;
+    }
   }
   return e + D.e_zero;
 }

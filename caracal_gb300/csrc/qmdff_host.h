@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include "bead_rows.cuh"
 #include "qmdff.cuh"
 
 struct cr_qmdff {
@@ -32,9 +33,10 @@ struct QmdffNpt {
 };
 
 // e[b] (with E_zero) and g = dV/dq for nbeads beads of d_q(3, n, nbeads);
-// npt: per-trajectory boxes and the virial (NULL: the force field's box).
+// npt: per-trajectory boxes and the virial (NULL: the force field's box);
+// rows: the rows that the nbeads evaluations read and write.
 int qmdff_launch(const cr_qmdff* ff, const double* d_q, int nbeads, double* d_e, double* d_g, int precision,
-                 cudaStream_t s, const QmdffNpt* npt = nullptr);
+                 cudaStream_t s, const QmdffNpt* npt = nullptr, cr::BeadRows rows = cr::all_rows());
 
 // Plain-form derivatives for the adjoint (bonds, angles, torsions, NCI pairs):
 // energy, gradient and H w per bead (d_e, d_g, d_dew may be NULL) ...
@@ -49,8 +51,9 @@ int qmdff_vjp_launch(const cr_qmdff* ff, const double* d_q, const double* d_v, i
 int qmdff_nlin(const cr_qmdff* ff);
 
 // dE-EVB of two force fields (csrc/evb.cu): e, g <- EVB energy and gradient;
-// e2, g2 are scratch of the same sizes for the second force field.
+// e2, g2 are scratch of the same sizes for the second force field.  The force
+// fields take the rows of `rows`; nbeads counts all rows.
 struct cr_evb;
 int evb_launch(const cr_evb* evb, const double* d_q, int nbeads, double* d_e, double* d_g, double* d_e2,
-               double* d_g2, int precision, cudaStream_t s);
+               double* d_g2, int precision, cudaStream_t s, cr::BeadRows rows = cr::all_rows());
 cr_qmdff* evb_first(const cr_evb* evb);

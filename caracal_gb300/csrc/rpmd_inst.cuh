@@ -44,11 +44,11 @@ struct RunsOf {
     }
     return cudaErrorInvalidValue;
   }
-  static cudaError_t egrad(bool mixed, int nbeads, const double* q, double* V, double* g, cudaStream_t st) {
+  static cudaError_t egrad(bool mixed, int nbeads, BeadRows rows, const double* q, double* V, double* g, cudaStream_t st) {
     const int bs = 128, nb = (nbeads + bs - 1) / bs;
     if (nbeads <= 0) return cudaSuccess;
-    if (mixed) egrad_kernel<PES, true><<<nb, bs, 0, st>>>(nbeads, q, V, g);
-    else egrad_kernel<PES, false><<<nb, bs, 0, st>>>(nbeads, q, V, g);
+    if (mixed) egrad_kernel<PES, true><<<nb, bs, 0, st>>>(nbeads, rows, q, V, g);
+    else egrad_kernel<PES, false><<<nb, bs, 0, st>>>(nbeads, rows, q, V, g);
     return cudaGetLastError();
   }
   static constexpr PesRuns table() { return PesRuns{MAXTPB, &run, &set_smem, &egrad}; }

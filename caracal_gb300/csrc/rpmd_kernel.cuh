@@ -30,6 +30,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "bead_rows.cuh"
 #include "cr_common.cuh"
 
 namespace cr {
@@ -835,20 +836,26 @@ __global__ void __launch_bounds__(256) rpmd_run_kernel(StepParams prm, int istep
   }
 }
 
-// One thread per bead: V and dV/dq.
+// One thread per evaluated bead: V and dV/dq.
 template <class PES, bool MIXED>
-__global__ void egrad_kernel(int nbeads_total, const double* q, double* V, double* g) {
+__global__ void egrad_kernel(int nbeads_total, BeadRows rows, const double* q, double* V, double* g) {
   constexpr int NC = 3 * PES::N;
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nbeads_total) return;
+  const size_t r = rows.row(b), r2 = rows.twin(b);
   double qq[NC], gg[NC], v;
 #pragma unroll
-  for (int c = 0; c < NC; ++c) qq[c] = q[(size_t)b * NC + c];
+  for (int c = 0; c < NC; ++c) qq[c] = q[r * NC + c];
   if (MIXED) PES::template egrad<float>(qq, v, gg);
   else PES::template egrad<double>(qq, v, gg);
-  V[b] = v;
+  V[r] = v;
 #pragma unroll
-  for (int c = 0; c < NC; ++c) g[(size_t)b * NC + c] = gg[c];
+  for (int c = 0; c < NC; ++c) g[r * NC + c] = gg[c];
+  if (r2 != r) {
+    V[r2] = v;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) g[r2 * NC + c] = gg[c];
+  }
 }
 
 }  // namespace cr

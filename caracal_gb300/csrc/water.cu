@@ -16,7 +16,7 @@ namespace cr {
 // the energy sum.
 template <bool MIXED>
 __global__ void __launch_bounds__(water::kMaxAtoms)
-    water_egrad_kernel(water::Dev D, int nbeads, const double* q, double* e, double* g) {
+    water_egrad_kernel(water::Dev D, int nbeads, BeadRows rows, const double* q, double* e, double* g) {
   extern __shared__ double wsm[];
   const int n = D.n, n3 = 3 * n, tid = threadIdx.x;
   double* xs = wsm;
@@ -24,7 +24,8 @@ __global__ void __launch_bounds__(water::kMaxAtoms)
   float2* hl = reinterpret_cast<float2*>(gi + n3);
   double* red = reinterpret_cast<double*>(hl + n3);
   for (int b = blockIdx.x; b < nbeads; b += gridDim.x) {
-    const double* qb = q + (size_t)b * n3;
+    const size_t r = rows.row(b), r2 = rows.twin(b);
+    const double* qb = q + r * n3;
     for (int k = tid; k < n3; k += blockDim.x) {
       const double v = qb[k];
       xs[k] = v;
@@ -41,10 +42,16 @@ __global__ void __launch_bounds__(water::kMaxAtoms)
     if (tid < n) {
       double f[3] = {gi[3 * tid], gi[3 * tid + 1], gi[3 * tid + 2]};
       en += MIXED ? water::pairs_mixed(D, xs, hl, tid, f) : water::pairs_plain(D, xs, tid, f);
-      double* gb = g + (size_t)b * n3 + 3 * tid;
+      double* gb = g + r * n3 + 3 * tid;
       gb[0] = f[0];
       gb[1] = f[1];
       gb[2] = f[2];
+      if (r2 != r) {
+        double* g2 = g + r2 * n3 + 3 * tid;
+        g2[0] = f[0];
+        g2[1] = f[1];
+        g2[2] = f[2];
+      }
     }
     // energy: warp shuffles, then the warps in order (deterministic)
     for (int o = 16; o >= 1; o >>= 1) en += __shfl_down_sync(0xffffffffu, en, o);
@@ -53,7 +60,8 @@ __global__ void __launch_bounds__(water::kMaxAtoms)
     if (tid == 0) {
       double s = 0.0;
       for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-      e[b] = s;
+      e[r] = s;
+      if (r2 != r) e[r2] = s;
     }
     __syncthreads();
   }
@@ -68,7 +76,7 @@ size_t water_smem(int n) { return (size_t)3 * n * (8 + 8 + 8) + 32 * 8; }
 }  // namespace
 
 int water_launch(const cr_water* w, const double* d_q, int nbeads, double* d_e, double* d_g, int precision,
-                 cudaStream_t s) {
+                 cudaStream_t s, cr::BeadRows rows) {
   if (precision != CR_PREC_MIXED && precision != CR_PREC_FP64) return cr_set_error(CR_ERR_ARG, "unknown precision");
   const size_t smem = water_smem(w->dev.n);
   auto kern = precision == CR_PREC_MIXED ? cr::water_egrad_kernel<true> : cr::water_egrad_kernel<false>;
@@ -76,7 +84,7 @@ int water_launch(const cr_water* w, const double* d_q, int nbeads, double* d_e, 
   if (nbeads <= 0) return CR_OK;
   const int threads = (w->dev.n + 31) / 32 * 32;
   const int grid = std::min(nbeads, 1 << 20);
-  kern<<<grid, threads, smem, s>>>(w->dev, nbeads, d_q, d_e, d_g);
+  kern<<<grid, threads, smem, s>>>(w->dev, nbeads, rows, d_q, d_e, d_g);
   CR_TRY_CUDA(cudaGetLastError());
   return CR_OK;
 }
