@@ -1321,8 +1321,12 @@ __device__ inline void pair_batches_mixed(const Dev& D, const BeadPos& X, Grad<f
 
 // Shared memory per warp (bytes): coordinates (3n doubles), the FP32 split
 // (hi, lo) (3n float pairs) and the gradient (3n doubles, or (sum,
-// compensation) float pairs and the 3n floats of the pair sum).
-__host__ __device__ inline size_t warp_smem_bytes(int n) { return (size_t)3 * n * (8 + 4 + 4 + 8 + 4); }
+// compensation) float pairs and the 3n floats of the pair sum), in whole
+// 16-byte units: the warps' regions follow one another, and 84 n bytes are no
+// multiple of a double for odd n.
+__host__ __device__ inline size_t warp_smem_bytes(int n) {
+  return ((size_t)3 * n * (8 + 4 + 4 + 8 + 4) + 15) / 16 * 16;
+}
 
 // Energy (with E_zero) and gradient (times gscale) of one bead by one warp.
 // ws: the warp's shared memory with the bead's FP64 coordinates in its first
