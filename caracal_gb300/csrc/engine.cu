@@ -181,6 +181,8 @@ struct cr_engine {
   int N = 0, NC = 0, P = 0, T = 0, G = 1, H = 1;
   int block = 32, grid = 1;
   int tpb = 1;  // threads per bead of the persistent step kernel
+  int gpb = 1;  // trajectories per block of that kernel
+  int threads = 32;  // threads that its blocks launch
   size_t smem = 0;
   int istep = 0;
   int launches = 0;
@@ -189,6 +191,8 @@ struct cr_engine {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double *d_q = nullptr, *d_p = nullptr, *d_f = nullptr, *d_epot = nullptr, *d_V = nullptr;
   double *d_pile = nullptr, *d_q0 = nullptr;
+  cr::Limbs* d_maps = nullptr;  // StepParams::ke, ko and pile
+  double* d_parts = nullptr;    // StepParams::psym and panti
   double* d_circ = nullptr;  // [3][P] circulant propagator rows (nm_mode 1)
   int* d_status = nullptr;
   // recrossing children
@@ -217,7 +221,7 @@ struct cr_engine {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   bool split_ready = false;  // split_prepare done
-  // umbrella windows (graph path, analytic surfaces)
+  // umbrella windows (analytic surfaces)
   double *d_umb = nullptr;   // [T] centres, [T] force constants, [T] xsum, [T] xsum2, [T][nbins] histogram
   int* d_umb_flag = nullptr; // [2]: sampling switch, constant 0
   int umb_sampling = 0;      // host copy of the sampling switch
@@ -376,6 +380,50 @@ void build_pile(int P, double beta, double dt, double tau0, std::vector<double>&
   }
 }
 
+// The persistent kernel's linear maps as limbs under one exponent each:
+// the propagator blocks on folded rows x_l + x_{M-l}, x_l - x_{M-l} of the
+// distinct beads (odd P: on the rows themselves; a bead that stands for two
+// counts twice), and the PILE circulants between the carried beads.
+void persistent_maps(cr_engine* e, const cr::PropDims& pd, const std::vector<double>& ke, const std::vector<double>& ko,
+                     const std::vector<double>& pile, std::vector<cr::Limbs>& maps, size_t& off_ko, size_t& off_pile) {
+  cr::StepParams& s = e->prm;
+  const int P = e->P, pair = e->cfg.nm_mode == 0 ? 1 : 0, U = pair ? P / 2 + 1 : P;
+  s.pair = pair;
+  s.U = U;
+  s.guard = cr::fixed_guard(pd.nu);
+  s.pguard = cr::fixed_guard(U);
+  std::vector<double> me(ke), mo(ko);
+  mo.resize((size_t)3 * pd.nr * pd.nv);
+  for (size_t x = 0; x < me.size(); ++x)
+    if (x % pd.nu != 0) me[x] *= 2.0;
+  for (size_t x = 0; x < mo.size(); ++x)
+    if (x % pd.nv != 0) mo[x] *= 2.0;
+  const size_t ne = (size_t)pd.nr * pd.nu, no = (size_t)pd.nr * pd.nv;
+  for (int w = 0; w < 3; ++w) {
+    std::vector<double> both(me.begin() + w * ne, me.begin() + (w + 1) * ne);
+    both.insert(both.end(), mo.begin() + w * no, mo.begin() + (w + 1) * no);
+    s.ek[w] = cr::fixed_exponent(both);
+  }
+  for (int w = 0; w < 3; ++w)
+    cr::fixed_limbs(std::vector<double>(me.begin() + w * ne, me.begin() + (w + 1) * ne), s.ek[w], maps);
+  off_ko = maps.size();
+  for (int w = 0; w < 3; ++w)
+    cr::fixed_limbs(std::vector<double>(mo.begin() + w * no, mo.begin() + (w + 1) * no), s.ek[w], maps);
+  off_pile = maps.size();
+  if (e->cfg.thermostat != CR_THERMO_PILE) return;
+  for (int w = 0; w < 2; ++w) {
+    std::vector<double> m((size_t)U * U);
+    for (int l = 0; l < U; ++l)
+      for (int j = 0; j < U; ++j) {
+        double v = pile[(size_t)w * P + ((j - l) % P + P) % P];
+        if (pair && l > 0 && 2 * l != P) v += pile[(size_t)w * P + (j + l) % P];
+        m[(size_t)l * U + j] = v;
+      }
+    s.ep[w] = cr::fixed_exponent(m);
+    cr::fixed_limbs(m, s.ep[w], maps);
+  }
+}
+
 // Persistent run of nsteps steps.  dev_step: the first step index is read
 // from the device counter, which a second launch then advances (so the pair
 // can be replayed from a graph); the shared-memory limit is then set by the
@@ -385,13 +433,13 @@ int launch_run(cr_engine* e, int nsteps, bool dev_step = false) {
   if (!r) return fail(CR_ERR_UNSUPPORTED, "PES not built");
   const bool mixed = e->cfg.precision == CR_PREC_MIXED;
   if (!dev_step) {
-    CR_CUDA(r->set_smem(mixed, e->tpb, e->smem));
-    CR_CUDA(r->run(e->prm, mixed, e->tpb, e->grid, e->block, e->smem, e->stream, e->istep, nsteps));
+    CR_CUDA(r->set_smem(mixed, e->smem));
+    CR_CUDA(r->run(e->prm, mixed, (e->T + e->gpb - 1) / e->gpb, e->threads, e->smem, e->stream, e->istep, nsteps));
     return CR_OK;
   }
   cr::StepParams prm = e->prm;
   prm.istep_dev = e->d_istep;
-  CR_CUDA(r->run(prm, mixed, e->tpb, e->grid, e->block, e->smem, e->stream, 0, nsteps));
+  CR_CUDA(r->run(prm, mixed, (e->T + e->gpb - 1) / e->gpb, e->threads, e->smem, e->stream, 0, nsteps));
   cr::advance_by_kernel<<<1, 1, 0, e->stream>>>(e->d_istep, nsteps);
   CR_CUDA(cudaGetLastError());
   return CR_OK;
@@ -414,9 +462,12 @@ int launch_group(cr_engine* e, int t0, int tn, cudaStream_t st) {
   prm.epot += t0;
   prm.status += t0;
   prm.vnh += 4 * (size_t)t0;
+  if (prm.panti) {
+    prm.psym += (size_t)t0 * prm.U * e->NC;
+    prm.panti += (size_t)t0 * prm.U * e->NC;
+  }
   if (prm.side) prm.side += (size_t)t0 * prm.side_stride;
-  const int groups = e->block / (e->G * e->tpb);
-  CR_CUDA(r->run(prm, e->cfg.precision == CR_PREC_MIXED, e->tpb, (tn + groups - 1) / groups, e->block, e->smem, st,
+  CR_CUDA(r->run(prm, e->cfg.precision == CR_PREC_MIXED, (tn + e->gpb - 1) / e->gpb, e->threads, e->smem, st,
                  e->istep, 1));
   return CR_OK;
 }
@@ -424,7 +475,7 @@ int launch_group(cr_engine* e, int t0, int tn, cudaStream_t st) {
 int set_run_smem(cr_engine* e) {
   const cr::PesRuns* r = cr::pes_runs(e->cfg.pes);
   if (!r) return fail(CR_ERR_UNSUPPORTED, "PES not built");
-  CR_CUDA(r->set_smem(e->cfg.precision == CR_PREC_MIXED, e->tpb, e->smem));
+  CR_CUDA(r->set_smem(e->cfg.precision == CR_PREC_MIXED, e->smem));
   return CR_OK;
 }
 
@@ -438,7 +489,7 @@ int launch_forces(cr_engine* e) {
 }
 
 // Forces of the large-molecule path from an analytic surface (constrained
-// parents and umbrella windows step through the graph path).
+// parents step through the graph path).
 int egrad_launch(cr_engine* e, cr::BeadRows rows, double* V, double* f) {
   const cr::PesRuns* r = cr::pes_runs(e->cfg.pes);
   if (!r) return fail(CR_ERR_UNSUPPORTED, "PES not built");
@@ -525,12 +576,11 @@ cr::SplitParams split_params_range(const cr_engine* e, int t0, int tn) {
 
 // The kernels of one step of the large-molecule path for the trajectories
 // of s (s = split_params_range(e, t0, tn)) on stream st; the caller advances
-// the device step counter.  Constrained parents and umbrella windows step
-// every trajectory at once on e->stream.  *nl counts the launches.
+// the device step counter.  Constrained parents step every trajectory at once
+// on e->stream.  *nl counts the launches.
 int split_group_launches(cr_engine* e, const cr::SplitParams& s, int t0, int tn, cudaStream_t st, int* nl) {
   const bool whole = t0 == 0 && tn == e->T && st == e->stream;
-  if ((e->parent || s.umbrella) && !whole)
-    return fail(CR_ERR_UNSUPPORTED, "constrained parents and umbrella windows step every trajectory at once");
+  if (e->parent && !whole) return fail(CR_ERR_UNSUPPORTED, "constrained parents step every trajectory at once");
   const int cw = cr::split_chunk(e->P);
   const dim3 grid((e->NC + cw - 1) / cw, tn);
   // under the Berendsen barostat the reference applies no Nose-Hoover chain
@@ -556,7 +606,7 @@ int split_group_launches(cr_engine* e, const cr::SplitParams& s, int t0, int tn,
   rc = split_forces_range(e, t0, tn, true, s.V, s.f, st);
   if (rc) return rc;
   n += e->evb ? 3 : 1;
-  if (s.umbrella) {  // src/verlet.f90:1043-1046
+  if (s.umbrella) {  // a parent that also has windows (src/verlet.f90:1043-1046)
     switch (e->N) {
       case 3: cr::split_umbrella_kernel<3><<<tn, 64, 0, st>>>(s); break;
       case 6: cr::split_umbrella_kernel<6><<<tn, 64, 0, st>>>(s); break;
@@ -681,8 +731,13 @@ int split_run(cr_engine* e, int nsteps) {
   return CR_OK;
 }
 
+// Steps by the persistent kernel: the analytic surfaces except constrained
+// parents (umbrella windows included, although their engines count as graph-path
+// ones in the API: no launch shape to set).
+bool persistent(const cr_engine* e) { return !e->ff && !e->evb && !e->water && !e->parent; }
+
 int dispatch_run(cr_engine* e, int nsteps) {
-  if (e->split) return split_run(e, nsteps);
+  if (!persistent(e)) return split_run(e, nsteps);
   return launch_run(e, nsteps);
 }
 
@@ -697,41 +752,83 @@ int dispatch_forces(cr_engine* e) {
   return launch_forces(e);
 }
 
-// Launch shape for `block` threads per block and `tpb` threads per bead
-// (block a multiple of G tpb, at most 256): false if the surface has no such
-// variant or the group scratch of block/(G tpb) trajectories does not fit.
-bool set_launch_shape(cr_engine* e, int block, int tpb) {
+// Launch shape of `groups` trajectories per block with tpb threads per carried
+// bead: U tpb threads per trajectory (U distinct beads), rounded up to a warp.
+// The nominal block size counts a thread for every bead of the group of
+// G = next_pow2(P), as the API does.  false if the surface has no such variant
+// or the block is too large for the kernel.
+bool apply_shape(cr_engine* e, int groups, int tpb) {
   const cr::PesRuns* r = cr::pes_runs(e->cfg.pes);
   if (!r || (tpb != 1 && tpb != 2 && tpb != 4) || tpb > r->max_tpb) return false;
-  const int GT = e->G * tpb;
-  if (block < GT || block % GT || block > 256) return false;
-  const size_t smem = cr::step_smem_doubles(e->P, e->G, e->NC, block / GT, tpb) * sizeof(double);
-  if (smem > 200 * 1024) return false;
-  e->block = block;
+  const cr::PropDims d = cr::prop_dims(e->P);
+  const int U = e->prm.U;
+  int gpb = std::min(groups, e->T);
+  while (gpb > 1 && cr::step_smem_bytes(d, U, e->NC, gpb) > 220 * 1024) --gpb;
+  const size_t smem = cr::step_smem_bytes(d, U, e->NC, gpb);
+  const int threads = (gpb * U * tpb + 31) / 32 * 32;
+  if (smem > 220 * 1024 || threads > 256) return false;
+  e->block = groups * e->G * tpb;
   e->tpb = tpb;
-  e->grid = (e->T + block / GT - 1) / (block / GT);
+  e->grid = (e->T + groups - 1) / groups;
+  e->gpb = gpb;
+  e->threads = threads;
   e->smem = smem;
+  e->prm.gpb = gpb;
+  e->prm.subs = tpb;
   return true;
 }
 
-// Launch shape: a tiny batch is latency-bound, so it is spread one warp per
-// SM; a large batch uses 128-thread blocks, shrunk until the shared memory
-// fits; one thread per bead.
+// The same for the API's `block` threads per block: a multiple of G tpb, at
+// most 256, its scratch by the API's rule within 200 KB.
+bool set_launch_shape(cr_engine* e, int block, int tpb) {
+  const int GT = e->G * tpb;
+  if (GT < 1 || block < GT || block % GT || block > 256) return false;
+  const cr::PropDims d = cr::prop_dims(e->P);
+  const size_t nominal = 8 * ((size_t)3 * d.nr * (d.nu + d.nv) + 2 * (size_t)e->P +
+                              (block / GT) * ((size_t)2 * e->NC * e->G + (size_t)2 * e->NC * (d.su + d.sv) +
+                                              (size_t)((GT + 31) / 32) * 32));
+  if (nominal > 200 * 1024) return false;
+  return apply_shape(e, block / GT, tpb);
+}
+
+// Built-in launch shape.  A batch of at most a trajectory per scheduler is
+// latency-bound: one trajectory per block, with as many threads per bead as the
+// surface has.  A larger one takes the number of trajectories per block with
+// the least work per scheduler: SMs in whole blocks, resident blocks as
+// registers and shared memory allow, a wave costing its warps per scheduler.
 void choose_launch(cr_engine* e) {
-  const int G = e->G;
   int sms = 152;
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long threads = (long long)e->T * G;
-  int block = (threads <= (long long)sms * 128) ? 32 : 128;
-  if (block < G) block = G;
-  if (block > 256) block = 256;
-  while (block > G && cr::step_smem_doubles(e->P, G, e->NC, block / G) * 8 > 200 * 1024) block /= 2;
-  e->block = block;
-  e->tpb = 1;
-  const int groups = block / G;
-  e->grid = (e->T + groups - 1) / groups;
-  e->smem = cr::step_smem_doubles(e->P, G, e->NC, groups) * sizeof(double);
+  const cr::PesRuns* r = cr::pes_runs(e->cfg.pes);
+  const bool mixed = e->cfg.precision == CR_PREC_MIXED;
+  if (e->T <= 4 * sms)
+    for (int tpb = r ? r->max_tpb : 1; tpb >= 1; tpb /= 2)
+      if (e->G * tpb <= 256 && apply_shape(e, 1, tpb)) return;
+  double best = 0.0;
+  int pick = 1;
+  for (int groups = 1; groups * e->prm.U <= 256 && groups <= 256; ++groups) {
+    if (!apply_shape(e, groups, 1) || e->gpb != std::min(groups, e->T)) continue;
+    int res = 1;
+    if (!r || r->resident(mixed, e->threads, e->smem, &res) != cudaSuccess || res < 1) res = 1;
+    const int blocks = (e->T + groups - 1) / groups, per_sm = (blocks + sms - 1) / sms;
+    const double w = e->threads / 128.0;  // warps per scheduler of one block
+    auto wave = [&](int n) { return n == 0 ? 0.0 : 0.35 + std::max(0.65, 0.65 * n * w); };
+    const double cost = (per_sm / res) * wave(res) + wave(per_sm % res);
+    // among equals the fuller block, up to two warps: more small blocks than
+    // schedulers would share some of them
+    if (best == 0.0 || cost < 0.99 * best || (cost < 1.01 * best && e->threads <= 64)) {
+      best = cost;
+      pick = groups;
+    }
+  }
+  // a second thread per bead, in blocks of about two warps, where all of them
+  // fit the SMs at once (H3 1100 x 16 plain 64.2 -> 59.5 us per step, OH + H2
+  // 1000 x 24 plain 60.5 -> 56.2)
+  if (r && r->max_tpb > 1 && (long long)e->T * e->prm.U * 2 <= (long long)sms * 256 &&
+      apply_shape(e, std::max(1, 32 / e->prm.U), 2))
+    return;
+  apply_shape(e, pick, 1);
 }
 
 }  // namespace
@@ -952,7 +1049,6 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
   e->T = cfg->ntraj;
   e->G = next_pow2(e->P);
   e->H = e->P / 2 + 1;
-  if (!e->split) choose_launch(e);
 
   auto cleanup_fail = [&](int code) {
     cr_engine_destroy(e);
@@ -986,6 +1082,14 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
   std::vector<double> circ;
   if (cfg->nm_mode == 1) build_circulant(e->P, cfg->beta, cfg->dt, circ);
   else circ.assign((size_t)3 * e->P, 0.0);
+  // the persistent kernel's maps on the carried beads, as limbs (fixed_map.cuh)
+  std::vector<cr::Limbs> maps;
+  size_t map_ko = 0, map_pile = 0;
+  if (!e->split) persistent_maps(e, pd, ke, ko, pile, maps, map_ko, map_pile);
+  if (!maps.empty() &&
+      (cudaMalloc(&e->d_maps, maps.size() * sizeof(cr::Limbs)) != cudaSuccess ||
+       cudaMemcpy(e->d_maps, maps.data(), maps.size() * sizeof(cr::Limbs), cudaMemcpyHostToDevice) != cudaSuccess))
+    return cleanup_fail(fail(CR_ERR_CUDA, "upload of the step maps failed"));
   if (cudaMalloc(&e->d_ke, ke.size() * 8) != cudaSuccess || cudaMalloc(&e->d_ko, ko.size() * 8) != cudaSuccess ||
       cudaMalloc(&e->d_pile, pile.size() * 8) != cudaSuccess || cudaMalloc(&e->d_circ, circ.size() * 8) != cudaSuccess)
     return cleanup_fail(fail(CR_ERR_CUDA, "device allocation of the tables failed"));
@@ -1113,8 +1217,6 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
   cr::StepParams& s = e->prm;
   s.T = e->T;
   s.P = e->P;
-  s.G = e->G;
-  s.H = e->H;
   s.thermostat = cfg->thermostat;
   s.andersen_step = cfg->andersen_step > 0 ? cfg->andersen_step : 1;
   s.transrot = cfg->transrot ? 1 : 0;
@@ -1133,18 +1235,28 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
   s.nhc = nhc;
   s.vnh = e->d_vnh;
   s.pd = pd;
-  s.pow2_P = (e->P & (e->P - 1)) == 0 ? 1 : 0;
   s.inv_P = 1.0 / e->P;
+  s.wsum = tm;
   s.nm_mode = cfg->nm_mode;
   s.circ = e->d_circ;
-  s.ke = e->d_ke;
-  s.ko = e->d_ko;
-  s.pile = e->d_pile;
+  s.ke = e->d_maps;
+  s.ko = e->d_maps + map_ko;
+  s.pile = e->d_maps + map_pile;
+  s.pile_b = e->d_pile + e->P;
   s.q = e->d_q;
   s.p = e->d_p;
   s.f = e->d_f;
   s.epot = e->d_epot;
   s.status = e->d_status;
+  if (s.pair && e->P > 2 && (cfg->thermostat == CR_THERMO_ANDERSEN || cfg->thermostat == CR_THERMO_PILE)) {
+    const size_t n = (size_t)e->T * s.U * e->NC;
+    if (cudaMalloc(&e->d_parts, 2 * n * 8) != cudaSuccess ||
+        cudaMemsetAsync(e->d_parts, 0, 2 * n * 8, e->stream) != cudaSuccess)
+      return cleanup_fail(fail(CR_ERR_CUDA, "device allocation of the momentum parts failed"));
+    s.psym = e->d_parts;
+    s.panti = e->d_parts + n;
+  }
+  choose_launch(e);
   *out = e;
   return CR_OK;
 }
@@ -1182,6 +1294,8 @@ int cr_engine_destroy(cr_engine* e) {
   cudaFree(e->d_status);
   cudaFree(e->d_q0);
   cudaFree(e->d_pile);
+  cudaFree(e->d_maps);
+  cudaFree(e->d_parts);
   cudaFree(e->d_side);
   cudaFree(e->d_w);
   cudaFree(e->d_kappa);
@@ -1366,7 +1480,7 @@ static int engine_run_async(cr_engine* e, int nsteps) {
   if (rc) return rc;
   CR_CUDA(cudaEventRecord(e->ev1, e->stream));
   e->istep += nsteps;
-  e->launches = e->split ? e->step_launches * nsteps : 1;
+  e->launches = persistent(e) ? 1 : e->step_launches * nsteps;
   return CR_OK;
 }
 
@@ -1745,6 +1859,9 @@ int cr_engine_set_umbrella(cr_engine* e, const cr_recross* rc, const double* cen
   e->sp.umbrella = 1;
   e->sp.umb = u;
   e->sp.xi = x;
+  e->prm.umb_on = 1;
+  e->prm.umb = u;
+  e->prm.xi = x;
   if (e->graph_exec) {
     cudaGraphExecDestroy(e->graph_exec);
     e->graph_exec = nullptr;
@@ -1882,17 +1999,13 @@ int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* th
                             cudaMemcpyDeviceToDevice, e->stream);
     return err;
   };
-  const int block0 = e->block, tpb0 = e->tpb, istep0 = e->istep;
-  int best = block0, best_tpb = tpb0, rc = CR_OK;
+  const int groups0 = e->block / (e->G * e->tpb), tpb0 = e->tpb, istep0 = e->istep;
+  int best = groups0, best_tpb = tpb0, rc = CR_OK;
   float best_ms = 0.f;
   cudaError_t err = copy_state(true);
   for (int tpb = 1; tpb <= 4 && rc == CR_OK && err == cudaSuccess; tpb *= 2) {
-    const int cand[] = {e->G * tpb, 32, 64, 128, 256};
-    for (int k = 0; k < 5 && rc == CR_OK && err == cudaSuccess; ++k) {
-      const int b = cand[k];
-      bool seen = false;
-      for (int i = 0; i < k; ++i) seen |= cand[i] == b;
-      if (seen || !set_launch_shape(e, b, tpb)) continue;
+    for (int m = 1; m * e->prm.U * tpb <= 256 && rc == CR_OK && err == cudaSuccess; m += m < 8 ? 1 : m / 4) {
+      if (!apply_shape(e, m, tpb)) continue;
       // one untimed step (first launch of this shape), then the timed run
       for (int rep = 0; rep < 2 && rc == CR_OK; ++rep) {
         if ((rc = engine_run_async(e, rep == 0 ? 1 : nsteps))) break;
@@ -1903,7 +2016,7 @@ int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* th
           cudaEventElapsedTime(&ms, e->ev0, e->ev1);
           if (best_ms == 0.f || ms < best_ms) {
             best_ms = ms;
-            best = b;
+            best = m;
             best_tpb = tpb;
           }
         }
@@ -1917,16 +2030,16 @@ int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* th
   cudaFree(save_st);
   e->istep = istep0;
   if (rc) {
-    set_launch_shape(e, block0, tpb0);
+    apply_shape(e, groups0, tpb0);
     return rc;
   }
   if (err != cudaSuccess) {
-    set_launch_shape(e, block0, tpb0);
+    apply_shape(e, groups0, tpb0);
     return fail(CR_ERR_CUDA, cudaGetErrorString(err));
   }
-  set_launch_shape(e, best, best_tpb);
+  apply_shape(e, best, best_tpb);
   drop_graph(e);
-  if (threads_per_block) *threads_per_block = best;
+  if (threads_per_block) *threads_per_block = e->block;
   if (threads_per_bead) *threads_per_bead = best_tpb;
   if (ms_per_step) *ms_per_step = best_ms / nsteps;
   return CR_OK;
@@ -2126,12 +2239,12 @@ struct cr_batch {
 namespace {
 
 int batch_prepare(cr_engine* e) {
-  if (e->split) return split_prepare(e);
+  if (!persistent(e)) return split_prepare(e);
   return set_run_smem(e);
 }
 
 int batch_branch(cr_engine* e, int len) {
-  if (e->split) {
+  if (!persistent(e)) {
     for (int n = 0; n < len; ++n) {
       int rc = split_step_launches(e);
       if (rc) return rc;

@@ -15,12 +15,14 @@ namespace cr {
 struct StepParams;
 
 struct PesRuns {
-  int max_tpb;  // largest threads-per-bead variant of the step kernel built for the surface
-  // rpmd_run_kernel<surface, mixed, tpb><<<grid, block, smem, st>>>(prm, istep, nsteps)
-  cudaError_t (*run)(const StepParams& prm, bool mixed, int tpb, int grid, int block, size_t smem,
-                     cudaStream_t st, int istep, int nsteps);
+  int max_tpb;  // most threads per bead of the step kernel on the surface
+  // rpmd_run_kernel<surface, mixed><<<grid, block, smem, st>>>(prm, istep, nsteps)
+  cudaError_t (*run)(const StepParams& prm, bool mixed, int grid, int block, size_t smem, cudaStream_t st, int istep,
+                     int nsteps);
   // dynamic shared-memory limit of that kernel (set outside a stream capture)
-  cudaError_t (*set_smem)(bool mixed, int tpb, size_t smem);
+  cudaError_t (*set_smem)(bool mixed, size_t smem);
+  // blocks of that many threads and bytes that an SM holds
+  cudaError_t (*resident)(bool mixed, int block, size_t smem, int* blocks);
   // egrad_kernel<surface, mixed>: V and dV/dq of nbeads evaluations at the rows of `rows`
   cudaError_t (*egrad)(bool mixed, int nbeads, BeadRows rows, const double* q, double* V, double* g, cudaStream_t st);
 };

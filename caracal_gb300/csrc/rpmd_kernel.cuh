@@ -6,32 +6,39 @@
 // cosine "normal modes", forces, 1/2 kick, Andersen or PILE thermostat,
 // NaN check, `transrot`.
 //
-// Thread layout: a trajectory owns a group of G = next_pow2(P) consecutive
-// threads, bead j on lane j of the group (lanes j >= P idle).  Groups of
-// G <= 32 live inside one warp; G = 64 or 128 span 2 or 4 warps.
+// Distinct beads.  Caracal's modes C = sqrt(1/P) cos(2 pi j k/P) (src/rfft.f90,
+// src/irfft.f90), a per-mode 2x2 rotation (src/verlet.f90:405-454) and C again
+// give a linear map p' = K1 p + m K2 q, q' = K3 p / m + K1 q with
+// K[j][l] = K[-j][l] = K[j][-l]: its output is the same for beads j and P - j,
+// and it reads only the sums x_l + x_{P-l}.  From the first drift on, positions,
+// gradients and momenta of the two agree, so the kernel carries the U = P/2 + 1
+// distinct beads (all P where nm_mode 1 uses orthonormal modes): the starting
+// state enters as its symmetric part, sums over beads weigh the pairs twice, and
+// what a thermostat adds to the antisymmetric part of p -- which the next
+// drift removes -- is kept only where the run ends on it.
 //
-// Bead coupling.  Caracal applies C = sqrt(1/P) cos(2 pi j k/P) (src/rfft.f90,
-// src/irfft.f90), a per-mode 2x2 rotation (src/verlet.f90:405-454), and C
-// again.  The composite is linear: p' = K1 p + m K2 q, q' = K3 p / m + K1 q
-// with K = C diag(poly) C.  Since poly(k) = poly(P-k), K[j][l] = K[-j][l] =
-// K[j][-l]: beads j and P-j get the same output and only the P/2+1
-// symmetrised inputs s_l = x_l + x_{-l} matter.  For even P (M = P/2),
-// C[M-r][k] = (-1)^k C[r][k], so with K = Ke + Ko split by mode parity,
-// K[r] = Ke[r] + Ko[r] and K[M-r] = Ke[r] - Ko[r]; Ke is even and Ko odd
-// under l -> M-l.  One pass over u_l = s_l + s_{M-l}, v_l = s_l - s_{M-l}
-// gives rows r and M-r together.  The group's lanes share the (coordinate,
-// row pair) tasks, so each unique output is computed once: per coordinate
-// 4 (M/2+1)(M+1) FP64 FMAs for the whole ring polymer, against 4 P (M+1)
-// when every bead computes its own row.
+// Thread layout: a block holds several trajectories; thread b serves bead
+// b mod U of trajectory b / U for the surface, and every other stage is a set
+// of tasks (coordinate rows, row pairs, sums) shared by all threads of the
+// block through shared memory, where q, p and the gradient stay during the
+// run.  The state out of the registers leaves them to the surface.
+//
+// The linear maps run on the integer pipe (fixed_map.cuh).  For even P
+// (M = P/2), C[M-r][k] = (-1)^k C[r][k], so with K = Ke + Ko split by mode
+// parity, K[r] = Ke[r] + Ko[r] and K[M-r] = Ke[r] - Ko[r]; Ke is even and Ko
+// odd under l -> M-l: one pass over x_l + x_{M-l} and x_l - x_{M-l} gives rows
+// r and M - r together.
 //
 // PILE (new; Caracal has Andersen and Nose-Hoover only) uses the orthonormal
 // real normal modes; O^T diag(c) O is circulant, so each half step is two
-// length-P circular convolutions: p' = a * p + sqrt(mP/beta) b * eta.
+// length-P circular convolutions: p' = a * p + sqrt(mP/beta) b * eta, folded
+// onto the distinct beads.
 #pragma once
 #include <cuda_runtime.h>
 
 #include "bead_rows.cuh"
 #include "cr_common.cuh"
+#include "fixed_map.cuh"
 
 namespace cr {
 
@@ -101,9 +108,9 @@ __device__ inline double xi_bimolec_value(const XiDev& x, const double* c) {
   for (int k = 0; k < x.nreac2; ++k)
     for (int d = 0; d < 3; ++d) c2[d] = fma(x.w2[k], c[3 * x.reac2[k] + d], c2[d]);
   const double Red[3] = {c2[0] - c1[0], c2[1] - c1[1], c2[2] - c1[2]};
-  const double rf = sqrt(Rf[0] * Rf[0] + Rf[1] * Rf[1] + Rf[2] * Rf[2]);
-  const double rb = sqrt(Rb[0] * Rb[0] + Rb[1] * Rb[1] + Rb[2] * Rb[2]);
-  const double reds = sqrt(Red[0] * Red[0] + Red[1] * Red[1] + Red[2] * Red[2]);
+  const double rf = fx::sqrt(Rf[0] * Rf[0] + Rf[1] * Rf[1] + Rf[2] * Rf[2]);
+  const double rb = fx::sqrt(Rb[0] * Rb[0] + Rb[1] * Rb[1] + Rb[2] * Rb[2]);
+  const double reds = fx::sqrt(Red[0] * Red[0] + Red[1] * Red[1] + Red[2] * Red[2]);
   const double s1 = (rb - x.break_ref) - (rf - x.form_ref);
   return x.xi_ideal * s1 + (1.0 - x.xi_ideal) * (x.r_inf - reds);
 }
@@ -191,11 +198,26 @@ __host__ __device__ inline double nhc_scale(const NhcParams& c, double eksum, do
   return scale;
 }
 
+// Umbrella windows (verlet with constrain = 0, src/umbrella.f90 mode 0).
+struct UmbrellaDev {
+  const double* center;  // [T] xi of each trajectory's window
+  const double* kforce;  // [T] force constant (Eh)
+  double beta;           // 1 / (k_B T) of the fs term
+  const int* sampling;   // device flag: 1 while the statistics are collected
+  double* xsum;          // [T] sum of xi over the sampled steps
+  double* xsum2;         // [T] sum of xi^2
+  int nbins;             // histogram of xi over [lo, hi) (0: none)
+  double lo, hi;
+  double* hist;          // [T][nbins]
+};
+
 struct StepParams {
   int T;           // trajectories in the launch
   int P;           // beads
-  int G;           // threads per trajectory (power of two >= P)
-  int H;           // P/2 + 1
+  int U;           // beads carried: P/2 + 1 distinct ones, or all P (nm_mode 1)
+  int pair;        // 1: bead j stands for j and P - j too
+  int gpb;         // trajectories per block
+  int subs;        // threads per carried bead
   int thermostat;  // CR_THERMO_*
   int andersen_step;
   int transrot;
@@ -205,18 +227,26 @@ struct StepParams {
   double half_dt;
   double beta;
   double totmass;  // Caracal's transrot total mass (P^2 sum m)
+  double wsum;     // P sum m
   double mass[kMaxAtoms];
   double inv_mass[kMaxAtoms];
   double sigma[kMaxAtoms];    // sqrt(m P / beta): Andersen / PILE noise scale
   PropDims pd;
-  const double* ke;    // [3][nr][nu]: K1, K2, K3 (unit mass), even-mode part (odd P: unique rows)
-  const double* ko;    // [3][nr][nv]: odd-mode part
-  const double* pile;  // [2][P]: circulant a (c1) and b (c2)
+  const Limbs* ke;     // [3][nr][nu]: K1, K2, K3 (unit mass) on folded rows, even-mode part (odd P: all modes)
+  const Limbs* ko;     // [3][nr][nv]: odd-mode part
+  int ek[3];           // their exponents
+  int guard;           // guard bits of the folded rows (fixed_map.cuh)
+  const Limbs* pile;   // [2][U][U] friction and noise maps on the carried beads, [w][l][j]
+  int ep[2];
+  int pguard;
+  const double* pile_b;  // [P] noise circulant (the antisymmetric part at the end of a run)
   NhcParams nhc;
   double* vnh;         // [T][4] Nose-Hoover chain velocities
   double* q;           // [T][P][N][3]
   double* p;
   double* f;
+  double* psym;        // [T][U][N][3] symmetric and antisymmetric part of p as the last run left
+  double* panti;       // them after a draw (NULL: no thermostat draws, or no pairs)
   double* epot;        // [T]
   int* status;         // [T]
   // recrossing children: after each step, side[t*side_stride + istep-side_step0-1]
@@ -226,124 +256,21 @@ struct StepParams {
   int side_stride;
   unsigned char* side;
   XiDev xi;
+  // umbrella windows: bias towards the trajectory's window after the forces
+  int umb_on;
+  UmbrellaDev umb;
   // step counter on the device (a launch replayed from a CUDA graph reads its
   // first step index here); NULL: the launch argument
   const int* istep_dev;
-  int pow2_P;     // P is a power of two: centroids multiply by inv_P (exact)
   double inv_P;
   // nm_mode 1 (orthonormal normal modes): K1, K2, K3 are circulant, row j
-  // holds circ[w][(j - l) mod P] (unit mass); loaded where Ke sits in shared memory
+  // holds circ[w][(j - l) mod P] (unit mass)
   int nm_mode;
   const double* circ;  // [3][P]
 };
 
-// Sum over the G lanes of a group (deterministic tree).  red: per-group
-// shared scratch of (G/32) * NV doubles, used only when G > 32.
-template <int NV>
-__device__ inline void group_sum(double (&v)[NV], int G, double* red, int lane_in_group) {
-  const int w = G < 32 ? G : 32;
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
-    if (o < w) {
-#pragma unroll
-      for (int i = 0; i < NV; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
-    }
-  }
-  if (G > 32) {
-    const int nw = G / 32, wid = lane_in_group / 32;
-    __syncthreads();
-    if ((lane_in_group & 31) == 0) {
-#pragma unroll
-      for (int i = 0; i < NV; ++i) red[wid * NV + i] = v[i];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      double s = red[i];
-      for (int k = 1; k < nw; ++k) s += red[k * NV + i];
-      v[i] = s;
-    }
-  }
-}
-
-// Allreduce over a group of G <= 32 lanes by reduce-scatter and all-gather:
-// at each butterfly level (offset O = G/2 .. 1) a lane keeps half of the
-// values it holds (the lower half if its bit O is clear) and adds the
-// partner's copy of that half, so the FP64 adds per lane total about NV
-// instead of NV log2(G); each sum is then read from the lane holding it.
-// The summation order is fixed (deterministic), not that of group_sum.
-template <int N, int O, int NV>
-__device__ __forceinline__ void rs_levels(double (&v)[NV], int lane) {
-  if constexpr (O >= 1) {
-    constexpr int H = (N + 1) / 2;
-    const bool b = (lane & O) != 0;
-#pragma unroll
-    for (int i = 0; i < H; ++i) {
-      const double hi = (i < N - H) ? v[H + i] : 0.0;
-      const double send = b ? v[i] : hi;
-      const double keep = b ? hi : v[i];
-      v[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
-    }
-    rs_levels<H, O / 2, NV>(v, lane);
-  }
-}
-
-struct RsSrc {
-  int lane, idx;
-};
-// Which lane (within the group) ends up holding the sum of value c, and at
-// which slot, after rs_levels<NV, G/2>.  Every level halves the held set to
-// ceil(n/2) slots on both sides of the split (the upper half of an odd set
-// carries one empty slot), as rs_levels does.
-__host__ __device__ constexpr RsSrc rs_src(int NV, int G, int c) {
-  int n = NV, lo = 0, lane = 0;
-  for (int o = G / 2; o >= 1; o /= 2) {
-    const int h = (n + 1) / 2;
-    if (c - lo >= h) {
-      lane |= o;
-      lo += h;
-    }
-    n = h;
-  }
-  return RsSrc{lane, c - lo};
-}
-
-template <int NV, int G>
-__device__ inline void rs_allreduce(double (&v)[NV], int lane_in_group) {
-  rs_levels<NV, G / 2, NV>(v, lane_in_group);
-  const int base = (int)(threadIdx.x & 31u) & ~(G - 1);
-  double out[NV];
-#pragma unroll
-  for (int c = 0; c < NV; ++c) {
-    const RsSrc src = rs_src(NV, G, c);
-    out[c] = __shfl_sync(0xffffffffu, v[src.idx], base + src.lane);
-  }
-#pragma unroll
-  for (int c = 0; c < NV; ++c) v[c] = out[c];
-}
-
-// Sum over the G lanes of a group, on every lane: reduce-scatter for groups
-// inside one warp, the tree of group_sum for groups spanning warps.
-template <int NV>
-__device__ inline void group_allreduce(double (&v)[NV], int G, double* red, int lane_in_group) {
-  switch (G) {
-    case 32: rs_allreduce<NV, 32>(v, lane_in_group); return;
-    case 16: rs_allreduce<NV, 16>(v, lane_in_group); return;
-    case 8: rs_allreduce<NV, 8>(v, lane_in_group); return;
-    case 4: rs_allreduce<NV, 4>(v, lane_in_group); return;
-    case 2: rs_allreduce<NV, 2>(v, lane_in_group); return;
-    case 1: return;
-    default: group_sum<NV>(v, G, red, lane_in_group);
-  }
-}
-
 // Non-finite test on the exponent bits (integer pipe, no FP64 compare).
 __device__ inline bool nonfinite_bits(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
-
-__device__ inline void group_sync(int G) {
-  if (G > 32) __syncthreads();
-  else __syncwarp();
-}
 
 // Gauss-Jordan inverse with full pivoting of a 3x3 matrix (the algorithm of
 // Caracal's invert, src/invert.f90:38-124).  Returns false if singular.
@@ -378,7 +305,7 @@ __device__ inline bool invert3(double (&a)[3][3]) {
     indxr[i] = irow;
     indxc[i] = icol;
     if (a[icol][icol] == 0.0) return false;
-    double ipivot = 1.0 / a[icol][icol];
+    double ipivot = fx::rcp(a[icol][icol]);
     a[icol][icol] = 1.0;
 #pragma unroll
     for (int j = 0; j < 3; ++j) a[icol][j] *= ipivot;
@@ -406,433 +333,672 @@ __device__ inline bool invert3(double (&a)[3][3]) {
   return true;
 }
 
-// Dynamic shared memory layout (doubles):
-//   [0, 3 nr (nu + nv))            propagator blocks Ke, Ko of K1, K2, K3
-//   then 2P                        PILE circulant vectors a, b
-//   then per group: xs[2 NC][G] (reused as the outputs [2 NC][P/2+1]),
-//                   u[2 NC][su], v[2 NC][sv], red[(GT/32) * 32] with GT = G TPB
-__host__ __device__ inline size_t step_group_doubles(int P, int G, int NC, int tpb = 1) {
-  const PropDims d = prop_dims(P);
-  return (size_t)2 * NC * G + (size_t)2 * NC * (d.su + d.sv) + (size_t)((G * tpb + 31) / 32) * 32;
-}
-__host__ __device__ inline size_t step_smem_doubles(int P, int G, int NC, int groups, int tpb = 1) {
-  const PropDims d = prop_dims(P);
-  return (size_t)3 * d.nr * (d.nu + d.nv) + 2 * (size_t)P + step_group_doubles(P, G, NC, tpb) * groups;
+// transrot's move from the fifteen moment sums over beads and atoms (sum p;
+// sum w x; sum x cross p; sum w x x^T as xx, xy, xz, yy, yz, zz): p <- p - m (b +
+// va cross x) with b in mv[0..2], va in mv[3..5].  The second moments about
+// Caracal's rotation centre xt come from the raw ones by the parallel-axis
+// identity C = S - xt Sx^T - Sx xt^T + W xt xt^T, W = sum w.  false: singular.
+__device__ inline bool transrot_move(const double* tot, double tm, double W, bool two_atoms, double* mv) {
+  const double itm = fx::rcp(tm);
+  const double vt[3] = {tot[0] * itm, tot[1] * itm, tot[2] * itm};
+  const double xt[3] = {tot[3] * itm, tot[4] * itm, tot[5] * itm};
+  const double cxx = tot[9] - 2.0 * xt[0] * tot[3] + W * xt[0] * xt[0];
+  const double cxy = tot[10] - xt[0] * tot[4] - tot[3] * xt[1] + W * xt[0] * xt[1];
+  const double cxz = tot[11] - xt[0] * tot[5] - tot[3] * xt[2] + W * xt[0] * xt[2];
+  const double cyy = tot[12] - 2.0 * xt[1] * tot[4] + W * xt[1] * xt[1];
+  const double cyz = tot[13] - xt[1] * tot[5] - tot[4] * xt[2] + W * xt[1] * xt[2];
+  const double czz = tot[14] - 2.0 * xt[2] * tot[5] + W * xt[2] * xt[2];
+  const double mang[3] = {tot[6] - (xt[1] * vt[2] - xt[2] * vt[1]) * tm,
+                          tot[7] - (xt[2] * vt[0] - xt[0] * vt[2]) * tm,
+                          tot[8] - (xt[0] * vt[1] - xt[1] * vt[0]) * tm};
+  double ten[3][3] = {{cyy + czz, -cxy, -cxz}, {-cxy, cxx + czz, -cyz}, {-cxz, -cyz, cxx + cyy}};
+  if (two_atoms) {
+    ten[0][0] += 0.000001;
+    ten[1][1] += 0.000001;
+    ten[2][2] += 0.000001;
+  }
+  if (!invert3(ten)) return false;
+  double va[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) va[a] = ten[a][0] * mang[0] + ten[a][1] * mang[1] + ten[a][2] * mang[2];
+  mv[0] = vt[0] - (va[1] * xt[2] - va[2] * xt[1]);
+  mv[1] = vt[1] - (va[2] * xt[0] - va[0] * xt[2]);
+  mv[2] = vt[2] - (va[0] * xt[1] - va[1] * xt[0]);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) mv[3 + a] = va[a];
+  return true;
 }
 
-// Threads per bead (TPB = 1, 2, 4).  A trajectory owns GT = G TPB
-// consecutive threads: thread l of the group serves bead j = l mod G as its
-// sub-thread s = l / G.  Sub-thread s owns the atoms a with a mod TPB = s:
-// their q, p, f stay in its registers (slot 3 (a / TPB) + d), and it does
-// their share of every per-coordinate stage (kicks, the PILE convolutions,
-// the propagator's output rows, Andersen, the NaN check, the transrot moment
-// sums), so those stages cost 1/TPB per thread; the propagator's
-// (coordinate, row) tasks are shared by all GT threads.  The surface needs
-// the whole bead, so every sub-thread gathers the bead's coordinates
-// through shared memory and evaluates it (the same instructions side by
-// side; no exchange of forces).  Worth it where the batch is too small to
-// fill the GPU and the integrator dominates the bead's work (H3, OH + H2);
-// TPB = 1 is the one-thread-per-bead kernel.
-template <int TPB>
-__host__ __device__ constexpr int own_slot(int c) { return 3 * ((c / 3) / TPB) + c % 3; }
+__device__ __forceinline__ Limbs ldg_limbs(const Limbs* p) {
+  const int2 v = __ldg(reinterpret_cast<const int2*>(p));
+  return Limbs{v.x, v.y};
+}
 
-template <class PES, bool MIXED, int TPB>
-__global__ void __launch_bounds__(256) rpmd_run_kernel(StepParams prm, int istep_arg, int nsteps) {
+// Umbrella bias at the centroid c (src/umbrella.f90:100-176, mode 0): the
+// gradient of 1/2 k (xi - xi0)^2 - (1/beta) log fs with xi = s0 / (s0 - s1)
+// (calc_xi mode 1, src/calc_xi.f90:63-279) and fs^2 = sum dxi^2/m / (2 pi beta),
+// i.e. k (xi - xi0) dxi - H(dxi/m) / (beta sum dxi^2/m), into bias.  xi depends
+// on c through three vectors only (forming bond, breaking bond, distance of the
+// reactants), so dxi and the Hessian-vector product are combinations of their
+// unit vectors n and of the derivatives t = (u - n (n.u)) / r of n along u.
+// Returns xi.  dxi: scratch of 3 N, which may be c.
+template <int N>
+__device__ inline double umbrella_bias(const XiDev& x, const double* c, const double* mass, const double* inv_mass,
+                                       double center, double kforce, double beta, double* dxi, double* bias) {
+  // v[0] forming bond, v[1] breaking bond, v[2] second reactant - first
+  double v[3][3], r[3], ir[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    v[0][d] = c[3 * x.form0 + d] - c[3 * x.form1 + d];
+    v[1][d] = c[3 * x.brk0 + d] - c[3 * x.brk1 + d];
+    v[2][d] = 0.0;
+  }
+  // a vector's part on the atoms: y += J^T w
+  auto spread = [&](int k, double w0, double w1, double w2, double* y) {
+    const double w[3] = {w0, w1, w2};
+    if (k < 2) {
+      const int p = k == 0 ? x.form0 : x.brk0, m = k == 0 ? x.form1 : x.brk1;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        y[3 * p + d] += w[d];
+        y[3 * m + d] -= w[d];
+      }
+    } else {
+      for (int i = 0; i < x.nreac2; ++i)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) y[3 * x.reac2[i] + d] = fma(x.w2[i], w[d], y[3 * x.reac2[i] + d]);
+      for (int i = 0; i < x.nreac1; ++i)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) y[3 * x.reac1[i] + d] = fma(-x.w1[i], w[d], y[3 * x.reac1[i] + d]);
+    }
+  };
+  for (int i = 0; i < x.nreac2; ++i)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) v[2][d] = fma(x.w2[i], c[3 * x.reac2[i] + d], v[2][d]);
+  for (int i = 0; i < x.nreac1; ++i)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) v[2][d] = fma(-x.w1[i], c[3 * x.reac1[i] + d], v[2][d]);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    fx::sqrt_rsqrt(v[k][0] * v[k][0] + v[k][1] * v[k][1] + v[k][2] * v[k][2], r[k], ir[k]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) v[k][d] *= ir[k];  // unit vector
+  }
+  const double s1 = (r[1] - x.break_ref) - (r[0] - x.form_ref), s0 = x.r_inf - r[2];
+  const double iD = fx::rcp(s0 - s1), iD2 = iD * iD;
+  // dxi = s0/D^2 (n_b - n_f) + s1/D^2 n_e on the vectors' atoms
+  const double a0 = s0 * iD2, a1 = s1 * iD2;
+  for (int i = 0; i < 3 * N; ++i) dxi[i] = bias[i] = 0.0;
+  spread(0, -a0 * v[0][0], -a0 * v[0][1], -a0 * v[0][2], dxi);
+  spread(1, a0 * v[1][0], a0 * v[1][1], a0 * v[1][2], dxi);
+  spread(2, a1 * v[2][0], a1 * v[2][1], a1 * v[2][2], dxi);
+  // along u = dxi / m: the vectors' changes, r' = n.u, n' = t
+  double fs = 0.0;
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double y = dxi[3 * i + d];
+      fs = fma(y * y, inv_mass[i], fs);
+    }
+  double u[3][3], rp[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    u[0][d] = dxi[3 * x.form0 + d] * inv_mass[x.form0] - dxi[3 * x.form1 + d] * inv_mass[x.form1];
+    u[1][d] = dxi[3 * x.brk0 + d] * inv_mass[x.brk0] - dxi[3 * x.brk1 + d] * inv_mass[x.brk1];
+    u[2][d] = 0.0;
+  }
+  for (int i = 0; i < x.nreac2; ++i)
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      u[2][d] = fma(x.w2[i] * inv_mass[x.reac2[i]], dxi[3 * x.reac2[i] + d], u[2][d]);
+  for (int i = 0; i < x.nreac1; ++i)
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      u[2][d] = fma(-x.w1[i] * inv_mass[x.reac1[i]], dxi[3 * x.reac1[i] + d], u[2][d]);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    rp[k] = v[k][0] * u[k][0] + v[k][1] * u[k][1] + v[k][2] * u[k][2];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) u[k][d] = (u[k][d] - v[k][d] * rp[k]) * ir[k];  // t
+  }
+  const double s1p = rp[1] - rp[0], s0p = -rp[2], Dp = s0p - s1p;
+  const double coef = -fx::rcp(beta * fs);
+  const double b0 = coef * iD2 * s0p, b1 = coef * iD2 * s0, e0 = coef * iD2 * s1p, e1 = coef * iD2 * s1;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const double sg = k == 0 ? -1.0 : 1.0;
+    spread(k, sg * (b0 * v[k][0] + b1 * u[k][0]), sg * (b0 * v[k][1] + b1 * u[k][1]),
+           sg * (b0 * v[k][2] + b1 * u[k][2]), bias);
+  }
+  spread(2, e0 * v[2][0] + e1 * u[2][0], e0 * v[2][1] + e1 * u[2][1], e0 * v[2][2] + e1 * u[2][2], bias);
+  const double xi = s0 * iD, kd = kforce * (xi - center) - 2.0 * coef * Dp * iD;
+  for (int i = 0; i < 3 * N; ++i) bias[i] = fma(kd, dxi[i], bias[i]);
+  return xi;
+}
+
+// Sampling statistics of one trajectory's xi.
+__device__ inline void umbrella_sample(const UmbrellaDev& u, size_t t, double xi) {
+  u.xsum[t] = u.xsum[t] + xi;
+  u.xsum2[t] = u.xsum2[t] + xi * xi;
+  if (u.nbins > 0) {
+    const double y = (xi - u.lo) / (u.hi - u.lo) * u.nbins;
+    if (y >= 0.0 && y < u.nbins) u.hist[t * u.nbins + (int)y] += 1.0;
+  }
+}
+
+// Dynamic shared memory: the propagator's limbs (3 nr (nu + nv)), then for the
+// gpb trajectories of the block, each array over all of them:
+//   q, p, f   [NC][U] doubles
+//   area      [2 NC][U]: limbs of the folded rows, PILE limbs, partial sums
+//   sums      [16] doubles, move [8] doubles, chain velocities [4] doubles
+//   exponent of each row [2 NC] int, status int
+__host__ __device__ inline size_t step_group_bytes(int U, int NC) {
+  return (size_t)(5 * NC * U + 16 + 8 + 4) * 8 + ((size_t)(2 * NC + 1) * 4 + 7) / 8 * 8;
+}
+__host__ __device__ inline size_t step_smem_bytes(const PropDims& d, int U, int NC, int groups) {
+  return (size_t)3 * d.nr * (d.nu + d.nv) * 8 + step_group_bytes(U, NC) * groups;
+}
+
+// Threads per bead (TPB = 1, 2, 4).  subs threads share a carried bead: the
+// task stages spread over all gpb U subs threads of the block, the surface is
+// evaluated by the first gpb U.  Worth it where the batch is too small to fill
+// the GPU and the integrator weighs as much as the surface (H3, OH + H2).  The
+// sums do not depend on the block's shape or on subs.
+template <class PES, bool MIXED>
+__global__ void __launch_bounds__(256) rpmd_run_kernel(const __grid_constant__ StepParams prm, int istep_arg, int nsteps) {
   const int istep0 = prm.istep_dev ? *prm.istep_dev : istep_arg;
   constexpr int N = PES::N;
   constexpr int NC = 3 * N;
-  constexpr int NL = 3 * ((N + TPB - 1) / TPB);  // coordinate slots per sub-thread
+  constexpr int NQ = (NC + 3) / 4;  // Philox blocks per bead
   extern __shared__ double smem[];
-  const int P = prm.P, G = prm.G, H = prm.H;
-  const int GT = G * TPB;
-  const int groups = blockDim.x / GT;
-  const int grp = threadIdx.x / GT;
-  const int lg = threadIdx.x % GT;          // thread within the group
-  const int j = (TPB == 1) ? lg : lg % G;   // bead
-  const int sub = (TPB == 1) ? 0 : lg / G;  // sub-thread
-  const int t = blockIdx.x * groups + grp;
-  const bool active = (t < prm.T) && (j < P);
-  // does this sub-thread own coordinate c (c a compile-time loop index)
-  auto mine = [&](int c) { return TPB == 1 || (c / 3) % TPB == sub; };
-
+  const int P = prm.P, U = prm.U, gpb = prm.gpb;
+  const int tid = threadIdx.x, nth = blockDim.x;
+  const int t_first = blockIdx.x * gpb;
+  const int ng = min(gpb, prm.T - t_first);  // trajectories of this block
+  const int nb = ng * U, rows = ng * NC, flat = rows * U;
   const PropDims pd = prm.pd;
   const int nke = 3 * pd.nr * pd.nu, nko = 3 * pd.nr * pd.nv;
-  double* s_ke = smem;
-  double* s_ko = s_ke + nke;
-  double* s_pile = s_ko + nko;
-  double* s_grp = s_pile + 2 * P + step_group_doubles(P, G, NC, TPB) * grp;
-  double* xs = s_grp;                      // [2][NC][G]; after the fold: outputs [2][NC][H]
-  double* su = xs + 2 * NC * G;            // [2 NC][su]
-  double* sv = su + 2 * NC * pd.su;        // [2 NC][sv]
-  double* red = sv + 2 * NC * pd.sv;       // [(GT/32)][32]
+  Limbs* s_ke = reinterpret_cast<Limbs*>(smem);
+  Limbs* s_ko = s_ke + nke;
+  double* sq = smem + nke + nko;
+  double* sp = sq + gpb * NC * U;
+  double* sf = sp + gpb * NC * U;
+  double* area = sf + gpb * NC * U;
+  Limbs* limbs = reinterpret_cast<Limbs*>(area);
+  double* ssum = area + 2 * gpb * NC * U;
+  double* smove = ssum + 16 * gpb;
+  double* svnh = smove + 8 * gpb;
+  int* sexp = reinterpret_cast<int*>(svnh + 4 * gpb);
+  int* sstat = sexp + 2 * NC * gpb;
 
-  if (prm.nm_mode) {
-    for (int x = threadIdx.x; x < 3 * P; x += blockDim.x) s_ke[x] = prm.circ[x];  // 3 P <= nke
-  } else {
-    for (int x = threadIdx.x; x < nke; x += blockDim.x) s_ke[x] = prm.ke[x];
-    for (int x = threadIdx.x; x < nko; x += blockDim.x) s_ko[x] = prm.ko[x];
+  if (!prm.nm_mode) {
+    for (int x = tid; x < nke; x += nth) s_ke[x] = prm.ke[x];
+    for (int x = tid; x < nko; x += nth) s_ko[x] = prm.ko[x];
   }
-  if (prm.thermostat == CR_THERMO_PILE)
-    for (int x = threadIdx.x; x < 2 * P; x += blockDim.x) s_pile[x] = prm.pile[x];
-
-  double q[NL], p[NL], f[NL];
-#pragma unroll
-  for (int k = 0; k < NL; ++k) { q[k] = 0.0; p[k] = 0.0; f[k] = 0.0; }
-  const size_t base = ((size_t)t * P + j) * NC;
-  if (active) {
-#pragma unroll
+  // the bead of this thread (threads below nb subs)
+  const int sub = nb > 0 ? tid / nb : 0;
+  const int b = tid - sub * nb, g = b / U, j = b - g * U;
+  const bool bead = sub == 0;                    // evaluates the surface
+  const bool worker = sub < prm.subs;            // shares the bead's stages
+  const int t = t_first + g;
+  // does a carried bead stand for two
+  auto twin_of = [&](int k) { return prm.pair && k > 0 && 2 * k != P ? P - k : k; };
+  // sum over all P beads of a row of carried ones, in bead order
+  auto bead_sum = [&](const double* x) {
+    if (!prm.pair) {
+      double r = x[0];
+      for (int k = 1; k < U; ++k) r += x[k];
+      return r;
+    }
+    double in = 0.0;
+    for (int k = 1; k <= (P - 1) / 2; ++k) in += x[k];
+    double r = fma(2.0, in, x[0]);
+    if (U > 1 && (P & 1) == 0) r += x[U - 1];
+    return r;
+  };
+  const size_t row_a = ((size_t)t * P + j) * NC, row_b = ((size_t)t * P + twin_of(j)) * NC;
+  const size_t row_u = ((size_t)t * U + j) * NC;
+  double ek_anti = 0.0;  // kinetic share of the antisymmetric starting momenta
+  if (bead) {
     for (int c = 0; c < NC; ++c) {
-      if (!mine(c)) continue;
-      q[own_slot<TPB>(c)] = prm.q[base + c];
-      p[own_slot<TPB>(c)] = prm.p[base + c];
-      f[own_slot<TPB>(c)] = prm.f[base + c];
+      const int x = (g * NC + c) * U + j;
+      double q = prm.q[row_a + c], p = prm.p[row_a + c], f = prm.f[row_a + c];
+      if (row_b != row_a) {
+        const double pb = prm.p[row_b + c], d = 0.5 * (p - pb);
+        ek_anti = fma(d * d, prm.inv_mass[c / 3], ek_anti);
+        q = 0.5 * (q + prm.q[row_b + c]);
+        // the symmetric part; where p is still what the last run left, exactly
+        // the one that it carried, so that a run in pieces is the run in one
+        double ps = 0.5 * (p + pb);
+        if (prm.panti) {
+          const double s = prm.psym[row_u + c], a = prm.panti[row_u + c];
+          if (p == s + a && pb == s - a) ps = s;
+        }
+        p = ps;
+        f = 0.5 * (f + prm.f[row_b + c]);
+      }
+      sq[x] = q;
+      sp[x] = p;
+      sf[x] = f;
     }
   }
-  const uint32_t traj_key = prm.traj0 + (uint32_t)t;
-  int status = 0;
+  for (int x = tid; x < gpb; x += nth) sstat[x] = 0;
+  const bool nhc = prm.thermostat == CR_THERMO_NHC, pile = prm.thermostat == CR_THERMO_PILE;
+  if (nhc && tid < ng)
+    for (int k = 0; k < 4; ++k) svnh[4 * tid + k] = prm.vnh[4 * (size_t)(t_first + tid) + k];
   double vbead = 0.0;
-  const bool nhc = prm.thermostat == CR_THERMO_NHC;
-  double vnh[4] = {0.0, 0.0, 0.0, 0.0};
-  if (nhc && t < prm.T) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) vnh[k] = prm.vnh[4 * (size_t)t + k];
-  }
+  bool anti_left = false;  // the run ends with an antisymmetric part of p (prm.panti)
   __syncthreads();
 
-  // nhc (src/nhc.f90): group sum of p.p/(2m)/P/P, the chain, one scale.
-  auto nhc_half = [&]() {
-    double ek[1] = {0.0};
-    if (active) {
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        if (!mine(3 * i)) continue;
-        const int k = own_slot<TPB>(3 * i);
-        const double pp = p[k] * p[k] + p[k + 1] * p[k + 1] + p[k + 2] * p[k + 2];
-        ek[0] = ek[0] + pp / (2.0 * prm.mass[i]) / P / P;
+  // nhc (src/nhc.f90): sum of p.p/(2m)/P/P, the chain, one scale
+  auto nhc_half = [&](double extra) {
+    if (bead) {
+      double ek = extra;
+      for (int c = 0; c < NC; ++c) {
+        const double p = sp[(g * NC + c) * U + j];
+        ek = fma(p * p, prm.inv_mass[c / 3], ek);
       }
+      area[g * U + j] = ek;
     }
-    group_sum<1>(ek, GT, red, lg);
-    const double sc = nhc_scale(prm.nhc, ek[0], vnh);
-#pragma unroll
-    for (int k = 0; k < NL; ++k) p[k] = sc * p[k];
+    __syncthreads();
+    if (tid < ng) {
+      double v[4];
+      for (int k = 0; k < 4; ++k) v[k] = svnh[4 * tid + k];
+      const double ek = bead_sum(area + tid * U) * (0.5 * prm.inv_P * prm.inv_P);
+      smove[8 * tid] = nhc_scale(prm.nhc, ek, v);
+      for (int k = 0; k < 4; ++k) svnh[4 * tid + k] = v[k];
+    }
+    __syncthreads();
+    for (int x = tid; x < flat; x += nth) sp[x] = smove[8 * (x / (NC * U))] * sp[x];
+    __syncthreads();
   };
 
-  // PILE half step on p (in place); eta from the per-bead Gaussian stream.
-  auto pile_half = [&](uint32_t step, uint32_t tag) {
-    double eta[NC];
-    normals_bead<NC>(prm.seed, traj_key, (uint32_t)j, step, tag, eta);
-    group_sync(GT);
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      if (!mine(c)) continue;
-      xs[c * G + j] = p[own_slot<TPB>(c)];
-      xs[(NC + c) * G + j] = active ? eta[c] : 0.0;
+  // the deviates of bead k and its twin for coordinates 4 i .. 4 i + 3
+  auto quad = [&](int gg, int k, int i, uint32_t step, uint32_t tag, double (&za)[4], double (&zb)[4]) {
+    const uint32_t key = prm.traj0 + (uint32_t)(t_first + gg);
+    const uint4 r = philox4x32_10(make_uint4((uint32_t)i, (uint32_t)k, step, tag), prm.seed, key);
+    bm_pair(r.x, r.y, za[0], za[1]);
+    bm_pair(r.z, r.w, za[2], za[3]);
+    const int kt = twin_of(k);
+    if (kt == k) {
+      for (int d = 0; d < 4; ++d) zb[d] = za[d];
+    } else {
+      const uint4 w = philox4x32_10(make_uint4((uint32_t)i, (uint32_t)kt, step, tag), prm.seed, key);
+      bm_pair(w.x, w.y, zb[0], zb[1]);
+      bm_pair(w.z, w.w, zb[2], zb[3]);
     }
-    group_sync(GT);
-    const double* a = s_pile;
-    const double* b = s_pile + P;
-    if (j < P) {
-      double acc_p[NL], acc_e[NL];
+  };
+
+  // PILE half step on p; the limbs of p's rows, then those of the deviates'
+  // symmetric part (|eta| < 8: one exponent for all)
+  constexpr int kEtaExp = 1025;
+  auto pile_half = [&](uint32_t step, uint32_t tag, bool last) {
+    Limbs* le = limbs + flat;
+    for (int x = tid; x < rows; x += nth) {
+      const double* r = sp + x * U;
+      int e = 0;
+      for (int k = 0; k < U; ++k) e = max(e, exponent_field(r[k]));
+      sexp[x] = e;
+      for (int k = 0; k < U; ++k) limbs[x * U + k] = to_limbs(to_fixed(r[k], e, prm.pguard + 1));
+    }
+    for (int x = tid; x < nb * NQ; x += nth) {
+      const int i = x / nb, y = x - i * nb, gg = y / U, k = y - gg * U;
+      double za[4], zb[4];
+      quad(gg, k, i, step, tag, za, zb);
 #pragma unroll
-      for (int k = 0; k < NL; ++k) { acc_p[k] = 0.0; acc_e[k] = 0.0; }
-      int m = j;  // (j - l) mod P
-      for (int l = 0; l < P; ++l) {
-        const double al = a[m], bl = b[m];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          if (!mine(c)) continue;
-          const int k = own_slot<TPB>(c);
-          acc_p[k] = fma(al, xs[c * G + l], acc_p[k]);
-          acc_e[k] = fma(bl, xs[(NC + c) * G + l], acc_e[k]);
-        }
-        m = (m == 0) ? P - 1 : m - 1;
+      for (int d = 0; d < 4; ++d)
+        if (4 * i + d < NC)
+          le[(gg * NC + 4 * i + d) * U + k] = to_limbs(to_fixed(za[d], kEtaExp, prm.pguard + 1) +
+                                                       to_fixed(zb[d], kEtaExp, prm.pguard + 1));
+    }
+    __syncthreads();
+    for (int x = tid; x < flat; x += nth) {
+      const int r = x / U, k = x - r * U;
+      FixedSum a{0, 0}, e{0, 0};
+      const Limbs* ka = prm.pile + k;
+      const Limbs* kb = ka + U * U;
+      for (int l = 0; l < U; ++l) {
+        a.add(limbs[r * U + l], ldg_limbs(ka + l * U));
+        e.add(le[r * U + l], ldg_limbs(kb + l * U));
       }
+      const int c = r % NC;
+      double v = from_fixed(a.value(), prm.ep[0] + sexp[r] - 1077 + prm.pguard);
+      if (sexp[r] == kFixedNan) v = __longlong_as_double(0x7ff8000000000000ll);
+      // half the sum of the two deviates: one bit of the exponent
+      sp[x] = fma(prm.sigma[c / 3], from_fixed(e.value(), prm.ep[1] + kEtaExp - 1078 + prm.pguard), v);
+    }
+    __syncthreads();
+    if (last && prm.panti) {
+      // b * (the deviates' antisymmetric part), which the next drift would remove
+      for (int x = tid; x < nb * NQ; x += nth) {
+        const int i = x / nb, y = x - i * nb, gg = y / U, k = y - gg * U;
+        double za[4], zb[4];
+        quad(gg, k, i, step, tag, za, zb);
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        if (!mine(c)) continue;
-        const int k = own_slot<TPB>(c);
-        p[k] = acc_p[k] + prm.sigma[c / 3] * acc_e[k];
+        for (int d = 0; d < 4; ++d)
+          if (4 * i + d < NC) area[(gg * NC + 4 * i + d) * U + k] = 0.5 * (za[d] - zb[d]);
       }
+      __syncthreads();
+      for (int x = tid; x < flat; x += nth) {
+        const int r = x / U, k = x - r * U, c = r % NC;
+        double acc = 0.0;
+        for (int l = 1; l <= (P - 1) / 2; ++l)
+          acc = fma(prm.pile_b[k >= l ? k - l : k - l + P] - prm.pile_b[k + l >= P ? k + l - P : k + l], area[r * U + l], acc);
+        prm.panti[((size_t)(t_first + r / NC) * U + k) * NC + c] = twin_of(k) == k ? 0.0 : prm.sigma[c / 3] * acc;
+      }
+      __syncthreads();
     }
   };
 
   for (int n = 1; n <= nsteps; ++n) {
     const int istep = istep0 + n;
-    if (nhc) nhc_half();  // src/verlet.f90:186-208
-    if (prm.thermostat == CR_THERMO_PILE) pile_half((uint32_t)istep, TAG_PILE_A);
+    const bool last = n == nsteps;
+    if (nhc) nhc_half(n == 1 ? ek_anti : 0.0);  // src/verlet.f90:186-208
+    if (pile) pile_half((uint32_t)istep, TAG_PILE_A, false);
 
     // 1/2 kick (src/verlet.f90:216-218)
-#pragma unroll
-    for (int k = 0; k < NL; ++k) p[k] = p[k] - prm.half_dt * f[k];
+    for (int x = tid; x < flat; x += nth) sp[x] = fma(-prm.half_dt, sf[x], sp[x]);
+    __syncthreads();
 
     // free ring polymer (src/verlet.f90:377-463): Caracal's cosine modes, or
     // orthonormal normal modes where nm_mode is set
-    group_sync(GT);
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      if (!mine(c)) continue;
-      xs[c * G + j] = p[own_slot<TPB>(c)];
-      xs[(NC + c) * G + j] = q[own_slot<TPB>(c)];
-    }
-    group_sync(GT);
     if (prm.nm_mode) {
-      // orthonormal normal modes: bead j's row of the circulant K1, K2, K3
-      if (j < P) {
-        const double* c1 = s_ke;
-        const double* c2 = s_ke + P;
-        const double* c3 = s_ke + 2 * P;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          if (!mine(c)) continue;
-          double a1p = 0.0, a1q = 0.0, a2q = 0.0, a3p = 0.0;
-          int m = j;  // (j - l) mod P
-          for (int l = 0; l < P; ++l) {
-            const double xp = xs[c * G + l], xq = xs[(NC + c) * G + l];
-            a1p = fma(c1[m], xp, a1p);
-            a1q = fma(c1[m], xq, a1q);
-            a2q = fma(c2[m], xq, a2q);
-            a3p = fma(c3[m], xp, a3p);
-            m = (m == 0) ? P - 1 : m - 1;
-          }
-          p[own_slot<TPB>(c)] = fma(prm.mass[c / 3], a2q, a1p);
-          q[own_slot<TPB>(c)] = fma(prm.inv_mass[c / 3], a3p, a1q);
+      for (int x = tid; x < flat; x += nth) {
+        const int r = x / U, k = x - r * U, c = r % NC;
+        const double* xp = sp + r * U;
+        const double* xq = sq + r * U;
+        double a1p = 0.0, a1q = 0.0, a2q = 0.0, a3p = 0.0;
+        int m = k;  // (k - l) mod P
+        for (int l = 0; l < P; ++l) {
+          const double c1 = __ldg(prm.circ + m), c2 = __ldg(prm.circ + P + m), c3 = __ldg(prm.circ + 2 * P + m);
+          a1p = fma(c1, xp[l], a1p);
+          a1q = fma(c1, xq[l], a1q);
+          a2q = fma(c2, xq[l], a2q);
+          a3p = fma(c3, xp[l], a3p);
+          m = (m == 0) ? P - 1 : m - 1;
         }
+        area[x] = fma(prm.mass[c / 3], a2q, a1p);
+        area[flat + x] = fma(prm.inv_mass[c / 3], a3p, a1q);
+      }
+      __syncthreads();
+      for (int x = tid; x < flat; x += nth) {
+        const double qn = area[flat + x];
+        sp[x] = area[x];
+        sq[x] = qn;
+        if (nonfinite_bits(qn)) atomicOr(&sstat[x / (NC * U)], CR_TRAJ_NONFINITE);
       }
     } else {
-      // Caracal's transform: fold each coordinate's P values into u (and v): tasks (cc, l)
-      for (int idx = lg; idx < 2 * NC * pd.nu; idx += GT) {
-        const int cc = idx / pd.nu, l = idx - cc * pd.nu;
-        const double* x = xs + cc * G;
-        const double a = sym_at(x, l, P);
-        if (pd.split && 2 * l != pd.M) {
-          const double b = sym_at(x, pd.M - l, P);
-          su[cc * pd.su + l] = a + b;
-          if (l < pd.nv) sv[cc * pd.sv + l] = a - b;
+      // fold: rows of q, then of p, into limbs: x_l + x_{M-l}, x_l - x_{M-l}
+      for (int x = tid; x < 2 * rows; x += nth) {
+        const double* r = x < rows ? sq + x * U : sp + (x - rows) * U;
+        Limbs* o = limbs + x * U;
+        int e = 0;
+        for (int k = 0; k < U; ++k) e = max(e, exponent_field(r[k]));
+        sexp[x] = e;
+        if (pd.split) {
+          for (int l = 0; l < pd.nu; ++l) {
+            const int64_t a = to_fixed(r[l], e, prm.guard);
+            const int64_t c = 2 * l == pd.M ? 0 : to_fixed(r[pd.M - l], e, prm.guard);
+            o[l] = to_limbs(a + c);
+            if (l < pd.nv) o[pd.nu + l] = to_limbs(a - c);
+          }
         } else {
-          su[cc * pd.su + l] = a;
+          for (int l = 0; l < U; ++l) o[l] = to_limbs(to_fixed(r[l], e, prm.guard));
         }
       }
-      group_sync(GT);
-      // row pairs (r, M - r) of every coordinate: tasks (c, r); outputs into xs
-      for (int idx = lg; idx < NC * pd.nr; idx += GT) {
-        const int c = idx / pd.nr, r = idx - c * pd.nr;
-        const double* k1e = s_ke + (0 * pd.nr + r) * pd.nu;
-        const double* k2e = s_ke + (1 * pd.nr + r) * pd.nu;
-        const double* k3e = s_ke + (2 * pd.nr + r) * pd.nu;
-        const double* up = su + c * pd.su;
-        const double* uq = su + (NC + c) * pd.su;
-        double e1q = 0.0, e1p = 0.0, e2q = 0.0, e3p = 0.0;
+      __syncthreads();
+      // rows r and M - r of every coordinate
+      for (int x = tid; x < rows * pd.nr; x += nth) {
+        const int y = x / pd.nr, r = x - y * pd.nr, c = y % NC;
+        const Limbs* uq = limbs + y * U;
+        const Limbs* up = limbs + (rows + y) * U;
+        const Limbs* k1 = s_ke + r * pd.nu;
+        const Limbs* k2 = k1 + pd.nr * pd.nu;
+        const Limbs* k3 = k2 + pd.nr * pd.nu;
+        FixedSum a1q{0, 0}, a1p{0, 0}, a2q{0, 0}, a3p{0, 0};
         for (int l = 0; l < pd.nu; ++l) {
-          const double a1 = k1e[l], a2 = k2e[l], a3 = k3e[l], xq = uq[l], xp = up[l];
-          e1q = fma(a1, xq, e1q);
-          e1p = fma(a1, xp, e1p);
-          e2q = fma(a2, xq, e2q);
-          e3p = fma(a3, xp, e3p);
+          const Limbs vq = uq[l], vp = up[l], w1 = k1[l];
+          a1q.add(vq, w1);
+          a1p.add(vp, w1);
+          a2q.add(vq, k2[l]);
+          a3p.add(vp, k3[l]);
         }
-        double o1q = 0.0, o1p = 0.0, o2q = 0.0, o3p = 0.0;
+        const int64_t e1q = a1q.value(), e1p = a1p.value(), e2q = a2q.value(), e3p = a3p.value();
+        int64_t o1q = 0, o1p = 0, o2q = 0, o3p = 0;
         if (pd.nv > 0) {
-          const double* k1o = s_ko + (0 * pd.nr + r) * pd.nv;
-          const double* k2o = s_ko + (1 * pd.nr + r) * pd.nv;
-          const double* k3o = s_ko + (2 * pd.nr + r) * pd.nv;
-          const double* vp = sv + c * pd.sv;
-          const double* vq = sv + (NC + c) * pd.sv;
+          a1q = a1p = a2q = a3p = FixedSum{0, 0};
+          uq += pd.nu;
+          up += pd.nu;
+          k1 = s_ko + r * pd.nv;
+          k2 = k1 + pd.nr * pd.nv;
+          k3 = k2 + pd.nr * pd.nv;
           for (int l = 0; l < pd.nv; ++l) {
-            const double a1 = k1o[l], a2 = k2o[l], a3 = k3o[l], xq = vq[l], xp = vp[l];
-            o1q = fma(a1, xq, o1q);
-            o1p = fma(a1, xp, o1p);
-            o2q = fma(a2, xq, o2q);
-            o3p = fma(a3, xp, o3p);
+            const Limbs vq = uq[l], vp = up[l], w1 = k1[l];
+            a1q.add(vq, w1);
+            a1p.add(vp, w1);
+            a2q.add(vq, k2[l]);
+            a3p.add(vp, k3[l]);
           }
+          o1q = a1q.value();
+          o1p = a1p.value();
+          o2q = a2q.value();
+          o3p = a3p.value();
         }
         const double m = prm.mass[c / 3], im = prm.inv_mass[c / 3];
-        xs[c * H + r] = fma(m, e2q + o2q, e1p + o1p);
-        xs[(NC + c) * H + r] = fma(im, e3p + o3p, e1q + o1q);
-        if (pd.split && 2 * r != pd.M) {
-          xs[c * H + pd.M - r] = fma(m, e2q - o2q, e1p - o1p);
-          xs[(NC + c) * H + pd.M - r] = fma(im, e3p - o3p, e1q - o1q);
+        const int sq_e = sexp[y] - 1078 + prm.guard, sp_e = sexp[rows + y] - 1078 + prm.guard;
+        const bool bad = sexp[y] == kFixedNan || sexp[rows + y] == kFixedNan;
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          const int k = h == 0 ? r : pd.M - r;
+          if (h == 1 && !(pd.split && 2 * r != pd.M)) break;
+          const double pn = fma(m, from_fixed(e2q + o2q, prm.ek[1] + sq_e), from_fixed(e1p + o1p, prm.ek[0] + sp_e));
+          const double qn = fma(im, from_fixed(e3p + o3p, prm.ek[2] + sp_e), from_fixed(e1q + o1q, prm.ek[0] + sq_e));
+          sp[y * U + k] = bad ? nan : pn;
+          sq[y * U + k] = bad ? nan : qn;
+          // NaN / Inf check of the step (src/verlet.f90:1256-1275)
+          if (bad || nonfinite_bits(qn)) atomicOr(&sstat[y / NC], CR_TRAJ_NONFINITE);
+          o1q = -o1q;
+          o1p = -o1p;
+          o2q = -o2q;
+          o3p = -o3p;
         }
       }
-      group_sync(GT);
-      if (j < P) {
-        const int row = (j <= P - j) ? j : P - j;
+    }
+    __syncthreads();
+
+    // per-bead forces (src/verlet.f90:772-777)
+    if (bead) {
+      double q[NC], gr[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          if (!mine(c)) continue;
-          p[own_slot<TPB>(c)] = xs[c * H + row];
-          q[own_slot<TPB>(c)] = xs[(NC + c) * H + row];
-        }
-      }
+      for (int c = 0; c < NC; ++c) q[c] = sq[(g * NC + c) * U + j];
+      if (MIXED) PES::template egrad<float>(q, vbead, gr);
+      else PES::template egrad<double>(q, vbead, gr);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) sf[(g * NC + c) * U + j] = gr[c];
     }
 
-    // per-bead forces (src/verlet.f90:772-777); with TPB > 1 the bead's
-    // coordinates are first gathered from its sub-threads
-    double g[NC];
-    if constexpr (TPB == 1) {
-      if (MIXED) PES::template egrad<float>(q, vbead, g);
-      else PES::template egrad<double>(q, vbead, g);
-#pragma unroll
-      for (int c = 0; c < NC; ++c) f[c] = active ? g[c] : 0.0;
-    } else {
-      group_sync(GT);
-#pragma unroll
-      for (int c = 0; c < NC; ++c)
-        if (mine(c)) xs[c * G + j] = q[own_slot<TPB>(c)];
-      group_sync(GT);
-      double qb[NC];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) qb[c] = xs[c * G + j];
-      if (MIXED) PES::template egrad<float>(qb, vbead, g);
-      else PES::template egrad<double>(qb, vbead, g);
-#pragma unroll
-      for (int c = 0; c < NC; ++c)
-        if (mine(c)) f[own_slot<TPB>(c)] = active ? g[c] : 0.0;
-      if (sub != 0) vbead = 0.0;  // the bead's energy counts once
+    // umbrella windows (src/verlet.f90:1043-1046): the bias at the centroid on
+    // every bead's gradient
+    if (prm.umb_on) {
+      double* bias = area + rows;
+      for (int x = tid; x < rows; x += nth) area[x] = bead_sum(sq + x * U) * prm.inv_P;
+      __syncthreads();
+      if (tid < ng) {
+        const int tt = t_first + tid;
+        const double xi = umbrella_bias<N>(prm.xi, area + tid * NC, prm.mass, prm.inv_mass, prm.umb.center[tt],
+                                           prm.umb.kforce[tt], prm.umb.beta, area + tid * NC, bias + tid * NC);
+        if (*prm.umb.sampling) umbrella_sample(prm.umb, (size_t)tt, xi);
+      }
+      __syncthreads();
+      for (int x = tid; x < flat; x += nth) sf[x] += bias[x / U];
     }
-    if (!active) vbead = 0.0;
 
     // reaction coordinate of the centroid (umbrella mode 1 of a child step,
     // src/verlet.f90:1049-1050 -> src/umbrella.f90:115-117)
     if (prm.xi_on) {
-      double cq[NC];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) cq[c] = (active && mine(c)) ? q[own_slot<TPB>(c)] : 0.0;
-      group_allreduce<NC>(cq, GT, red, lg);
-      if (active && lg == 0) {
-        // centroid: a multiplication by 1/P where P is a power of two (exact), else the division
-#pragma unroll
-        for (int c = 0; c < NC; ++c) cq[c] = prm.pow2_P ? cq[c] * prm.inv_P : cq[c] / P;
-        const double xi = xi_bimolec_value<N>(prm.xi, cq);
-        prm.side[(size_t)t * prm.side_stride + (istep - prm.side_step0 - 1)] = xi > 0.0 ? 1 : 0;
+      for (int x = tid; x < rows; x += nth) area[x] = bead_sum(sq + x * U) * prm.inv_P;
+      __syncthreads();
+      if (tid < ng) {
+        const double xi = xi_bimolec_value<N>(prm.xi, area + tid * NC);
+        prm.side[(size_t)(t_first + tid) * prm.side_stride + (istep - prm.side_step0 - 1)] = xi > 0.0 ? 1 : 0;
       }
     }
+    __syncthreads();
 
     // 1/2 kick (src/verlet.f90:1060-1062)
-#pragma unroll
-    for (int k = 0; k < NL; ++k) p[k] = p[k] - prm.half_dt * f[k];
+    for (int x = tid; x < flat; x += nth) sp[x] = fma(-prm.half_dt, sf[x], sp[x]);
+    __syncthreads();
 
-    if (nhc) nhc_half();  // src/verlet.f90:1085-1106
+    if (nhc) nhc_half(0.0);  // src/verlet.f90:1085-1106
 
     // Andersen (src/verlet.f90:1159-1165): full resample every andersen_step
     if (prm.thermostat == CR_THERMO_ANDERSEN && (istep % prm.andersen_step) == 0) {
-      double z[NC];
-      normals_bead<NC>(prm.seed, traj_key, (uint32_t)j, (uint32_t)istep, TAG_ANDERSEN, z);
+      for (int x = tid; x < nb * NQ; x += nth) {
+        const int i = x / nb, y = x - i * nb, gg = y / U, k = y - gg * U, kt = twin_of(k);
+        double za[4], zb[4];
+        quad(gg, k, i, (uint32_t)istep, TAG_ANDERSEN, za, zb);
 #pragma unroll
-      for (int c = 0; c < NC; ++c)
-        if (mine(c)) p[own_slot<TPB>(c)] = active ? z[c] * prm.sigma[c / 3] : 0.0;
+        for (int d = 0; d < 4; ++d) {
+          const int c = 4 * i + d;
+          if (c >= NC) continue;
+          const double s = prm.sigma[c / 3];
+          sp[(gg * NC + c) * U + k] = kt == k ? za[d] * s : 0.5 * (za[d] + zb[d]) * s;
+          if (last && prm.panti)
+            prm.panti[((size_t)(t_first + gg) * U + k) * NC + c] = kt == k ? 0.0 : 0.5 * (za[d] - zb[d]) * s;
+        }
+      }
+      anti_left = last && prm.panti;
+      __syncthreads();
     }
-    if (prm.thermostat == CR_THERMO_PILE) pile_half((uint32_t)istep, TAG_PILE_B);
-
-    // NaN / Inf check (src/verlet.f90:1256-1275)
-#pragma unroll
-    for (int k = 0; k < NL; ++k)
-      if (nonfinite_bits(q[k])) status |= CR_TRAJ_NONFINITE;
+    if (pile) {
+      pile_half((uint32_t)istep, TAG_PILE_B, last);
+      anti_left = last && prm.panti;
+    }
 
     // transrot (src/transrot.f90:36-237): removed COM velocity and rotation
-    // centre both carry Caracal's extra 1/P (total mass P^2 sum m).
+    // centre both carry Caracal's extra 1/P (total mass P^2 sum m).  Fifteen
+    // raw moments per bead, in four parts that the bead's threads share, summed
+    // over beads; the second moments about the centre by the parallel axis.
     if (prm.transrot) {
-      double vel[NL];
+      double* part = area;  // [ng][16][U]
+      if (worker) {
+        double* o = part + (g * 16) * U + j;
+        const double* bq = sq + g * NC * U + j;
+        const double* bp = sp + g * NC * U + j;
+        for (int k = sub; k < 4; k += prm.subs) {
+          double a[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+          if (k == 0) {
 #pragma unroll
-      for (int c = 0; c < NC; ++c)
-        if (mine(c)) vel[own_slot<TPB>(c)] = p[own_slot<TPB>(c)] * prm.inv_mass[c / 3];
-      double s1[6] = {0, 0, 0, 0, 0, 0};
+            for (int i = 0; i < N; ++i)
 #pragma unroll
-      for (int i = 0; i < N; ++i) {
-        if (!mine(3 * i)) continue;
-        const int k = own_slot<TPB>(3 * i);
-        const double w = prm.mass[i];
+              for (int d = 0; d < 3; ++d) {
+                a[d] += bp[(3 * i + d) * U];
+                a[3 + d] = fma(prm.mass[i], bq[(3 * i + d) * U], a[3 + d]);
+              }
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          s1[d] = fma(vel[k + d], w, s1[d]);
-          s1[3 + d] = fma(q[k + d], w, s1[3 + d]);
+            for (int d = 0; d < 6; ++d) o[d * U] = a[d];
+          } else if (k == 1) {
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+              const double q0 = bq[(3 * i) * U], q1 = bq[(3 * i + 1) * U], q2 = bq[(3 * i + 2) * U];
+              const double p0 = bp[(3 * i) * U], p1 = bp[(3 * i + 1) * U], p2 = bp[(3 * i + 2) * U];
+              a[0] = fma(q1, p2, fma(-q2, p1, a[0]));
+              a[1] = fma(q2, p0, fma(-q0, p2, a[1]));
+              a[2] = fma(q0, p1, fma(-q1, p0, a[2]));
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) o[(6 + d) * U] = a[d];
+          } else if (k == 2) {
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+              const double q0 = bq[(3 * i) * U], w = prm.mass[i] * q0;
+              a[0] = fma(w, q0, a[0]);
+              a[1] = fma(w, bq[(3 * i + 1) * U], a[1]);
+              a[2] = fma(w, bq[(3 * i + 2) * U], a[2]);
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) o[(9 + d) * U] = a[d];
+          } else {
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+              const double q1 = bq[(3 * i + 1) * U], q2 = bq[(3 * i + 2) * U], w = prm.mass[i] * q1;
+              a[0] = fma(w, q1, a[0]);
+              a[1] = fma(w, q2, a[1]);
+              a[2] = fma(prm.mass[i] * q2, q2, a[2]);
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) o[(12 + d) * U] = a[d];
+          }
         }
       }
-      if (!active) {
-#pragma unroll
-        for (int k = 0; k < 6; ++k) s1[k] = 0.0;
+      __syncthreads();
+      for (int x = tid; x < 15 * ng; x += nth) {
+        const int gg = x / 15, v = x - 15 * gg;
+        ssum[16 * gg + v] = bead_sum(part + (gg * 16 + v) * U);
       }
-      group_allreduce<6>(s1, GT, red, lg);
-      const double itm = 1.0 / prm.totmass;
-      const double vt[3] = {s1[0] * itm, s1[1] * itm, s1[2] * itm};
-      const double xt[3] = {s1[3] * itm, s1[4] * itm, s1[5] * itm};
-      double s2[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll
-      for (int i = 0; i < N; ++i) {
-        if (!mine(3 * i)) continue;
-        const int k = own_slot<TPB>(3 * i);
-        const double w = prm.mass[i];
-        const double* qq = &q[k];
-        const double* vv = &vel[k];
-        s2[0] = fma(qq[1] * vv[2] - qq[2] * vv[1], w, s2[0]);
-        s2[1] = fma(qq[2] * vv[0] - qq[0] * vv[2], w, s2[1]);
-        s2[2] = fma(qq[0] * vv[1] - qq[1] * vv[0], w, s2[2]);
-        const double xd = qq[0] - xt[0], yd = qq[1] - xt[1], zd = qq[2] - xt[2];
-        s2[3] = fma(xd * xd, w, s2[3]);
-        s2[4] = fma(xd * yd, w, s2[4]);
-        s2[5] = fma(xd * zd, w, s2[5]);
-        s2[6] = fma(yd * yd, w, s2[6]);
-        s2[7] = fma(yd * zd, w, s2[7]);
-        s2[8] = fma(zd * zd, w, s2[8]);
-      }
-      if (!active) {
-#pragma unroll
-        for (int k = 0; k < 9; ++k) s2[k] = 0.0;
-      }
-      group_allreduce<9>(s2, GT, red, lg);
-      const double tm = prm.totmass;
-      double mang[3] = {s2[0] - (xt[1] * vt[2] - xt[2] * vt[1]) * tm,
-                        s2[1] - (xt[2] * vt[0] - xt[0] * vt[2]) * tm,
-                        s2[2] - (xt[0] * vt[1] - xt[1] * vt[0]) * tm};
-      double ten[3][3] = {{s2[6] + s2[8], -s2[4], -s2[5]},
-                          {-s2[4], s2[3] + s2[8], -s2[7]},
-                          {-s2[5], -s2[7], s2[3] + s2[6]}};
-      if (N <= 2) {
-        ten[0][0] += 0.000001;
-        ten[1][1] += 0.000001;
-        ten[2][2] += 0.000001;
-      }
-      if (!invert3(ten)) {
-        status |= CR_TRAJ_SINGULAR_INERTIA;
-      } else {
-        double va[3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a) va[a] = ten[a][0] * mang[0] + ten[a][1] * mang[1] + ten[a][2] * mang[2];
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-          if (!mine(3 * i)) continue;
-          double* vv = &vel[own_slot<TPB>(3 * i)];
-          const double* qq = &q[own_slot<TPB>(3 * i)];
-          vv[0] -= vt[0];
-          vv[1] -= vt[1];
-          vv[2] -= vt[2];
-          const double xd = qq[0] - xt[0], yd = qq[1] - xt[1], zd = qq[2] - xt[2];
-          vv[0] = vv[0] - va[1] * zd + va[2] * yd;
-          vv[1] = vv[1] - va[2] * xd + va[0] * zd;
-          vv[2] = vv[2] - va[0] * yd + va[1] * xd;
+      __syncthreads();
+      if (tid < ng) {
+        double tot[15];
+        for (int k = 0; k < 15; ++k) tot[k] = ssum[16 * tid + k];
+        double* mv = smove + 8 * tid;
+        mv[6] = 0.0;
+        if (!transrot_move(tot, prm.totmass, prm.wsum, N <= 2, mv)) {
+          mv[6] = 1.0;
+          atomicOr(&sstat[tid], CR_TRAJ_SINGULAR_INERTIA);
         }
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-          if (mine(c)) p[own_slot<TPB>(c)] = active ? vel[own_slot<TPB>(c)] * prm.mass[c / 3] : 0.0;
       }
+      __syncthreads();
+      if (worker) {
+        const double* mv = smove + 8 * g;
+        if (mv[6] == 0.0) {
+          double* bp = sp + g * NC * U + j;
+          const double* bq = sq + g * NC * U + j;
+          for (int i = sub; i < N; i += prm.subs) {
+            const double w = prm.mass[i], q0 = bq[3 * i * U], q1 = bq[(3 * i + 1) * U], q2 = bq[(3 * i + 2) * U];
+            const double u0 = mv[0] + fma(mv[4], q2, -mv[5] * q1);
+            const double u1 = mv[1] + fma(mv[5], q0, -mv[3] * q2);
+            const double u2 = mv[2] + fma(mv[3], q1, -mv[4] * q0);
+            bp[3 * i * U] = fma(-w, u0, bp[3 * i * U]);
+            bp[(3 * i + 1) * U] = fma(-w, u1, bp[(3 * i + 1) * U]);
+            bp[(3 * i + 2) * U] = fma(-w, u2, bp[(3 * i + 2) * U]);
+          }
+        }
+      }
+      __syncthreads();
     }
   }
 
-  // potential energy of the last step, summed over beads
-  double e[1] = {vbead};
-  group_sum<1>(e, GT, red, lg);
-  if (active) {
-#pragma unroll
+  // the state of every bead, the potential energy of the last step
+  if (bead) {
+    area[g * U + j] = vbead;
     for (int c = 0; c < NC; ++c) {
-      if (!mine(c)) continue;
-      prm.q[base + c] = q[own_slot<TPB>(c)];
-      prm.p[base + c] = p[own_slot<TPB>(c)];
-      prm.f[base + c] = f[own_slot<TPB>(c)];
+      const int x = (g * NC + c) * U + j;
+      const double q = sq[x], p = sp[x], f = sf[x];
+      prm.q[row_a + c] = q;
+      prm.f[row_a + c] = f;
+      if (row_b != row_a) {
+        double a = 0.0;
+        if (anti_left) {
+          a = prm.panti[row_u + c];
+          prm.psym[row_u + c] = p;
+        }
+        prm.p[row_a + c] = p + a;
+        prm.p[row_b + c] = p - a;
+        prm.q[row_b + c] = q;
+        prm.f[row_b + c] = f;
+      } else {
+        prm.p[row_a + c] = p;
+      }
     }
-    if (lg == 0) prm.epot[t] = e[0];
-    if (lg == 0 && nhc) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) prm.vnh[4 * (size_t)t + k] = vnh[k];
-    }
-    if (status) atomicOr(&prm.status[t], status);
+  }
+  __syncthreads();
+  if (tid < ng) {
+    const int tt = t_first + tid;
+    prm.epot[tt] = bead_sum(area + tid * U);
+    if (nhc)
+      for (int k = 0; k < 4; ++k) prm.vnh[4 * (size_t)tt + k] = svnh[4 * tid + k];
+    if (sstat[tid]) atomicOr(&prm.status[tt], sstat[tid]);
   }
 }
 

@@ -33,19 +33,6 @@
 
 namespace cr {
 
-// Umbrella windows (verlet with constrain = 0, src/umbrella.f90 mode 0).
-struct UmbrellaDev {
-  const double* center;  // [T] xi of each trajectory's window
-  const double* kforce;  // [T] force constant (Eh)
-  double beta;           // 1 / (k_B T) of the fs term
-  const int* sampling;   // device flag: 1 while the statistics are collected
-  double* xsum;          // [T] sum of xi over the sampled steps
-  double* xsum2;         // [T] sum of xi^2
-  int nbins;             // histogram of xi over [lo, hi) (0: none)
-  double lo, hi;
-  double* hist;          // [T][nbins]
-};
-
 struct SplitParams {
   int T, P, N, NC;
   int M;          // P / 2
@@ -751,37 +738,10 @@ __global__ void split_solve_kernel(SplitParams s, int S) {
   s.epot[t] = tot[15] + (shake_fail ? 100000.0 : 0.0);
   double* mv = s.fmove + (size_t)t * kMoveDoubles;
   if (s.transrot) {
-    const double itm = 1.0 / s.totmass, tm = s.totmass, W = s.wsum;
-    const double vt[3] = {tot[0] * itm, tot[1] * itm, tot[2] * itm};
-    const double xt[3] = {tot[3] * itm, tot[4] * itm, tot[5] * itm};
-    // centred second moments xx, xy, xz, yy, yz, zz
-    const double cxx = tot[9] - 2.0 * xt[0] * tot[3] + W * xt[0] * xt[0];
-    const double cxy = tot[10] - xt[0] * tot[4] - tot[3] * xt[1] + W * xt[0] * xt[1];
-    const double cxz = tot[11] - xt[0] * tot[5] - tot[3] * xt[2] + W * xt[0] * xt[2];
-    const double cyy = tot[12] - 2.0 * xt[1] * tot[4] + W * xt[1] * xt[1];
-    const double cyz = tot[13] - xt[1] * tot[5] - tot[4] * xt[2] + W * xt[1] * xt[2];
-    const double czz = tot[14] - 2.0 * xt[2] * tot[5] + W * xt[2] * xt[2];
-    const double mang[3] = {tot[6] - (xt[1] * vt[2] - xt[2] * vt[1]) * tm,
-                            tot[7] - (xt[2] * vt[0] - xt[0] * vt[2]) * tm,
-                            tot[8] - (xt[0] * vt[1] - xt[1] * vt[0]) * tm};
-    double ten[3][3] = {{cyy + czz, -cxy, -cxz}, {-cxy, cxx + czz, -cyz}, {-cxz, -cyz, cxx + cyy}};
-    if (s.N <= 2) {
-      ten[0][0] += 0.000001;
-      ten[1][1] += 0.000001;
-      ten[2][2] += 0.000001;
-    }
-    if (!invert3(ten)) {
+    mv[9] = 0.0;
+    if (!transrot_move(tot, s.totmass, s.wsum, s.N <= 2, mv)) {
       status |= CR_TRAJ_SINGULAR_INERTIA;
       mv[9] = 1.0;
-    } else {
-      double va[3];
-      for (int a = 0; a < 3; ++a) va[a] = ten[a][0] * mang[0] + ten[a][1] * mang[1] + ten[a][2] * mang[2];
-      // p <- m (v - vt - va x (x - xt)) = p - m (b + va x x), b = vt - va x xt
-      mv[0] = vt[0] - (va[1] * xt[2] - va[2] * xt[1]);
-      mv[1] = vt[1] - (va[2] * xt[0] - va[0] * xt[2]);
-      mv[2] = vt[2] - (va[0] * xt[1] - va[1] * xt[0]);
-      for (int a = 0; a < 3; ++a) mv[3 + a] = va[a];
-      mv[9] = 0.0;
     }
   }
   if (status) s.status[t] |= status;
@@ -911,67 +871,12 @@ __global__ void split_sum_beads_kernel(int T, int P, const double* V, double* ep
 }
 
 
-// BIMOLEC reaction coordinate of umbrella sampling (calc_xi mode 1,
-// src/calc_xi.f90:63-279): xi = s0 / (s0 - s1) and its gradient
-// (s0 ds1 - s1 ds0) / (s0 - s1)^2.  T = Dual gives, with dual coordinates
-// c + eps u, the Hessian-vector product in the eps parts of dxi.
-template <int N, class T>
-__device__ inline T xi_umbrella(const XiDev& x, const T* c, const double* mass, T* dxi) {
-  constexpr int NC = 3 * N;
-  T Rf[3], Rb[3];
-  for (int d = 0; d < 3; ++d) {
-    Rf[d] = c[3 * x.form0 + d] - c[3 * x.form1 + d];
-    Rb[d] = c[3 * x.brk0 + d] - c[3 * x.brk1 + d];
-  }
-  const T rf = sqrt(Rf[0] * Rf[0] + Rf[1] * Rf[1] + Rf[2] * Rf[2]);
-  const T rb = sqrt(Rb[0] * Rb[0] + Rb[1] * Rb[1] + Rb[2] * Rb[2]);
-  T s1 = T(0.0);
-  s1 = s1 + (rb - x.break_ref) / 1.0;
-  s1 = s1 - (rf - x.form_ref) / 1.0;
-  T c1[3] = {T(0.0), T(0.0), T(0.0)}, c2[3] = {T(0.0), T(0.0), T(0.0)};
-  for (int k = 0; k < x.nreac1; ++k)
-    for (int d = 0; d < 3; ++d) c1[d] = c1[d] + mass[x.reac1[k]] * c[3 * x.reac1[k] + d] / x.mreac1;
-  for (int k = 0; k < x.nreac2; ++k)
-    for (int d = 0; d < 3; ++d) c2[d] = c2[d] + mass[x.reac2[k]] * c[3 * x.reac2[k] + d] / x.mreac2;
-  const T Red[3] = {c2[0] - c1[0], c2[1] - c1[1], c2[2] - c1[2]};
-  const T reds = sqrt(Red[0] * Red[0] + Red[1] * Red[1] + Red[2] * Red[2]);
-  T s0 = T(0.0);
-  s0 = s0 + (x.r_inf - reds);
-  s0 = s0 / 1.0;
-  T ds1[NC], ds0[NC];
-  for (int i = 0; i < NC; ++i) ds1[i] = ds0[i] = T(0.0);
-  T ri = 1.0 / rf;
-  for (int d = 0; d < 3; ++d) {
-    ds1[3 * x.form0 + d] = ds1[3 * x.form0 + d] - Rf[d] * ri / 1.0;
-    ds1[3 * x.form1 + d] = ds1[3 * x.form1 + d] + Rf[d] * ri / 1.0;
-  }
-  ri = 1.0 / rb;
-  for (int d = 0; d < 3; ++d) {
-    ds1[3 * x.brk0 + d] = ds1[3 * x.brk0 + d] + Rb[d] * ri / 1.0;
-    ds1[3 * x.brk1 + d] = ds1[3 * x.brk1 + d] - Rb[d] * ri / 1.0;
-  }
-  ri = 1.0 / reds;
-  for (int k = 0; k < x.nreac1; ++k) {
-    const int a = x.reac1[k];
-    for (int d = 0; d < 3; ++d) ds0[3 * a + d] = ds0[3 * a + d] + Red[d] * ri * mass[a] / x.mreac1 / 1.0;
-  }
-  for (int k = 0; k < x.nreac2; ++k) {
-    const int a = x.reac2[k];
-    for (int d = 0; d < 3; ++d) ds0[3 * a + d] = ds0[3 * a + d] + (-1.0) * Red[d] * ri * mass[a] / x.mreac2 / 1.0;
-  }
-  const T D = s0 - s1;
-  for (int i = 0; i < NC; ++i) dxi[i] = (s0 * ds1[i] - s1 * ds0[i]) / (D * D);
-  return s0 / D;
-}
-
-// Umbrella bias after the forces (src/umbrella.f90:100-176): at the centroid,
-// every bead's gradient gets k (xi - xi0) dxi, then the gradient of
-// -(1/beta) log fs, (-1/beta) / (2 pi beta fs^2) H dxi/m with H the Hessian
-// of xi (a dual-number pass along u = dxi/m).  One block per trajectory.
+// Umbrella bias outside a step (mdinit's forces, src/mdinit.f90:96-100): one
+// block per trajectory.
 template <int N>
 __global__ void split_umbrella_kernel(SplitParams s) {
   constexpr int NC = 3 * N;
-  __shared__ double cq[NC], ka[NC], kb[NC];
+  __shared__ double cq[NC], dxi[NC], bias[NC];
   const int t = blockIdx.x, P = s.P;
   const size_t tb = (size_t)t * P * NC;
   for (int c = threadIdx.x; c < NC; c += blockDim.x) {
@@ -981,37 +886,11 @@ __global__ void split_umbrella_kernel(SplitParams s) {
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    double dxi[NC];
-    const double xi = xi_umbrella<N, double>(s.xi, cq, s.mass, dxi);
-    Dual cd[NC], hd[NC];
-    for (int c = 0; c < NC; ++c) cd[c] = Dual(cq[c], dxi[c] / s.mass[c / 3]);
-    xi_umbrella<N, Dual>(s.xi, cd, s.mass, hd);
-    const double delta = xi - s.umb.center[t], kf = s.umb.kforce[t];
-    const double pi = 3.1415926535897932384;
-    double fs2 = 0.0;
-    for (int l = 0; l < 3; ++l)
-      for (int m = 0; m < N; ++m) fs2 = fs2 + dxi[3 * m + l] * dxi[3 * m + l] / s.mass[m];
-    const double coeff1 = 2.0 * pi * s.umb.beta;
-    fs2 = fs2 / coeff1;
-    const double coeff2 = -1.0 / s.umb.beta;
-    for (int c = 0; c < NC; ++c) {
-      ka[c] = kf * delta * dxi[c];
-      kb[c] = hd[c].d * coeff2 / (coeff1 * fs2);
-    }
-    if (*s.umb.sampling) {
-      s.umb.xsum[t] = s.umb.xsum[t] + xi;
-      s.umb.xsum2[t] = s.umb.xsum2[t] + xi * xi;
-      if (s.umb.nbins > 0) {
-        const double u = (xi - s.umb.lo) / (s.umb.hi - s.umb.lo) * s.umb.nbins;
-        if (u >= 0.0 && u < s.umb.nbins) s.umb.hist[(size_t)t * s.umb.nbins + (int)u] += 1.0;
-      }
-    }
+    const double xi = umbrella_bias<N>(s.xi, cq, s.mass, s.inv_mass, s.umb.center[t], s.umb.kforce[t], s.umb.beta, dxi, bias);
+    if (*s.umb.sampling) umbrella_sample(s.umb, (size_t)t, xi);
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < P * NC; idx += blockDim.x) {
-    const int c = idx % NC;
-    s.f[tb + idx] = (s.f[tb + idx] + ka[c]) + kb[c];
-  }
+  for (int idx = threadIdx.x; idx < P * NC; idx += blockDim.x) s.f[tb + idx] += bias[idx % NC];
 }
 
 }  // namespace cr
