@@ -193,6 +193,7 @@ struct cr_engine {
   double *d_pile = nullptr, *d_q0 = nullptr;
   cr::Limbs* d_maps = nullptr;  // StepParams::ke, ko and pile
   double* d_parts = nullptr;    // StepParams::psym and panti
+  int64_t* d_ring = nullptr;    // FastRing::tab
   double* d_circ = nullptr;  // [3][P] circulant propagator rows (nm_mode 1)
   int* d_status = nullptr;
   // recrossing children
@@ -345,6 +346,24 @@ void build_fast_drift(int P, double beta, double dt, std::vector<double>& tab) {
       tab[(size_t)3 * (M + 1) + N / 2 - 1 + k] = 1.0 / (2.0 * std::cos(kPi * (2 * k + 1) / (2.0 * N)));
 }
 
+
+// Tables of the fast transforms in fixed point (ring_fast.cuh): (w_k / 2) times
+// pc, pd, pq of mode_tables as Q62 under the exponents 0, eb, ec.
+void build_fast_ring(int P, double beta, double dt, std::vector<int64_t>& tab, int& eb, int& ec) {
+  const int M = P / 2;
+  std::vector<double> C, diag[3];
+  mode_tables(P, beta, dt, C, diag);
+  std::vector<double> t[3];
+  for (int w = 0; w < 3; ++w)
+    for (int k = 0; k <= M; ++k) t[w].push_back((k == 0 || k == M ? 0.5 : 1.0) * diag[w][(size_t)k]);
+  eb = cr::fixed_exponent(t[2]);
+  ec = cr::fixed_exponent(t[1]);
+  const double* v[3] = {t[0].data(), t[2].data(), t[1].data()};
+  const int e[3] = {0, eb, ec};
+  tab.clear();
+  for (int w = 0; w < 3; ++w)
+    for (int k = 0; k <= M; ++k) tab.push_back((int64_t)std::llrint(std::ldexp(v[w][k], 62 - e[w])));
+}
 
 // PILE-L circulant vectors a (friction) and b (noise) of O^T diag(c) O with O
 // the orthonormal real normal-mode matrix; gamma_0 = 1/tau0, gamma_k = 2 w_k.
@@ -762,11 +781,15 @@ bool apply_shape(cr_engine* e, int groups, int tpb) {
   if (!r || (tpb != 1 && tpb != 2 && tpb != 4) || tpb > r->max_tpb) return false;
   const cr::PropDims d = cr::prop_dims(e->P);
   const int U = e->prm.U;
-  int gpb = std::min(groups, e->T);
-  while (gpb > 1 && cr::step_smem_bytes(d, U, e->NC, gpb) > 220 * 1024) --gpb;
+  // where the block would be too large, fewer threads per bead, then fewer
+  // trajectories (the results do not depend on either)
+  int subs = tpb, gpb = std::min(groups, e->T);
+  while (subs > 1 && U * subs > cr::kStepThreads) subs /= 2;
+  auto fits = [&](int n) { return n * U * subs <= cr::kStepThreads && cr::step_smem_bytes(d, U, e->NC, n) <= 220 * 1024; };
+  while (gpb > 1 && !fits(gpb)) --gpb;
+  if (!fits(gpb)) return false;
   const size_t smem = cr::step_smem_bytes(d, U, e->NC, gpb);
-  const int threads = (gpb * U * tpb + 31) / 32 * 32;
-  if (smem > 220 * 1024 || threads > 256) return false;
+  const int threads = (gpb * U * subs + 31) / 32 * 32;
   e->block = groups * e->G * tpb;
   e->tpb = tpb;
   e->grid = (e->T + groups - 1) / groups;
@@ -774,7 +797,7 @@ bool apply_shape(cr_engine* e, int groups, int tpb) {
   e->threads = threads;
   e->smem = smem;
   e->prm.gpb = gpb;
-  e->prm.subs = tpb;
+  e->prm.subs = subs;
   return true;
 }
 
@@ -807,7 +830,7 @@ void choose_launch(cr_engine* e) {
       if (e->G * tpb <= 256 && apply_shape(e, 1, tpb)) return;
   double best = 0.0;
   int pick = 1;
-  for (int groups = 1; groups * e->prm.U <= 256 && groups <= 256; ++groups) {
+  for (int groups = 1; groups * e->prm.U <= cr::kStepThreads; ++groups) {
     if (!apply_shape(e, groups, 1) || e->gpb != std::min(groups, e->T)) continue;
     int res = 1;
     if (!r || r->resident(mixed, e->threads, e->smem, &res) != cudaSuccess || res < 1) res = 1;
@@ -1256,6 +1279,19 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
     s.psym = e->d_parts;
     s.panti = e->d_parts + n;
   }
+  // fast transforms from 32 beads on: a row's transform is one chain of some
+  // hundred products on one lane, which 16 beads do not repay (H3 64 x 16 PILE
+  // mixed 36 us per step against 32 with the matrix products on all lanes; CH4 + H
+  // 4096 x 32 mixed 102 against 122, CH4 + OH 512 x 64 mixed 80 against 118)
+  if (s.pair && (e->P == 32 || e->P == 64)) {
+    std::vector<int64_t> tab;
+    build_fast_ring(e->P, cfg->beta, cfg->dt, tab, s.fast.eb, s.fast.ec);
+    if (cudaMalloc(&e->d_ring, tab.size() * 8) != cudaSuccess ||
+        cudaMemcpy(e->d_ring, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess)
+      return cleanup_fail(fail(CR_ERR_CUDA, "upload of the ring tables failed"));
+    s.fast.tab = e->d_ring;
+    s.fast_M = e->P / 2;
+  }
   choose_launch(e);
   *out = e;
   return CR_OK;
@@ -1296,6 +1332,7 @@ int cr_engine_destroy(cr_engine* e) {
   cudaFree(e->d_pile);
   cudaFree(e->d_maps);
   cudaFree(e->d_parts);
+  cudaFree(e->d_ring);
   cudaFree(e->d_side);
   cudaFree(e->d_w);
   cudaFree(e->d_kappa);
@@ -2004,7 +2041,7 @@ int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* th
   float best_ms = 0.f;
   cudaError_t err = copy_state(true);
   for (int tpb = 1; tpb <= 4 && rc == CR_OK && err == cudaSuccess; tpb *= 2) {
-    for (int m = 1; m * e->prm.U * tpb <= 256 && rc == CR_OK && err == cudaSuccess; m += m < 8 ? 1 : m / 4) {
+    for (int m = 1; m * e->prm.U * tpb <= cr::kStepThreads && rc == CR_OK && err == cudaSuccess; m += m < 8 ? 1 : m / 4) {
       if (!apply_shape(e, m, tpb)) continue;
       // one untimed step (first launch of this shape), then the timed run
       for (int rep = 0; rep < 2 && rc == CR_OK; ++rep) {

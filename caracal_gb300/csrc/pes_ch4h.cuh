@@ -4,7 +4,7 @@
 // (bohr/Hartree user units, no relabelling: src/util_ch4h.f CARTOU, CARTTOR,
 // EUNITZERO, RTOCART, DEDCOU are identities).
 //
-// One thread evaluates one bead.  Routines restated: POT_ch4h :161,
+// Four lanes evaluate one bead.  Routines restated: POT_ch4h :161,
 // coorden :287, switchf :1545, refangles :367, stretch :506, opbend :713,
 // calcdelta :986, opforce :1240, ipbend :865, ipforce :1350; constants from
 // BLOCK DATA PTPACM_ch4h with PREPOT_ch4h's unit factors (all REAL(8)).
@@ -45,34 +45,39 @@ struct Par {
   static constexpr bool sphi_cut = true;                     // switchf's rch < 3.8 condition on sphi
 };
 
-template <class F>
-__device__ inline void egrad(const double (&qb)[18], double& V, double (&g)[18]) {
-  methane::Bonds<F> G;
-  F tch[4][3];
+// Lane i of a quad (i = lane & 3; every lane of the warp takes part): the
+// energy on all four, the gradient by put(coordinate, value), each coordinate
+// from one lane.
+template <class F, class Get, class Put>
+__device__ inline void egrad(const Get& x, int i, double& V, const Put& put) {
+  methane::Bond<F> G;
   if constexpr (std::is_same<F, float>::value) {
     methane::Pairs X;
-    ff x[18], gx[18];
-    methane::scaled_pairs(qb, x);
-    methane::bond_vectors(x, G, X, tch);
-    const float vs = methane::stretch_pairs<Par>(G, X);
-    const float vb = methane::bends<float, Par>(tch, &X, G);
-    V = ff_to_double(vs + vb) * 0.03812;
-#pragma unroll
-    for (int k = 0; k < 18; ++k) gx[k] = ff{0.f, 0.f};
-    methane::chain(G, X, gx);
+    ff g[9], none;
+    methane::bond_vectors(x, i, G, X);
+    const float vs = methane::stretch_pairs<Par>(G, X, i, ff{0.f, 0.f}, none);
+    const float vb = methane::bends<float, Par>(&X, G, i);
+    V = ff_to_double(methane::quad_sum(vs + vb)) * 0.03812;
+    methane::chain(G, X, g);
     constexpr ff kUnit = ff_const(0.0201723);
 #pragma unroll
-    for (int k = 0; k < 18; ++k) g[k] = ff_to_double(ff_float(gx[k] * kUnit));
+    for (int d = 0; d < 3; ++d) {
+      put(3 * methane::NH(i) + d, ff_to_double(ff_float(g[d] * kUnit)));
+      const ff h = i == 0 ? g[3 + d] : g[6 + d];
+      if (i < 2) put(3 * (i == 0 ? methane::NC : methane::NB) + d, ff_to_double(ff_float(h * kUnit)));
+    }
   } else {
-    methane::bond_vectors(qb, G, tch);
-    const double vs = methane::stretch_plain<Par>(G);
-    const double vb = methane::bends<double, Par>(tch, nullptr, G);
-    V = (vs + vb) * 0.03812;
-#pragma unroll
-    for (int k = 0; k < 18; ++k) g[k] = 0.0;
+    double g[9], none;
+    methane::bond_vectors(x, i, G);
+    const double vs = methane::stretch_plain<Par>(G, i, 0.0, none);
+    const double vb = methane::bends<double, Par>(nullptr, G, i);
+    V = methane::quad_sum(vs + vb) * 0.03812;
     methane::chain(G, g);
 #pragma unroll
-    for (int k = 0; k < 18; ++k) g[k] *= 0.0201723;
+    for (int d = 0; d < 3; ++d) {
+      put(3 * methane::NH(i) + d, g[d] * 0.0201723);
+      if (i < 2) put(3 * (i == 0 ? methane::NC : methane::NB) + d, (i == 0 ? g[3 + d] : g[6 + d]) * 0.0201723);
+    }
   }
 }
 
@@ -80,9 +85,10 @@ __device__ inline void egrad(const double (&qb)[18], double& V, double (&g)[18])
 
 struct PesCH4H {
   static constexpr int N = 6;
-  template <class F>
-  __device__ static inline void egrad(const double (&q)[18], double& V, double (&g)[18]) {
-    ch4h::egrad<F>(q, V, g);
+  static constexpr int kLanes = 4;  // per bead
+  template <class F, class Get, class Put>
+  __device__ static inline void egrad(const Get& x, int i, double& V, const Put& put) {
+    ch4h::egrad<F>(x, i, V, put);
   }
 };
 

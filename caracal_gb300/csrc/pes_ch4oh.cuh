@@ -7,7 +7,7 @@
 // routines differ from CH4 + OH's only in the pyramid angle of refangles and
 // the uncut sphi of switchf (ParCH4OH / ParGeH4OH below).
 //
-// One thread evaluates one bead.  Routines restated (src/egrad_ch4oh.f):
+// Four lanes evaluate one bead.  Routines restated (src/egrad_ch4oh.f):
 // POT_ch4oh :157, coorden :288, refangles :374, stretch :517, opbend :782,
 // ipbend :938, calcdelta :1177, opforce :1435, ipforce :1549, switchf :1748;
 // constants from BLOCK DATA PTPACM_ch4oh :2007 with PREPOT_ch4oh's unit
@@ -85,136 +85,109 @@ struct ParGeH4OH : ParXH4OH {
 
 constexpr int NB = methane::NB, NO = 6;
 
-// O-H Morse stretch (stretch_ch4oh :602-605, :620-632, :711-716): the energy,
-// dV/dr in dr.
-template <class K>
-__device__ inline double morse(double r, double& dr) {
-  const double e = fx::exp(-K::ahh * (r - K::r0hh)), om = 1.0 - e;
-  dr = (2.0 * K::ahh * K::d1hh) * om * e;
-  return K::d1hh * (om * om);
-}
-// its 1 - exp(-a (r - r0)) near the minimum in float pairs; dr = dV/dr / r
-template <class K>
-__device__ inline float morse(ff r, ff& dr) {
-  constexpr ff kA = ff_const(K::ahh), kR0 = ff_const(K::r0hh);
-  const ff e = ff_exp(-(kA * (r - kR0))), om = ff_from(1.f) - e;
-  dr = (ff_const(2.0 * K::ahh * K::d1hh) * om * e) / r;
-  return ff_float(ff_const(K::d1hh) * (om * om));
-}
-
-// H(i)-O-H(O) bends (ipbend_ch4oh :1061-1172): the energy; dV/dr(BH_i) into G,
-// the gradient across the bonds on H_i and H(O) into gh, go.
+// H(i)-O-H(O) bend of lane i (ipbend_ch4oh :1061-1172): the energy; dV/dr(BH_i)
+// into G, the gradient across the bonds on H_i and H(O) into gh, go.
 template <class F, class K>
-__device__ inline F hoh_bends(const F (&tno)[3], F rno, F irno, const ff* xno, ff xrno, const methane::Pairs* X,
-                              methane::Bonds<F>& G, F (&gh)[4][3], F (&go)[3]) {
+__device__ inline F hoh_bend(const F (&tno)[3], F irno, const ff* xno, ff xrno, const methane::Pairs* X,
+                             methane::Bond<F>& G, F (&gh)[3], F (&go)[3]) {
   constexpr bool kPair = std::is_same<F, float>::value;
-  F V = F(0);
-#pragma unroll
-  for (int d = 0; d < 3; ++d) go[d] = F(0);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const F* tb = G.tbh[i];
-    F cosine, dang;
-    if constexpr (kPair) {
-      // angle - anh2oeq as asin(sin(angle - anh2oeq)) from a float-pair
-      // cosine: a small difference of two ~1.8 rad angles
-      const ff* xb = X->tbh[i];
-      const ff rbh = ff_sqrt(xb[0] * xb[0] + xb[1] * xb[1] + xb[2] * xb[2]);
-      ff c = -((xno[0] * xb[0] + xno[1] * xb[1] + xno[2] * xb[2]) / (xrno * rbh));
-      if (c.hi > 1.f) c = ff_from(1.f);
-      if (c.hi < -1.f) c = ff_from(-1.f);
-      constexpr ff kCosEq = ff_const(-0.25398078034139054), kSinEq = ff_const(0.9672092654731852);
-      const ff y = ff_sqrt(ff_from(1.f) - c * c) * kCosEq - c * kSinEq;  // sin(angle - anh2oeq)
-      cosine = ff_float(c);
-      dang = fabsf(y.hi) < 0.9f ? asinf(y.hi) + y.lo * methane::m_rsqrt<float>(1.f - y.hi * y.hi)
-                                : acosf(cosine) - F(anh2oeq);
-    } else {
-      cosine = -methane::dot3(tno, tb) * (irno * G.irbh[i]);
-      cosine = fmin(F(1), fmax(F(-1), cosine));
-      dang = methane::m_acos<F>(cosine) - F(anh2oeq);
-    }
-    const F arga = F(alph2o) * (G.rbh[i] - F(K::r0hh));
-    F t, ds;  // tanh(arga), -alph2o / cosh(arga)^2 (also past the cutoff)
-    methane::tanh_switch(arga, F(alph2o), t, ds);
-    const F fk = (arga < F(19.0)) ? F(fkh2oeq) * (F(1) - t) : F(0);
-    const F h = F(0.5) * dang * dang, dstda = fk * dang;
-    V += fk * h;
-    G.drbh[i] += F(fkh2oeq) * ds * h;
-    const F xp = tno[1] * tb[2] - tno[2] * tb[1];
-    const F yp = tno[2] * tb[0] - tno[0] * tb[2];
-    const F zp = tno[0] * tb[1] - tno[1] * tb[0];
-    F rp = methane::m_sqrt<F>(xp * xp + yp * yp + zp * zp);
-    if (rp < F(1.0e-6)) rp = F(1.0e-6);
-    const F k = methane::m_div<F>(dstda, rp);
-    const F ta = k * (G.irbh[i] * G.irbh[i]), tc = k * (irno * irno);
-    gh[i][0] = -ta * (tb[1] * zp - tb[2] * yp);
-    gh[i][1] = -ta * (tb[2] * xp - tb[0] * zp);
-    gh[i][2] = -ta * (tb[0] * yp - tb[1] * xp);
-    go[0] -= tc * (tno[1] * zp - tno[2] * yp);
-    go[1] -= tc * (tno[2] * xp - tno[0] * zp);
-    go[2] -= tc * (tno[0] * yp - tno[1] * xp);
+  const F* tb = G.tbh;
+  F cosine, dang;
+  if constexpr (kPair) {
+    // angle - anh2oeq as asin(sin(angle - anh2oeq)) from a float-pair
+    // cosine: a small difference of two ~1.8 rad angles
+    const ff* xb = X->tbh;
+    const ff rbh = ff_sqrt(xb[0] * xb[0] + xb[1] * xb[1] + xb[2] * xb[2]);
+    ff c = -((xno[0] * xb[0] + xno[1] * xb[1] + xno[2] * xb[2]) / (xrno * rbh));
+    if (c.hi > 1.f) c = ff_from(1.f);
+    if (c.hi < -1.f) c = ff_from(-1.f);
+    constexpr ff kCosEq = ff_const(-0.25398078034139054), kSinEq = ff_const(0.9672092654731852);
+    const ff y = ff_sqrt(ff_from(1.f) - c * c) * kCosEq - c * kSinEq;  // sin(angle - anh2oeq)
+    cosine = ff_float(c);
+    dang = fabsf(y.hi) < 0.9f ? asinf(y.hi) + y.lo * methane::m_rsqrt<float>(1.f - y.hi * y.hi)
+                              : acosf(cosine) - F(anh2oeq);
+  } else {
+    cosine = -methane::dot3(tno, tb) * (irno * G.irbh);
+    cosine = fmin(F(1), fmax(F(-1), cosine));
+    dang = methane::m_acos<F>(cosine) - F(anh2oeq);
   }
-  return V;
+  const F arga = F(alph2o) * (G.rbh - F(K::r0hh));
+  F t, ds;  // tanh(arga), -alph2o / cosh(arga)^2 (also past the cutoff)
+  methane::tanh_switch(arga, F(alph2o), t, ds);
+  const F fk = (arga < F(19.0)) ? F(fkh2oeq) * (F(1) - t) : F(0);
+  const F h = F(0.5) * dang * dang, dstda = fk * dang;
+  G.drbh += F(fkh2oeq) * ds * h;
+  const F xp = tno[1] * tb[2] - tno[2] * tb[1];
+  const F yp = tno[2] * tb[0] - tno[0] * tb[2];
+  const F zp = tno[0] * tb[1] - tno[1] * tb[0];
+  F rp = methane::m_sqrt<F>(xp * xp + yp * yp + zp * zp);
+  if (rp < F(1.0e-6)) rp = F(1.0e-6);
+  const F k = methane::m_div<F>(dstda, rp);
+  const F ta = k * (G.irbh * G.irbh), tc = k * (irno * irno);
+  gh[0] = -ta * (tb[1] * zp - tb[2] * yp);
+  gh[1] = -ta * (tb[2] * xp - tb[0] * zp);
+  gh[2] = -ta * (tb[0] * yp - tb[1] * xp);
+  go[0] = -tc * (tno[1] * zp - tno[2] * yp);
+  go[1] = -tc * (tno[2] * xp - tno[0] * zp);
+  go[2] = -tc * (tno[0] * yp - tno[1] * xp);
+  return fk * h;
 }
 
-template <class F, class K>
-__device__ inline void egrad(const double (&qb)[21], double& V, double (&g)[21]) {
-  methane::Bonds<F> G;
-  F tch[4][3], tno[3], gh[4][3], go[3], rno, irno;
+// Lane i of a quad, as in ch4h::egrad.  The O-H Morse stretch (stretch_ch4oh
+// :602-605, :620-632, :711-716) is evaluated on every lane, its energy counted
+// on lane 0; its 1 - exp(-a (r - r0)) near the minimum in float pairs too.
+template <class F, class K, class Get, class Put>
+__device__ inline void egrad(const Get& x, int i, double& V, const Put& put) {
+  methane::Bond<F> G;
+  F tno[3], gh[3], go[3], rno, irno;
   if constexpr (std::is_same<F, float>::value) {
     methane::Pairs X;
-    ff x[21], gx[21], xno[3], dno;
-    methane::scaled_pairs(qb, x);
-    methane::bond_vectors(x, G, X, tch);
+    ff g[9], xno[3], eoh;
+    methane::bond_vectors(x, i, G, X);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      xno[d] = x[3 * NO + d] - x[3 * NB + d];
+      xno[d] = methane::scaled_pair(x(3 * NO + d)) - methane::scaled_pair(x(3 * NB + d));
       tno[d] = ff_float(xno[d]);
     }
     const ff xrno = ff_sqrt(xno[0] * xno[0] + xno[1] * xno[1] + xno[2] * xno[2]);
     methane::m_root(methane::dot3(tno, tno), rno, irno);
-    float v = methane::stretch_pairs<K>(G, X) + morse<K>(xrno, dno);
-    v += methane::bends<float, K>(tch, &X, G);
-    v += hoh_bends<float, K>(tno, rno, irno, xno, xrno, &X, G, gh, go);
-    V = ff_to_double(v) * 0.03812;
-#pragma unroll
-    for (int k = 0; k < 21; ++k) gx[k] = ff{0.f, 0.f};
-    methane::chain(G, X, gx);
+    constexpr ff kA = ff_const(K::ahh), kR0 = ff_const(K::r0hh);
+    float v = methane::stretch_pairs<K>(G, X, i, -(kA * (xrno - kR0)), eoh);
+    const ff om = ff_from(1.f) - eoh, dno = (ff_const(2.0 * K::ahh * K::d1hh) * om * eoh) / xrno;
+    if (i == 0) v += ff_float(ff_const(K::d1hh) * (om * om));
+    v += methane::bends<float, K>(&X, G, i);
+    v += hoh_bend<float, K>(tno, irno, xno, xrno, &X, G, gh, go);
+    V = ff_to_double(methane::quad_sum(v)) * 0.03812;
+    methane::chain(G, X, g);
+    constexpr ff kUnit = ff_const(0.0201723);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const ff t = xno[d] * dno;
-      gx[3 * NB + d] += -t - (gh[0][d] + gh[1][d] + gh[2][d] + gh[3][d] + go[d]);
-      gx[3 * NO + d] += t + go[d];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) gx[3 * methane::NH(i) + d] += gh[i][d];
+      const float so = methane::quad_sum(go[d]), sh = methane::quad_sum(gh[d]);
+      put(3 * methane::NH(i) + d, ff_to_double(ff_float((g[d] + gh[d]) * kUnit)));
+      const ff h = i == 0 ? g[3 + d] : i == 1 ? g[6 + d] - (t + (sh + so)) : t + so;
+      if (i < 3) put(3 * (i == 0 ? methane::NC : i == 1 ? NB : NO) + d, ff_to_double(ff_float(h * kUnit)));
     }
-    constexpr ff kUnit = ff_const(0.0201723);
-#pragma unroll
-    for (int k = 0; k < 21; ++k) g[k] = ff_to_double(ff_float(gx[k] * kUnit));
   } else {
-    methane::bond_vectors(qb, G, tch);
+    double g[9], eoh;
+    methane::bond_vectors(x, i, G);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) tno[d] = qb[3 * NO + d] * 0.52918 - qb[3 * NB + d] * 0.52918;
+    for (int d = 0; d < 3; ++d) tno[d] = x(3 * NO + d) * 0.52918 - x(3 * NB + d) * 0.52918;
     methane::m_root(methane::dot3(tno, tno), rno, irno);
-    double dno;
-    double v = methane::stretch_plain<K>(G) + morse<K>(rno, dno);
-    v += methane::bends<double, K>(tch, nullptr, G);
-    v += hoh_bends<double, K>(tno, rno, irno, nullptr, ff{0.f, 0.f}, nullptr, G, gh, go);
-    V = v * 0.03812;
-#pragma unroll
-    for (int k = 0; k < 21; ++k) g[k] = 0.0;
+    double v = methane::stretch_plain<K>(G, i, -K::ahh * (rno - K::r0hh), eoh);
+    const double om = 1.0 - eoh, dno = (2.0 * K::ahh * K::d1hh) * om * eoh * irno;
+    if (i == 0) v += K::d1hh * (om * om);
+    v += methane::bends<double, K>(nullptr, G, i);
+    v += hoh_bend<double, K>(tno, irno, nullptr, ff{0.f, 0.f}, nullptr, G, gh, go);
+    V = methane::quad_sum(v) * 0.03812;
     methane::chain(G, g);
-    dno *= irno;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const double t = fma(tno[d], dno, go[d]);
-      g[3 * NB + d] -= t + (gh[0][d] + gh[1][d] + gh[2][d] + gh[3][d]);
-      g[3 * NO + d] += t;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) g[3 * methane::NH(i) + d] += gh[i][d];
+      const double so = methane::quad_sum(go[d]), sh = methane::quad_sum(gh[d]), t = fma(tno[d], dno, so);
+      put(3 * methane::NH(i) + d, (g[d] + gh[d]) * 0.0201723);
+      const double h = i == 0 ? g[3 + d] : i == 1 ? g[6 + d] - (t + sh) : t;
+      if (i < 3) put(3 * (i == 0 ? methane::NC : i == 1 ? NB : NO) + d, h * 0.0201723);
     }
-#pragma unroll
-    for (int k = 0; k < 21; ++k) g[k] *= 0.0201723;
   }
 }
 
@@ -222,9 +195,10 @@ __device__ inline void egrad(const double (&qb)[21], double& V, double (&g)[21])
 
 struct PesCH4OH {
   static constexpr int N = 7;
-  template <class F>
-  __device__ static inline void egrad(const double (&q)[21], double& V, double (&g)[21]) {
-    ch4oh::egrad<F, ch4oh::ParCH4OH>(q, V, g);
+  static constexpr int kLanes = 4;  // per bead
+  template <class F, class Get, class Put>
+  __device__ static inline void egrad(const Get& x, int i, double& V, const Put& put) {
+    ch4oh::egrad<F, ch4oh::ParCH4OH>(x, i, V, put);
   }
 };
 
@@ -233,9 +207,10 @@ struct PesCH4OH {
 // roles (Ge in C's place) with its own constants.
 struct PesGeH4OH {
   static constexpr int N = 7;
-  template <class F>
-  __device__ static inline void egrad(const double (&q)[21], double& V, double (&g)[21]) {
-    ch4oh::egrad<F, ch4oh::ParGeH4OH>(q, V, g);
+  static constexpr int kLanes = 4;
+  template <class F, class Get, class Put>
+  __device__ static inline void egrad(const Get& x, int i, double& V, const Put& put) {
+    ch4oh::egrad<F, ch4oh::ParGeH4OH>(x, i, V, put);
   }
 };
 

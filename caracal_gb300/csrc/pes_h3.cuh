@@ -407,6 +407,7 @@ __device__ inline void pote(const F (&R)[3], const double (&Rd)[3], F& V, F (&dV
 // the displacements to float and evaluates the surface in float.
 struct PesH3 {
   static constexpr int N = 3;
+  static constexpr int kLanes = 1;  // per bead
   template <class F>
   __device__ static inline void egrad(const double (&q)[9], double& V, double (&g)[9]) {
     F d[3][3];  // d[0]=q2-q1 (AB), d[1]=q1-q3 (AC), d[2]=q3-q2 (BC)

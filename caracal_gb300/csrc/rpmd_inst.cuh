@@ -1,35 +1,36 @@
 // The PesRuns table of one analytic surface: instantiates its persistent
 // step kernel and its force kernel (both precision forms); MAXTPB is the
-// largest number of threads per bead that the surface's engines take.  Included once per surface, by rpmd_<surface>.cu.
+// largest number of threads per bead that the surface's engines take, BP and
+// BM the resident blocks per SM of the plain and mixed step kernels.  Included once per surface, by rpmd_<surface>.cu.
 #pragma once
 #include "pes_runs.h"
 #include "rpmd_kernel.cuh"
 
 namespace cr {
 
-template <class PES, int MAXTPB>
+template <class PES, int MAXTPB, int BP, int BM>
 struct RunsOf {
   static cudaError_t run(const StepParams& prm, bool mixed, int grid, int block, size_t smem, cudaStream_t st,
                          int istep, int nsteps) {
-    if (mixed) rpmd_run_kernel<PES, true><<<grid, block, smem, st>>>(prm, istep, nsteps);
-    else rpmd_run_kernel<PES, false><<<grid, block, smem, st>>>(prm, istep, nsteps);
+    if (mixed) rpmd_run_kernel<PES, true, BM><<<grid, block, smem, st>>>(prm, istep, nsteps);
+    else rpmd_run_kernel<PES, false, BP><<<grid, block, smem, st>>>(prm, istep, nsteps);
     return cudaGetLastError();
   }
   static cudaError_t set_smem(bool mixed, size_t smem) {
-    return mixed ? cudaFuncSetAttribute(rpmd_run_kernel<PES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                 : cudaFuncSetAttribute(rpmd_run_kernel<PES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return mixed ? cudaFuncSetAttribute(rpmd_run_kernel<PES, true, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                 : cudaFuncSetAttribute(rpmd_run_kernel<PES, false, BP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   }
   static cudaError_t resident(bool mixed, int block, size_t smem, int* blocks) {
     cudaError_t err = set_smem(mixed, smem);
     if (err != cudaSuccess) return err;
-    return mixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, rpmd_run_kernel<PES, true>, block, smem)
-                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, rpmd_run_kernel<PES, false>, block, smem);
+    return mixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, rpmd_run_kernel<PES, true, BM>, block, smem)
+                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, rpmd_run_kernel<PES, false, BP>, block, smem);
   }
   static cudaError_t egrad(bool mixed, int nbeads, BeadRows rows, const double* q, double* V, double* g, cudaStream_t st) {
-    const int bs = 128, nb = (nbeads + bs - 1) / bs;
+    const int bs = 128 / PES::kLanes, nb = (nbeads + bs - 1) / bs;
     if (nbeads <= 0) return cudaSuccess;
-    if (mixed) egrad_kernel<PES, true><<<nb, bs, 0, st>>>(nbeads, rows, q, V, g);
-    else egrad_kernel<PES, false><<<nb, bs, 0, st>>>(nbeads, rows, q, V, g);
+    if (mixed) egrad_kernel<PES, true><<<nb, 128, 0, st>>>(nbeads, rows, q, V, g);
+    else egrad_kernel<PES, false><<<nb, 128, 0, st>>>(nbeads, rows, q, V, g);
     return cudaGetLastError();
   }
   static constexpr PesRuns table() { return PesRuns{MAXTPB, &run, &set_smem, &resident, &egrad}; }

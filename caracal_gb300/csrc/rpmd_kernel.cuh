@@ -39,6 +39,7 @@
 #include "bead_rows.cuh"
 #include "cr_common.cuh"
 #include "fixed_map.cuh"
+#include "ring_fast.cuh"
 
 namespace cr {
 
@@ -236,6 +237,8 @@ struct StepParams {
   const Limbs* ko;     // [3][nr][nv]: odd-mode part
   int ek[3];           // their exponents
   int guard;           // guard bits of the folded rows (fixed_map.cuh)
+  int fast_M;          // P / 2 where the free ring polymer takes the fast transforms (ring_fast.cuh), else 0
+  FastRing fast;
   const Limbs* pile;   // [2][U][U] friction and noise maps on the carried beads, [w][l][j]
   int ep[2];
   int pguard;
@@ -490,22 +493,40 @@ __device__ inline void umbrella_sample(const UmbrellaDev& u, size_t t, double xi
 // gpb trajectories of the block, each array over all of them:
 //   q, p, f   [NC][U] doubles
 //   area      [2 NC][U]: limbs of the folded rows, PILE limbs, partial sums
-//   sums      [16] doubles, move [8] doubles, chain velocities [4] doubles
+//   energies  [U] doubles, sums [16] doubles, move [8] doubles, chain velocities [4] doubles
 //   exponent of each row [2 NC] int, status int
 __host__ __device__ inline size_t step_group_bytes(int U, int NC) {
-  return (size_t)(5 * NC * U + 16 + 8 + 4) * 8 + ((size_t)(2 * NC + 1) * 4 + 7) / 8 * 8;
+  return (size_t)((5 * NC + 1) * U + 16 + 8 + 4) * 8 + ((size_t)(2 * NC + 1) * 4 + 7) / 8 * 8;
 }
 __host__ __device__ inline size_t step_smem_bytes(const PropDims& d, int U, int NC, int groups) {
   return (size_t)3 * d.nr * (d.nu + d.nv) * 8 + step_group_bytes(U, NC) * groups;
 }
+
+// The free ring polymer of the block's rows by fast transforms: lanes 2 y and
+// 2 y + 1 take row y of q and of p.
+template <int M, int NC>
+__device__ __noinline__ void ring_rows(const StepParams& prm, double* sq, double* sp, int rows, int* sstat) {
+  for (int x0 = threadIdx.x & ~31; x0 < 2 * rows; x0 += blockDim.x) {
+    const int x = x0 + (threadIdx.x & 31), y = x >> 1;
+    const bool active = x < 2 * rows, isp = x & 1;
+    const int i = active ? (y % NC) / 3 : 0;
+    const bool fine = ring::row<M>((isp ? sp : sq) + (active ? y : 0) * (M + 1), 1, isp, active,
+                                   isp ? prm.mass[i] : prm.inv_mass[i], prm.fast);
+    if (!fine) atomicOr(&sstat[y / NC], CR_TRAJ_NONFINITE);
+  }
+}
+
+// Most threads of a block of the step kernel; MINB blocks stay resident per SM
+// (the registers follow: 255 for 2, 168 for 3, 128 for 4).
+constexpr int kStepThreads = 128;
 
 // Threads per bead (TPB = 1, 2, 4).  subs threads share a carried bead: the
 // task stages spread over all gpb U subs threads of the block, the surface is
 // evaluated by the first gpb U.  Worth it where the batch is too small to fill
 // the GPU and the integrator weighs as much as the surface (H3, OH + H2).  The
 // sums do not depend on the block's shape or on subs.
-template <class PES, bool MIXED>
-__global__ void __launch_bounds__(256) rpmd_run_kernel(const __grid_constant__ StepParams prm, int istep_arg, int nsteps) {
+template <class PES, bool MIXED, int MINB>
+__global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __grid_constant__ StepParams prm, int istep_arg, int nsteps) {
   const int istep0 = prm.istep_dev ? *prm.istep_dev : istep_arg;
   constexpr int N = PES::N;
   constexpr int NC = 3 * N;
@@ -525,7 +546,8 @@ __global__ void __launch_bounds__(256) rpmd_run_kernel(const __grid_constant__ S
   double* sf = sp + gpb * NC * U;
   double* area = sf + gpb * NC * U;
   Limbs* limbs = reinterpret_cast<Limbs*>(area);
-  double* ssum = area + 2 * gpb * NC * U;
+  double* svb = area + 2 * gpb * NC * U;  // bead energies
+  double* ssum = svb + gpb * U;
   double* smove = ssum + 16 * gpb;
   double* svnh = smove + 8 * gpb;
   int* sexp = reinterpret_cast<int*>(svnh + 4 * gpb);
@@ -538,8 +560,8 @@ __global__ void __launch_bounds__(256) rpmd_run_kernel(const __grid_constant__ S
   // the bead of this thread (threads below nb subs)
   const int sub = nb > 0 ? tid / nb : 0;
   const int b = tid - sub * nb, g = b / U, j = b - g * U;
-  const bool bead = sub == 0;                    // evaluates the surface
   const bool worker = sub < prm.subs;            // shares the bead's stages
+  const bool bead = sub == 0;                    // evaluates the surface
   const int t = t_first + g;
   // does a carried bead stand for two
   auto twin_of = [&](int k) { return prm.pair && k > 0 && 2 * k != P ? P - k : k; };
@@ -586,7 +608,6 @@ __global__ void __launch_bounds__(256) rpmd_run_kernel(const __grid_constant__ S
   const bool nhc = prm.thermostat == CR_THERMO_NHC, pile = prm.thermostat == CR_THERMO_PILE;
   if (nhc && tid < ng)
     for (int k = 0; k < 4; ++k) svnh[4 * tid + k] = prm.vnh[4 * (size_t)(t_first + tid) + k];
-  double vbead = 0.0;
   bool anti_left = false;  // the run ends with an antisymmetric part of p (prm.panti)
   __syncthreads();
 
@@ -727,6 +748,9 @@ __global__ void __launch_bounds__(256) rpmd_run_kernel(const __grid_constant__ S
         sq[x] = qn;
         if (nonfinite_bits(qn)) atomicOr(&sstat[x / (NC * U)], CR_TRAJ_NONFINITE);
       }
+    } else if (prm.fast_M) {
+      if (prm.fast_M == 16) ring_rows<16, NC>(prm, sq, sp, rows, sstat);
+      else ring_rows<32, NC>(prm, sq, sp, rows, sstat);
     } else {
       // fold: rows of q, then of p, into limbs: x_l + x_{M-l}, x_l - x_{M-l}
       for (int x = tid; x < 2 * rows; x += nth) {
@@ -756,6 +780,7 @@ __global__ void __launch_bounds__(256) rpmd_run_kernel(const __grid_constant__ S
         const Limbs* k2 = k1 + pd.nr * pd.nu;
         const Limbs* k3 = k2 + pd.nr * pd.nu;
         FixedSum a1q{0, 0}, a1p{0, 0}, a2q{0, 0}, a3p{0, 0};
+#pragma unroll 4
         for (int l = 0; l < pd.nu; ++l) {
           const Limbs vq = uq[l], vp = up[l], w1 = k1[l];
           a1q.add(vq, w1);
@@ -772,6 +797,7 @@ __global__ void __launch_bounds__(256) rpmd_run_kernel(const __grid_constant__ S
           k1 = s_ko + r * pd.nv;
           k2 = k1 + pd.nr * pd.nv;
           k3 = k2 + pd.nr * pd.nv;
+#pragma unroll 4
           for (int l = 0; l < pd.nv; ++l) {
             const Limbs vq = uq[l], vp = up[l], w1 = k1[l];
             a1q.add(vq, w1);
@@ -808,12 +834,31 @@ __global__ void __launch_bounds__(256) rpmd_run_kernel(const __grid_constant__ S
     __syncthreads();
 
     // per-bead forces (src/verlet.f90:772-777)
-    if (bead) {
-      double q[NC], gr[NC];
+    if constexpr (PES::kLanes > 1) {
+      // kLanes lanes per bead, whole warps; a last partial pass repeats its
+      // first bead without storing
+      constexpr int L = PES::kLanes;
+      for (int b0 = 0; b0 < nb; b0 += nth / L) {
+        const int y = b0 + tid / L;
+        if (b0 + (tid & ~31) / L >= nb) break;  // none of the warp's
+        const bool store = y < nb;
+        const int yb = store ? y : b0, yg = yb / U, off = yg * NC * U + (yb - yg * U);
+        double v;
+        auto get = [&](int c) { return sq[off + c * U]; };
+        auto put = [&](int c, double x) {
+          if (store) sf[off + c * U] = x;
+        };
+        if (MIXED) PES::template egrad<float>(get, tid % L, v, put);
+        else PES::template egrad<double>(get, tid % L, v, put);
+        if (store && tid % L == 0) svb[yb] = v;
+      }
+    } else if (bead) {
+      double q[NC], gr[NC], v;
 #pragma unroll
       for (int c = 0; c < NC; ++c) q[c] = sq[(g * NC + c) * U + j];
-      if (MIXED) PES::template egrad<float>(q, vbead, gr);
-      else PES::template egrad<double>(q, vbead, gr);
+      if (MIXED) PES::template egrad<float>(q, v, gr);
+      else PES::template egrad<double>(q, v, gr);
+      svb[b] = v;
 #pragma unroll
       for (int c = 0; c < NC; ++c) sf[(g * NC + c) * U + j] = gr[c];
     }
@@ -971,7 +1016,6 @@ __global__ void __launch_bounds__(256) rpmd_run_kernel(const __grid_constant__ S
 
   // the state of every bead, the potential energy of the last step
   if (bead) {
-    area[g * U + j] = vbead;
     for (int c = 0; c < NC; ++c) {
       const int x = (g * NC + c) * U + j;
       const double q = sq[x], p = sp[x], f = sf[x];
@@ -995,32 +1039,47 @@ __global__ void __launch_bounds__(256) rpmd_run_kernel(const __grid_constant__ S
   __syncthreads();
   if (tid < ng) {
     const int tt = t_first + tid;
-    prm.epot[tt] = bead_sum(area + tid * U);
+    prm.epot[tt] = bead_sum(svb + tid * U);
     if (nhc)
       for (int k = 0; k < 4; ++k) prm.vnh[4 * (size_t)tt + k] = svnh[4 * tid + k];
     if (sstat[tid]) atomicOr(&prm.status[tt], sstat[tid]);
   }
 }
 
-// One thread per evaluated bead: V and dV/dq.
+// PES::kLanes threads per evaluated bead: V and dV/dq.
 template <class PES, bool MIXED>
 __global__ void egrad_kernel(int nbeads_total, BeadRows rows, const double* q, double* V, double* g) {
-  constexpr int NC = 3 * PES::N;
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nbeads_total) return;
+  constexpr int NC = 3 * PES::N, L = PES::kLanes;
+  const int x = blockIdx.x * blockDim.x + threadIdx.x, e = x / L;
+  if (L == 1 && e >= nbeads_total) return;
+  const bool store = e < nbeads_total;  // a quad's shuffles need whole warps
+  const int b = store ? e : nbeads_total - 1;
   const size_t r = rows.row(b), r2 = rows.twin(b);
-  double qq[NC], gg[NC], v;
+  double v;
+  if constexpr (L > 1) {
+    auto get = [&](int c) { return q[r * NC + c]; };
+    auto put = [&](int c, double y) {
+      if (!store) return;
+      g[r * NC + c] = y;
+      if (r2 != r) g[r2 * NC + c] = y;
+    };
+    if (MIXED) PES::template egrad<float>(get, x % L, v, put);
+    else PES::template egrad<double>(get, x % L, v, put);
+  } else {
+    double qq[NC], gg[NC];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) qq[c] = q[r * NC + c];
-  if (MIXED) PES::template egrad<float>(qq, v, gg);
-  else PES::template egrad<double>(qq, v, gg);
-  V[r] = v;
+    for (int c = 0; c < NC; ++c) qq[c] = q[r * NC + c];
+    if (MIXED) PES::template egrad<float>(qq, v, gg);
+    else PES::template egrad<double>(qq, v, gg);
 #pragma unroll
-  for (int c = 0; c < NC; ++c) g[r * NC + c] = gg[c];
-  if (r2 != r) {
-    V[r2] = v;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) g[r2 * NC + c] = gg[c];
+    for (int c = 0; c < NC; ++c) {
+      g[r * NC + c] = gg[c];
+      if (r2 != r) g[r2 * NC + c] = gg[c];
+    }
+  }
+  if (store && x % L == 0) {
+    V[r] = v;
+    if (r2 != r) V[r2] = v;
   }
 }
 
