@@ -489,14 +489,82 @@ __device__ inline void umbrella_sample(const UmbrellaDev& u, size_t t, double xi
   }
 }
 
+// Bead sums of one atom's rows (row0 .. row0 + 2 of q and of p) in fixed point:
+// v = 0..2 p, 3..5 q, 6..11 q_a p_b for (a, b) = (y z), (z y), (z x), (x z), (x y),
+// (y x), 12..17 q_a q_b for xx, xy, xz, yy, yz, zz.  pair: interior beads count
+// twice.
+constexpr int kMoments = 18;
+__device__ inline double atom_moment(const Limbs* q, const Limbs* p, const int* eq, const int* ep, int row0, int v, int U,
+                                     int P, int pair, int guard) {
+  const int ends = pair && U > 1 && (P & 1) == 0 ? U - 1 : 0;  // the last bead that counts once
+  const int in = pair ? (P - 1) / 2 : U - 1;                     // beads 1 .. in, then `ends`
+  int ex;
+  int64_t s;
+  bool bad;
+  if (v < 6) {
+    const int r = row0 + v % 3;
+    const Limbs* x = (v < 3 ? p : q) + r * U;
+    auto at = [&](int l) { return ((int64_t)x[l].hi << kLimbBits) + x[l].lo; };
+    int64_t a = 0;
+    for (int l = 1; l <= in; ++l) a += at(l);
+    s = (pair ? 2 * a : a) + at(0) + (ends ? at(ends) : 0);
+    const int e = (v < 3 ? ep : eq)[r];
+    bad = e == kFixedNan;
+    ex = e - 1078 + guard;
+  } else {
+    const int a = v < 12 ? (v == 6 || v == 11 ? 1 : v == 7 || v == 8 ? 2 : 0) : (v < 15 ? 0 : v < 17 ? 1 : 2);
+    const int b = v < 12 ? (v == 6 || v == 9 ? 2 : v == 7 || v == 10 ? 1 : 0)
+                         : (v == 12 ? 0 : v == 13 || v == 15 ? 1 : 2);
+    const Limbs* x = q + (row0 + a) * U;
+    const Limbs* y = (v < 12 ? p : q) + (row0 + b) * U;
+    FixedSum m{0, 0}, o{0, 0};
+#pragma unroll 4
+    for (int l = 1; l <= in; ++l) m.add(x[l], y[l]);
+    o.add(x[0], y[0]);
+    if (ends) o.add(x[ends], y[ends]);
+    s = (pair ? 2 * m.value() : m.value()) + o.value();
+    const int ea = eq[row0 + a], eb = (v < 12 ? ep : eq)[row0 + b];
+    bad = ea == kFixedNan || eb == kFixedNan;
+    ex = ea + eb + 2 * (guard - 1078) + 2 * kLimbBits;
+  }
+  const double r = from_fixed(s, ex);
+  return bad ? __longlong_as_double(0x7ff8000000000000ll) : r;
+}
+
+// transrot's move from the moment sums over beads and atoms (sum p; sum m x; x
+// cross p; sum m x x^T as xx, xy, xz, yy, yz, zz), lane d = 0, 1, 2 of a quad
+// taking component d: p <- p - m (b + va cross x).  With S = sum m x, M
+// Caracal's total mass and W = sum m, the centre S/M gives the centred moments
+// S_ab - (2/M - W/M^2) S_a S_b and the angular momentum L - S x (sum p) / M; the
+// inertia system is solved by cofactors.  false: singular.
+__device__ inline bool transrot_quad(const double* tot, int lane, double tm, double W, double& bb, double& va) {
+  const int d = lane < 3 ? lane : 0, e = d == 2 ? 0 : d + 1, f = d == 0 ? 2 : d - 1;
+  const double itm = fx::rcp(tm), kap = fma(-W * itm, itm, 2.0 * itm);
+  const double Sd = tot[3 + d], Se = tot[3 + e], Sf = tot[3 + f];
+  // centred second moments: dd and the product of the other two axes
+  const int dd = d == 0 ? 9 : d == 1 ? 12 : 14, ef = d == 0 ? 13 : d == 1 ? 11 : 10;
+  const double cdd = fma(-kap * Sd, Sd, tot[dd]), cef = fma(-kap * Se, Sf, tot[ef]);
+  const double L = fma(-itm, fma(Se, tot[f], -Sf * tot[e]), tot[6 + d]);
+  auto at = [](double x, int src) { return __shfl_sync(0xffffffffu, x, src, 4); };
+  // row d of the tensor: tdd, and t between the other two axes
+  const double tdd = at(cdd, e) + at(cdd, f), tef = -cef;
+  const double tee = at(tdd, e), tff = at(tdd, f), tde = at(tef, f), tdf = at(tef, e);
+  const double Cdd = fma(tee, tff, -tef * tef), Cde = fma(tdf, tef, -tde * tff), Cdf = at(Cde, f);
+  const double det = at(fma(tdd, Cdd, fma(tde, Cde, tdf * Cdf)), 0);
+  va = fma(Cdd, L, fma(Cde, at(L, e), Cdf * at(L, f))) * fx::rcp(det);
+  const double ve = at(va, e), vf = at(va, f);
+  bb = fma(-ve, Sf, fma(vf, Se, tot[d])) * itm;
+  return det != 0.0;
+}
+
 // Dynamic shared memory: the propagator's limbs (3 nr (nu + nv)), then for the
 // gpb trajectories of the block, each array over all of them:
 //   q, p, f   [NC][U] doubles
 //   area      [2 NC][U]: limbs of the folded rows, PILE limbs, partial sums
-//   energies  [U] doubles, sums [16] doubles, move [8] doubles, chain velocities [4] doubles
+//   energies  [U] doubles, transrot sums per atom [18 N] doubles, sums [16] doubles, move [8] doubles, chain velocities [4] doubles
 //   exponent of each row [2 NC] int, status int
 __host__ __device__ inline size_t step_group_bytes(int U, int NC) {
-  return (size_t)((5 * NC + 1) * U + 16 + 8 + 4) * 8 + ((size_t)(2 * NC + 1) * 4 + 7) / 8 * 8;
+  return (size_t)((5 * NC + 1) * U + 6 * NC + 16 + 8 + 4) * 8 + ((size_t)(2 * NC + 1) * 4 + 7) / 8 * 8;
 }
 __host__ __device__ inline size_t step_smem_bytes(const PropDims& d, int U, int NC, int groups) {
   return (size_t)3 * d.nr * (d.nu + d.nv) * 8 + step_group_bytes(U, NC) * groups;
@@ -547,7 +615,8 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
   double* area = sf + gpb * NC * U;
   Limbs* limbs = reinterpret_cast<Limbs*>(area);
   double* svb = area + 2 * gpb * NC * U;  // bead energies
-  double* ssum = svb + gpb * U;
+  double* smom = svb + gpb * U;
+  double* ssum = smom + gpb * 6 * NC;
   double* smove = ssum + 16 * gpb;
   double* svnh = smove + 8 * gpb;
   int* sexp = reinterpret_cast<int*>(svnh + 4 * gpb);
@@ -560,7 +629,6 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
   // the bead of this thread (threads below nb subs)
   const int sub = nb > 0 ? tid / nb : 0;
   const int b = tid - sub * nb, g = b / U, j = b - g * U;
-  const bool worker = sub < prm.subs;            // shares the bead's stages
   const bool bead = sub == 0;                    // evaluates the surface
   const int t = t_first + g;
   // does a carried bead stand for two
@@ -922,93 +990,68 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
     }
 
     // transrot (src/transrot.f90:36-237): removed COM velocity and rotation
-    // centre both carry Caracal's extra 1/P (total mass P^2 sum m).  Fifteen
-    // raw moments per bead, in four parts that the bead's threads share, summed
-    // over beads; the second moments about the centre by the parallel axis.
+    // centre both carry Caracal's extra 1/P (total mass P^2 sum m)
     if (prm.transrot) {
-      double* part = area;  // [ng][16][U]
-      if (worker) {
-        double* o = part + (g * 16) * U + j;
-        const double* bq = sq + g * NC * U + j;
-        const double* bp = sp + g * NC * U + j;
-        for (int k = sub; k < 4; k += prm.subs) {
-          double a[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-          if (k == 0) {
-#pragma unroll
-            for (int i = 0; i < N; ++i)
-#pragma unroll
-              for (int d = 0; d < 3; ++d) {
-                a[d] += bp[(3 * i + d) * U];
-                a[3 + d] = fma(prm.mass[i], bq[(3 * i + d) * U], a[3 + d]);
-              }
-#pragma unroll
-            for (int d = 0; d < 6; ++d) o[d * U] = a[d];
-          } else if (k == 1) {
-#pragma unroll
-            for (int i = 0; i < N; ++i) {
-              const double q0 = bq[(3 * i) * U], q1 = bq[(3 * i + 1) * U], q2 = bq[(3 * i + 2) * U];
-              const double p0 = bp[(3 * i) * U], p1 = bp[(3 * i + 1) * U], p2 = bp[(3 * i + 2) * U];
-              a[0] = fma(q1, p2, fma(-q2, p1, a[0]));
-              a[1] = fma(q2, p0, fma(-q0, p2, a[1]));
-              a[2] = fma(q0, p1, fma(-q1, p0, a[2]));
-            }
-#pragma unroll
-            for (int d = 0; d < 3; ++d) o[(6 + d) * U] = a[d];
-          } else if (k == 2) {
-#pragma unroll
-            for (int i = 0; i < N; ++i) {
-              const double q0 = bq[(3 * i) * U], w = prm.mass[i] * q0;
-              a[0] = fma(w, q0, a[0]);
-              a[1] = fma(w, bq[(3 * i + 1) * U], a[1]);
-              a[2] = fma(w, bq[(3 * i + 2) * U], a[2]);
-            }
-#pragma unroll
-            for (int d = 0; d < 3; ++d) o[(9 + d) * U] = a[d];
-          } else {
-#pragma unroll
-            for (int i = 0; i < N; ++i) {
-              const double q1 = bq[(3 * i + 1) * U], q2 = bq[(3 * i + 2) * U], w = prm.mass[i] * q1;
-              a[0] = fma(w, q1, a[0]);
-              a[1] = fma(w, q2, a[1]);
-              a[2] = fma(prm.mass[i] * q2, q2, a[2]);
-            }
-#pragma unroll
-            for (int d = 0; d < 3; ++d) o[(12 + d) * U] = a[d];
-          }
-        }
+      // rows of q and p as limbs; per atom the bead sums of p, q, q_a p_b and
+      // q_a q_b in fixed point (in FP64 some 20 instructions per bead and atom, and the
+      // solve on one lane: per step H3 64 x 16 PILE mixed 32.2 -> 24.8 us, OH + H2 1000 x 24
+      // plain 61 -> 51 us)
+      for (int x = tid; x < 2 * rows; x += nth) {
+        const double* r = x < rows ? sq + x * U : sp + (x - rows) * U;
+        Limbs* o = limbs + x * U;
+        int e = 0;
+        for (int l = 0; l < U; ++l) e = max(e, exponent_field(r[l]));
+        sexp[x] = e;
+        for (int l = 0; l < U; ++l) o[l] = to_limbs(to_fixed(r[l], e, prm.pguard));
       }
       __syncthreads();
+      for (int x = tid; x < ng * N * kMoments; x += nth) {
+        const int y = x / kMoments, v = x - y * kMoments;  // y: trajectory and atom
+        smom[x] = atom_moment(limbs, limbs + flat, sexp, sexp + rows, 3 * y, v, U, P, prm.pair, prm.pguard);
+      }
+      __syncthreads();
+      // over the atoms: sum p, sum m q, q x p, sum m q q^T
       for (int x = tid; x < 15 * ng; x += nth) {
         const int gg = x / 15, v = x - 15 * gg;
-        ssum[16 * gg + v] = bead_sum(part + (gg * 16 + v) * U);
-      }
-      __syncthreads();
-      if (tid < ng) {
-        double tot[15];
-        for (int k = 0; k < 15; ++k) tot[k] = ssum[16 * tid + k];
-        double* mv = smove + 8 * tid;
-        mv[6] = 0.0;
-        if (!transrot_move(tot, prm.totmass, prm.wsum, N <= 2, mv)) {
-          mv[6] = 1.0;
-          atomicOr(&sstat[tid], CR_TRAJ_SINGULAR_INERTIA);
+        const double* mo = smom + gg * N * kMoments;
+        double a = 0.0;
+        if (v < 3) {
+          for (int i = 0; i < N; ++i) a += mo[i * kMoments + v];
+        } else if (v < 6) {
+          for (int i = 0; i < N; ++i) a = fma(prm.mass[i], mo[i * kMoments + v], a);
+        } else if (v < 9) {
+          for (int i = 0; i < N; ++i) a += mo[i * kMoments + 2 * v - 6] - mo[i * kMoments + 2 * v - 5];
+        } else {
+          for (int i = 0; i < N; ++i) a = fma(prm.mass[i], mo[i * kMoments + v + 3], a);
         }
+        ssum[16 * gg + v] = a;
       }
       __syncthreads();
-      if (worker) {
-        const double* mv = smove + 8 * g;
-        if (mv[6] == 0.0) {
-          double* bp = sp + g * NC * U + j;
-          const double* bq = sq + g * NC * U + j;
-          for (int i = sub; i < N; i += prm.subs) {
-            const double w = prm.mass[i], q0 = bq[3 * i * U], q1 = bq[(3 * i + 1) * U], q2 = bq[(3 * i + 2) * U];
-            const double u0 = mv[0] + fma(mv[4], q2, -mv[5] * q1);
-            const double u1 = mv[1] + fma(mv[5], q0, -mv[3] * q2);
-            const double u2 = mv[2] + fma(mv[3], q1, -mv[4] * q0);
-            bp[3 * i * U] = fma(-w, u0, bp[3 * i * U]);
-            bp[(3 * i + 1) * U] = fma(-w, u1, bp[(3 * i + 1) * U]);
-            bp[(3 * i + 2) * U] = fma(-w, u2, bp[(3 * i + 2) * U]);
+      for (int x0 = 0; x0 < ng; x0 += nth / 4) {
+        const int gg = x0 + tid / 4;
+        if (x0 + (tid & ~31) / 4 >= ng) break;
+        const bool real = gg < ng;
+        double* mv = smove + 8 * (real ? gg : x0);
+        double bb, va;
+        const bool ok = transrot_quad(ssum + 16 * (real ? gg : x0), tid & 3, prm.totmass, prm.wsum, bb, va);
+        if (real && (tid & 3) < 3) {
+          mv[tid & 3] = bb;
+          mv[3 + (tid & 3)] = va;
+          if ((tid & 3) == 0) {
+            mv[6] = ok ? 0.0 : 1.0;
+            if (!ok) atomicOr(&sstat[gg], CR_TRAJ_SINGULAR_INERTIA);
           }
         }
+      }
+      __syncthreads();
+      for (int x = tid; x < flat; x += nth) {
+        const int r = x / U, gg = r / NC, c = r - gg * NC, d = c % 3;
+        const int e = d == 2 ? 0 : d + 1, f = d == 0 ? 2 : d - 1;
+        const double* mv = smove + 8 * gg;
+        if (mv[6] != 0.0) continue;
+        const double qe = sq[x + (e - d) * U], qf = sq[x + (f - d) * U];
+        const double u = mv[d] + fma(mv[3 + e], qf, -mv[3 + f] * qe);
+        sp[x] = fma(-prm.mass[c / 3], u, sp[x]);
       }
       __syncthreads();
     }
