@@ -50,24 +50,31 @@ template <> __device__ inline double m_exp<double>(double x) { return fx::exp(x)
 template <> __device__ inline float m_exp<float>(float x) { return expf(x); }
 template <class F> __device__ inline F m_rcp(F x);
 template <> __device__ inline double m_rcp<double>(double x) { return fx::rcp(x); }
-template <> __device__ inline float m_rcp<float>(float x) { return 1.f / x; }
+template <> __device__ inline float m_rcp<float>(float x) { return f_rcp(x); }
 template <class F> __device__ inline F m_div(F a, F b);
 template <> __device__ inline double m_div<double>(double a, double b) { return fx::div(a, b); }
-template <> __device__ inline float m_div<float>(float a, float b) { return a / b; }
+template <> __device__ inline float m_div<float>(float a, float b) { return a * f_rcp(b); }
 template <class F> __device__ inline F m_sqrt(F x);
 template <> __device__ inline double m_sqrt<double>(double x) { return fx::sqrt(x); }
-template <> __device__ inline float m_sqrt<float>(float x) { return sqrtf(x); }
+template <> __device__ inline float m_sqrt<float>(float x) {
+  float r, ir;
+  f_root(x, r, ir);
+  return r;
+}
 template <class F> __device__ inline F m_rsqrt(F x);
 template <> __device__ inline double m_rsqrt<double>(double x) { return fx::rsqrt(x); }
-template <> __device__ inline float m_rsqrt<float>(float x) { return rsqrtf(x); }
+template <> __device__ inline float m_rsqrt<float>(float x) {
+  float r, ir;
+  f_root(x, r, ir);
+  return ir;
+}
 template <class F> __device__ inline F m_acos(F x);
 template <> __device__ inline double m_acos<double>(double x) { return fx::acos(x); }
 template <> __device__ inline float m_acos<float>(float x) { return acosf(x); }
 // sqrt and its reciprocal
 __device__ inline void m_root(double x, double& r, double& ir) { fx::sqrt_rsqrt(x, r, ir); }
 __device__ inline void m_root(float x, float& r, float& ir) {
-  r = sqrtf(x);
-  ir = 1.f / r;
+  f_root(x, r, ir);
 }
 
 // methane H i (0..3, nnh order) -> atom index; X and the attacking atom B
@@ -212,7 +219,7 @@ __device__ inline float stretch_pairs(const Bond<float>& G, Pairs& X, int i, ff 
   if (arga < 19.0f) {
     constexpr ff A1 = ff_const(K::a1ch), B1 = ff_const(K::b1ch);
     ach = A1 + B1 / (ff_from(1.f) + e2);
-    const float s = 2.f * e2.hi / (1.f + e2.hi);  // 1 - tanh(arga)
+    const float s = 2.f * e2.hi * f_rcp(1.f + e2.hi);  // 1 - tanh(arga)
     dach = float(K::b1ch * K::c1ch * 0.125) * (s * (2.f - s));
   }
   const ff ecb2 = ecb1 * ecb1;
