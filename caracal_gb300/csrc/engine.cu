@@ -836,7 +836,15 @@ void choose_launch(cr_engine* e) {
     if (!r || r->resident(mixed, e->threads, e->smem, &res) != cudaSuccess || res < 1) res = 1;
     const int blocks = (e->T + groups - 1) / groups, per_sm = (blocks + sms - 1) / sms;
     const double w = e->threads / 128.0;  // warps per scheduler of one block
-    auto wave = [&](int n) { return n == 0 ? 0.0 : 0.35 + std::max(0.65, 0.65 * n * w); };
+    // a surface on quads: the passes of a block's threads over its beads, each a
+    // latency and an issue share (CH4 + H 1000 x 32: 2 and 4 trajectories per block 36.5
+    // us per step mixed and 120 plain, 7 per block 41.6 and 134; 4096 x 32 mixed: 7
+    // per block 78 us, 4 per block 114)
+    const int passes = r && r->lanes > 1 ? (groups * e->prm.U * r->lanes + e->threads - 1) / e->threads : 0;
+    auto wave = [&](int n) {
+      if (n == 0) return 0.0;
+      return passes ? passes * (0.15 + 0.1 * n * w) : 0.35 + std::max(0.65, 0.65 * n * w);
+    };
     const double cost = (per_sm / res) * wave(res) + wave(per_sm % res);
     // among equals the fuller block, up to two warps: more small blocks than
     // schedulers would share some of them

@@ -16,6 +16,7 @@ struct StepParams;
 
 struct PesRuns {
   int max_tpb;  // most threads per bead of the step kernel on the surface
+  int lanes;    // threads that evaluate a bead together (PES::kLanes)
   // rpmd_run_kernel<surface, mixed><<<grid, block, smem, st>>>(prm, istep, nsteps)
   cudaError_t (*run)(const StepParams& prm, bool mixed, int grid, int block, size_t smem, cudaStream_t st, int istep,
                      int nsteps);

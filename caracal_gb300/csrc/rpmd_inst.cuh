@@ -33,7 +33,7 @@ struct RunsOf {
     else egrad_kernel<PES, false><<<nb, 128, 0, st>>>(nbeads, rows, q, V, g);
     return cudaGetLastError();
   }
-  static constexpr PesRuns table() { return PesRuns{MAXTPB, &run, &set_smem, &resident, &egrad}; }
+  static constexpr PesRuns table() { return PesRuns{MAXTPB, PES::kLanes, &run, &set_smem, &resident, &egrad}; }
 };
 
 }  // namespace cr
