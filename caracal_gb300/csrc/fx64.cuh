@@ -21,7 +21,8 @@
 // Methods: reciprocal and reciprocal square root by one third-order Newton
 // step from the FP32 hardware estimate; exp2 by 16 tabulated powers of two and
 // the Taylor series of 2^z, z < 1/16; log2 by 2 atanh((m-1)/(m+1)); arc sine
-// by its Taylor series with the half-angle reduction.  The constants are those
+// by its Taylor series with the half-angle reduction; sine, cosine and erf by
+// Taylor series to an absolute 2^-58.  The constants are those
 // series' coefficients, scaled.
 #pragma once
 #include <cmath>
@@ -31,6 +32,8 @@
 #ifdef __CUDACC__
 #include <cuda_runtime.h>
 #endif
+
+#include "fx64_erf.cuh"
 
 namespace cr {
 namespace fx {
@@ -117,6 +120,15 @@ FX_FN u64 mulh(u64 a, u64 b) {
   return (u64)ah * bh + (t >> 32) + (u >> 32);
 }
 
+// floor(a b / 2^64)
+FX_FN u64 mulh_exact(u64 a, u64 b) {
+#ifdef __CUDA_ARCH__
+  return __umul64hi(a, b);
+#else
+  return (u64)(((unsigned __int128)a * b) >> 64);
+#endif
+}
+
 // +-M 2^(e - 63), M with its top bit set, to the nearest double (e in the
 // normal range; a carry out of the significand moves the exponent)
 FX_FN double pack(u64 sign, int e, u64 M) {
@@ -170,6 +182,7 @@ FX_SLOW double slow_exp(double x) { return std::exp(x); }
 FX_SLOW double slow_log(double x) { return std::log(x); }
 FX_SLOW double slow_pow(double x, double y) { return std::pow(x, y); }
 FX_SLOW double slow_acos(double x) { return std::acos(x); }
+FX_SLOW double slow_asin(double x) { return std::asin(x); }
 
 // biased exponent within [lo, hi] (one unsigned comparison)
 FX_FN bool within(int e, int lo, int hi) { return (u32)(e - lo) <= (u32)(hi - lo); }
@@ -332,19 +345,20 @@ FX_FN u64 log2_q57(u64 M, int e, bool& neg) {
   return (u64)(neg ? -v : v);
 }
 
-// x^y for positive x in [2^-30, 2^30] and 2^-10 <= |y| < 2; out of that range pow
+// x^y for positive x in [2^-30, 2^30] and 2^-10 <= |y| < 16; out of that range pow
 FX_FN double pow(double x, double y) {
   const u64 b = bits(x), by = bits(y);
   const int eb = (int)(u32)(b >> 52), ey = expo(by) - 1023;
-  if (!within(eb, 1023 - 30, 1023 + 30) || !within(ey, -10, 0)) return slow_pow(x, y);
+  if (!within(eb, 1023 - 30, 1023 + 30) || !within(ey, -10, 3)) return slow_pow(x, y);
   bool neg;
   const u64 L = log2_q57(signif(b), eb - 1023, neg);  // Q57
-  const u64 Y = signif(by) >> (1 - ey);               // |y|: Q62
+  const int s = ey > 0 ? ey : 0;
+  const u64 Y = signif(by) >> (1 - (ey - s));         // |y| 2^-s: Q62
   if (by >> 63) neg = !neg;
   // L Y: Q119 in 128 bits
-  const u64 hi = mulh(L, Y), lo = L * Y;              // hi Q55
-  int n = (int)(hi >> 55);
-  u64 f = (hi << 9) | (lo >> 55);
+  const u64 hi = mulh_exact(L, Y), lo = L * Y;              // hi Q55
+  int n = (int)(hi >> (55 - s));
+  u64 f = (hi << (9 + s)) | (lo >> (55 - s));
   if (neg) {
     n = -n - (f != 0 ? 1 : 0);
     f = 0 - f;
@@ -352,17 +366,9 @@ FX_FN double pow(double x, double y) {
   return pack(0, n, exp2_frac(f));
 }
 
-// arc cosine of |x| <= 1 - 2^-24; outside acos.  About 130 cycles per warp
-// against 1415 of the FP64 function.  asin(u) = u P(4 u^2) for u <= 1/2, P the
-// Taylor series of asin(s)/s to s^52 (error 2^-61); beyond 1/2 the half-angle
-// form 2 asin(sqrt((1 - |x|) / 2)).
-FX_FN double acos(double x) {
-  const u64 b = bits(x);
-  const int e = expo(b) - 1023;
-  const bool small = e < -1;
-  const u64 X = e < -62 ? 0 : signif(b) >> (e < 0 ? -e : 0);  // |x|, Q63
-  const u64 Z = small ? mulh(X, X) << 2 : 0x8000000000000000ull - X;  // u^2, Q64
-  if (e >= 0 || (!small && Z < 0x0000008000000000ull)) return slow_acos(x);
+// P(4 Z 2^-64) of asin(u) = u P(4 u^2), u^2 = Z 2^-64 <= 1/4: the Taylor series of
+// asin(s)/s to s^52 (error 2^-61), Q63
+FX_FN u64 asin_poly(u64 Z) {
   const u64 w = (Z >= 0x4000000000000000ull ? 0x3fffffffffffffffull : Z) << 2;
   const u32 w32 = (u32)(w >> 32);
   u32 s = 1u;
@@ -391,7 +397,32 @@ FX_FN double acos(double x) {
   a = 0x002db6db6db6db6eull + mulh(a, w);
   a = 0x0133333333333333ull + mulh(a, w);
   a = 0x0aaaaaaaaaaaaaabull + mulh(a, w);
-  a = 0x8000000000000000ull + (mulh(a, w) >> 1);  // P, Q63
+  return 0x8000000000000000ull + (mulh(a, w) >> 1);
+}
+
+// arc sine of |x| < 1/2; outside asin
+FX_FN double asin(double x) {
+  const u64 b = bits(x);
+  const int e = expo(b) - 1023;
+  if (e < -31) return e < -1022 ? slow_asin(x) : x;
+  if (e >= -1) return slow_asin(x);
+  const u64 M = signif(b), X = M >> -e;
+  const u64 A = mulh(M, asin_poly(mulh(X, X) << 2));  // asin|x| 2^-e, Q62 in [1, 2.1)
+  const int lz = clz64(A);
+  return pack(b & 0x8000000000000000ull, e + 1 - lz, A << lz);
+}
+
+// arc cosine of |x| <= 1 - 2^-24; outside acos.  About 130 cycles per warp
+// against 1415 of the FP64 function.  asin_poly for u <= 1/2; beyond, the half-angle
+// form 2 asin(sqrt((1 - |x|) / 2)).
+FX_FN double acos(double x) {
+  const u64 b = bits(x);
+  const int e = expo(b) - 1023;
+  const bool small = e < -1;
+  const u64 X = e < -62 ? 0 : signif(b) >> (e < 0 ? -e : 0);  // |x|, Q63
+  const u64 Z = small ? mulh(X, X) << 2 : 0x8000000000000000ull - X;  // u^2, Q64
+  if (e >= 0 || (!small && Z < 0x0000008000000000ull)) return slow_acos(x);
+  const u64 a = asin_poly(Z);
   u64 V;
   int ex = 1;
   if (small) {
@@ -410,6 +441,114 @@ FX_FN double acos(double x) {
   }
   const int lz = clz64(V);
   return pack(0, ex - lz, V << lz);
+}
+
+FX_SLOW double slow_sin(double x) { return std::sin(x); }
+FX_SLOW double slow_cos(double x) { return std::cos(x); }
+FX_SLOW double slow_erf(double x) { return std::erf(x); }
+
+// V 2^-63 as a double
+FX_FN double from_q63(u64 V, u64 sign) {
+  const int lz = clz64(V);
+  return V == 0 ? 0.0 : pack(sign, -lz, V << lz);
+}
+
+// sin(x) and cos(x) to 2^-58 absolute (|x| 2^-65 from the 64-bit 2 / pi on top; not
+// relative to a small sine) for |x| < 1024.  x 2/pi = n + f with |f| <= 1/2, then
+// the Taylor series in v = 2 |f|: sum (-1)^k (pi/4)^k v^k / k!, the upper terms in 32
+// bits.  About 130 cycles per warp for both against 1274 for either FP64 function.
+FX_FN void sincos(double x, double& sn, double& cs) {
+  const u64 b = bits(x);
+  const int e = expo(b) - 1023;
+  if (e > 9) {
+    sn = slow_sin(x);
+    cs = slow_cos(x);
+    return;
+  }
+  const u64 C = 0xa2f9836e4e44152aull;  // 2 / pi, Q64
+  const u64 M = signif(b), hi = mulh_exact(M, C), lo = M * C;
+  u32 n = 0;
+  u64 f;  // fraction of |x| 2/pi, Q64
+  if (e >= 0) {
+    n = (u32)(hi >> (63 - e));
+    f = (hi << (1 + e)) | (lo >> (63 - e));
+  } else {
+    f = e < -64 ? 0 : hi >> (-1 - e);
+  }
+  const bool up = (f >> 63) != 0;
+  n += up;
+  u64 v = up ? 0 - f : f;
+  v = v >> 63 ? ~0ull : v << 1;
+  const u64 w = mulh(v, v);
+  const u32 w32 = (u32)(w >> 32);
+  u32 t = 23531u - mulh32(53u, w32);
+  t = 8011021u - mulh32(t, w32);
+  t = 2025968632u - mulh32(t, w32);
+  u64 a = 0x00000541e0d21fbaull - (((u64)t * w32) >> 28);
+  a = 0x000265a599cc57b1ull - mulh(a, w);
+  a = 0x00a335e33bad570full - mulh(a, w);
+  a = 0x14abbce625be52bfull - mulh(a, w);
+  a = 0xc90fdaa22168c235ull - mulh(a, w);
+  const u64 S = mulh(a, v) >> 1;  // Q63
+  t = 1155u - mulh32(2u, w32);
+  t = 449417u - mulh32(t, w32);
+  t = 132599337u - mulh32(t, w32);
+  a = 0x000000069b47ca88ull * 16 + 1 - (((u64)t * w32) >> 28);
+  a = 0x00003c3ea0d12375ull - mulh(a, w);
+  a = 0x00155d3c7e3cbffaull - mulh(a, w);
+  a = 0x040f07c206d6b0edull - mulh(a, w);
+  a = 0x4ef4f326f9177969ull - mulh(a, w);
+  const u64 c = 0x8000000000000000ull - (mulh(a, w) >> 1);
+  const u64 top = 0x8000000000000000ull, neg = b & top;
+  const u64 sS = up ? top : 0;  // sign of sin(f)
+  const bool odd = n & 1, half = (n & 2) != 0;
+  // n = 0: (S, c); 1: (c, -S); 2: (-S, -c); 3: (-c, S)
+  const u64 s1 = (half ? top : 0), c1 = ((n + 1) & 2) ? top : 0;
+  sn = from_q63(odd ? c : S, (odd ? s1 : s1 ^ sS) ^ neg);
+  cs = from_q63(odd ? S : c, odd ? c1 ^ sS : c1);
+}
+
+#ifdef __CUDACC__
+FX_TABLE ErfRow kErf[48] = {FX_ERF_ROWS};
+#endif
+FX_FN const ErfRow& erf_row(int j) {
+#if defined(__CUDACC__) && defined(__CUDA_ARCH__)
+  return kErf[j];
+#else
+  static const ErfRow host[48] = {FX_ERF_ROWS};
+  return host[j];
+#endif
+}
+
+// erf(x) to 2^-58 absolute: a Taylor series about the nearest of 48 centres on
+// [0, 6); beyond erf.  About 120 cycles per warp against 3025.
+FX_FN double erf(double x) {
+  const u64 b = bits(x);
+  const int e = expo(b) - 1023;
+  const u64 X = e > 2 ? ~0ull : e < -60 ? 0 : signif(b) >> (3 - e);  // |x|, Q60
+  const int j = (int)(X >> 57);
+  if (j >= 48) return slow_erf(x);
+  const ErfRow& r = erf_row(j);
+  const int64_t z = (int64_t)((X << 7) ^ 0x8000000000000000ull);  // Q63
+  const int32_t zh = (int32_t)(z >> 32);
+  auto m32 = [zh](int32_t a) { return (int32_t)(((int64_t)a * zh) >> 31); };
+  // a z / 2^63
+  auto m64 = [z](int64_t a) {
+    u64 p = mulh((u64)a, (u64)z);
+    if (a < 0) p -= (u64)z;
+    if (z < 0) p -= (u64)a;
+    return (int64_t)(p << 1);
+  };
+  int32_t t = r.d[3] + m32(r.d[4]);
+  t = r.d[2] + m32(t);
+  t = r.d[1] + m32(t);
+  t = r.d[0] + m32(t);
+  int64_t a = r.c[6] + (((int64_t)t * zh) >> 31);
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+  for (int k = 5; k >= 0; --k) a = r.c[k] + m64(a);
+  return from_q63((u64)(a < 0 ? 0 : a) << 1, b & 0x8000000000000000ull);
 }
 
 }  // namespace fx

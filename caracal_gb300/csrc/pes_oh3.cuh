@@ -12,12 +12,16 @@
 // of R1 (1 - exp(-b (R - Re)) cancels near its minimum) and the H2 LEPS term
 // (its Coulomb and exchange parts cancel) in double-FP32 arithmetic
 // (ff32.cuh) from the FP64 distances split into float pairs, the rest FP32.
+// FP64 exponentials, reciprocals and roots run on the integer pipe (fx64.cuh),
+// 1 - tanh and its derivative come from one exponential: 1000 x 24 plain 51 -> 33
+// us per step, 4096 x 32 mixed 100 -> 82.
 #pragma once
 #include <cuda_runtime.h>
 
 #include <type_traits>
 
 #include "ff32.cuh"
+#include "fx64.cuh"
 
 namespace cr {
 namespace oh3 {
@@ -37,11 +41,15 @@ struct K {
 
 template <class F>
 __device__ inline F sq(F x) { return x * x; }
+__device__ inline double oexp(double x) { return fx::exp(x); }
+__device__ inline float oexp(float x) { return expf(x); }
+__device__ inline double orcp(double x) { return fx::rcp(x); }
+__device__ inline float orcp(float x) { return f_rcp(x); }
 
 // Morse D (1 - exp(-B (R - T)))^2 and its derivative
 template <class F>
 __device__ inline void morse(F d, F b, F t, F r, F& v, F& dv) {
-  const F ex = exp(-b * (r - t));
+  const F ex = oexp(-b * (r - t));
   const F u = F(1) - ex;
   v = d * (u * u);
   dv = F(2) * b * d * u * ex;
@@ -59,18 +67,20 @@ __device__ inline F v3pot(const F (&r)[3], F (&dedr)[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     do4z[i] = de[i] / F(4) / zpo;
-    x[i] = exp(-be[i] * (r[i] - re[i]));
+    x[i] = oexp(-be[i] * (r[i] - re[i]));
     e = e + do4z[i] * (zp3 * x[i] - top3z) * x[i];
     exch[i] = do4z[i] * (op3z * x[i] - tzp3) * x[i];
   }
-  const F rad = sqrt(sq(exch[0] - exch[1]) + sq(exch[1] - exch[2]) + sq(exch[2] - exch[0]));
+  F rad, irad;
+  fx::sqrt_rsqrt(sq(exch[0] - exch[1]) + sq(exch[1] - exch[2]) + sq(exch[2] - exch[0]), rad, irad);
   const F is2 = F(0.70710678118654752440);
+  irad *= is2;
   e = e - rad * is2;
   const F s = exch[0] + exch[1] + exch[2];
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const F b = be[i] * do4z[i] * F(2);
-    dedr[i] = b * x[i] * ((F(3) * exch[i] - s) * is2 * (op3z * x[i] - zp3) / rad - zp3 * x[i] + op3z);
+    dedr[i] = b * x[i] * ((F(3) * exch[i] - s) * irad * (op3z * x[i] - zp3) - zp3 * x[i] + op3z);
   }
   return e;
 }
@@ -118,9 +128,9 @@ template <class F>
 __device__ inline F v4pot(const F (&r)[4], F (&dedr)[4]) {
   const F a0 = F(K::alp[0]), a1 = F(K::alp[1]), a2 = F(K::alp[2]), a3 = F(K::alp[3]);
   const F c0 = F(K::clam[0]), c1 = F(K::clam[1]), c2 = F(K::clam[2]), c3 = F(K::clam[3]);
-  const F t1 = exp(-(c0 * sq(r[0] - a0)) - c0 * sq(r[1] - a0) - c2 * sq(r[2] - a2) - c2 * sq(r[3] - a2)) *
+  const F t1 = oexp(-(c0 * sq(r[0] - a0)) - c0 * sq(r[1] - a0) - c2 * sq(r[2] - a2) - c2 * sq(r[3] - a2)) *
                F(K::acon[0]);
-  const F t2 = exp(-(c1 * sq(r[0] - a1)) - c1 * sq(r[1] - a1) - c3 * sq(r[2] - a3) - c3 * sq(r[3] - a3)) *
+  const F t2 = oexp(-(c1 * sq(r[0] - a1)) - c1 * sq(r[1] - a1) - c3 * sq(r[2] - a3) - c3 * sq(r[3] - a3)) *
                F(K::acon[1]);
   dedr[0] = F(-2) * (t1 * c0 * (r[0] - a0) + t2 * c1 * (r[0] - a1));
   dedr[1] = F(-2) * (t1 * c0 * (r[1] - a0) + t2 * c1 * (r[1] - a1));
@@ -129,9 +139,9 @@ __device__ inline F v4pot(const F (&r)[4], F (&dedr)[4]) {
   return t1 + t2;
 }
 
-// Water-like term of (OH, OH', HH): Q1 Q2 Q3 P, Q = 1 - tanh(gam s / 2)
-// (2 / (1 + exp(2x)) for 15 <= x < 43, 0 beyond; where Q = 0 the derivative
-// is 0); derivatives returned in the argument order
+// Water-like term of (OH, OH', HH): Q1 Q2 Q3 P, Q = 1 - tanh(x) = 2 / (1 + exp(2x)),
+// x = gam s / 2, 0 from x = 43 on; dQ/dx = -1/cosh^2 x = -Q (2 - Q);
+// derivatives returned in the argument order
 template <class F>
 __device__ inline F vh2o(const F (&r)[3], F (&dedr)[3]) {
   const F gam[3] = {F(K::gam[0]), F(K::gam[1]), F(K::gam[2])};
@@ -141,32 +151,20 @@ __device__ inline F vh2o(const F (&r)[3], F (&dedr)[3]) {
   s[1] = r[2] - F(K::rehh);
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const F x = F(0.5) * gam[i] * s[i];
-    if (x < F(15)) {
-      q[i] = F(1) - tanh(x);
-    } else if (x < F(43)) {
-      q[i] = F(2) / (F(1) + exp(F(2) * x));
-    } else {
-      q[i] = F(0);
-      dq[i] = F(0);
-      continue;
-    }
-    const F ch = cosh(x);
-    dq[i] = F(-0.5) * gam[i] / (ch * ch);
+    const F x2 = gam[i] * s[i];
+    q[i] = x2 < F(86) ? F(2) * orcp(F(1) + oexp(x2)) : F(0);
+    dq[i] = F(-0.5) * gam[i] * (q[i] * (F(2) - q[i]));
   }
   const F c0 = F(K::con[0]), c1 = F(K::con[1]), c2 = F(K::con[2]), c3 = F(K::con[3]), c4 = F(K::con[4]),
           c5 = F(K::con[5]), c6 = F(K::con[6]);
   const F p = c0 + c1 * (s[0] + s[2]) + c2 * s[1] + F(0.5) * c3 * (s[0] * s[0] + s[2] * s[2]) +
               F(0.5) * c4 * s[1] * s[1] + c5 * s[1] * (s[0] + s[2]) + c6 * s[0] * s[2];
-  const F e = q[0] * q[1] * q[2] * p;
+  const F q12 = q[1] * q[2], q02 = q[0] * q[2], q01 = q[0] * q[1], qa = q01 * q[2], e = qa * p;
   const F dp[3] = {c1 + c3 * s[0] + c5 * s[1] + c6 * s[2], c2 + c4 * s[1] + c5 * (s[0] + s[2]),
                    c1 + c3 * s[2] + c5 * s[1] + c6 * s[0]};
-  F d[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) d[i] = q[i] == F(0) ? F(0) : e * (dq[i] / q[i] + (dp[i] / p));
-  dedr[0] = d[0];
-  dedr[1] = d[2];
-  dedr[2] = d[1];
+  dedr[0] = fma(dq[0] * q12, p, qa * dp[0]);
+  dedr[1] = fma(dq[2] * q01, p, qa * dp[2]);
+  dedr[2] = fma(dq[1] * q02, p, qa * dp[1]);
   return e;
 }
 
@@ -277,13 +275,13 @@ struct PesOH3 {
   template <class F>
   __device__ static inline void egrad(const double (&q)[12], double& V, double (&g)[12]) {
     constexpr int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {1, 2, 3, 2, 3, 3};  // R_k = |q_pb - q_pa|
-    double d[6][3], Rd[6];
+    double d[6][3], Rd[6], iRd[6];
     F R[6], dv[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
 #pragma unroll
       for (int x = 0; x < 3; ++x) d[k][x] = q[3 * pb[k] + x] - q[3 * pa[k] + x];
-      Rd[k] = sqrt(d[k][0] * d[k][0] + d[k][1] * d[k][1] + d[k][2] * d[k][2]);
+      fx::sqrt_rsqrt(d[k][0] * d[k][0] + d[k][1] * d[k][1] + d[k][2] * d[k][2], Rd[k], iRd[k]);
       R[k] = (F)Rd[k];
     }
     double dvd[6];
@@ -301,7 +299,7 @@ struct PesOH3 {
     for (int x = 0; x < 12; ++x) g[x] = 0.0;
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
-      const double u = dvd[k] / Rd[k];
+      const double u = dvd[k] * iRd[k];
 #pragma unroll
       for (int x = 0; x < 3; ++x) {
         g[3 * pa[k] + x] -= u * d[k][x];
