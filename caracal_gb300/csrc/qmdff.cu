@@ -120,83 +120,101 @@ namespace cr {
 
 // MINB: blocks of kQmdffWarps warps kept resident per SM (the register cap
 // follows: 65536 / (MINB * 128) per thread).  The FP64 form trades spills for
-// occupancy differently from the mixed form; the autotuner below picks.
+// occupancy differently from the mixed form; the autotuner below picks.  Mixed: a
+// warp per bead; FP64: a block per bead (kTeam).
+static_assert(kQmdffWarps == qmdff::kTeam, "an FP64 block is one team");
 template <bool MIXED, int MINB, int MODE = qmdff::kFree>
 __global__ void __launch_bounds__(kQmdffWarps * 32, MINB)
     qmdff_egrad_kernel(qmdff::Dev D, int nbeads, BeadRows rows, const double* q, double* e, double* g) {
   extern __shared__ double qsm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n3 = 3 * D.n;
-  double* ws = qsm + (size_t)warp * (qmdff::warp_smem_bytes(D.n) / sizeof(double));
-  for (int b = blockIdx.x * kQmdffWarps + warp; b < nbeads; b += gridDim.x * kQmdffWarps) {
-    const size_t r = rows.row(b), r2 = rows.twin(b);
-    const double* qb = q + r * n3;
-    for (int a = lane; a < n3; a += 32) ws[a] = qb[a];
-    __syncwarp();
-    const double v = qmdff::warp_egrad<MIXED, MODE>(D, ws, g + r * n3, g + r2 * n3, 1.0, lane, r, r2);
-    if (lane == 0) {
-      e[r] = v;
-      if (r2 != r) e[r2] = v;
+  if constexpr (MIXED) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double* ws = qsm + (size_t)warp * (qmdff::warp_smem_bytes(D.n) / sizeof(double));
+    for (int b = blockIdx.x * kQmdffWarps + warp; b < nbeads; b += gridDim.x * kQmdffWarps) {
+      const size_t r = rows.row(b), r2 = rows.twin(b);
+      const double* qb = q + r * n3;
+      for (int a = lane; a < n3; a += 32) ws[a] = qb[a];
+      __syncwarp();
+      const double v = qmdff::warp_egrad<MODE>(D, ws, g + r * n3, g + r2 * n3, lane, r, r2);
+      if (lane == 0) {
+        e[r] = v;
+        if (r2 != r) e[r2] = v;
+      }
+      __syncwarp();
     }
-    __syncwarp();
+  } else {
+    for (int b = blockIdx.x; b < nbeads; b += gridDim.x) {
+      const size_t r = rows.row(b), r2 = rows.twin(b);
+      const double* qb = q + r * n3;
+      for (int a = threadIdx.x; a < n3; a += kQmdffWarps * 32) qsm[a] = qb[a];
+      const double v = qmdff::team_egrad<MODE>(D, qsm, g + r * n3, g + r2 * n3, r, r2);
+      if (threadIdx.x == 0) {
+        e[r] = v;
+        if (r2 != r) e[r2] = v;
+      }
+      __syncthreads();
+    }
   }
 }
 
 // Energy, gradient and Hessian-vector product H w per bead (plain form, dual
-// coordinates); dew[b] = w . grad E.
+// coordinates), a block per bead; dew[b] = w . grad E.
 __global__ void __launch_bounds__(kQmdffWarps * 32)
     qmdff_hvp_kernel(qmdff::Dev D, int nbeads, const double* q, const double* w, double* e, double* g, double* hw,
                      double* dew) {
   extern __shared__ double qsm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n3 = 3 * D.n;
-  double* ws = qsm + (size_t)warp * (qmdff::warp_hvp_smem_bytes(D.n) / sizeof(double));
-  for (int b = blockIdx.x * kQmdffWarps + warp; b < nbeads; b += gridDim.x * kQmdffWarps) {
+  for (int b = blockIdx.x; b < nbeads; b += gridDim.x) {
     const double* qb = q + (size_t)b * n3;
     const double* wb = w + (size_t)b * n3;
-    for (int a = lane; a < n3; a += 32) {
-      ws[a] = qb[a];
-      ws[n3 + a] = wb[a];
+    for (int a = threadIdx.x; a < n3; a += kQmdffWarps * 32) {
+      qsm[a] = qb[a];
+      qsm[n3 + a] = wb[a];
     }
-    __syncwarp();
     double de = 0.0;
-    const double v = qmdff::warp_hvp(D, ws, g ? g + (size_t)b * n3 : nullptr, hw + (size_t)b * n3, de, lane);
-    if (lane == 0) {
+    const double v = qmdff::team_hvp(D, qsm, g ? g + (size_t)b * n3 : nullptr, hw + (size_t)b * n3, de);
+    if (threadIdx.x == 0) {
       if (e) e[b] = v;
       if (dew) dew[b] = de;
     }
-    __syncwarp();
+    __syncthreads();
   }
 }
 
 // Per bead b and linear parameter t: out[b][t] = alpha_b (v_b . grad E_t|unit)
-// + beta_b E_t|unit (alpha = 1, beta = 0 where the weights are NULL).
+// + beta_b E_t|unit (alpha = 1, beta = 0 where the weights are NULL), a block per bead.
 __global__ void __launch_bounds__(kQmdffWarps * 32)
     qmdff_vjp_kernel(qmdff::Dev D, qmdff::Tables<double> U, int nbeads, int nlin, const double* q, const double* v,
                      const double* alpha, const double* beta, double* out) {
   extern __shared__ double qsm[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n3 = 3 * D.n;
-  double* xs = qsm + (size_t)warp * 2 * n3;
-  double* vs = xs + n3;
-  for (int b = blockIdx.x * kQmdffWarps + warp; b < nbeads; b += gridDim.x * kQmdffWarps) {
-    for (int a = lane; a < n3; a += 32) {
-      xs[a] = q[(size_t)b * n3 + a];
-      vs[a] = v[(size_t)b * n3 + a];
-    }
-    __syncwarp();
-    qmdff::warp_param_vjp(D, U, xs, vs, alpha ? alpha[b] : 1.0, beta ? beta[b] : 0.0, out + (size_t)b * nlin, lane);
-    __syncwarp();
+  const int n3 = 3 * D.n, b = blockIdx.x;
+  for (int a = threadIdx.x; a < n3; a += kQmdffWarps * 32) {
+    qsm[a] = q[(size_t)b * n3 + a];
+    qsm[n3 + a] = v[(size_t)b * n3 + a];
   }
+  __syncthreads();
+  qmdff::team_param_vjp(D, U, qsm, qsm + n3, alpha ? alpha[b] : 1.0, beta ? beta[b] : 0.0, out + (size_t)b * nlin);
 }
 
-// acc[t] += scale * sum_b in[b][t], the beads summed in order (deterministic).
-__global__ void sum_rows_kernel(int nrows, int ncols, const double* in, double scale, double* acc) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ncols) return;
+// acc[t] += scale * sum_b in[b][t]: 32 columns per block, eight rows at a time in
+// eight partial sums, added in order (deterministic).
+constexpr int kSumCols = 32, kSumRows = 8;
+__global__ void __launch_bounds__(kSumCols * kSumRows) sum_rows_kernel(int nrows, int ncols, const double* in, double scale, double* acc) {
+  __shared__ double part[kSumRows][kSumCols];
+  const int x = threadIdx.x, y = threadIdx.y, t = blockIdx.x * kSumCols + x;
   double s = 0.0;
-  for (int r = 0; r < nrows; ++r) s += in[(size_t)r * ncols + t];
-  acc[t] += scale * s;
+  if (t < ncols) {
+#pragma unroll 4
+    for (int r = y; r < nrows; r += kSumRows) s += in[(size_t)r * ncols + t];
+  }
+  part[y][x] = s;
+  __syncthreads();
+  if (y == 0 && t < ncols) {
+    s = 0.0;
+    for (int k = 0; k < kSumRows; ++k) s += part[k][x];
+    acc[t] += scale * s;
+  }
 }
 
 }  // namespace cr
@@ -204,11 +222,10 @@ __global__ void sum_rows_kernel(int nrows, int ncols, const double* in, double s
 int qmdff_hvp_launch(const cr_qmdff* ff, const double* d_q, const double* d_w, int nbeads, double* d_e, double* d_g,
                      double* d_hw, double* d_dew, cudaStream_t s) {
   if (ff->nterm[4] > 0) return cr_set_error(CR_ERR_UNSUPPORTED, "second derivatives of H/halogen-bond terms are not built");
-  const size_t smem = (size_t)kQmdffWarps * cr::qmdff::warp_hvp_smem_bytes(ff->n);
+  const size_t smem = cr::qmdff::team_hvp_smem_bytes(ff->n);
   CR_TRY_CUDA(cudaFuncSetAttribute(cr::qmdff_hvp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (nbeads == 0) return CR_OK;
-  int grid = (nbeads + kQmdffWarps - 1) / kQmdffWarps;
-  if (grid > 1 << 20) grid = 1 << 20;
+  const int grid = std::min(nbeads, 1 << 20);
   cr::qmdff_hvp_kernel<<<grid, kQmdffWarps * 32, smem, s>>>(ff->dev, nbeads, d_q, d_w, d_e, d_g, d_hw, d_dew);
   CR_TRY_CUDA(cudaGetLastError());
   return CR_OK;
@@ -221,18 +238,17 @@ int qmdff_vjp_launch(const cr_qmdff* ff, const double* d_q, const double* d_v, i
                      cudaStream_t s) {
   if (ff->nterm[4] > 0) return cr_set_error(CR_ERR_UNSUPPORTED, "parameter gradients of H/halogen-bond terms are not built");
   const int nlin = qmdff_nlin(ff);
-  const size_t smem = (size_t)kQmdffWarps * 2 * 3 * ff->n * sizeof(double);
+  const size_t smem = (size_t)2 * 3 * ff->n * sizeof(double);
   CR_TRY_CUDA(cudaFuncSetAttribute(cr::qmdff_vjp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (nlin == 0) return CR_OK;
   const size_t n3 = (size_t)3 * ff->n;
   for (int b0 = 0; b0 < nbeads; b0 += scratch_beads) {
     const int nb = std::min(scratch_beads, nbeads - b0);
-    const int grid = (nb + kQmdffWarps - 1) / kQmdffWarps;
-    cr::qmdff_vjp_kernel<<<grid, kQmdffWarps * 32, smem, s>>>(ff->dev, ff->unit, nb, nlin, d_q + b0 * n3, d_v + b0 * n3,
+    cr::qmdff_vjp_kernel<<<nb, kQmdffWarps * 32, smem, s>>>(ff->dev, ff->unit, nb, nlin, d_q + b0 * n3, d_v + b0 * n3,
                                                               d_alpha ? d_alpha + b0 : nullptr,
                                                               d_beta ? d_beta + b0 : nullptr, d_scratch);
     CR_TRY_CUDA(cudaGetLastError());
-    cr::sum_rows_kernel<<<(nlin + 127) / 128, 128, 0, s>>>(nb, nlin, d_scratch, scale, d_acc);
+    cr::sum_rows_kernel<<<(nlin + cr::kSumCols - 1) / cr::kSumCols, dim3(cr::kSumCols, cr::kSumRows), 0, s>>>(nb, nlin, d_scratch, scale, d_acc);
     CR_TRY_CUDA(cudaGetLastError());
   }
   return CR_OK;
@@ -255,11 +271,18 @@ const QmdffKernel kNptKernels[2] = {cr::qmdff_egrad_kernel<false, 3, cr::qmdff::
                                     cr::qmdff_egrad_kernel<true, 5, cr::qmdff::kNpt>};
 constexpr int kTuneMinBeads = 2048;  // smaller batches keep the default
 
+// Blocks and dynamic shared memory of the force kernel's forms.
+int egrad_grid(int prec, int nbeads) {
+  return std::min(prec == 1 ? (nbeads + kQmdffWarps - 1) / kQmdffWarps : nbeads, 1 << 20);
+}
+size_t egrad_smem(int prec, int n) {
+  return prec == 1 ? (size_t)kQmdffWarps * cr::qmdff::warp_smem_bytes(n) : cr::qmdff::team_smem_bytes(n);
+}
+
 int launch_dev(const cr::qmdff::Dev& D, int prec, int v, cr::BeadRows rows, const double* d_q, int nbeads, double* d_e, double* d_g,
                cudaStream_t s) {
-  const size_t smem = (size_t)kQmdffWarps * cr::qmdff::warp_smem_bytes(D.n);
-  int grid = (nbeads + kQmdffWarps - 1) / kQmdffWarps;
-  if (grid > 1 << 20) grid = 1 << 20;
+  const size_t smem = egrad_smem(prec, D.n);
+  const int grid = egrad_grid(prec, nbeads);
   const QmdffKernel k = D.periodic ? kBoxKernels[prec] : kKernels[prec][v];
   k<<<grid, kQmdffWarps * 32, smem, s>>>(D, nbeads, rows, d_q, d_e, d_g);
   CR_TRY_CUDA(cudaGetLastError());
@@ -278,12 +301,11 @@ int launch_npt(const cr_qmdff* ff, int prec, const QmdffNpt& npt, cr::BeadRows r
   D.tbox = npt.tbox;
   D.tbox_beads = npt.beads_per_box;
   D.vir = npt.vir;
-  const size_t smem = (size_t)kQmdffWarps * cr::qmdff::warp_smem_bytes(D.n);
+  const size_t smem = egrad_smem(prec, D.n);
   if (smem > 48 * 1024)
     CR_TRY_CUDA(cudaFuncSetAttribute(kNptKernels[prec], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (nbeads <= 0) return CR_OK;
-  int grid = (nbeads + kQmdffWarps - 1) / kQmdffWarps;
-  if (grid > 1 << 20) grid = 1 << 20;
+  const int grid = egrad_grid(prec, nbeads);
   kNptKernels[prec]<<<grid, kQmdffWarps * 32, smem, s>>>(D, nbeads, rows, d_q, d_e, d_g);
   CR_TRY_CUDA(cudaGetLastError());
   return CR_OK;
@@ -297,7 +319,7 @@ int qmdff_launch_kinds(const cr_qmdff* ff, unsigned mask, bool ezero, const doub
                        double* d_g, int precision, cudaStream_t s) {
   if (precision != CR_PREC_MIXED && precision != CR_PREC_FP64) return cr_set_error(CR_ERR_ARG, "unknown precision");
   const int prec = precision == CR_PREC_MIXED ? 1 : 0;
-  const size_t smem = (size_t)kQmdffWarps * cr::qmdff::warp_smem_bytes(ff->n);
+  const size_t smem = egrad_smem(prec, ff->n);
   if (smem > 48 * 1024) {
     for (int v = 0; v < kVariants; ++v)
       CR_TRY_CUDA(cudaFuncSetAttribute(kKernels[prec][v], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -365,7 +387,7 @@ int qmdff_launch(const cr_qmdff* ff_c, const double* d_q, int nbeads, double* d_
   if (precision != CR_PREC_MIXED && precision != CR_PREC_FP64) return cr_set_error(CR_ERR_ARG, "unknown precision");
   const int prec = precision == CR_PREC_MIXED ? 1 : 0;
   if (npt) return launch_npt(ff, prec, *npt, rows, d_q, nbeads, d_e, d_g, s);
-  const size_t smem = (size_t)kQmdffWarps * cr::qmdff::warp_smem_bytes(ff->n);
+  const size_t smem = egrad_smem(prec, ff->n);
   // the attribute is set even for nbeads = 0, so a caller can prepare the
   // kernels before a stream capture
   if (smem > 48 * 1024) {
@@ -490,12 +512,14 @@ int cr_qmdff_create(const cr_qmdff_def* d, cr_qmdff** out) {
     const int z1 = d->at[i1] - 1, z2 = d->at[i2] - 1;
     const size_t e12 = (size_t)z1 + 94 * (size_t)z2;  // (iz1, iz2) column-major
     double* v = &vpair[(size_t)kVPair * m];
-    v[0] = d->r0094[e12];
-    v[1] = d->c66ab[(size_t)i2 + (size_t)n * i1];     // c66ab(i2, i1)
-    v[2] = d->sr42[e12];
-    v[3] = d->zab[e12];
-    v[4] = d->r0ab[e12];
-    v[5] = d->eps2[nk - 1];
+    const double R0 = d->r0094[e12], c6 = d->c66ab[(size_t)i2 + (size_t)n * i1], eps2 = d->eps2[nk - 1];  // c66ab(i2, i1)
+    const double R02 = R0 * R0, R06 = R02 * R02 * R02;
+    v[0] = R06;
+    v[1] = R06 * R02;
+    v[2] = eps2 * c6;
+    v[3] = eps2 * c6 * d->sr42[e12];
+    v[4] = eps2 * d->zab[e12];
+    v[5] = d->r0ab[e12];
     v[6] = d->zahn ? d->q[i1] * d->q[i2] : d->q[i1] * d->q[i2] * d->eps1[nk - 1];
   }
 
@@ -593,26 +617,19 @@ int cr_qmdff_create(const cr_qmdff_def* d, cr_qmdff** out) {
   up(vtors, &D.d.vtors);
   up(vpair, &D.d.vpair);
   std::vector<float> frad = to_float(rad), fvbond = to_float(vbond), fvangl = to_float(vangl),
-                     fvtors = to_float(vtors), fvpair = to_float(vpair);
+                     fvtors = to_float(vtors);
   up(frad, &D.f.rad);
   up(fvbond, &D.f.vbond);
   up(fvangl, &D.f.vangl);
   up(fvtors, &D.f.vtors);
-  up(fvpair, &D.f.vpair);
   // mixed-form pair constants (pair_mixed)
   std::vector<float> fpair((size_t)kVPair * d->nnci);
   for (int m = 0; m < d->nnci; ++m) {
     const double* v = &vpair[(size_t)kVPair * m];
     float* o = &fpair[(size_t)kVPair * m];
-    const double R02 = v[0] * v[0], R06 = R02 * R02 * R02;
-    o[0] = (float)R06;
-    o[1] = (float)(R06 * R02);
-    o[2] = (float)(v[5] * v[1]);
-    o[3] = (float)(v[5] * v[1] * v[2]);
-    o[4] = (float)(v[5] * v[3]);
-    o[5] = (float)(v[4] * 1.4426950408889634074);  // log2(e)
-    o[6] = (float)v[6];
-    o[7] = (float)v[4];
+    for (int k = 0; k < kVPair; ++k) o[k] = (float)v[k];
+    o[5] = (float)(v[5] * 1.4426950408889634074);  // log2(e)
+    o[7] = (float)v[5];
   }
   up(fpair, &D.fpair);
   if (rc != CR_OK) {
@@ -687,7 +704,7 @@ int cr_qmdff_create(const cr_qmdff_def* d, cr_qmdff** out) {
   for (int m = 0; m < d->nangl; ++m) uangl[(size_t)kVAngl * m + 1] = 1.0;
   for (int m = 0; m < d->ntors; ++m) utors[(size_t)14 * m + 1] = 1.0;
   for (int m = 0; m < d->nnci; ++m) {
-    upair[(size_t)kVPair * m + 5] = 0.0;
+    for (int k = 2; k < 5; ++k) upair[(size_t)kVPair * m + k] = 0.0;
     upair[(size_t)kVPair * m + 6] = 1.0;
   }
   ff->unit.rad = D.d.rad;

@@ -1,4 +1,4 @@
-// QMDFF force field on the GB300: one warp per bead.
+// QMDFF force field on the GB300: one warp per bead in the mixed form, four in FP64.
 //
 // Drop-in for Caracal's per-bead QMDFF gradient (src/gradient.f90:342-358:
 // ff_eg src/ff_eg.f90:41-629, ff_nonb src/ff_nonb.f90:34-889, E_zero shift),
@@ -31,7 +31,7 @@ namespace qmdff {
 
 constexpr int kMaxAtoms = 1024;
 constexpr int kVAngl = 4;   // theta0, k, cos(theta0), linear flag
-constexpr int kVPair = 8;   // R0, C6, sr42, zab, alpha, eps2, qq (eps1 q_i q_j or q_i q_j), 0
+constexpr int kVPair = 8;   // R0^6, R0^8, eps2 C6, eps2 C6 sr42, eps2 zab, alpha, qq (eps1 q_i q_j or q_i q_j), 0
 
 // Per-term parameter tables in the arithmetic type of the form.
 template <class F>
@@ -114,7 +114,7 @@ struct Dev {
   // bond_mixed): per bond kBondSer (hi, lo) pairs: 1/r0^2, r0^2, (use flag,
   // 0), the kBondPoly coefficients
   const float2* bser;
-  // mixed form, NCI pairs with their constants folded (pair_mixed): per pair
+  // mixed form, NCI pairs with their constants folded (pair_mixed_v): per pair
   // kVPair floats R0^6, R0^8, eps2 C6, eps2 C6 sr42, eps2 zab,
   // alpha log2(e), qq, alpha, each rounded once from FP64
   const float* fpair;
@@ -150,39 +150,10 @@ __device__ inline FF ff_of(float2 v) { return FF{v.x, v.y}; }
 template <class F> __device__ inline F q_sqrt(F x);
 template <> __device__ inline double q_sqrt<double>(double x) { return sqrt(x); }
 template <> __device__ inline float q_sqrt<float>(float x) { return sqrtf(x); }
-template <class F> __device__ inline F q_exp(F x);
-template <> __device__ inline double q_exp<double>(double x) { return exp(x); }
-template <> __device__ inline float q_exp<float>(float x) { return expf(x); }
-template <class F> __device__ inline F q_acos(F x);
-template <> __device__ inline double q_acos<double>(double x) { return acos(x); }
-template <> __device__ inline float q_acos<float>(float x) { return acosf(x); }
-template <class F> __device__ inline F q_asin(F x);
-template <> __device__ inline double q_asin<double>(double x) { return asin(x); }
-template <> __device__ inline float q_asin<float>(float x) { return asinf(x); }
-template <class F> __device__ inline F q_erf(F x);
-template <> __device__ inline double q_erf<double>(double x) { return erf(x); }
-template <> __device__ inline float q_erf<float>(float x) { return erff(x); }
 template <class F> __device__ inline F q_erfc(F x);
 template <> __device__ inline double q_erfc<double>(double x) { return erfc(x); }
 template <> __device__ inline float q_erfc<float>(float x) { return erfcf(x); }
-template <class F> __device__ inline F q_sin(F x);
-template <> __device__ inline double q_sin<double>(double x) { return sin(x); }
-template <> __device__ inline float q_sin<float>(float x) { return sinf(x); }
-template <class F> __device__ inline F q_cos(F x);
-template <> __device__ inline double q_cos<double>(double x) { return cos(x); }
-template <> __device__ inline float q_cos<float>(float x) { return cosf(x); }
-template <class F> __device__ inline F q_pow(F x, double p);
-template <> __device__ inline double q_pow<double>(double x, double p) { return pow(x, p); }
-// dual coordinates (Hessian-vector products of the plain form)
-template <> __device__ inline Dual q_sqrt<Dual>(Dual x) { return sqrt(x); }
-template <> __device__ inline Dual q_exp<Dual>(Dual x) { return exp(x); }
-template <> __device__ inline Dual q_acos<Dual>(Dual x) { return acos(x); }
-template <> __device__ inline Dual q_asin<Dual>(Dual x) { return asin(x); }
-template <> __device__ inline Dual q_erf<Dual>(Dual x) { return erf(x); }
 template <> __device__ inline Dual q_erfc<Dual>(Dual x) { return erfc(x); }
-template <> __device__ inline Dual q_sin<Dual>(Dual x) { return sin(x); }
-template <> __device__ inline Dual q_cos<Dual>(Dual x) { return cos(x); }
-template <> __device__ inline Dual q_pow<Dual>(Dual x, double p) { return pow(x, p); }
 
 // |x| < 1e-14 and |x| > 1e-14 as the reference tests its FP64 denominators;
 // for FP32 the same sets of values without a conversion (1e-14 is not a
@@ -191,11 +162,6 @@ template <class F> __device__ inline bool below_1em14(F x) { return fabs((double
 template <> __device__ inline bool below_1em14<float>(float x) { return fabsf(x) <= 1e-14f; }
 template <class F> __device__ inline bool above_1em14(F x) { return fabs((double)ad::val(x)) > 1e-14; }
 template <> __device__ inline bool above_1em14<float>(float x) { return fabsf(x) > 1e-14f; }
-
-// Parameter type of a term evaluated in arithmetic type F (dual coordinates
-// read FP64 parameters).
-template <class F> struct ParamOf { using type = F; };
-template <> struct ParamOf<Dual> { using type = double; };
 
 template <class F>
 __device__ inline void cross(const F* a, const F* b, F* c) {
@@ -300,16 +266,12 @@ __device__ inline void scatter(const Contrib<float>& c, Grad<float>& G, bool dis
 }
 
 // abdamp (src/abdamp.f90:36-51); the cutoff prefactor is the REAL(4) product 3.0*3.5710642
-template <class F>
-__device__ inline void abdamp(F radi, F radj, F r2, F& damp, F& ddamp) {
-  const F pre = (F)(double)(3.0f * 3.5710642f);
-  const F s = radi + radj;
-  const F rcut = pre * (s * s);
-  const F x = r2 / rcut;
-  const F rr = x * x;
-  if constexpr (std::is_same<F, float>::value) damp = __frcp_rn(1.0f + rr);  // = 1/(1 + rr), correctly rounded
-  else damp = F(1) / (F(1) + rr);
-  ddamp = F(-4) * rr * (damp * damp) / r2;
+__device__ inline void abdamp(float radi, float radj, float r2, float& damp, float& ddamp) {
+  const float s = radi + radj;
+  const float x = r2 / ((3.0f * 3.5710642f) * (s * s));
+  const float rr = x * x;
+  damp = __frcp_rn(1.0f + rr);  // = 1/(1 + rr), correctly rounded
+  ddamp = -4.0f * rr * (damp * damp) / r2;
 }
 
 // A bead's coordinates: FP64, and (mixed form) the FP32 split x = hi + lo.
@@ -387,32 +349,7 @@ __device__ inline void disp<float>(const BeadPos& X, int a, int b, float* v) {
   }
 }
 
-// Bond stretch, generalised Lennard-Jones (src/ff_eg.f90:87-163):
-// e = k (1 + (r0/r)^a - 2 (r0/r)^(a/2)).
-template <class F>
-__device__ inline F bond_plain(const Dev& D, const Tables<typename ParamOf<F>::type>& T, const BeadPos& x, int m,
-                               Contrib<F>& c) {
-  const int i = D.bond[2 * m], j = D.bond[2 * m + 1];
-  F rb[3];
-  disp<F>(x, i, j, rb);
-  const F r2 = rb[0] * rb[0] + rb[1] * rb[1] + rb[2] * rb[2];
-  const F r = q_sqrt<F>(r2);
-  const auto* v = &T.vbond[3 * m];
-  const double rij = v[0], kij = v[1], aai = v[2];
-  const F pa2 = q_pow<F>(rij / r, aai / 2), pa = pa2 * pa2;
-  const F fac = aai * kij * (-pa + pa2) / r2;
-  c.na = 2;
-  c.a[0] = i;
-  c.a[1] = j;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    c.g[0][d] = fac * rb[d];
-    c.g[1][d] = -fac * rb[d];
-  }
-  return kij * (1. + pa - 2. * pa2);
-}
-
-// Mixed form: with u = (r0/r)^(a/2) = exp(-(a/2) log1p(x)), x = (r - r0)/r0
+// Bond stretch of the mixed form (src/ff_eg.f90:87-163): with u = (r0/r)^(a/2) = exp(-(a/2) log1p(x)), x = (r - r0)/r0
 // taken from the FP64 r^2 - r0^2, e = k (1 - u)^2 and the gradient factor
 // a k u (1 - u) / r^2 are free of the cancellation in 1 + u^2 - 2u.
 // Bond stretches carry the largest forces of a molecule, so FP32 roundings
@@ -490,10 +427,10 @@ __device__ inline float bond_mixed(const Dev& D, const BeadPos& x, int m, Contri
   return kij * omu * omu;
 }
 
-// Angle bend with abdamp damping (src/ff_eg.f90:167-299).
-template <class F>
-__device__ inline F angle_term(const Dev& D, const Tables<typename ParamOf<F>::type>& T, const BeadPos& x, int m,
-                               Contrib<F>& c) {
+// Angle bend with abdamp damping (src/ff_eg.f90:167-299), mixed form.
+__device__ inline float angle_mixed(const Dev& D, const BeadPos& x, int m, Contrib<float>& c) {
+  using F = float;
+  const Tables<float>& T = D.f;
   const int j = D.angl[3 * m], i = D.angl[3 * m + 1], k = D.angl[3 * m + 2];
   const auto* v = &T.vangl[kVAngl * m];
   const F c0 = v[0], kijk = v[1], cc0 = v[2];
@@ -511,10 +448,10 @@ __device__ inline F angle_term(const Dev& D, const Tables<typename ParamOf<F>::t
   // harmonic-cosine form as sqrt((1 - c)(1 + c)), free of cancellation away
   // from c = +-1 (where the linear form is used)
   F theta = F(0);
-  if (!std::is_same<F, float>::value || v[3] != F(0)) theta = q_acos<F>(cosa);
+  if (v[3] != F(0)) theta = acosf(cosa);
   F dampij, damp2ij, dampjk, damp2jk;
-  abdamp<F>(T.rad[i], T.rad[j], rab2, dampij, damp2ij);
-  abdamp<F>(T.rad[k], T.rad[j], rcb2, dampjk, damp2jk);
+  abdamp(T.rad[i], T.rad[j], rab2, dampij, damp2ij);
+  abdamp(T.rad[k], T.rad[j], rcb2, dampjk, damp2jk);
   const F damp = dampij * dampjk;
   F ea, deddt;
   if (v[3] != F(0)) {  // linear reference angle: harmonic in theta
@@ -524,9 +461,7 @@ __device__ inline F angle_term(const Dev& D, const Tables<typename ParamOf<F>::t
   } else {
     const F dd = cosa - cc0;
     ea = kijk * (dd * dd);
-    F sth;
-    if constexpr (std::is_same<F, float>::value) sth = sqrtf((1.0f - cosa) * (1.0f + cosa));
-    else sth = q_sin<F>(theta);
+    const F sth = sqrtf((1.0f - cosa) * (1.0f + cosa));
     deddt = F(2) * kijk * sth * (cc0 - cosa);
   }
   F deda[3], dedc[3];
@@ -549,45 +484,21 @@ __device__ inline F angle_term(const Dev& D, const Tables<typename ParamOf<F>::t
   return ea * damp;
 }
 
-// Torsion angle phi in [0, pi] of i-j-k-l (valijkl, src/valijkl.f90) with
-// its cosine and sine.  FP64: Caracal's acos of the normalised plane normals.
-// FP32: atan2(|rb| |na . rc|, na . nb), accurate near 0 and pi.
-template <class F>
-__device__ inline F dihedral(const F* ra, const F* rb, const F* rc, F* na, F* nb, F& nan_, F& nbn,
-                             F& cosphi, F& sinphi) {
+// Torsion angle phi in [0, pi] of i-j-k-l (valijkl, src/valijkl.f90) with its
+// cosine and sine, as atan2(|rb| |na . rc|, na . nb), accurate near 0 and pi.
+__device__ inline float dihedral(const float* ra, const float* rb, const float* rc, float* na, float* nb, float& nan_,
+                                 float& nbn, float& cosphi, float& sinphi) {
   cross(ra, rb, na);
   cross(rb, rc, nb);
-  nan_ = q_sqrt<F>(dot3(na, na));
-  nbn = q_sqrt<F>(dot3(nb, nb));
-  F phi;
-  if constexpr (!std::is_same<F, float>::value) {
-    F a[3] = {na[0], na[1], na[2]}, b[3] = {nb[0], nb[1], nb[2]};
-    if (fabs(ad::val(nan_)) > 1e-14) {
-      const F o = 1.0 / nan_;
-      a[0] *= o;
-      a[1] *= o;
-      a[2] *= o;
-    }
-    if (fabs(ad::val(nbn)) > 1e-14) {
-      const F o = 1.0 / nbn;
-      b[0] *= o;
-      b[1] *= o;
-      b[2] *= o;
-    }
-    F s = a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
-    if (fabs(fabs(ad::val(s)) - 1.0) < 1e-14) s = ad::val(s) >= 0 ? F(1.0) : F(-1.0);
-    phi = q_acos<F>(s);
-    cosphi = q_cos<F>(phi);
-    sinphi = q_sin<F>(phi);
-  } else {
-    const float cn = dot3(na, nb);
-    const float sn = sqrtf(dot3(rb, rb)) * fabsf(dot3(na, rc));
-    phi = atan2f(sn, cn);
-    const float den = nan_ * nbn;
-    const float id = den > 0.f ? __frcp_rn(den) : 0.f;
-    cosphi = den > 0.f ? cn * id : 1.f;
-    sinphi = den > 0.f ? sn * id : 0.f;
-  }
+  nan_ = sqrtf(dot3(na, na));
+  nbn = sqrtf(dot3(nb, nb));
+  const float cn = dot3(na, nb);
+  const float sn = sqrtf(dot3(rb, rb)) * fabsf(dot3(na, rc));
+  const float phi = atan2f(sn, cn);
+  const float den = nan_ * nbn;
+  const float id = den > 0.f ? __frcp_rn(den) : 0.f;
+  cosphi = den > 0.f ? cn * id : 1.f;
+  sinphi = den > 0.f ? sn * id : 0.f;
   return phi;
 }
 
@@ -600,13 +511,12 @@ __device__ inline F tors_virial(const F* vab, const F* vcb, const F* vdc, const 
 }
 
 // Torsions (erf-blended cosine series, src/ff_eg.f90:303-440) and
-// inversions (tors type 2, src/ff_eg.f90:441-618).
-template <class F>
-__device__ inline F torsion_term(const Dev& D, const Tables<typename ParamOf<F>::type>& T, const BeadPos& x, int m,
-                                 Contrib<F>& c, F* vir = nullptr) {
+// inversions (tors type 2, src/ff_eg.f90:441-618), mixed form.
+__device__ inline float torsion_mixed(const Dev& D, const BeadPos& x, int m, Contrib<float>& c, float* vir = nullptr) {
+  using F = float;
+  const Tables<float>& T = D.f;
   const F pi = (F)3.1415926535897932384626433832795029;
   const F pi2 = (F)6.28318530717958623199592693708837;
-  const F spi = (F)1.77245385090551599275151910313925;
   const int i = D.tors[6 * m], j = D.tors[6 * m + 1], k = D.tors[6 * m + 2], l = D.tors[6 * m + 3];
   const int nt = D.tors[6 * m + 4], type = D.tors[6 * m + 5];
   const auto* vt = &T.vtors[14 * m];
@@ -622,16 +532,15 @@ __device__ inline F torsion_term(const Dev& D, const Tables<typename ParamOf<F>:
     disp<F>(x, i, j, vab);
     disp<F>(x, j, k, vcb);
     disp<F>(x, k, l, vdc);
-    abdamp<F>(T.rad[i], T.rad[j], dot3(vab, vab), dampij, d2ij);
-    abdamp<F>(T.rad[k], T.rad[j], dot3(vcb, vcb), dampjk, d2jk);
-    abdamp<F>(T.rad[k], T.rad[l], dot3(vdc, vdc), dampX, d2X);
+    abdamp(T.rad[i], T.rad[j], dot3(vab, vab), dampij, d2ij);
+    abdamp(T.rad[k], T.rad[j], dot3(vcb, vcb), dampjk, d2jk);
+    abdamp(T.rad[k], T.rad[l], dot3(vdc, vdc), dampX, d2X);
     // dphidr (src/dphidr.f90): ra = r_j - r_i, rb = r_k - r_j, rc = r_l - r_k
     const F ra[3] = {-vab[0], -vab[1], -vab[2]}, rb[3] = {-vcb[0], -vcb[1], -vcb[2]};
     const F rc[3] = {-vdc[0], -vdc[1], -vdc[2]};
     F na[3], nb[3], nan_, nbn, cosphi, sinphi;
-    const F phi = dihedral<F>(ra, rb, rc, na, nb, nan_, nbn, cosphi, sinphi);
-    const F nenner = nan_ * nbn * sinphi;
-    if constexpr (std::is_same<F, float>::value) {
+    const F phi = dihedral(ra, rb, rc, na, nb, nan_, nbn, cosphi, sinphi);
+    {
       // FP32: dphi/dr without the division by sin(phi) of dphidr.f90, whose
       // numerator cancels as phi -> 0 or pi (planar groups); the same
       // derivative, written with the plane normals (Blondel and Karplus,
@@ -658,62 +567,19 @@ __device__ inline F torsion_term(const Dev& D, const Tables<typename ParamOf<F>:
           ddc[d] = -fb * nb[d] - uv;
         }
       }
-    } else if (below_1em14(nenner)) {
-#pragma unroll
-      for (int d = 0; d < 3; ++d) dda[d] = ddb[d] = ddc[d] = ddd[d] = F(0);
-    } else {
-      F on, rba_, rab_;
-      if constexpr (std::is_same<F, float>::value) {
-        on = __frcp_rn(nenner);
-        rba_ = nbn * __frcp_rn(nan_);
-        rab_ = nan_ * __frcp_rn(nbn);
-      } else {
-        on = F(1) / nenner;
-        rba_ = nbn / nan_;
-        rab_ = nan_ / nbn;
-      }
-      const F rapb[3] = {ra[0] + rb[0], ra[1] + rb[1], ra[2] + rb[2]};
-      const F rbpc[3] = {rb[0] + rc[0], rb[1] + rc[1], rb[2] + rc[2]};
-      F t_rab[3], t_rba[3], t_rac[3], t_rbb[3], t_rbc[3], t_raa[3], rapba[3], rapbb[3], rbpca[3], rbpcb[3];
-      cross(na, rb, t_rab);
-      cross(nb, ra, t_rba);
-      cross(na, rc, t_rac);
-      cross(nb, rb, t_rbb);
-      cross(nb, rc, t_rbc);
-      cross(na, ra, t_raa);
-      cross(rapb, na, rapba);
-      cross(rapb, nb, rapbb);
-      cross(rbpc, na, rbpca);
-      cross(rbpc, nb, rbpcb);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        dda[d] = on * (cosphi * rba_ * t_rab[d] - t_rbb[d]);
-        ddb[d] = on * (cosphi * (rba_ * rapba[d] + rab_ * t_rbc[d]) - (t_rac[d] + rapbb[d]));
-        ddc[d] = on * (cosphi * (rba_ * t_raa[d] + rab_ * rbpcb[d]) - (t_rba[d] + rbpca[d]));
-        ddd[d] = on * (cosphi * rab_ * t_rbb[d] - t_rab[d]);
-      }
     }
     et = F(0);
     dij = F(0);
     const F phipi = phi - pi;
-    const F ef = q_erf<F>(phipi);
-    F expo;
-    if constexpr (std::is_same<F, float>::value) expo = q_exp<F>(-(phipi * phipi)) * 0.564189583547756286948f;  // 1/sqrt(pi)
-    else expo = q_exp<F>(-(phipi * phipi)) / spi;
+    const F ef = erff(phipi);
+    const F expo = expf(-(phipi * phipi)) * 0.564189583547756286948f;  // 1/sqrt(pi)
     for (int it = 0; it < nt; ++it) {
       const F rn = vt[2 + 3 * it], ph = vt[3 + 3 * it], vn = vt[4 + 3 * it];
       const F c1 = rn * (phi - phi0) + ph;
       const F c2 = rn * (phi + phi0 - pi2) + ph;
       F x1cos, x2cos, x1sin, x2sin;
-      if constexpr (std::is_same<F, float>::value) {
-        sincosf(c1, &x1sin, &x1cos);
-        sincosf(c2, &x2sin, &x2cos);
-      } else {
-        x1cos = q_cos<F>(c1);
-        x2cos = q_cos<F>(c2);
-        x1sin = q_sin<F>(c1);
-        x2sin = q_sin<F>(c2);
-      }
+      sincosf(c1, &x1sin, &x1cos);
+      sincosf(c2, &x2sin, &x2cos);
       const F e1 = vn * (F(1) + x1cos), e2 = vn * (F(1) + x2cos);
       et = et + F(0.5) * (F(1) - ef) * e1 + (F(0.5) + F(0.5) * ef) * e2;
       dij = dij - expo * e1 - F(0.5) * (F(1) - ef) * vn * x1sin * rn + expo * e2 -
@@ -739,9 +605,9 @@ __device__ inline F torsion_term(const Dev& D, const Tables<typename ParamOf<F>:
   disp<F>(x, j, i, vab);
   disp<F>(x, j, k, vcb);
   disp<F>(x, j, l, vdc);
-  abdamp<F>(T.rad[i], T.rad[j], dot3(vab, vab), dampij, d2ij);
-  abdamp<F>(T.rad[k], T.rad[j], dot3(vcb, vcb), dampjk, d2jk);
-  abdamp<F>(T.rad[j], T.rad[l], dot3(vdc, vdc), dampX, d2X);
+  abdamp(T.rad[i], T.rad[j], dot3(vab, vab), dampij, d2ij);
+  abdamp(T.rad[k], T.rad[j], dot3(vcb, vcb), dampjk, d2jk);
+  abdamp(T.rad[j], T.rad[l], dot3(vdc, vdc), dampX, d2X);
   const F re[3] = {-vab[0], -vab[1], -vab[2]};  // r_i - r_j
   const F rd[3] = {-vcb[0], -vcb[1], -vcb[2]};  // r_k - r_j
   F rv[3];
@@ -749,26 +615,8 @@ __device__ inline F torsion_term(const Dev& D, const Tables<typename ParamOf<F>:
   F rn[3];
   cross(re, rd, rn);
   const F rnn = q_sqrt<F>(dot3(rn, rn)), rvn = q_sqrt<F>(dot3(rv, rv));
-  F om;
-  if constexpr (!std::is_same<F, float>::value) {
-    F a[3] = {rn[0], rn[1], rn[2]}, b[3] = {rv[0], rv[1], rv[2]};
-    if (fabs(ad::val(rnn)) > 1e-14) {
-      const F o = 1.0 / rnn;
-      a[0] *= o;
-      a[1] *= o;
-      a[2] *= o;
-    }
-    if (fabs(ad::val(rvn)) > 1e-14) {
-      const F o = 1.0 / rvn;
-      b[0] *= o;
-      b[1] *= o;
-      b[2] *= o;
-    }
-    om = q_asin<F>(a[0] * b[0] + a[1] * b[1] + a[2] * b[2]);
-  } else {
-    om = q_asin<F>(fmin(F(1), fmax(F(-1), dot3(rn, rv) / (rnn * rvn))));
-  }
-  const F sinom = q_sin<F>(om), cosom = q_cos<F>(om);
+  const F om = asinf(fmin(F(1), fmax(F(-1), dot3(rn, rv) / (rnn * rvn))));
+  const F sinom = sinf(om), cosom = cosf(om);
   const F rdme[3] = {rd[0] - re[0], rd[1] - re[1], rd[2] - re[2]};
   F rve[3], rne[3], rdv[3], rdn[3], rvdme[3], rndme[3];
   cross(rv, re, rve);
@@ -792,7 +640,7 @@ __device__ inline F torsion_term(const Dev& D, const Tables<typename ParamOf<F>:
     for (int d = 0; d < 3; ++d) dda[d] = ddb[d] = ddc[d] = ddd[d] = F(0);
   }
   const F damp = dampjk * dampij * dampX;
-  if constexpr (std::is_same<F, float>::value) {
+  {
     // FP32: the differences of cosines as products of sines, cos a - cos b
     // = -2 sin((a+b)/2) sin((a-b)/2) and 1 - cos a = 2 sin^2(a/2): near
     // omega = phi0 the reference's forms cancel to a few bits in float,
@@ -807,14 +655,6 @@ __device__ inline F torsion_term(const Dev& D, const Tables<typename ParamOf<F>:
       et = vt[1] * (dd * dd);
       dij = -2.f * vt[1] * sinf(om) * dd * damp;
     }
-  } else if (vt[2] > F(1e-6)) {
-    const F c1 = (om - phi0) + pi;
-    et = (F(1) + q_cos<F>(c1)) * vt[1];
-    dij = -q_sin<F>(c1) * vt[1] * damp;
-  } else {
-    const F dd = q_cos<F>(om) - q_cos<F>(phi0);
-    et = vt[1] * (dd * dd);
-    dij = F(2) * vt[1] * q_sin<F>(om) * (q_cos<F>(phi0) - q_cos<F>(om)) * damp;
   }
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -845,83 +685,14 @@ __device__ inline void load_pair_params(const double* p, double* v) {
     v[2 * k + 1] = t.y;
   }
 }
-__device__ inline void load_pair_params(const double* p, Dual* v) {
-  double t[kVPair];
-  load_pair_params(p, t);
-#pragma unroll
-  for (int k = 0; k < kVPair; ++k) v[k] = Dual(t[k]);
-}
 
-// One NCI pair (src/ff_nonb.f90): BJ-damped C6/C8 dispersion and, for
-// r < 25 bohr, exponential repulsion, both times eps2 (:79-193); Coulomb
-// within coul_cut (:337-416), eps1 q_i q_j / r or the Zahn form.
-template <class F>
-__device__ inline F pair_term(const Dev& D, const Tables<typename ParamOf<F>::type>& T, const BeadPos& x, int kp,
-                              Contrib<F>& c) {
-  const int2 ij = __ldg(reinterpret_cast<const int2*>(D.pair) + kp);
-  const int i1 = ij.x, i2 = ij.y;
-  F v[kVPair];
-  load_pair_params(&T.vpair[kVPair * kp], v);
-  F vab[3];
-  disp<F>(x, i1, i2, vab);
-  const F r2 = dot3(vab, vab);
-  F r, oner, it6, it8;
-  const F R0 = v[0], c6 = v[1], eps2 = v[5];
-  const F r4 = r2 * r2, r6 = r4 * r2;
-  const F R02 = R0 * R0, r06 = R02 * R02 * R02;
-  const F t6 = r6 + r06;
-  const F t8 = r6 * r2 + r06 * R0 * R0;
-  if constexpr (std::is_same<F, float>::value) {
-    // hardware approximations (a few ulp): the pair forces are ~1 % of the
-    // valence forces, far below the form's error budget
-    oner = rsqrtf(r2);
-    r = r2 * oner;
-    it6 = __fdividef(1.0f, t6);
-    it8 = __fdividef(1.0f, t8);
-  } else {
-    r = q_sqrt<F>(r2);
-    oner = F(1) / r;
-    it6 = F(1) / t6;
-    it8 = F(1) / t8;
-  }
-  const F ir2 = oner * oner;
-  const F c6t6 = c6 * it6, c6t8 = c6 * it8;
-  const F t27 = v[2] * c6t8;
-  // periodic: dispersion and repulsion only within vdw_cut (src/ff_nonb.f90:107)
-  const bool vdw = !x.pbc || !(r > (std::is_same<F, float>::value ? F(D.fvdw_cut) : F(D.vdw_cut)));
-  F e = vdw ? -(c6t6 + t27) * eps2 : F(0);
-  F drij = vdw ? eps2 * (c6t6 * F(6) * r4 * it6 + F(8) * t27 * r6 * it8) : F(0);
-  if (vdw && r < F(25)) {
-    const F alpha = v[4];
-    F ex;
-    if constexpr (std::is_same<F, float>::value) ex = __expf(-alpha * r);
-    else ex = q_exp<F>(-alpha * r);
-    const F t = v[3] * ex;
-    e = e + t * oner * eps2;
-    drij = drij - eps2 * t * (alpha * r + F(1)) * oner * ir2;
-  }
-  const F cut = std::is_same<F, float>::value ? F(D.fcoul_cut) : F(D.coul_cut);
-  if (!(r > cut)) {
-    F e0;
-    if (D.zahn) {
-      const F za = std::is_same<F, float>::value ? F(D.fzahn_a) : F(D.zahn_a);
-      const F zp = std::is_same<F, float>::value ? F(D.fzahn_par) : F(D.zahn_par);
-      e0 = v[6] * ((q_erfc<F>(za * r) * oner) - zp * (r - cut));
-    }
-    else e0 = v[6] * oner;
-    e = e + e0;
-    drij = drij - e0 * ir2;
-  }
-  c.na = 2;
-  c.a[0] = i1;
-  c.a[1] = i2;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    c.g[0][d] = vab[d] * drij;
-    c.g[1][d] = -vab[d] * drij;
-  }
-  return e;
-}
+}  // namespace qmdff
+}  // namespace cr
+
+#include "qmdff_plain.cuh"
+
+namespace cr {
+namespace qmdff {
 
 // FP32 hardware approximations (PTX rsqrt / rcp / ex2 .approx.ftz, relative
 // error about 2^-22): inputs here are normal numbers far from the limits.
@@ -941,7 +712,7 @@ __device__ inline float ex2_approx(float x) {
   return y;
 }
 
-// One NCI pair in the mixed form: the formulas of pair_term with the
+// One NCI pair in the mixed form: the formulas of pair_plain with the
 // per-pair constants folded into the table Dev::fpair (R0^6 and R0^8 of the
 // BJ damping, eps2 into the C6 / C8 and repulsion prefactors, alpha log2(e)
 // for a base-2 exponential).  The pair forces are ~1 % of the valence
@@ -980,13 +751,6 @@ __device__ inline float pair_mixed_v(const Dev& D, const BeadPos& x, int i1, int
   }
   if (vir) *vir = r2 * drij;  // vab . g_i1 with g_i1 = vab drij (NpT)
   return e;
-}
-
-__device__ inline float pair_mixed(const Dev& D, const BeadPos& x, int kp, Contrib<float>& c) {
-  const int2 ij = __ldg(reinterpret_cast<const int2*>(D.pair) + kp);
-  float v[kVPair];
-  load_pair_params(&D.fpair[kVPair * kp], v);
-  return pair_mixed_v(D, x, ij.x, ij.y, v, c);
 }
 
 // x^5, x^6, x^12 by products (the reference's real-exponent ** operators)
@@ -1153,27 +917,22 @@ __device__ __noinline__ F hb_term(const Dev& D, const Tables<F>&, const BeadPos&
   return xbond_term<F>(X, t.x, t.y, t.z, D.vhb[2 * k], c);
 }
 
-// Energy of one term of kind `kind` (0 bond, 1 angle, 2 torsion, 3 pair, 4 H/halogen bond).
-template <bool MIXED>
-__device__ inline typename std::conditional<MIXED, float, double>::type term(
-    const Dev& D, int kind, const BeadPos& x, int m, Contrib<typename std::conditional<MIXED, float, double>::type>& c) {
-  if constexpr (MIXED) {
-    switch (kind) {
-      case 0: return bond_mixed(D, x, m, c);
-      case 1: return angle_term<float>(D, D.f, x, m, c);
-      case 2: return torsion_term<float>(D, D.f, x, m, c);
-      case 3: return pair_mixed(D, x, m, c);
-      default: return hb_term<float>(D, D.f, x, m, c);
-    }
-  } else {
-    switch (kind) {
-      case 0: return bond_plain<double>(D, D.d, x, m, c);
-      case 1: return angle_term<double>(D, D.d, x, m, c);
-      case 2: return torsion_term<double>(D, D.d, x, m, c);
-      case 3: return pair_term<double>(D, D.d, x, m, c);
-      default: return hb_term<double>(D, D.d, x, m, c);
-    }
-  }
+// Energy of one term of kind KIND (0 bond, 1 angle, 2 torsion, 3 pair, 4 H/halogen
+// bond); vir: the torsions' virial trace.
+template <int KIND>
+__device__ inline float term(const Dev& D, const BeadPos& x, int m, Contrib<float>& c, float* vir) {
+  if constexpr (KIND == 0) return bond_mixed(D, x, m, c);
+  else if constexpr (KIND == 1) return angle_mixed(D, x, m, c);
+  else if constexpr (KIND == 2) return torsion_mixed(D, x, m, c, vir);
+  else return hb_term<float>(D, D.f, x, m, c);
+}
+template <int KIND>
+__device__ inline double term(const Dev& D, const BeadPos& x, int m, Contrib<double>& c, double* vir) {
+  if constexpr (KIND == 0) return bond_plain<double>(D, D.d, x, m, c);
+  else if constexpr (KIND == 1) return angle_plain<double>(D, D.d, x, m, c);
+  else if constexpr (KIND == 2) return torsion_plain<double>(D, D.d, x, m, c, vir);
+  else if constexpr (KIND == 3) return pair_plain<double>(D, D.d, x, m, c);
+  else return hb_term<double>(D, D.d, x, m, c);
 }
 
 // All batches of one term kind (NA atoms per term): each lane evaluates its
@@ -1234,31 +993,44 @@ __device__ inline F term_virial(const Dev& D, const BeadPos& X, int m, const Con
 // box), kNpt (each trajectory's box from Dev::tbox, and the virial).
 constexpr int kFree = 0, kBox = 1, kNpt = 2;
 
-template <bool MIXED, int KIND, int NA, int MODE>
+// Warps per bead of the FP64 forms.  An FP64 instruction holds its scheduler's
+// pipe 64 cycles and four warps fill an SM's four, so a bead is spread over them:
+// a small batch then takes a quarter of the time, a large one as long as with a
+// warp per bead.  Each warp sums into its own gradient; the four are added in
+// order.  With the terms of qmdff_plain.cuh, whole calls: the adjoint of 16 x 16
+// beads of C20H42 over 20 steps 47.4 -> 12.2 ms, C13H28 100 x 48, four steps 4.82 ->
+// 2.29 ms.
+constexpr int kTeam = 4;
+
+// the first batch of number b0 or more that falls to the warp
+template <int W>
+__device__ __forceinline__ int team_first(int b0, int warp) {
+  return W == 1 ? b0 : b0 + ((warp - b0) & (W - 1));
+}
+
+// W warps share a bead: this one takes the batches whose number is warp modulo W.
+template <bool MIXED, int KIND, int NA, int MODE, int W>
 __device__ inline void kind_batches(const Dev& D, const BeadPos& X,
                                     Grad<typename std::conditional<MIXED, float, double>::type>& G,
                                     typename std::conditional<MIXED, float, double>::type& es,
                                     typename std::conditional<MIXED, float, double>::type& ec,
-                                    typename std::conditional<MIXED, float, double>::type& wv, int lane) {
+                                    typename std::conditional<MIXED, float, double>::type& wv, int warp, int lane) {
   using F = typename std::conditional<MIXED, float, double>::type;
   const Schedule& S = D.sched[MIXED ? 1 : 0];
-  const int b0 = S.boff[KIND], nb = S.nb[KIND];
+  const int b0 = S.boff[KIND], b1 = b0 + S.nb[KIND];
   const bool distinct = D.distinct != 0;
-  for (int b = b0; b < b0 + nb; ++b) {
+  for (int b = team_first<W>(b0, warp); b < b1; b += W) {
     const int m = S.slot[32 * b + lane];
     const int col = S.color[32 * b + lane];
     const int ncol = S.ncol[b];
     Contrib<F> c;
     if (m >= 0) {
-      F v;
-      if constexpr (MODE == kNpt && KIND == 2) {  // the torsion's own vectors give its virial
-        F w;
-        if constexpr (MIXED) v = torsion_term<float>(D, D.f, X, m, c, &w);
-        else v = torsion_term<double>(D, D.d, X, m, c, &w);
+      F v, w = F(0);
+      if constexpr (MODE == kNpt && KIND == 2) v = term<KIND>(D, X, m, c, &w);  // the torsion's own vectors
+      else v = term<KIND>(D, X, m, c, (F*)nullptr);
+      if constexpr (MODE == kNpt) {
+        if constexpr (KIND != 2) w = term_virial<F, KIND>(D, X, m, c);
         wv += w;
-      } else {
-        v = term<MIXED>(D, KIND, X, m, c);
-        if constexpr (MODE == kNpt) wv += term_virial<F, KIND>(D, X, m, c);
       }
       if constexpr (MIXED) {  // compensated FP32 lane sum
         const F t = es + v;
@@ -1319,79 +1091,124 @@ __device__ inline void pair_batches_mixed(const Dev& D, const BeadPos& X, Grad<f
   }
 }
 
-// Shared memory per warp (bytes): coordinates (3n doubles), the FP32 split
-// (hi, lo) (3n float pairs) and the gradient (3n doubles, or (sum,
-// compensation) float pairs and the 3n floats of the pair sum), in whole
-// 16-byte units: the warps' regions follow one another, and 84 n bytes are no
-// multiple of a double for odd n.
+// Shared memory of a mixed-form warp (bytes): coordinates (3n doubles), the FP32
+// split (hi, lo) (3n float pairs) and the gradient ((sum, compensation) float
+// pairs and the 3n floats of the pair sum), in whole 16-byte units: the warps'
+// regions follow one another, and 84 n bytes are no multiple of a double for odd n.
 __host__ __device__ inline size_t warp_smem_bytes(int n) {
   return ((size_t)3 * n * (8 + 4 + 4 + 8 + 4) + 15) / 16 * 16;
 }
+// ... of an FP64 team: coordinates, kTeam gradients, the warps' energies and virials
+__host__ __device__ inline size_t team_smem_bytes(int n) { return ((size_t)3 * n * (1 + kTeam) + 2 * kTeam) * 8; }
 
-// Energy (with E_zero) and gradient (times gscale) of one bead by one warp.
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// The box of a launch's mode as a local copy: taking the address of the kernel
+// parameter D would move all of it from the constant bank to local memory.
+template <int MODE>
+__device__ inline const PBox* launch_box(const Dev& D, size_t bead, PBox& tb) {
+  if constexpr (MODE == kNpt) {  // this trajectory's box
+    tb = make_box(D.tbox + 3 * (size_t)(bead / (size_t)D.tbox_beads));
+    return &tb;
+  } else if constexpr (MODE == kBox) {
+    tb = D.box;
+    return &tb;
+  }
+  return nullptr;
+}
+
+// Energy (with E_zero) and gradient of one bead by one warp, mixed form.
 // ws: the warp's shared memory with the bead's FP64 coordinates in its first
 // 3n doubles; gout, gout2: the gradient destinations (gout2 = gout: one).  Returns the energy on every lane.
-template <bool MIXED, int MODE = kFree>
-__device__ inline double warp_egrad(const Dev& D, double* ws, double* gout, double* gout2, double gscale, int lane, size_t bead = 0,
-                                   size_t twin = 0) {
-  // MODE (kFree, kBox, kNpt): with kNpt the bead's trajectory box from D.tbox
-  // and the virial trace into D.vir (rows bead and twin)
-  using F = typename std::conditional<MIXED, float, double>::type;
+// MODE (kFree, kBox, kNpt): with kNpt the bead's trajectory box from D.tbox
+// and the virial trace into D.vir (rows bead and twin).
+template <int MODE = kFree>
+__device__ inline double warp_egrad(const Dev& D, double* ws, double* gout, double* gout2, int lane, size_t bead,
+                                    size_t twin) {
   const int n3 = 3 * D.n;
   double* xs = ws;
   float2* hl = (float2*)(ws + n3);
-  void* gs = hl + n3;
-  // the box as a local copy: taking the address of the kernel parameter D
-  // would move all of it from the constant bank to local memory
   PBox tb;
-  const PBox* pb = nullptr;
-  if constexpr (MODE == kNpt) {  // this trajectory's box
-    tb = make_box(D.tbox + 3 * (size_t)(bead / (size_t)D.tbox_beads));
-    pb = &tb;
-  } else if constexpr (MODE == kBox) {
-    tb = D.box;
-    pb = &tb;
+  const BeadPos X{xs, hl, nullptr, launch_box<MODE>(D, bead, tb)};
+  Grad<float> G;
+  for (int a = lane; a < n3; a += 32) {
+    const double v = xs[a];
+    const float h = __double2float_rn(v);
+    hl[a] = make_float2(h, __double2float_rn(v - (double)h));
   }
-  BeadPos X{xs, hl, nullptr, pb};
-  Grad<F> G;
-  if constexpr (MIXED) {
-    for (int a = lane; a < n3; a += 32) {
-      const double v = xs[a];
-      const float h = __double2float_rn(v);
-      hl[a] = make_float2(h, __double2float_rn(v - (double)h));
-    }
-    G.sk = (float2*)gs;
-    G.pr = (float*)(G.sk + n3);
-    for (int a = lane; a < n3; a += 32) {
-      G.sk[a] = make_float2(0.f, 0.f);
-      G.pr[a] = 0.f;
-    }
-  } else {
-    G.g = (double*)gs;
-    for (int a = lane; a < n3; a += 32) G.g[a] = 0.0;
+  G.sk = hl + n3;
+  G.pr = (float*)(G.sk + n3);
+  for (int a = lane; a < n3; a += 32) {
+    G.sk[a] = make_float2(0.f, 0.f);
+    G.pr[a] = 0.f;
   }
   __syncwarp();
-  F es = F(0), ec = F(0);  // compensated lane sum of term energies
-  F wv = F(0);             // lane sum of the terms' virial traces (NpT)
-  kind_batches<MIXED, 0, 2, MODE>(D, X, G, es, ec, wv, lane);
-  kind_batches<MIXED, 1, 3, MODE>(D, X, G, es, ec, wv, lane);
-  kind_batches<MIXED, 2, 4, MODE>(D, X, G, es, ec, wv, lane);
-  if constexpr (MIXED) pair_batches_mixed<MODE>(D, X, G, es, ec, wv, lane);
-  else kind_batches<MIXED, 3, 2, MODE>(D, X, G, es, ec, wv, lane);
-  kind_batches<MIXED, 4, 3, MODE>(D, X, G, es, ec, wv, lane);
+  float es = 0.f, ec = 0.f;  // compensated lane sum of term energies
+  float wv = 0.f;            // lane sum of the terms' virial traces (NpT)
+  kind_batches<true, 0, 2, MODE, 1>(D, X, G, es, ec, wv, 0, lane);
+  kind_batches<true, 1, 3, MODE, 1>(D, X, G, es, ec, wv, 0, lane);
+  kind_batches<true, 2, 4, MODE, 1>(D, X, G, es, ec, wv, 0, lane);
+  pair_batches_mixed<MODE>(D, X, G, es, ec, wv, lane);
+  kind_batches<true, 4, 3, MODE, 1>(D, X, G, es, ec, wv, 0, lane);
   for (int a = lane; a < n3; a += 32) {
-    const double v = gscale * G.get(a);
+    const double v = G.get(a);
     gout[a] = v;
     if (gout2 != gout) gout2[a] = v;
   }
-  double e = (double)es + (double)ec;
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+  const double e = warp_sum((double)es + (double)ec);
   if constexpr (MODE == kNpt) {
-    double w = (double)wv;
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    const double w = warp_sum((double)wv);
     if (lane == 0) {
+      D.vir[bead] = w;
+      if (twin != bead) D.vir[twin] = w;
+    }
+  }
+  return e + D.e_zero;
+}
+
+// The same in FP64 by a block of kTeam warps.  ws: the block's shared memory with
+// the coordinates in place (a barrier follows here).  The energy is thread 0's.
+template <int MODE = kFree>
+__device__ inline double team_egrad(const Dev& D, double* ws, double* gout, double* gout2, size_t bead, size_t twin) {
+  const int n3 = 3 * D.n, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  PBox tb;
+  const BeadPos X{ws, nullptr, nullptr, launch_box<MODE>(D, bead, tb)};
+  double* g = ws + n3;
+  double* red = g + kTeam * n3;
+  Grad<double> G{g + warp * n3};
+  for (int a = tid; a < kTeam * n3; a += kTeam * 32) g[a] = 0.0;
+  __syncthreads();
+  double es = 0.0, ec = 0.0, wv = 0.0;
+  kind_batches<false, 0, 2, MODE, kTeam>(D, X, G, es, ec, wv, warp, lane);
+  kind_batches<false, 1, 3, MODE, kTeam>(D, X, G, es, ec, wv, warp, lane);
+  kind_batches<false, 2, 4, MODE, kTeam>(D, X, G, es, ec, wv, warp, lane);
+  kind_batches<false, 3, 2, MODE, kTeam>(D, X, G, es, ec, wv, warp, lane);
+  kind_batches<false, 4, 3, MODE, kTeam>(D, X, G, es, ec, wv, warp, lane);
+  es = warp_sum(es);
+  if constexpr (MODE == kNpt) wv = warp_sum(wv);
+  if (lane == 0) {
+    red[warp] = es;
+    red[kTeam + warp] = wv;
+  }
+  __syncthreads();
+  for (int a = tid; a < n3; a += kTeam * 32) {
+    double v = g[a];
+#pragma unroll
+    for (int w = 1; w < kTeam; ++w) v += g[w * n3 + a];
+    gout[a] = v;
+    if (gout2 != gout) gout2[a] = v;
+  }
+  double e = 0.0, w = 0.0;
+#pragma unroll
+  for (int k = 0; k < kTeam; ++k) e += red[k];
+  if constexpr (MODE == kNpt) {
+#pragma unroll
+    for (int k = 0; k < kTeam; ++k) w += red[kTeam + k];
+    if (tid == 0) {
       D.vir[bead] = w;
       if (twin != bead) D.vir[twin] = w;
     }
@@ -1414,26 +1231,22 @@ struct GradDual {
   }
 };
 
-__device__ inline Dual term_dual(const Dev& D, int kind, const BeadPos& x, int m, Contrib<Dual>& c) {
-  switch (kind) {
-    case 0: return bond_plain<Dual>(D, D.d, x, m, c);
-    case 1: return angle_term<Dual>(D, D.d, x, m, c);
-    case 2: return torsion_term<Dual>(D, D.d, x, m, c);
-    default: return pair_term<Dual>(D, D.d, x, m, c);
-  }
-}
-
-// The plain form's schedule (sched[0]) with dual coordinates.
+// The plain form's schedule (sched[0]) with dual coordinates, by a team of warps.
 template <int KIND, int NA>
-__device__ inline void kind_batches_dual(const Dev& D, const BeadPos& X, GradDual& G, Dual& es, int lane) {
+__device__ inline void kind_batches_dual(const Dev& D, const BeadPos& X, GradDual& G, Dual& es, int warp, int lane) {
   const Schedule& S = D.sched[0];
-  const int b0 = S.boff[KIND], nb = S.nb[KIND];
-  for (int b = b0; b < b0 + nb; ++b) {
+  const int b0 = S.boff[KIND], b1 = b0 + S.nb[KIND];
+  for (int b = team_first<kTeam>(b0, warp); b < b1; b += kTeam) {
     const int m = S.slot[32 * b + lane];
     const int col = S.color[32 * b + lane];
     const int ncol = S.ncol[b];
     Contrib<Dual> c;
-    if (m >= 0) es += term_dual(D, KIND, X, m, c);
+    if (m >= 0) {
+      if constexpr (KIND == 0) es += bond_plain<Dual>(D, D.d, X, m, c);
+      else if constexpr (KIND == 1) es += angle_plain<Dual>(D, D.d, X, m, c);
+      else if constexpr (KIND == 2) es += torsion_plain<Dual>(D, D.d, X, m, c);
+      else es += pair_plain<Dual>(D, D.d, X, m, c);
+    }
     for (int k = 0; k < ncol; ++k) {
       if (m >= 0 && col == k) {
 #pragma unroll
@@ -1446,41 +1259,56 @@ __device__ inline void kind_batches_dual(const Dev& D, const BeadPos& X, GradDua
   }
 }
 
-// Shared memory per warp of warp_hvp: x, w, gradient, H w (3n doubles each).
-__host__ __device__ inline size_t warp_hvp_smem_bytes(int n) { return (size_t)12 * n * sizeof(double); }
+// Shared memory of team_hvp: x, w, kTeam gradients and H w (3n doubles each), the
+// warps' energies and derivatives.
+__host__ __device__ inline size_t team_hvp_smem_bytes(int n) {
+  return ((size_t)3 * n * (2 + 2 * kTeam) + 2 * kTeam) * 8;
+}
 
 // Energy (with E_zero), gradient and Hessian-vector product H w of one bead
-// by one warp.  ws: the warp's shared memory holding x (3n doubles) then w
-// (3n doubles).  dew receives the directional derivative w . grad E.
-__device__ inline double warp_hvp(const Dev& D, double* ws, double* gout, double* hout, double& dew, int lane) {
-  const int n3 = 3 * D.n;
-  double* xs = ws;
+// by a block of kTeam warps.  ws: the block's shared memory holding x (3n
+// doubles) then w (3n doubles; a barrier follows here).  dew receives the
+// directional derivative w . grad E.
+__device__ inline double team_hvp(const Dev& D, double* ws, double* gout, double* hout, double& dew) {
+  const int n3 = 3 * D.n, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   double* w = ws + n3;
-  GradDual G{w + n3, w + 2 * n3};
-  for (int a = lane; a < n3; a += 32) {
-    G.g[a] = 0.0;
-    G.h[a] = 0.0;
-  }
-  __syncwarp();
+  double* g = w + n3;
+  double* h = g + kTeam * n3;
+  double* red = h + kTeam * n3;
+  GradDual G{g + warp * n3, h + warp * n3};
+  for (int a = tid; a < 2 * kTeam * n3; a += kTeam * 32) g[a] = 0.0;
+  __syncthreads();
   PBox tb;
   if (D.periodic) tb = D.box;
-  BeadPos X{xs, nullptr, w, D.periodic ? &tb : nullptr};
+  const BeadPos X{ws, nullptr, w, D.periodic ? &tb : nullptr};
   Dual es(0.0);
-  kind_batches_dual<0, 2>(D, X, G, es, lane);
-  kind_batches_dual<1, 3>(D, X, G, es, lane);
-  kind_batches_dual<2, 4>(D, X, G, es, lane);
-  kind_batches_dual<3, 2>(D, X, G, es, lane);
-  for (int a = lane; a < n3; a += 32) {
-    if (gout) gout[a] = G.g[a];
-    hout[a] = G.h[a];
+  kind_batches_dual<0, 2>(D, X, G, es, warp, lane);
+  kind_batches_dual<1, 3>(D, X, G, es, warp, lane);
+  kind_batches_dual<2, 4>(D, X, G, es, warp, lane);
+  kind_batches_dual<3, 2>(D, X, G, es, warp, lane);
+  const double e1 = warp_sum(es.v), d1 = warp_sum(es.d);
+  if (lane == 0) {
+    red[warp] = e1;
+    red[kTeam + warp] = d1;
   }
-  double e = es.v, de = es.d;
+  __syncthreads();
+  for (int a = tid; a < n3; a += kTeam * 32) {
+    double gv = g[a], hv = h[a];
 #pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
-    e += __shfl_xor_sync(0xffffffffu, e, o);
-    de += __shfl_xor_sync(0xffffffffu, de, o);
+    for (int k = 1; k < kTeam; ++k) {
+      gv += g[k * n3 + a];
+      hv += h[k * n3 + a];
+    }
+    if (gout) gout[a] = gv;
+    hout[a] = hv;
   }
-  dew = de;
+  double e = 0.0;
+  dew = 0.0;
+#pragma unroll
+  for (int k = 0; k < kTeam; ++k) {
+    e += red[k];
+    dew += red[kTeam + k];
+  }
   return e + D.e_zero;
 }
 
@@ -1490,34 +1318,40 @@ __device__ inline double warp_hvp(const Dev& D, double* ws, double* gout, double
 // Coulomb product qq (vpair[6]: eps1 q_i q_j, or q_i q_j in the Zahn form).
 // Every term is linear in its parameter, so d/dtheta_t (v . grad E) is v .
 // grad E_t evaluated with theta_t = 1; the tables U hold the parameters with
-// those entries set to 1 (and, for pairs, eps2 = 0: Coulomb only).
-// Per term, out receives alpha * (v . grad E_t|unit) + beta * E_t|unit.
-__device__ inline void warp_param_vjp(const Dev& D, const Tables<double>& U, const double* xs, const double* vs,
-                                      double alpha, double beta, double* out, int lane) {
+// those entries set to 1 (and, for pairs, the eps2 ones to 0: Coulomb only).
+// Per term, out receives alpha * (v . grad E_t|unit) + beta * E_t|unit; the block's
+// threads take the terms of each kind in turn.
+template <int KIND>
+__device__ inline void team_vjp_kind(const Dev& D, const Tables<double>& U, const BeadPos& X, const double* vs,
+                                     double alpha, double beta, double* out) {
+  constexpr int NA = KIND == 1 ? 3 : KIND == 2 ? 4 : 2;
+  for (int m = threadIdx.x; m < D.nterm[KIND]; m += blockDim.x) {
+    Contrib<double> c;
+    double e;
+    if constexpr (KIND == 0) e = bond_plain<double>(D, U, X, m, c);
+    else if constexpr (KIND == 1) e = angle_plain<double>(D, U, X, m, c);
+    else if constexpr (KIND == 2) e = torsion_plain<double>(D, U, X, m, c);
+    else e = pair_plain<double>(D, U, X, m, c);
+    double s = 0.0;
+#pragma unroll
+    for (int a = 0; a < NA; ++a)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) s = fma(vs[3 * c.a[a] + d], c.g[a][d], s);
+    out[m] = alpha * s + beta * e;
+  }
+}
+__device__ inline void team_param_vjp(const Dev& D, const Tables<double>& U, const double* xs, const double* vs,
+                                      double alpha, double beta, double* out) {
   PBox tb;
   if (D.periodic) tb = D.box;
   const BeadPos X{xs, nullptr, nullptr, D.periodic ? &tb : nullptr};
-  int off = 0;
-#pragma unroll 1
-  for (int kind = 0; kind < 4; ++kind) {
-    const int nt = D.nterm[kind];
-    for (int m = lane; m < nt; m += 32) {
-      Contrib<double> c;
-      double e;
-      switch (kind) {
-        case 0: e = bond_plain<double>(D, U, X, m, c); break;
-        case 1: e = angle_term<double>(D, U, X, m, c); break;
-        case 2: e = torsion_term<double>(D, U, X, m, c); break;
-        default: e = pair_term<double>(D, U, X, m, c); break;
-      }
-      double s = 0.0;
-      for (int a = 0; a < c.na; ++a)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) s += vs[3 * c.a[a] + d] * c.g[a][d];
-      out[off + m] = alpha * s + beta * e;
-    }
-    off += nt;
-  }
+  team_vjp_kind<0>(D, U, X, vs, alpha, beta, out);
+  out += D.nterm[0];
+  team_vjp_kind<1>(D, U, X, vs, alpha, beta, out);
+  out += D.nterm[1];
+  team_vjp_kind<2>(D, U, X, vs, alpha, beta, out);
+  out += D.nterm[2];
+  team_vjp_kind<3>(D, U, X, vs, alpha, beta, out);
 }
 
 }  // namespace qmdff
