@@ -226,7 +226,6 @@ struct cr_engine {
   double *d_umb = nullptr;   // [T] centres, [T] force constants, [T] xsum, [T] xsum2, [T][nbins] histogram
   int* d_umb_flag = nullptr; // [2]: sampling switch, constant 0
   int umb_sampling = 0;      // host copy of the sampling switch
-  double* d_fdrift = nullptr;  // split_drift_fast_kernel table (SplitParams::fdrift)
   int fast_M = 0;              // P / 2 when the drift runs by fast cosine transforms, else 0
   double *d_fsum = nullptr, *d_fmove = nullptr;  // split finish scratch (SplitParams::fsum, fmove)
   int* d_fstat = nullptr;
@@ -326,27 +325,6 @@ void build_split_propagator(int P, double beta, double dt, const cr::PropDims& d
     }
 }
 
-// Table of split_drift_fast_kernel for even P = 2M: per mode k = 0..M the
-// weights w_k / P (w_0 = w_M = 1, else 2) times pc, pd, pq of mode_tables,
-// then the factors 1 / (2 cos(pi (2k+1) / (2N))) of Lee's type-III recursion
-// for N = 2, 4, ..., M/2 at [N/2 - 1 + k].
-void build_fast_drift(int P, double beta, double dt, std::vector<double>& tab) {
-  const int M = P / 2;
-  std::vector<double> C, diag[3];
-  mode_tables(P, beta, dt, C, diag);
-  tab.assign((size_t)cr::fast_drift_doubles(M), 0.0);
-  for (int k = 0; k <= M; ++k) {
-    const double w = (k == 0 || k == M) ? 1.0 / P : 2.0 / P;
-    tab[(size_t)k] = w * diag[0][(size_t)k];
-    tab[(size_t)(M + 1) + k] = w * diag[2][(size_t)k];
-    tab[(size_t)2 * (M + 1) + k] = w * diag[1][(size_t)k];
-  }
-  for (int N = 2; N <= M / 2; N *= 2)
-    for (int k = 0; k < N / 2; ++k)
-      tab[(size_t)3 * (M + 1) + N / 2 - 1 + k] = 1.0 / (2.0 * std::cos(kPi * (2 * k + 1) / (2.0 * N)));
-}
-
-
 // Tables of the fast transforms in fixed point (ring_fast.cuh): (w_k / 2) times
 // pc, pd, pq of mode_tables as Q62 under the exponents 0, eb, ec.
 void build_fast_ring(int P, double beta, double dt, std::vector<int64_t>& tab, int& eb, int& ec) {
@@ -363,6 +341,17 @@ void build_fast_ring(int P, double beta, double dt, std::vector<int64_t>& tab, i
   tab.clear();
   for (int w = 0; w < 3; ++w)
     for (int k = 0; k <= M; ++k) tab.push_back((int64_t)std::llrint(std::ldexp(v[w][k], 62 - e[w])));
+}
+
+// The same on the device, once per engine.
+bool upload_fast_ring(cr_engine* e, double beta, double dt, cr::FastRing& fast) {
+  std::vector<int64_t> tab;
+  build_fast_ring(e->P, beta, dt, tab, fast.eb, fast.ec);
+  if (!e->d_ring && (cudaMalloc(&e->d_ring, tab.size() * 8) != cudaSuccess ||
+                     cudaMemcpy(e->d_ring, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess))
+    return false;
+  fast.tab = e->d_ring;
+  return true;
 }
 
 // PILE-L circulant vectors a (friction) and b (noise) of O^T diag(c) O with O
@@ -586,7 +575,7 @@ cr::SplitParams split_params_range(const cr_engine* e, int t0, int tn) {
   s.epot += t0;
   s.status += t0;
   s.vnh += 4 * (size_t)t0;
-  const int S = cr::finish_slices(e->P * e->N);
+  const int S = cr::finish_slices(s.U * e->N);
   s.fsum += (size_t)t0 * S * cr::kFinishSums;
   s.fstat += (size_t)t0 * S;
   s.fmove += (size_t)t0 * cr::kMoveDoubles;
@@ -669,16 +658,15 @@ int split_group_launches(cr_engine* e, const cr::SplitParams& s, int t0, int tn,
   {
     // NaN check, transrot, epot: moments per slice, a solve per trajectory,
     // the momentum update per item
-    const int S = cr::finish_slices(e->P * e->N);
+    const int S = cr::finish_slices(s.U * e->N);
     cr::split_moments_kernel<<<dim3(S, tn), cr::kMomentThreads, 0, st>>>(s);
     CR_CUDA(cudaGetLastError());
     cr::split_solve_kernel<<<(tn + 127) / 128, 128, 0, st>>>(s, S);
     CR_CUDA(cudaGetLastError());
     n += 2;
     if (s.transrot) {
-      const long long items = (long long)tn * e->P * e->N;
-      const int grid = (int)std::min<long long>((items + cr::kMomentThreads - 1) / cr::kMomentThreads, 152LL * 16);
-      cr::split_apply_kernel<<<grid, cr::kMomentThreads, 0, st>>>(s);
+      const int blocks = (s.U * e->N + cr::kApplyItems - 1) / cr::kApplyItems;
+      cr::split_apply_kernel<<<dim3(tn, blocks), cr::kMomentThreads, 0, st>>>(s);
       CR_CUDA(cudaGetLastError());
       ++n;
     }
@@ -1171,15 +1159,19 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
     s.nv = pd.nv;
     s.su = pd.su;
     s.sv = pd.sv;
-    if (cudaMalloc(&e->d_mass, (size_t)N * 8) != cudaSuccess || cudaMalloc(&e->d_inv_mass, (size_t)N * 8) != cudaSuccess ||
+    std::vector<double> mass2 = e->mass;  // [N] masses, then [N] twice the masses
+    for (int i = 0; i < N; ++i) mass2.push_back(2.0 * e->mass[(size_t)i]);
+    if (cudaMalloc(&e->d_mass, (size_t)2 * N * 8) != cudaSuccess || cudaMalloc(&e->d_inv_mass, (size_t)N * 8) != cudaSuccess ||
         cudaMalloc(&e->d_sigma, (size_t)N * 8) != cudaSuccess || cudaMalloc(&e->d_istep, sizeof(int)) != cudaSuccess)
       return cleanup_fail(fail(CR_ERR_CUDA, "device allocation of the split tables failed"));
-    if (cudaMemcpy(e->d_mass, e->mass.data(), (size_t)N * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
+    if (cudaMemcpy(e->d_mass, mass2.data(), (size_t)2 * N * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(e->d_inv_mass, inv.data(), (size_t)N * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(e->d_sigma, sig.data(), (size_t)N * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(e->d_istep, 0, sizeof(int)) != cudaSuccess)
       return cleanup_fail(fail(CR_ERR_CUDA, "upload of the split tables failed"));
-    const size_t nsl = (size_t)e->T * cr::finish_slices(e->P * N);
+    s.pair = cfg->nm_mode == 0 && e->P > 2 ? 1 : 0;
+    s.U = s.pair ? e->P / 2 + 1 : e->P;
+    const size_t nsl = (size_t)e->T * cr::finish_slices(s.U * N);
     if (cudaMalloc(&e->d_fsum, nsl * cr::kFinishSums * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&e->d_fstat, nsl * sizeof(int)) != cudaSuccess ||
         cudaMalloc(&e->d_fmove, (size_t)e->T * cr::kMoveDoubles * sizeof(double)) != cudaSuccess)
@@ -1189,10 +1181,7 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
     const int P = e->P;
     if (pd.split && P >= 8 && P <= 64 && (P & (P - 1)) == 0 && cfg->thermostat != CR_THERMO_PILE &&
         cfg->nm_mode == 0) {
-      std::vector<double> tab;
-      build_fast_drift(P, cfg->beta, cfg->dt, tab);
-      if (cudaMalloc(&e->d_fdrift, tab.size() * 8) != cudaSuccess ||
-          cudaMemcpy(e->d_fdrift, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess)
+      if (!upload_fast_ring(e, cfg->beta, cfg->dt, s.fast))
         return cleanup_fail(fail(CR_ERR_CUDA, "upload of the fast drift table failed"));
       e->fast_M = P / 2;
     }
@@ -1211,6 +1200,7 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
     s.totmass = totmass;
     s.wsum = tm;
     s.mass = e->d_mass;
+    s.mass2 = e->d_mass + N;
     s.inv_mass = e->d_inv_mass;
     s.sigma = e->d_sigma;
     s.ke = e->d_ke;
@@ -1226,7 +1216,6 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
     s.nhc = nhc;
     s.vnh = e->d_vnh;
     s.fsum = e->d_fsum;
-    s.fdrift = e->d_fdrift;
     s.fstat = e->d_fstat;
     s.fmove = e->d_fmove;
     const bool pl = cfg->thermostat == CR_THERMO_PILE;
@@ -1292,12 +1281,8 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
   // mixed 36 us per step against 32 with the matrix products on all lanes; CH4 + H
   // 4096 x 32 mixed 102 against 122, CH4 + OH 512 x 64 mixed 80 against 118)
   if (s.pair && (e->P == 32 || e->P == 64)) {
-    std::vector<int64_t> tab;
-    build_fast_ring(e->P, cfg->beta, cfg->dt, tab, s.fast.eb, s.fast.ec);
-    if (cudaMalloc(&e->d_ring, tab.size() * 8) != cudaSuccess ||
-        cudaMemcpy(e->d_ring, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess)
+    if (!upload_fast_ring(e, cfg->beta, cfg->dt, s.fast))
       return cleanup_fail(fail(CR_ERR_CUDA, "upload of the ring tables failed"));
-    s.fast.tab = e->d_ring;
     s.fast_M = e->P / 2;
   }
   choose_launch(e);
@@ -1362,7 +1347,6 @@ int cr_engine_destroy(cr_engine* e) {
   cudaFree(e->d_umb);
   cudaFree(e->d_umb_flag);
   cudaFree(e->d_fsum);
-  cudaFree(e->d_fdrift);
   cudaFree(e->d_fstat);
   cudaFree(e->d_fmove);
   if (e->graph_exec) cudaGraphExecDestroy(e->graph_exec);

@@ -1,4 +1,4 @@
-// Free ring polymer of P = 2 M beads (M = 16, 32) by fast cosine
+// Free ring polymer of P = 2 M beads (M = 4, 8, 16, 32) by fast cosine
 // transforms in fixed point, on the integer pipe.
 //
 // Caracal's map on the distinct beads x_0 .. x_M is y = T_M(z) 2/P with
@@ -128,11 +128,11 @@ struct Dct1<2> {
 __device__ constexpr int log2i(int x) { return x <= 1 ? 0 : 1 + log2i(x / 2); }
 __device__ __forceinline__ int64_t shr(int64_t x, int n) { return x >> (n < 63 ? n : 63); }
 
-// One coordinate row x[0 .. M * stride] of q (isp 0) or p (isp 1), in place; msc
-// is 1/m for q, m for p.  Every lane of the warp takes part (active: its row is
-// real).  Returns whether the new row is finite.
-template <int M>
-__device__ __forceinline__ bool row(double* r, int stride, bool isp, bool active, double msc, const FastRing& T) {
+// One coordinate row, filled in by get, of q (isp 0) or p (isp 1) to put(0, .) ..
+// put(M, .); msc is 1/m for q, m for p.  Every lane of the warp takes part (active:
+// its row is real).  Returns whether the new row is finite.
+template <int M, class Get, class Put>
+__device__ __forceinline__ bool row(Get get, Put put, bool isp, bool active, double msc, const FastRing& T) {
   constexpr int kGuard = log2i(M) - 2, kBits = 56 - kGuard, kNone = -100000;
   int64_t x[M + 1], X[M + 1];
   double first = 0.0;
@@ -140,10 +140,10 @@ __device__ __forceinline__ bool row(double* r, int stride, bool isp, bool active
   {
     double v[M + 1];
 #pragma unroll
-    for (int l = 0; l <= M; ++l) {
-      v[l] = active ? r[l * stride] : 0.0;
-      e = max(e, exponent_field(v[l]));
-    }
+    for (int l = 0; l <= M; ++l) v[l] = 0.0;
+    if (active) get(v);
+#pragma unroll
+    for (int l = 0; l <= M; ++l) e = max(e, exponent_field(v[l]));
 #pragma unroll
     for (int l = 0; l <= M; ++l) x[l] = to_fixed(v[l], e, kGuard);
     if (!isp) first = v[0];
@@ -188,7 +188,7 @@ __device__ __forceinline__ bool row(double* r, int stride, bool isp, bool active
     double y = from_fixed(X[l], E - log2i(M)) + first;
     if (bad || obad) y = __longlong_as_double(0x7ff8000000000000ll);
     fine = fine && exponent_field(y) != 0x7ff;
-    r[l * stride] = y;
+    put(l, y);
   }
   return fine;
 }

@@ -28,7 +28,6 @@
 #include <cuda_runtime.h>
 
 #include "cr_common.cuh"
-#include "dual.cuh"
 #include "rpmd_kernel.cuh"
 
 namespace cr {
@@ -44,12 +43,14 @@ struct SplitParams {
   double half_dt, totmass;
   double wsum;             // sum of the masses over beads and atoms (P sum m)
   const double* mass;      // [N]
+  const double* mass2;     // [N] twice the masses
   const double* inv_mass;  // [N]
   const double* sigma;     // [N] sqrt(m P / beta)
   const double* ke;        // [3][nr][nu]: K1, K2, K3 (unit mass), even-mode part (or full rows)
   const double* ko;        // [3][nr][nv]: odd-mode part
   const double* pile;      // [2][P] circulant a, b
-  const double* fdrift;    // split_drift_fast_kernel: [3][M+1] mode coefficients, then M Lee factors
+  FastRing fast;           // split_drift_fast_kernel's mode tables
+  int pair, U;             // 1: after a drift rows l and P - l of q are equal (nm_mode 0, P > 2); U rows to visit
   double* q;
   double* p;
   double* f;               // dV/dq
@@ -312,139 +313,63 @@ __global__ void __launch_bounds__(kSplitBlock) split_drift_kernel(SplitParams s)
   }
 }
 
-// ---- free ring polymer by fast cosine transforms (even P = 2M, M = 4..32) ----
-// Caracal's map y = C D C x (C = sqrt(1/P) cos(2 pi j k / P)) depends on x
-// only through the fold s_0 = x_0, s_M = x_M, s_l = x_l + x_{P-l}, and
-// C x = T_M(s) / sqrt(P) with the type-I cosine transform
-//   T_M(s)_k = s_0 + (-1)^k s_M + sum_{l=1}^{M-1} s_l cos(pi k l / M),  k = 0..M.
-// The output is y_j = y_{P-j} = T_M(z)_j / sqrt(P), z_k = w_k D_k (C x)_k with
-// w_0 = w_M = 1, w_k = 2 otherwise.  T_M splits by the parity of k into
-// T_{M/2} of u_l = s_l + s_{M-l} (even k) and the type-III transform of size
-// M/2 of v_l = s_l - s_{M-l} (odd k); the type-III transform
-//   X_k = sum_{n<N} x_n cos(pi (2k+1) n / (2N))
-// follows Lee's recursion (B. G. Lee, IEEE Trans. ASSP 32 (1984) 1243):
-// G = (size N/2 of x_{2m}), H' = (size N/2 of x_{2m+1} + x_{2m-1}),
-// X_k = G_k + H'_k / (2 cos(pi (2k+1) / (2N))), X_{N-1-k} = G_k - (same).
-// For M = 32 that is ~210 FP64 operations per transform against 33^2 for the
-// matrix; the rounding error measured against extended precision is below
-// the matrix form's.
-template <int N>
-struct Dct3 {
-  __device__ static inline void run(const double (&x)[N], double (&X)[N], const double* lee) {
-    constexpr int H = N / 2;
-    double xe[H], z[H], G[H], Hh[H];
-#pragma unroll
-    for (int m = 0; m < H; ++m) {
-      xe[m] = x[2 * m];
-      z[m] = m > 0 ? x[2 * m + 1] + x[2 * m - 1] : x[1];
-    }
-    Dct3<H>::run(xe, G, lee);
-    Dct3<H>::run(z, Hh, lee);
-#pragma unroll
-    for (int k = 0; k < H; ++k) {
-      const double h = Hh[k] * lee[H - 1 + k];  // 1 / (2 cos(pi (2k+1) / (2N)))
-      X[k] = G[k] + h;
-      X[N - 1 - k] = G[k] - h;
-    }
-  }
-};
-template <>
-struct Dct3<1> {
-  __device__ static inline void run(const double (&x)[1], double (&X)[1], const double*) { X[0] = x[0]; }
-};
+// Row that equals row l after a drift (l itself: none).
+__device__ __forceinline__ int twin_row(const SplitParams& s, int l) {
+  return s.pair && l > 0 && 2 * l != s.P ? s.P - l : l;
+}
+__device__ __forceinline__ bool same_bits(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
 
+// Free ring-polymer step of P = 2 M = 8, 16, 32, 64 beads with the 1/2 kick before
+// it (no PILE) by fast transforms in fixed point (ring_fast.cuh): lanes 2 y and
+// 2 y + 1 of a warp take coordinate y of q and of p - dt/2 dV/dq, on the mean of
+// rows l and P - l (which mostly are equal: then nothing is added).  Block: 4 warps =
+// 64 coordinates; grid (ceil(NC / 64), T).  In FP64 the transforms were bound by
+// the FP64 pipe, some 900 instructions of 64 cycles per coordinate: 1024 x 64
+// C20H42 526 -> 281 us, where reading q, p, f and writing q, p takes 70.
 template <int M>
-struct Dct1 {
-  __device__ static inline void run(const double (&s)[M + 1], double (&y)[M + 1], const double* lee) {
-    constexpr int N = M / 2;
-    double u[N + 1], v[N], ye[N + 1], yo[N];
-    u[0] = s[0] + s[M];
-    v[0] = s[0] - s[M];
-#pragma unroll
-    for (int l = 1; l < N; ++l) {
-      u[l] = s[l] + s[M - l];
-      v[l] = s[l] - s[M - l];
-    }
-    u[N] = s[N];
-    Dct1<N>::run(u, ye, lee);
-    Dct3<N>::run(v, yo, lee);
-#pragma unroll
-    for (int k = 0; k <= N; ++k) y[2 * k] = ye[k];
-#pragma unroll
-    for (int k = 0; k < N; ++k) y[2 * k + 1] = yo[k];
-  }
-};
-template <>
-struct Dct1<2> {
-  __device__ static inline void run(const double (&s)[3], double (&y)[3], const double*) {
-    const double a = s[0] + s[2];
-    y[0] = a + s[1];
-    y[1] = s[0] - s[2];
-    y[2] = a - s[1];
-  }
-};
-
-// Entries of the fast-drift table for even P = 2M: A_k = w_k cos(w_k dt) / P,
-// B_k = w_k sin(w_k dt) / (w_k P) and C_k = -w_k w_k sin(w_k dt) / P per mode
-// k = 0..M (w the mode weight above), then the Lee factors of every size N
-// <= M/2 at [N/2 - 1 + k].
-__host__ __device__ inline int fast_drift_doubles(int M) { return 3 * (M + 1) + M; }
-
-// Free ring-polymer step of even P = 2M beads with the 1/2 kick before it
-// (no PILE): each warp takes 16 coordinates of one trajectory, lanes 0-15
-// transforming q and lanes 16-31 transforming p - dt/2 dV/dq of the same
-// coordinates; the 2x2 mode update exchanges the partner's coefficient by a
-// shuffle.  Block: 4 warps = 64 coordinates; grid (ceil(NC / 64), T).
-template <int M>
-__global__ void __launch_bounds__(128) split_drift_fast_kernel(SplitParams s) {
+__global__ void __launch_bounds__(128) split_drift_fast_kernel(const __grid_constant__ SplitParams s) {
   constexpr int P = 2 * M;
-  constexpr int kTab = 3 * (M + 1) + M;
-  __shared__ double tab[kTab];
-  for (int i = threadIdx.x; i < kTab; i += blockDim.x) tab[i] = s.fdrift[i];
-  __syncthreads();
-  const double* lee = tab + 3 * (M + 1);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int NC = s.NC, t = blockIdx.y;
-  const int c = (blockIdx.x * 4 + warp) * 16 + (lane & 15);
-  const bool isp = lane >= 16, active = c < NC;
-  const int atom = active ? c / 3 : 0;
-  const size_t tb = (size_t)t * P * NC + c;
-  // q enters relative to its bead-0 value: the constant vector is mode 0
-  // (K1 keeps it, K2 drops it), and the transforms then round on bead
-  // spreads instead of absolute positions
-  double x[M + 1], shift = 0.0;
+  const int c = (blockIdx.x * 4 + warp) * 16 + (lane >> 1);
+  const bool isp = lane & 1, active = c < NC;
+  const size_t tb = (size_t)t * P * NC + (active ? c : 0);
+  double* x = (isp ? s.p : s.q) + tb;
+  const double* f = s.f + tb;
+  const double hdt = isp ? s.half_dt : 0.0;
+  // kLoad rows at a time, so that their loads are in flight together
+  constexpr int kLoad = 11;
+  auto get = [&](double (&v)[M + 1]) {
 #pragma unroll
-  for (int l = 0; l <= M; ++l) x[l] = 0.0;
-  if (active) {
-    const double* src = isp ? s.p : s.q;
-    const double hdt = isp ? s.half_dt : 0.0;
-    if (!isp) shift = src[tb];
+    for (int l0 = 0; l0 <= M; l0 += kLoad) {
+      double xa[kLoad], xb[kLoad], fa[kLoad], fb[kLoad];
 #pragma unroll
-    for (int j = 0; j < P; ++j) {
-      const size_t g = tb + (size_t)j * NC;
-      const double v = fma(-hdt, s.f[g], src[g]) - shift;
-      x[j <= M ? j : P - j] += v;
+      for (int k = 0; k < kLoad; ++k) {
+        const int l = l0 + k;
+        if (l > M) continue;
+        const size_t a = (size_t)l * NC, b = (size_t)(l == 0 || l == M ? l : P - l) * NC;
+        xa[k] = x[a];
+        xb[k] = x[b];
+        fa[k] = isp ? f[a] : 0.0;
+        fb[k] = isp ? f[b] : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < kLoad; ++k) {
+        const int l = l0 + k;
+        if (l > M) continue;
+        v[l] = fma(-hdt, fa[k], xa[k]);
+        if (!(same_bits(xa[k], xb[k]) && same_bits(fa[k], fb[k]))) v[l] = 0.5 * (v[l] + fma(-hdt, fb[k], xb[k]));
+      }
     }
-  }
-  double X[M + 1];
-  Dct1<M>::run(x, X, lee);
-  // q' = A q + B p / m (lanes 0-15), p' = A p + C m q (lanes 16-31)
-  const double msc = isp ? s.mass[atom] : s.inv_mass[atom];
-  const double* coef = tab + (isp ? 2 : 1) * (M + 1);
-#pragma unroll
-  for (int k = 0; k <= M; ++k) {
-    const double other = __shfl_xor_sync(0xffffffffu, X[k], 16);
-    X[k] = fma(coef[k] * msc, other, tab[k] * X[k]);
-  }
-  Dct1<M>::run(X, x, lee);
-  if (!active) return;
-  double* dst = isp ? s.p : s.q;
-#pragma unroll
-  for (int j = 0; j <= M; ++j) {
-    const double y = x[j] + shift;
-    dst[tb + (size_t)j * NC] = y;
-    if (j > 0 && j < M) dst[tb + (size_t)(P - j) * NC] = y;
-  }
+  };
+  auto put = [&](int l, double y) {
+    x[(size_t)l * NC] = y;
+    if (l > 0 && l < M) x[(size_t)(P - l) * NC] = y;
+  };
+  const int atom = active ? c / 3 : 0;
+  ring::row<M>(get, put, isp, active, isp ? s.mass[atom] : s.inv_mass[atom], s.fast);
 }
 
 // mode 0: 1/2 kick and thermostat; 1: 1/2 kick only; 2: thermostat only (the
@@ -458,12 +383,21 @@ __global__ void __launch_bounds__(kSplitBlock) split_kick_kernel(SplitParams s, 
   const size_t tb = (size_t)t * P * NC + c0;
   const uint32_t traj = s.traj0 + (uint32_t)t;
   const double hdt = mode == 2 ? 0.0 : s.half_dt;
-  if (mode == 1) {
-    for (int idx = threadIdx.x; idx < P * cw; idx += blockDim.x) {
-      const int c = idx % cw, j = idx / cw;
-      const size_t g = tb + (size_t)j * NC + c;
-      s.p[g] = s.p[g] - s.half_dt * s.f[g];
+  // the kick alone: after the drift and the forces, rows l and P - l of p and f
+  // are equal (1024 x 64 C20H42 32 us)
+  auto kick = [&]() {
+    const int c = threadIdx.x % cw_max;
+    if (c >= cw) return;
+    for (int l = threadIdx.x / cw_max; l < s.U; l += kSplitBlock / cw_max) {
+      const size_t g = tb + (size_t)l * NC + c;
+      const double p = fma(-s.half_dt, s.f[g], s.p[g]);
+      s.p[g] = p;
+      const int k = twin_row(s, l);
+      if (k != l) s.p[tb + (size_t)k * NC + c] = p;
     }
+  };
+  if (mode == 1) {
+    kick();
     return;
   }
   if (s.thermostat == CR_THERMO_PILE) {
@@ -499,12 +433,7 @@ __global__ void __launch_bounds__(kSplitBlock) split_kick_kernel(SplitParams s, 
     }
     return;
   }
-  if (mode == 2) return;
-  for (int idx = threadIdx.x; idx < P * cw; idx += blockDim.x) {
-    const int c = idx % cw, j = idx / cw;
-    const size_t g = tb + (size_t)j * NC + c;
-    s.p[g] = s.p[g] - s.half_dt * s.f[g];
-  }
+  if (mode != 2) kick();
 }
 
 // ---- constrained parent (src/constrain_q.f90, src/constrain_p.f90) ----------
@@ -613,7 +542,9 @@ __global__ void split_parent_init_kernel(SplitParams s) {
 //   split_moments_kernel  grid (S, T): slice g of trajectory t's (bead, atom)
 //                         items -> 15 moment sums (sum w v, sum w x,
 //                         sum w x cross v, sum w x x^T), the bead energies
-//                         (slice 0), the NaN bits; fixed-order block sums
+//                         (slice 0), the NaN bits; fixed-order block sums.  Rows l
+//                         and P - l of q are equal after the drift, so an item
+//                         covers both with the sum of their momenta
 //   split_solve_kernel    one thread per trajectory: the S partials summed in
 //                         order, epot, status, and the 3x3 system for the
 //                         angular velocity (Gauss-Jordan, full pivoting)
@@ -621,8 +552,10 @@ __global__ void split_parent_init_kernel(SplitParams s) {
 //                         evaluated as p - m (b + va x x), b = vt - va x xt
 // The second moments about Caracal's rotation centre xt come from the raw
 // ones by the parallel-axis identity C = S - xt Sx^T - Sx xt^T + W xt xt^T,
-// W = sum w.  Traffic: q and p read twice, p written once.
+// W = sum w.  Traffic: half of q and p read twice, p written once; 1024 x 64 C20H42
+// 115, 12 and 71 us.
 constexpr int kMomentThreads = 256;
+constexpr int kApplyItems = 4 * kMomentThreads;  // items of one block of split_apply_kernel
 constexpr int kFinishSums = 16;   // 15 moments + sum of bead energies
 constexpr int kMoveDoubles = 10;  // b = vt - va x xt, va, (unused), skip flag per trajectory
 
@@ -635,12 +568,11 @@ __host__ __device__ inline int finish_slices(int items) {
 // Not NaN or infinite: exponent bits below all-ones (integer pipe only).
 __device__ inline bool finite_bits(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
 
-// Moment sums of one (bead, atom) item.  On this GPU the FP64 pipe bounds the
-// finish, so the sums use w v = p (momentum) and w x once: 21 FP64
-// operations per item.
-__device__ inline void finish_accumulate(const SplitParams& s, int a, const double (&q)[3], const double (&p)[3],
+// Moment sums of one (bead, atom) item of mass w and momentum p.  On this GPU the
+// FP64 pipe bounds the finish, so the sums use w v = p (momentum) and w x once: 21
+// FP64 operations per item.
+__device__ inline void finish_accumulate(double w, const double (&q)[3], const double (&p)[3],
                                          double (&acc)[kFinishSums], int& status) {
-  const double w = s.mass[a];
   const double wq[3] = {w * q[0], w * q[1], w * q[2]};
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -686,20 +618,22 @@ __global__ void __launch_bounds__(kMomentThreads) split_moments_kernel(SplitPara
   const int S = gridDim.x, g = blockIdx.x, t = blockIdx.y, P = s.P, N = s.N;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const size_t tb = (size_t)t * P * s.NC;
-  const int items = P * N;
+  const int items = s.U * N;
   const int lo = (int)((long long)items * g / S), hi = (int)((long long)items * (g + 1) / S);
   double acc[kFinishSums];
 #pragma unroll
   for (int j = 0; j < kFinishSums; ++j) acc[j] = 0.0;
   int status = 0;
   for (int i = lo + threadIdx.x; i < hi; i += kMomentThreads) {
+    const int l = i / N, a = i - l * N, k = twin_row(s, l);
     double q[3], p[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       q[d] = s.q[tb + 3 * (size_t)i + d];
       p[d] = s.p[tb + 3 * (size_t)i + d];
+      if (k != l) p[d] += s.p[tb + 3 * (size_t)(k * N + a) + d];
     }
-    finish_accumulate(s, i % N, q, p, acc, status);
+    finish_accumulate(k != l ? s.mass2[a] : s.mass[a], q, p, acc, status);
   }
   if (g == 0)
     for (int j = threadIdx.x; j < P; j += kMomentThreads) acc[15] += s.V[(size_t)t * P + j];
@@ -748,22 +682,26 @@ __global__ void split_solve_kernel(SplitParams s, int S) {
 }
 
 __global__ void __launch_bounds__(kMomentThreads) split_apply_kernel(SplitParams s) {
-  const int N = s.N, items = s.P * N;
-  const size_t total = (size_t)s.T * items;
-  for (size_t idx = (size_t)blockIdx.x * kMomentThreads + threadIdx.x; idx < total;
-       idx += (size_t)gridDim.x * kMomentThreads) {
-    const int t = (int)(idx / items), a = (int)(idx % items) % N;
-    const double* mv = s.fmove + (size_t)t * kMoveDoubles;
-    if (mv[9] != 0.0) continue;
-    const double* qq = s.q + 3 * idx;
-    double* pp = s.p + 3 * idx;
+  const int N = s.N, items = s.U * N, t = blockIdx.x;
+  const double* mv = s.fmove + (size_t)t * kMoveDoubles;
+  if (mv[9] != 0.0) return;
+  const double* q = s.q + (size_t)t * s.P * s.NC;
+  double* p = s.p + (size_t)t * s.P * s.NC;
+  const int lo = blockIdx.y * kApplyItems, hi = min(lo + kApplyItems, items);
+  for (int i = lo + threadIdx.x; i < hi; i += kMomentThreads) {
+    const int l = i / N, a = i - l * N, k = twin_row(s, l);
+    const double* qq = q + 3 * (size_t)i;
     const double w = s.mass[a];
-    const double u0 = mv[0] + fma(mv[4], qq[2], -mv[5] * qq[1]);
-    const double u1 = mv[1] + fma(mv[5], qq[0], -mv[3] * qq[2]);
-    const double u2 = mv[2] + fma(mv[3], qq[1], -mv[4] * qq[0]);
-    pp[0] = fma(-w, u0, pp[0]);
-    pp[1] = fma(-w, u1, pp[1]);
-    pp[2] = fma(-w, u2, pp[2]);
+    const double u[3] = {mv[0] + fma(mv[4], qq[2], -mv[5] * qq[1]), mv[1] + fma(mv[5], qq[0], -mv[3] * qq[2]),
+                         mv[2] + fma(mv[3], qq[1], -mv[4] * qq[0])};
+    double* pa = p + 3 * (size_t)i;
+    double* pb = p + 3 * (size_t)(k * N + a);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double x = pa[d], y = pb[d], r = fma(-w, u[d], x);
+      pa[d] = r;
+      if (k != l) pb[d] = same_bits(x, y) ? r : fma(-w, u[d], y);
+    }
   }
 }
 
@@ -777,9 +715,9 @@ __global__ void __launch_bounds__(kFinishBlock) split_nhc_kernel(SplitParams s) 
   double ek[1] = {0.0};
   for (int idx = threadIdx.x; idx < P * N; idx += blockDim.x) {
     const double* pp = s.p + tb + 3 * (size_t)idx;
-    const double w = s.mass[idx % N];
-    ek[0] = ek[0] + (pp[0] * pp[0] + pp[1] * pp[1] + pp[2] * pp[2]) / (2.0 * w) / P / P;
+    ek[0] = fma(pp[0] * pp[0] + pp[1] * pp[1] + pp[2] * pp[2], s.inv_mass[idx % N], ek[0]);
   }
+  ek[0] *= 0.5 / ((double)P * P);
   block_sum<1>(ek, red);
   if (threadIdx.x == 0) {
     double v[4];
