@@ -114,49 +114,72 @@ __global__ void init_children_kernel(int T, int P, uint32_t seed, uint32_t traj0
 }
 
 // Flux weight of each child (src/recross.f90:562-590): vs = dxi . sum_k p_k / m / P,
-// fs = sqrt(sum dxi^2 / m / (2 pi beta)), w = vs / fs, wpos = vs > 0.
+// fs = sqrt(sum dxi^2 / m / (2 pi beta)), w = vs / fs, wpos = vs > 0.  A block takes
+// kFluxChildren children: its warps sum over the beads, a lane per coordinate, then
+// a thread per child takes xi.  With a thread per child throughout, the chain of
+// uncoalesced loads and FP64 sums took 542 us for 4096 children of 32 beads.
+constexpr int kFluxChildren = 32, kFluxThreads = 256;
 template <int N>
-__global__ void child_flux_kernel(int T, int P, StepParams prm, const double* q, const double* p,
-                                  double* w, int* wpos) {
+__global__ void __launch_bounds__(kFluxThreads) child_flux_kernel(int T, int P, StepParams prm, const double* q,
+                                                                  const double* p, double* w, int* wpos) {
   constexpr int NC = 3 * N;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T) return;
-  double c[NC], dxi[NC];
-  for (int x = 0; x < NC; ++x) {
-    double acc = 0.0;
-    for (int k = 0; k < P; ++k) acc += q[((size_t)t * P + k) * NC + x];
-    c[x] = acc / P;
+  __shared__ double sq[kFluxChildren][NC], sp[kFluxChildren][NC];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t0 = blockIdx.x * kFluxChildren;
+  for (int g = warp; g < kFluxChildren && t0 + g < T; g += kFluxThreads / 32) {
+    if (lane >= NC) continue;
+    const size_t tb = (size_t)(t0 + g) * P * NC + lane;
+    double a = 0.0, b = 0.0;
+#pragma unroll 4
+    for (int k = 0; k < P; ++k) {
+      a += q[tb + (size_t)k * NC];
+      b += p[tb + (size_t)k * NC];
+    }
+    sq[g][lane] = a / P;
+    sp[g][lane] = b;
   }
+  __syncthreads();
+  const int g = threadIdx.x, t = t0 + g;
+  if (g >= kFluxChildren || t >= T) return;
+  double c[NC], dxi[NC];
+  for (int x = 0; x < NC; ++x) c[x] = sq[g][x];
   xi_bimolec<N>(prm.xi, c, prm.mass, dxi);
-  double vs = 0.0;
+  double vs = 0.0, fs = 0.0;
   for (int l = 0; l < 3; ++l)
-    for (int m = 0; m < N; ++m)
-      for (int o = 0; o < P; ++o) vs += dxi[3 * m + l] * p[((size_t)t * P + o) * NC + 3 * m + l] / prm.mass[m];
+    for (int m = 0; m < N; ++m) {
+      vs += dxi[3 * m + l] * sp[g][3 * m + l] / prm.mass[m];
+      fs += dxi[3 * m + l] * dxi[3 * m + l] / prm.mass[m];
+    }
   vs = vs / P;
-  double fs = 0.0;
-  for (int l = 0; l < 3; ++l)
-    for (int m = 0; m < N; ++m) fs += dxi[3 * m + l] * dxi[3 * m + l] / prm.mass[m];
   fs = sqrt(fs / (2.0 * 3.1415926535897932384 * prm.beta));
   w[t] = vs / fs;
   wpos[t] = vs > 0.0 ? 1 : 0;
 }
 
-// kappa(t) numerator and denominator, summed over trajectories in index order
-// (deterministic): num[s] = sum_t w[t] [xi_t > 0 after step s+1].
-__global__ void kappa_kernel(int T, int nsteps, int stride, const unsigned char* side, const double* w,
-                             const int* wpos, double* num, double* denom) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < nsteps) {
-    double acc = 0.0;
-    for (int t = 0; t < T; ++t)
-      if (side[(size_t)t * stride + s]) acc += w[t];
-    num[s] = acc;
-  } else if (s == nsteps) {
-    double acc = 0.0;
-    for (int t = 0; t < T; ++t)
-      if (wpos[t]) acc += w[t];
-    *denom = acc;
+// kappa(t) numerator and denominator: num[s] = sum_t w[t] [xi_t > 0 after step s+1],
+// and *denom = sum_t w[t] [wpos].  32 steps per block (a row of side is read
+// together), kKappaRows partial sums over the trajectories added in order
+// (deterministic).  One thread per step took 693 us for 4096 x 40 (the kernels alone).
+constexpr int kKappaRows = 32;
+__global__ void __launch_bounds__(32 * kKappaRows) kappa_kernel(int T, int nsteps, int stride, const unsigned char* side,
+                                                                const double* w, const int* wpos, double* num,
+                                                                double* denom) {
+  __shared__ double part[kKappaRows][32];
+  const int x = threadIdx.x, y = threadIdx.y, s = blockIdx.x * 32 + x;
+  double acc = 0.0;
+  if (s <= nsteps) {
+#pragma unroll 4
+    for (int t = y; t < T; t += kKappaRows) {
+      const bool on = s < nsteps ? side[(size_t)t * stride + s] != 0 : wpos[t] != 0;
+      acc += on ? w[t] : 0.0;
+    }
   }
+  part[y][x] = acc;
+  __syncthreads();
+  if (y != 0 || s > nsteps) return;
+  acc = 0.0;
+  for (int k = 0; k < kKappaRows; ++k) acc += part[k][x];
+  if (s < nsteps) num[s] = acc;
+  else *denom = acc;
 }
 
 // epot[t] = sum over beads of V[t][k]
@@ -2188,7 +2211,7 @@ int cr_engine_init_children(cr_engine* e, const double* q_parent) {
   CR_CUDA(cudaGetLastError());
   int rc = dispatch_forces(e);
   if (rc) return rc;
-  const int tb = 128, gb = (e->T + tb - 1) / tb;
+  const int tb = cr::kFluxThreads, gb = (e->T + cr::kFluxChildren - 1) / cr::kFluxChildren;
   switch (e->cfg.pes) {
     case CR_PES_H3:
     case CR_PES_BRH2:
@@ -2224,7 +2247,7 @@ int cr_engine_kappa(cr_engine* e, double* num, double* denom, double* weights, i
     *denom = 0.0;
     return CR_OK;
   }
-  cr::kappa_kernel<<<(ns + 1 + 127) / 128, 128, 0, e->stream>>>(e->T, ns, e->side_cap, e->d_side, e->d_w,
+  cr::kappa_kernel<<<ns / 32 + 1, dim3(32, cr::kKappaRows), 0, e->stream>>>(e->T, ns, e->side_cap, e->d_side, e->d_w,
                                                                   e->d_wpos, e->d_kappa, e->d_kappa + ns);
   CR_CUDA(cudaGetLastError());
   CR_CUDA(cudaMemcpyAsync(num, e->d_kappa, (size_t)ns * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
