@@ -5,6 +5,7 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -14,65 +15,62 @@
 namespace {
 
 using cr::qmdff::kVAngl;
+using cr::qmdff::kVBond;
 using cr::qmdff::kVPair;
+using cr::qmdff::kVTors;
 
-// Term schedule of one kind: batches of 32 lanes; within a batch, terms of
-// one colour touch disjoint atoms.  Greedy: each colour takes, in order, the
-// remaining terms that do not touch an atom already used by that colour,
-// until the batch holds 32 terms or has max_colours colours.  Every colour
-// costs one scatter round of the warp while an unfilled lane wastes a whole
-// term evaluation; on C20H42 the mixed form is fastest with at most 3
-// colours for bonds, 4 for angles and 6 for torsions (2.99 -> 2.66 ms per
-// 65 536 beads against 1 / 2 / 2: two colours left torsion batches half
-// empty); pairs use schedule_pairs.
-void schedule_kind(int nterm, int arity, int max_colours, const std::vector<int>& atoms,
-                   const std::vector<int>& order, int natoms, std::vector<int>& slot,
-                   std::vector<unsigned char>& color, std::vector<unsigned char>& ncol, int& nbatch,
-                   int& colours) {
-  std::vector<int> remaining = order;
-  std::vector<int> stamp((size_t)natoms, -1);
-  int stamp_id = 0;
-  nbatch = 0;
-  while (!remaining.empty()) {
-    std::vector<int> bt, bc;
-    int col = 0;
-    while ((int)bt.size() < 32 && !remaining.empty() && col < max_colours) {
-      ++stamp_id;
-      std::vector<int> rest;
-      rest.reserve(remaining.size());
-      for (int t : remaining) {
-        bool ok = (int)bt.size() < 32;
-        for (int a = 0; ok && a < arity; ++a)
-          if (stamp[(size_t)atoms[(size_t)t * arity + a]] == stamp_id) ok = false;
-        if (!ok) {
-          rest.push_back(t);
-          continue;
+// Segments of one kind (qmdff.cuh, Schedule): the terms cut into segments, and for
+// each coordinate the list of what a segment holds for it.
+struct ScheduleHost {
+  std::vector<int4> seg;
+  std::vector<int2> round;
+  std::vector<unsigned short> dst, ent;
+};
+void schedule_kind(bool mixed, int kind, int arity, const std::vector<int>& atoms, int natoms, ScheduleHost& h) {
+  const int C = cr::qmdff::segment_terms(mixed, kind), zero = cr::qmdff::buffer_values(mixed);
+  const int nterm = (int)atoms.size() / arity;
+  for (int t0 = 0; t0 < nterm; t0 += C) {
+    const int nt = std::min(nterm - t0, C);
+    // per atom the entries of its x component (y, z: C and 2 C further)
+    std::vector<std::vector<int>> list((size_t)natoms);
+    for (int i = 0; i < nt; ++i)
+      for (int a = 0; a < arity; ++a) {
+        std::vector<int>& l = list[(size_t)atoms[(size_t)(t0 + i) * arity + a]];
+        if (arity == 2) {  // the first atom's gradient (mixed-form bonds: hi, lo), the second's its negative
+          const int sign = a == 1 ? cr::qmdff::kNegate : 0;
+          l.push_back(i | sign);
+          if (mixed && kind == 0) l.push_back((3 * C + i) | sign);
+        } else {
+          l.push_back(3 * a * C + i);
         }
-        for (int a = 0; a < arity; ++a) stamp[(size_t)atoms[(size_t)t * arity + a]] = stamp_id;
-        bt.push_back(t);
-        bc.push_back(col);
       }
-      remaining.swap(rest);
-      ++col;
+    std::vector<int> by((size_t)natoms);
+    for (int a = 0; a < natoms; ++a) by[(size_t)a] = a;
+    std::stable_sort(by.begin(), by.end(), [&](int x, int y) { return list[(size_t)x].size() > list[(size_t)y].size(); });
+    int used = 0;  // coordinates with a list
+    while (used < natoms && !list[(size_t)by[(size_t)used]].empty()) ++used;
+    used *= 3;
+    const int rounds = (used + 31) / 32;
+    h.seg.push_back(make_int4(t0, nt, (int)h.round.size(), rounds));
+    for (int r = 0; r < rounds; ++r) {
+      const int steps = (int)list[(size_t)by[(size_t)(32 * r / 3)]].size();
+      h.round.push_back(make_int2((int)h.ent.size(), steps));
+      for (int x = 32 * r; x < 32 * r + 32; ++x)
+        h.dst.push_back((unsigned short)(x < used ? 3 * by[(size_t)(x / 3)] + x % 3 : cr::qmdff::kNoDst));
+      for (int k = 0; k < steps; ++k)
+        for (int x = 32 * r; x < 32 * r + 32; ++x) {
+          const std::vector<int>* l = x < used ? &list[(size_t)by[(size_t)(x / 3)]] : nullptr;
+          h.ent.push_back((unsigned short)(l && k < (int)l->size() ? (*l)[(size_t)k] + (x % 3) * C : zero));
+        }
     }
-    for (int l = 0; l < 32; ++l) {
-      slot.push_back(l < (int)bt.size() ? bt[(size_t)l] : -1);
-      color.push_back((unsigned char)(l < (int)bc.size() ? bc[(size_t)l] : 0));
-    }
-    ncol.push_back((unsigned char)col);
-    colours += col;
-    ++nbatch;
   }
-  (void)nterm;
 }
 
 // Pair terms: the circle method splits all atom pairs of n atoms (n even; a
 // dummy atom for odd n) into n-1 perfect matchings; the pairs of one
 // matching touch disjoint atoms, so each matching is one single-colour batch
 // (split in 32-lane pieces when n > 64).
-void schedule_pairs(int nterm, const std::vector<int>& atoms, int natoms, std::vector<int>& slot,
-                    std::vector<unsigned char>& color, std::vector<unsigned char>& ncol, int& nbatch,
-                    int& colours) {
+void schedule_pairs(int nterm, const std::vector<int>& atoms, int natoms, std::vector<int>& slot, int& nbatch) {
   const int m = natoms + (natoms & 1);  // players, even
   std::vector<std::vector<int>> rounds((size_t)(m > 1 ? m - 1 : 1));
   for (int t = 0; t < nterm; ++t) {
@@ -89,10 +87,7 @@ void schedule_pairs(int nterm, const std::vector<int>& atoms, int natoms, std::v
       for (int l = 0; l < 32; ++l) {
         const size_t k = k0 + (size_t)l;
         slot.push_back(k < rd.size() ? rd[k] : -1);
-        color.push_back(0);
       }
-      ncol.push_back(1);
-      colours += 1;
       ++nbatch;
     }
   }
@@ -136,24 +131,21 @@ std::vector<float> to_float(const std::vector<T>& v) {
 namespace cr {
 
 // MINB: blocks of kQmdffWarps warps kept resident per SM (the register cap
-// follows: 65536 / (MINB * 128) per thread).  The FP64 form trades spills for
+// follows: 65536 / (MINB * block) per thread).  The FP64 form trades spills for
 // occupancy differently from the mixed form; the autotuner below picks.  Mixed: a
 // warp per bead; FP64: a block per bead (kTeam).
-static_assert(kQmdffWarps == qmdff::kTeam, "an FP64 block is one team");
+constexpr int kQmdffThreads = kQmdffWarps * 32, kTeamThreads = qmdff::kTeam * 32;
 template <bool MIXED, int MINB, int MODE = qmdff::kFree>
-__global__ void __launch_bounds__(kQmdffWarps * 32, MINB)
+__global__ void __launch_bounds__(MIXED ? kQmdffThreads : kTeamThreads, MINB)
     qmdff_egrad_kernel(qmdff::Dev D, int nbeads, BeadRows rows, const double* q, double* e, double* g) {
   extern __shared__ double qsm[];
   const int n3 = 3 * D.n;
   if constexpr (MIXED) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* ws = qsm + (size_t)warp * (qmdff::warp_smem_bytes(D.n) / sizeof(double));
+    void* ws = qsm + (size_t)warp * (qmdff::warp_smem_bytes(D.n) / sizeof(double));
     for (int b = blockIdx.x * kQmdffWarps + warp; b < nbeads; b += gridDim.x * kQmdffWarps) {
       const size_t r = rows.row(b), r2 = rows.twin(b);
-      const double* qb = q + r * n3;
-      for (int a = lane; a < n3; a += 32) ws[a] = qb[a];
-      __syncwarp();
-      const double v = qmdff::warp_egrad<MODE>(D, ws, g + r * n3, g + r2 * n3, lane, r, r2);
+      const double v = qmdff::warp_egrad<MODE>(D, ws, q + r * n3, g + r * n3, g + r2 * n3, lane, r, r2);
       if (lane == 0) {
         e[r] = v;
         if (r2 != r) e[r2] = v;
@@ -164,7 +156,7 @@ __global__ void __launch_bounds__(kQmdffWarps * 32, MINB)
     for (int b = blockIdx.x; b < nbeads; b += gridDim.x) {
       const size_t r = rows.row(b), r2 = rows.twin(b);
       const double* qb = q + r * n3;
-      for (int a = threadIdx.x; a < n3; a += kQmdffWarps * 32) qsm[a] = qb[a];
+      for (int a = threadIdx.x; a < n3; a += kTeamThreads) qsm[a] = qb[a];
       const double v = qmdff::team_egrad<MODE>(D, qsm, g + r * n3, g + r2 * n3, r, r2);
       if (threadIdx.x == 0) {
         e[r] = v;
@@ -177,7 +169,7 @@ __global__ void __launch_bounds__(kQmdffWarps * 32, MINB)
 
 // Energy, gradient and Hessian-vector product H w per bead (plain form, dual
 // coordinates), a block per bead; dew[b] = w . grad E.
-__global__ void __launch_bounds__(kQmdffWarps * 32)
+__global__ void __launch_bounds__(kTeamThreads)
     qmdff_hvp_kernel(qmdff::Dev D, int nbeads, const double* q, const double* w, double* e, double* g, double* hw,
                      double* dew) {
   extern __shared__ double qsm[];
@@ -185,7 +177,7 @@ __global__ void __launch_bounds__(kQmdffWarps * 32)
   for (int b = blockIdx.x; b < nbeads; b += gridDim.x) {
     const double* qb = q + (size_t)b * n3;
     const double* wb = w + (size_t)b * n3;
-    for (int a = threadIdx.x; a < n3; a += kQmdffWarps * 32) {
+    for (int a = threadIdx.x; a < n3; a += kTeamThreads) {
       qsm[a] = qb[a];
       qsm[n3 + a] = wb[a];
     }
@@ -201,12 +193,12 @@ __global__ void __launch_bounds__(kQmdffWarps * 32)
 
 // Per bead b and linear parameter t: out[b][t] = alpha_b (v_b . grad E_t|unit)
 // + beta_b E_t|unit (alpha = 1, beta = 0 where the weights are NULL), a block per bead.
-__global__ void __launch_bounds__(kQmdffWarps * 32)
+__global__ void __launch_bounds__(kTeamThreads)
     qmdff_vjp_kernel(qmdff::Dev D, qmdff::Tables<double> U, int nbeads, int nlin, const double* q, const double* v,
                      const double* alpha, const double* beta, double* out) {
   extern __shared__ double qsm[];
   const int n3 = 3 * D.n, b = blockIdx.x;
-  for (int a = threadIdx.x; a < n3; a += kQmdffWarps * 32) {
+  for (int a = threadIdx.x; a < n3; a += kTeamThreads) {
     qsm[a] = q[(size_t)b * n3 + a];
     qsm[n3 + a] = v[(size_t)b * n3 + a];
   }
@@ -243,7 +235,7 @@ int qmdff_hvp_launch(const cr_qmdff* ff, const double* d_q, const double* d_w, i
   CR_TRY_CUDA(cudaFuncSetAttribute(cr::qmdff_hvp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (nbeads == 0) return CR_OK;
   const int grid = std::min(nbeads, 1 << 20);
-  cr::qmdff_hvp_kernel<<<grid, kQmdffWarps * 32, smem, s>>>(ff->dev, nbeads, d_q, d_w, d_e, d_g, d_hw, d_dew);
+  cr::qmdff_hvp_kernel<<<grid, cr::kTeamThreads, smem, s>>>(ff->dev, nbeads, d_q, d_w, d_e, d_g, d_hw, d_dew);
   CR_TRY_CUDA(cudaGetLastError());
   return CR_OK;
 }
@@ -261,7 +253,7 @@ int qmdff_vjp_launch(const cr_qmdff* ff, const double* d_q, const double* d_v, i
   const size_t n3 = (size_t)3 * ff->n;
   for (int b0 = 0; b0 < nbeads; b0 += scratch_beads) {
     const int nb = std::min(scratch_beads, nbeads - b0);
-    cr::qmdff_vjp_kernel<<<nb, kQmdffWarps * 32, smem, s>>>(ff->dev, ff->unit, nb, nlin, d_q + b0 * n3, d_v + b0 * n3,
+    cr::qmdff_vjp_kernel<<<nb, cr::kTeamThreads, smem, s>>>(ff->dev, ff->unit, nb, nlin, d_q + b0 * n3, d_v + b0 * n3,
                                                               d_alpha ? d_alpha + b0 : nullptr,
                                                               d_beta ? d_beta + b0 : nullptr, d_scratch);
     CR_TRY_CUDA(cudaGetLastError());
@@ -275,20 +267,21 @@ namespace {
 
 using QmdffKernel = void (*)(cr::qmdff::Dev, int, cr::BeadRows, const double*, double*, double*);
 constexpr int kVariants = 3;
-// [precision][variant]: blocks per SM 2 / 3 / 4 (FP64), 4 / 5 / 6 (mixed)
+// [precision][variant]: blocks per SM 1 / 2 / 3 (FP64), 4 / 5 / 6 (mixed)
 const QmdffKernel kKernels[2][kVariants] = {
-    {cr::qmdff_egrad_kernel<false, 2>, cr::qmdff_egrad_kernel<false, 3>, cr::qmdff_egrad_kernel<false, 4>},
+    {cr::qmdff_egrad_kernel<false, 1>, cr::qmdff_egrad_kernel<false, 2>, cr::qmdff_egrad_kernel<false, 3>},
     {cr::qmdff_egrad_kernel<true, 4>, cr::qmdff_egrad_kernel<true, 5>, cr::qmdff_egrad_kernel<true, 6>}};
 constexpr int kDefaultVariant = 1;
 // the force field's periodic box, and NpT (per-trajectory boxes and the
 // virial): one variant per form each
-const QmdffKernel kBoxKernels[2] = {cr::qmdff_egrad_kernel<false, 3, cr::qmdff::kBox>,
+const QmdffKernel kBoxKernels[2] = {cr::qmdff_egrad_kernel<false, 2, cr::qmdff::kBox>,
                                     cr::qmdff_egrad_kernel<true, 5, cr::qmdff::kBox>};
-const QmdffKernel kNptKernels[2] = {cr::qmdff_egrad_kernel<false, 3, cr::qmdff::kNpt>,
+const QmdffKernel kNptKernels[2] = {cr::qmdff_egrad_kernel<false, 2, cr::qmdff::kNpt>,
                                     cr::qmdff_egrad_kernel<true, 5, cr::qmdff::kNpt>};
 constexpr int kTuneMinBeads = 2048;  // smaller batches keep the default
 
-// Blocks and dynamic shared memory of the force kernel's forms.
+// Threads, blocks and dynamic shared memory of the force kernel's forms.
+int egrad_threads(int prec) { return prec == 1 ? cr::kQmdffThreads : cr::kTeamThreads; }
 int egrad_grid(int prec, int nbeads) {
   return std::min(prec == 1 ? (nbeads + kQmdffWarps - 1) / kQmdffWarps : nbeads, 1 << 20);
 }
@@ -301,7 +294,7 @@ int launch_dev(const cr::qmdff::Dev& D, int prec, int v, cr::BeadRows rows, cons
   const size_t smem = egrad_smem(prec, D.n);
   const int grid = egrad_grid(prec, nbeads);
   const QmdffKernel k = D.periodic ? kBoxKernels[prec] : kKernels[prec][v];
-  k<<<grid, kQmdffWarps * 32, smem, s>>>(D, nbeads, rows, d_q, d_e, d_g);
+  k<<<grid, egrad_threads(prec), smem, s>>>(D, nbeads, rows, d_q, d_e, d_g);
   CR_TRY_CUDA(cudaGetLastError());
   return CR_OK;
 }
@@ -323,7 +316,7 @@ int launch_npt(const cr_qmdff* ff, int prec, const QmdffNpt& npt, cr::BeadRows r
     CR_TRY_CUDA(cudaFuncSetAttribute(kNptKernels[prec], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (nbeads <= 0) return CR_OK;
   const int grid = egrad_grid(prec, nbeads);
-  kNptKernels[prec]<<<grid, kQmdffWarps * 32, smem, s>>>(D, nbeads, rows, d_q, d_e, d_g);
+  kNptKernels[prec]<<<grid, egrad_threads(prec), smem, s>>>(D, nbeads, rows, d_q, d_e, d_g);
   CR_TRY_CUDA(cudaGetLastError());
   return CR_OK;
 }
@@ -331,7 +324,7 @@ int launch_npt(const cr_qmdff* ff, int prec, const QmdffNpt& npt, cr::BeadRows r
 // The force kernel over a subset of the term kinds (bit k of mask: kind k =
 // bonds, angles, torsions, NCI pairs, H/halogen bonds), with or without
 // E_zero: the pieces of Caracal's QMDFF call site (src/gradient.f90:341-358).
-// The masked kinds' batch counts are set to zero in a copy of the schedule.
+// The masked kinds' segments are left out of a copy of the schedule.
 int qmdff_launch_kinds(const cr_qmdff* ff, unsigned mask, bool ezero, const double* d_q, int nbeads, double* d_e,
                        double* d_g, int precision, cudaStream_t s) {
   if (precision != CR_PREC_MIXED && precision != CR_PREC_FP64) return cr_set_error(CR_ERR_ARG, "unknown precision");
@@ -346,7 +339,10 @@ int qmdff_launch_kinds(const cr_qmdff* ff, unsigned mask, bool ezero, const doub
   cr::qmdff::Dev D = ff->dev;
   for (int p = 0; p < 2; ++p)
     for (int k = 0; k < cr::qmdff::kKinds; ++k)
-      if (!((mask >> k) & 1u)) D.sched[p].nb[k] = 0;
+      if (!((mask >> k) & 1u)) {
+        D.sched[p].seg1[k] = D.sched[p].seg0[k];
+        if (k == 3) D.sched[p].npair = 0;
+      }
   if (!ezero) D.e_zero = 0.0;
   const int v = ff->variant[prec] >= 0 ? ff->variant[prec] : kDefaultVariant;
   return launch_dev(D, prec, v, cr::all_rows(), d_q, nbeads, d_e, d_g, s);
@@ -502,42 +498,80 @@ int cr_qmdff_create(const cr_qmdff_def* d, cr_qmdff** out) {
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return cr_set_error(CR_ERR_NO_DEVICE, "no CUDA device");
 
   const double pi = 3.1415926535897932384626433832795029;
-  std::vector<double> rad((size_t)n), vbond(d->vbond, d->vbond + 3 * d->nbond), vtors(d->vtors, d->vtors + 14 * d->ntors);
-  for (int i = 0; i < n; ++i) rad[(size_t)i] = d->rad[d->at[i] - 1];
-  std::vector<double> vangl((size_t)kVAngl * d->nangl);
+  // the tables, value by value (qmdff.cuh, Tables); the torsions ordered by (type,
+  // nt), so a warp runs one code path
+  cr::qmdff::Dev devt{};
+  const int count[cr::qmdff::kKinds] = {d->nbond, d->nangl, d->ntors, d->nnci, d->nhb};
+  for (int k = 0; k < cr::qmdff::kKinds; ++k) devt.st[k] = (count[k] + 31) / 32 * 32;
+  const int* st = devt.st;
+  auto rad = [&](int atom) { return d->rad[d->at[atom] - 1]; };
+  // 1 / rcut of abdamp (src/abdamp.f90:36-51); its prefactor is the REAL(4) product 3.0*3.5710642
+  auto irc = [&](int a, int b) {
+    const double r = rad(a) + rad(b);
+    return 1.0 / ((double)(3.0f * 3.5710642f) * (r * r));
+  };
+  auto pack = [](int a, int b) { return (unsigned)a | (unsigned)b << 16; };
+  std::vector<double> vbond((size_t)kVBond * st[0]), vangl((size_t)kVAngl * st[1]), vtors((size_t)kVTors * st[2]),
+      vpair((size_t)kVPair * st[3]);
+  std::vector<unsigned> bond((size_t)st[0]), pair((size_t)st[3]);
+  std::vector<uint2> angl((size_t)st[1]);
+  std::vector<uint4> tors((size_t)st[2]);
+  std::vector<int> atoms[cr::qmdff::kKinds];  // per term in the order of its gradient
+  for (int m = 0; m < d->nbond; ++m) {
+    const int i = d->bond[2 * m] - 1, j = d->bond[2 * m + 1] - 1;
+    bond[(size_t)m] = pack(i, j);
+    for (int c = 0; c < 3; ++c) vbond[(size_t)c * st[0] + m] = d->vbond[3 * m + c];
+    atoms[0].insert(atoms[0].end(), {i, j});
+  }
   for (int m = 0; m < d->nangl; ++m) {
+    const int j = d->angl[3 * m] - 1, i = d->angl[3 * m + 1] - 1, k = d->angl[3 * m + 2] - 1;
+    angl[(size_t)m] = make_uint2(pack(i, j), (unsigned)k);
     const double th0 = d->vangl[2 * m];
-    vangl[(size_t)kVAngl * m] = th0;
-    vangl[(size_t)kVAngl * m + 1] = d->vangl[2 * m + 1];
-    vangl[(size_t)kVAngl * m + 2] = std::cos(th0);
-    vangl[(size_t)kVAngl * m + 3] = (pi - th0 < 1e-6) ? 1.0 : 0.0;
+    const double v[kVAngl] = {th0, d->vangl[2 * m + 1], std::cos(th0), (pi - th0 < 1e-6) ? 1.0 : 0.0, irc(i, j), irc(k, j)};
+    for (int c = 0; c < kVAngl; ++c) vangl[(size_t)c * st[1] + m] = v[c];
+    atoms[1].insert(atoms[1].end(), {i, j, k});
   }
-  std::vector<int> bond((size_t)2 * d->nbond), angl((size_t)3 * d->nangl), tors((size_t)6 * d->ntors),
-      pair((size_t)2 * d->nnci);
-  for (int m = 0; m < 2 * d->nbond; ++m) bond[(size_t)m] = d->bond[m] - 1;
-  for (int m = 0; m < 3 * d->nangl; ++m) angl[(size_t)m] = d->angl[m] - 1;
-  for (int m = 0; m < d->ntors; ++m) {
-    for (int a = 0; a < 4; ++a) tors[(size_t)6 * m + a] = d->tors[6 * m + a] - 1;
-    tors[(size_t)6 * m + 4] = d->tors[6 * m + 4];
-    tors[(size_t)6 * m + 5] = d->tors[6 * m + 5];
+  std::vector<int> order((size_t)d->ntors);
+  for (int m = 0; m < d->ntors; ++m) order[(size_t)m] = m;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+    return d->tors[6 * x + 5] * 8 + d->tors[6 * x + 4] < d->tors[6 * y + 5] * 8 + d->tors[6 * y + 4];
+  });
+  for (int x = 0; x < d->ntors; ++x) {
+    const int m = order[(size_t)x], *t = d->tors + 6 * m;
+    const int i = t[0] - 1, j = t[1] - 1, k = t[2] - 1, l = t[3] - 1, type = t[5];
+    // what the kernels tell apart: inversions (2) and torsions, which have 0..4 terms
+    tors[(size_t)x] = make_uint4(pack(i, j), pack(k, l), (unsigned)(type == 2 ? 2 * 256 : t[4] + 256), (unsigned)m);
+    for (int c = 0; c < 14; ++c) vtors[(size_t)c * st[2] + x] = d->vtors[14 * m + c];
+    vtors[(size_t)14 * st[2] + x] = irc(i, j);
+    vtors[(size_t)15 * st[2] + x] = irc(k, j);
+    vtors[(size_t)16 * st[2] + x] = type != 2 ? irc(k, l) : irc(j, l);
+    atoms[2].insert(atoms[2].end(), {i, j, k, l});
   }
-  std::vector<double> vpair((size_t)kVPair * d->nnci, 0.0);
+  // a pair's class: what depends on its elements and its category alone
+  struct PairClass {
+    int z1, z2, nk;
+    bool operator<(const PairClass& o) const { return std::tie(z1, z2, nk) < std::tie(o.z1, o.z2, o.nk); }
+  };
+  std::map<PairClass, int> classes;
+  std::vector<float4> pclass;
+  std::vector<int> class_of((size_t)d->nnci);
   for (int m = 0; m < d->nnci; ++m) {
     const int i1 = d->nci[3 * m] - 1, i2 = d->nci[3 * m + 1] - 1, nk = d->nci[3 * m + 2];
-    pair[(size_t)2 * m] = i1;
-    pair[(size_t)2 * m + 1] = i2;
+    pair[(size_t)m] = pack(i1, i2);
+    atoms[3].insert(atoms[3].end(), {i1, i2});
     const int z1 = d->at[i1] - 1, z2 = d->at[i2] - 1;
     const size_t e12 = (size_t)z1 + 94 * (size_t)z2;  // (iz1, iz2) column-major
-    double* v = &vpair[(size_t)kVPair * m];
     const double R0 = d->r0094[e12], c6 = d->c66ab[(size_t)i2 + (size_t)n * i1], eps2 = d->eps2[nk - 1];  // c66ab(i2, i1)
-    const double R02 = R0 * R0, R06 = R02 * R02 * R02;
-    v[0] = R06;
-    v[1] = R06 * R02;
-    v[2] = eps2 * c6;
-    v[3] = eps2 * c6 * d->sr42[e12];
-    v[4] = eps2 * d->zab[e12];
-    v[5] = d->r0ab[e12];
-    v[6] = d->zahn ? d->q[i1] * d->q[i2] : d->q[i1] * d->q[i2] * d->eps1[nk - 1];
+    const double R02 = R0 * R0, R06 = R02 * R02 * R02, alpha = d->r0ab[e12];
+    const double v[kVPair] = {R06, R06 * R02, eps2 * c6, eps2 * c6 * d->sr42[e12], eps2 * d->zab[e12], alpha,
+                              d->zahn ? d->q[i1] * d->q[i2] : d->q[i1] * d->q[i2] * d->eps1[nk - 1]};
+    for (int c = 0; c < kVPair; ++c) vpair[(size_t)c * st[3] + m] = v[c];
+    const auto at = classes.emplace(PairClass{z1, z2, nk}, (int)classes.size());
+    class_of[(size_t)m] = at.first->second;
+    if (at.second) {
+      pclass.push_back(make_float4((float)v[0], (float)v[1], (float)d->sr42[e12], (float)v[4]));
+      pclass.push_back(make_float4((float)(alpha * 1.4426950408889634074), (float)alpha, 0.f, 0.f));  // log2(e)
+    }
   }
 
   // H/halogen bonds: A, B, H (0-based) and the kind (src/ff_hb.f90:71-78)
@@ -556,69 +590,31 @@ int cr_qmdff_create(const cr_qmdff_def* d, cr_qmdff** out) {
   ff->nterm[3] = d->nnci;
   ff->nterm[4] = d->nhb;
 
-  // schedules (plain, mixed): torsions grouped by (type, nt) so a batch runs
-  // one code path
-  std::vector<int> slot[2];
-  std::vector<unsigned char> color[2], ncol[2];
+  for (int m = 0; m < d->nhb; ++m)
+    for (int a = 0; a < 3; ++a) atoms[4].push_back(hb[(size_t)4 * m + a]);
+  ScheduleHost sched[2];
+  std::vector<int> mixed_pairs;
   cr::qmdff::Dev& D = ff->dev;
+  D = devt;
   D.n = n;
-  bool distinct = true;
-  for (int form = 0; form < 2; ++form) {
-    int boff = 0;
+  for (int form = 0; form < 2; ++form)
     for (int kind = 0; kind < cr::qmdff::kKinds; ++kind) {
-      std::vector<int> order((size_t)ff->nterm[kind]);
-      for (int m = 0; m < ff->nterm[kind]; ++m) order[(size_t)m] = m;
-      std::vector<int> atoms;
-      int arity = 2;
-      if (kind == 0) atoms = bond;
-      if (kind == 1) {
-        arity = 3;
-        atoms = angl;
-      }
-      if (kind == 2) {
-        arity = 4;
-        atoms.resize((size_t)4 * d->ntors);
-        for (int m = 0; m < d->ntors; ++m)
-          for (int a = 0; a < 4; ++a) atoms[(size_t)4 * m + a] = tors[(size_t)6 * m + a];
-        std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-          const int kx = tors[(size_t)6 * x + 5] * 8 + tors[(size_t)6 * x + 4];
-          const int ky = tors[(size_t)6 * y + 5] * 8 + tors[(size_t)6 * y + 4];
-          return kx < ky;
-        });
-      }
-      if (kind == 3) atoms = pair;
-      if (kind == 4) {
-        arity = 3;
-        atoms.resize((size_t)3 * d->nhb);
-        for (int m = 0; m < d->nhb; ++m)
-          for (int a = 0; a < 3; ++a) atoms[(size_t)3 * m + a] = hb[(size_t)4 * m + a];
-      }
-      int nb = 0;
-      int* colours = form == 1 ? &ff->ncolors : &ff->ncolors_fp64;
-      if (form == 1 && kind == 3) {
-        schedule_pairs(ff->nterm[kind], atoms, n, slot[form], color[form], ncol[form], nb, *colours);
-      } else {
-        const int max_colours = form == 0 ? 255 : (kind == 0 ? 3 : kind == 1 ? 4 : kind == 2 ? 6 : 2);
-        schedule_kind(ff->nterm[kind], arity, max_colours, atoms, order, n, slot[form], color[form], ncol[form], nb,
-                      *colours);
-      }
-      if (form == 0)
-        for (int m = 0; m < ff->nterm[kind]; ++m)
-          for (int x = 0; x < arity; ++x)
-            for (int y = x + 1; y < arity; ++y)
-              if (atoms[(size_t)m * arity + x] == atoms[(size_t)m * arity + y]) distinct = false;
-      D.sched[form].nb[kind] = nb;
-      D.sched[form].boff[kind] = boff;
-      boff += nb;
+      const int arity = kind == 0 || kind == 3 ? 2 : kind == 2 ? 4 : 3;
+      cr::qmdff::Schedule& S = D.sched[form];
+      S.seg0[kind] = (int)sched[form].seg.size();
+      if (form == 1 && kind == 3) schedule_pairs(ff->nterm[kind], atoms[kind], n, mixed_pairs, S.npair);
+      else schedule_kind(form == 1, kind, arity, atoms[kind], n, sched[form]);
+      S.seg1[kind] = (int)sched[form].seg.size();
+      if (form == 1) ff->batches[kind] = kind == 3 ? S.npair : (ff->nterm[kind] + 31) / 32;
     }
-  }
 
   Arena arena;
   auto up = [&](auto& h, auto** dp) { arena.add(h, dp); };
   for (int form = 0; form < 2; ++form) {
-    up(slot[form], &D.sched[form].slot);
-    up(color[form], &D.sched[form].color);
-    up(ncol[form], &D.sched[form].ncol);
+    up(sched[form].seg, &D.sched[form].seg);
+    up(sched[form].round, &D.sched[form].round);
+    up(sched[form].dst, &D.sched[form].dst);
+    up(sched[form].ent, &D.sched[form].ent);
   }
   up(bond, &D.bond);
   up(angl, &D.angl);
@@ -626,27 +622,27 @@ int cr_qmdff_create(const cr_qmdff_def* d, cr_qmdff** out) {
   up(pair, &D.pair);
   up(hb, &D.hb);
   up(vhb, &D.vhb);
-  up(rad, &D.d.rad);
-  up(vbond, &D.d.vbond);
-  up(vangl, &D.d.vangl);
-  up(vtors, &D.d.vtors);
-  up(vpair, &D.d.vpair);
-  std::vector<float> frad = to_float(rad), fvbond = to_float(vbond), fvangl = to_float(vangl),
-                     fvtors = to_float(vtors);
-  up(frad, &D.f.rad);
-  up(fvbond, &D.f.vbond);
-  up(fvangl, &D.f.vangl);
-  up(fvtors, &D.f.vtors);
-  // mixed-form pair constants (pair_mixed)
-  std::vector<float> fpair((size_t)kVPair * d->nnci);
-  for (int m = 0; m < d->nnci; ++m) {
-    const double* v = &vpair[(size_t)kVPair * m];
-    float* o = &fpair[(size_t)kVPair * m];
-    for (int k = 0; k < kVPair; ++k) o[k] = (float)v[k];
-    o[5] = (float)(v[5] * 1.4426950408889634074);  // log2(e)
-    o[7] = (float)v[5];
-  }
+  up(vbond, &D.d.bond);
+  up(vangl, &D.d.angl);
+  up(vtors, &D.d.tors);
+  up(vpair, &D.d.pair);
+  std::vector<float> fvbond = to_float(vbond), fvangl = to_float(vangl), fvtors = to_float(vtors);
+  up(fvbond, &D.f.bond);
+  up(fvangl, &D.f.angl);
+  up(fvtors, &D.f.tors);
+  std::vector<uint4> fpair;
+  auto bits = [](double x) {
+    const float f = (float)x;
+    unsigned u;
+    std::memcpy(&u, &f, 4);
+    return u;
+  };
+  for (int m : mixed_pairs)
+    fpair.push_back(m < 0 ? make_uint4(0, cr::qmdff::kNoPair, 0, 0)
+                          : make_uint4(pair[(size_t)m], (unsigned)class_of[(size_t)m], bits(vpair[(size_t)2 * st[3] + m]),
+                                       bits(vpair[(size_t)6 * st[3] + m])));
   up(fpair, &D.fpair);
+  up(pclass, &D.pclass);
   D.coul_cut = d->coul_cut;
   D.zahn = d->zahn ? 1 : 0;
   D.zahn_a = d->zahn_a;
@@ -655,7 +651,6 @@ int cr_qmdff_create(const cr_qmdff_def* d, cr_qmdff** out) {
   D.fzahn_a = (float)d->zahn_a;
   D.fzahn_par = (float)d->zahn_par;
   D.e_zero = d->e_zero;
-  D.distinct = distinct ? 1 : 0;
   for (int k = 0; k < cr::qmdff::kKinds; ++k) D.nterm[k] = ff->nterm[k];
   // mixed form bond polynomial: a k u (1 - u) / r^2 = t H(t), t = r^2/r0^2 - 1,
   // H(t) = (a k / r0^2) [(1+t)^-(a/4+1) - (1+t)^-(a/2+1)] / t interpolated
@@ -667,7 +662,7 @@ int cr_qmdff_create(const cr_qmdff_def* d, cr_qmdff** out) {
     using cr::qmdff::kBondSer;
     const double T = cr::qmdff::kBondSerMaxT;
     const int nn = 48;
-    std::vector<float2> bser((size_t)kBondSer * std::max(d->nbond, 1), make_float2(0.f, 0.f));
+    std::vector<float2> bser((size_t)kBondSer * st[0], make_float2(0.f, 0.f));
     std::vector<double> node((size_t)nn), basis((size_t)kBondPoly * nn);
     for (int k = 0; k < nn; ++k) {
       node[(size_t)k] = std::cos(pi * (k + 0.5) / nn);
@@ -679,10 +674,10 @@ int cr_qmdff_create(const cr_qmdff_def* d, cr_qmdff** out) {
       return make_float2(hi, (float)(v - (double)hi));
     };
     for (int m = 0; m < d->nbond; ++m) {
-      const double r0 = vbond[(size_t)3 * m], kk = vbond[(size_t)3 * m + 1], aa = vbond[(size_t)3 * m + 2];
-      float2* row = &bser[(size_t)kBondSer * m];
-      row[0] = split(1.0 / (r0 * r0));
-      row[1] = split(r0 * r0);
+      const double r0 = d->vbond[3 * m], kk = d->vbond[3 * m + 1], aa = d->vbond[3 * m + 2];
+      auto row = [&](int c) -> float2& { return bser[(size_t)c * st[0] + m]; };
+      row(0) = split(1.0 / (r0 * r0));
+      row(1) = split(r0 * r0);
       if (!(aa > 0.0) || aa > 20.0 || !(r0 > 0.0)) continue;
       const double p1 = aa / 4.0 + 1.0, p2 = aa / 2.0 + 1.0, scale = aa * kk / (r0 * r0);
       std::vector<double>& mono = of_exponent[aa];
@@ -714,30 +709,27 @@ int cr_qmdff_create(const cr_qmdff_def* d, cr_qmdff** out) {
           }
         }
       }
-      row[2] = make_float2(1.0f, 0.0f);
-      for (int n = 0; n < kBondPoly; ++n) row[3 + n] = split(scale * mono[(size_t)n]);
+      row(2) = make_float2(1.0f, 0.0f);
+      for (int n = 0; n < kBondPoly; ++n) row(3 + n) = split(scale * mono[(size_t)n]);
     }
     up(bser, &D.bser);
   }
   // unit tables of the linear parameters (parameter gradients)
   std::vector<double> ubond = vbond, uangl = vangl, utors = vtors, upair = vpair;
-  for (int m = 0; m < d->nbond; ++m) ubond[(size_t)3 * m + 1] = 1.0;
-  for (int m = 0; m < d->nangl; ++m) uangl[(size_t)kVAngl * m + 1] = 1.0;
-  for (int m = 0; m < d->ntors; ++m) utors[(size_t)14 * m + 1] = 1.0;
-  for (int m = 0; m < d->nnci; ++m) {
-    for (int k = 2; k < 5; ++k) upair[(size_t)kVPair * m + k] = 0.0;
-    upair[(size_t)kVPair * m + 6] = 1.0;
-  }
-  up(ubond, &ff->unit.vbond);
-  up(uangl, &ff->unit.vangl);
-  up(utors, &ff->unit.vtors);
-  up(upair, &ff->unit.vpair);
+  std::fill_n(ubond.begin() + st[0], st[0], 1.0);
+  std::fill_n(uangl.begin() + st[1], st[1], 1.0);
+  std::fill_n(utors.begin() + st[2], st[2], 1.0);
+  std::fill_n(upair.begin() + (size_t)2 * st[3], (size_t)3 * st[3], 0.0);
+  std::fill_n(upair.begin() + (size_t)6 * st[3], st[3], 1.0);
+  up(ubond, &ff->unit.bond);
+  up(uangl, &ff->unit.angl);
+  up(utors, &ff->unit.tors);
+  up(upair, &ff->unit.pair);
   const int rc = arena.upload(ff);
   if (rc != CR_OK) {
     cr_qmdff_destroy(ff);
     return rc;
   }
-  ff->unit.rad = D.d.rad;
   *out = ff;
   return CR_OK;
 }
@@ -787,9 +779,12 @@ int cr_qmdff_set_periodic(cr_qmdff* ff, const double* box_ang, double coul_cut_a
 
 int cr_qmdff_schedule_info(const cr_qmdff* ff, int* batches, int* colors) {
   if (!ff) return cr_set_error(CR_ERR_ARG, "NULL force field");
-  if (batches)
-    for (int k = 0; k < cr::qmdff::kKinds; ++k) batches[k] = ff->dev.sched[1].nb[k];
-  if (colors) *colors = ff->ncolors;
+  int n = 0;
+  for (int k = 0; k < cr::qmdff::kKinds; ++k) {
+    if (batches) batches[k] = ff->batches[k];
+    n += ff->batches[k];
+  }
+  if (colors) *colors = n;  // one pass each
   return CR_OK;
 }
 

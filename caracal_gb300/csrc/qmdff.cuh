@@ -3,11 +3,10 @@
 // Drop-in for Caracal's per-bead QMDFF gradient (src/gradient.f90:342-358:
 // ff_eg src/ff_eg.f90:41-629, ff_nonb src/ff_nonb.f90:34-889, E_zero shift),
 // non-periodic, one molecule.  A bead's coordinates and gradient live in the
-// warp's shared memory.  The host packs the terms of each kind into batches
-// of 32 (one term per lane) and colours each batch so that no atom appears
-// twice within a colour; a lane computes its term, then the warp scatters the
-// term gradients colour by colour.  No atomics, fixed accumulation order:
-// results are deterministic run to run.
+// warp's shared memory.  A lane evaluates a term and writes its gradient into a
+// buffer in shared memory; once a segment of terms is done, every coordinate
+// sums what the segment holds for it, along lists that the host prepared.  No
+// atomics, fixed accumulation order: results are deterministic run to run.
 //
 // Precision: the plain form computes every term in FP64 with Caracal's
 // formulas (divisions by a shared denominator taken as one reciprocal).  The
@@ -30,30 +29,60 @@ namespace cr {
 namespace qmdff {
 
 constexpr int kMaxAtoms = 1024;
-constexpr int kVAngl = 4;   // theta0, k, cos(theta0), linear flag
-constexpr int kVPair = 8;   // R0^6, R0^8, eps2 C6, eps2 C6 sr42, eps2 zab, alpha, qq (eps1 q_i q_j or q_i q_j), 0
 
-// Per-term parameter tables in the arithmetic type of the form.
+// Values per term in the tables: bonds r0, k, a; angles theta0, k, cos(theta0),
+// linear flag, 1 / rcut of its two bonds' damping (abdamp); torsions phi0, V, (rn,
+// phase, Vn) x 4, 1 / rcut of its three; pairs R0^6, R0^8, eps2 C6, eps2 C6 sr42, eps2
+// zab, alpha, qq (eps1 q_i q_j or q_i q_j).
+constexpr int kVBond = 3, kVAngl = 6, kVTors = 17, kVPair = 7;
+constexpr int kVClass = 8;  // mixed-form pair classes (Dev::pclass)
+
+// Term tables in the arithmetic type of the form, value by value (value c of term m
+// of kind k at [c st[k] + m]): the lanes of a warp, which take consecutive terms,
+// read consecutive words.  With a term's values side by side the mixed
+// force kernel waited for its tables a third of the time (1024 x 64 C20H42, 33
+// distinct beads each: 1190 -> 940 us with the gather below).
 template <class F>
 struct Tables {
-  const F* rad;    // covalent radius per atom (bohr)
-  const F* vbond;  // 3 per bond: r0, k, a
-  const F* vangl;  // kVAngl per angle
-  const F* vtors;  // 14 per torsion: phi0, V, (rn, phase, Vn) x 4
-  const F* vpair;  // kVPair per NCI pair
+  const F* bond;
+  const F* angl;
+  const F* tors;
+  const F* pair;  // (the mixed form's pairs: Dev::fpair)
 };
 
 constexpr int kKinds = 5;  // bonds, angles, torsions, NCI pairs, H/halogen bonds
 
-// Warp schedule of the terms: batches of 32 slots (one term per lane) with
-// the colour of each slot; no atom appears twice within a colour.
+// Schedule of the terms of one form.  A segment is as many terms of a kind as the
+// gradient buffer holds; its gather works in rounds of 32 coordinates (the atoms
+// with the most terms first, so that a round's lists are of like length), each
+// lane summing its coordinate's list.  Written so, a term's gradient costs one
+// store per component and one load and sum per component and atom; scattered
+// colour by colour, as the terms of a batch share atoms, it cost a round of the
+// warp per colour: a third of the mixed kernel's instructions and two thirds of the
+// FP64 kernel's time.
 struct Schedule {
-  int nb[kKinds];    // batches per kind
-  int boff[kKinds];  // first batch of each kind
-  const int* slot;             // [batches][32]: term index or -1
-  const unsigned char* color;  // [batches][32]
-  const unsigned char* ncol;   // [batches]
+  int seg0[kKinds], seg1[kKinds];  // segments of each kind
+  const int4* seg;                 // first term, terms, first round, rounds
+  const int2* round;               // first list entry (32 per step), steps
+  const unsigned short* dst;       // [rounds][32]: coordinate, or kNoDst
+  const unsigned short* ent;       // buffer offset, kNegate for the negative; the offset past the buffer holds 0
+  int npair;                       // batches of 32 NCI pairs of the mixed form (Dev::fpair)
 };
+constexpr int kNoDst = 0xffff, kNegate = 0x8000;
+constexpr unsigned kNoPair = 0xffffffffu;
+__device__ __forceinline__ int lo16(unsigned x) { return (int)(x & 0xffffu); }
+__device__ __forceinline__ int hi16(unsigned x) { return (int)(x >> 16); }
+
+// Values per term in the buffer (a bond or pair: one atom's gradient, the mixed
+// form's bonds as (hi, lo); the other atom's is its negative), and the terms of a
+// segment.
+__host__ __device__ constexpr int term_values(bool mixed, int kind) {
+  return kind == 0 ? (mixed ? 6 : 3) : kind == 2 ? 12 : kind == 3 ? 3 : 9;
+}
+__host__ __device__ constexpr int segment_terms(bool mixed, int kind) {
+  return mixed ? (kind == 0 ? 64 : 32) : (kind == 0 || kind == 3 ? 1024 : 256);
+}
+__host__ __device__ constexpr int buffer_values(bool mixed) { return mixed ? 384 : 3072; }
 
 // A periodic box (src/box_image.f90): edges and halves in bohr, and for the
 // mixed form the edges as (hi, lo) float pairs and the halves in FP32.
@@ -79,15 +108,13 @@ __host__ __device__ inline PBox make_box(const double* len) {
 
 struct Dev {
   int n;
-  // [0] plain form: full 32-term batches, as many colours as needed (an FP64
-  // term costs far more than a scatter round); [1] mixed form: NCI pairs in
-  // round-robin matchings (one colour), bonds up to 3 colours, angles 4,
-  // torsions 6, H/halogen bonds 2.
+  // [0] plain form, [1] mixed form
   Schedule sched[2];
-  const int* bond;   // 2 per bond (0-based)
-  const int* angl;   // 3 per angle (centre, i, k)
-  const int* tors;   // 6 per torsion: i, j, k, l, nt, type
-  const int* pair;   // 2 per NCI pair
+  int st[kKinds];       // stride of the tables
+  const unsigned* bond; // atoms (0-based) in 16 bits each: i, j
+  const uint2* angl;    // i, centre; k
+  const uint4* tors;    // i, j; k, l; nt + 256 type; number in the definition (the terms are ordered by type and nt)
+  const unsigned* pair; // i, j
   const int* hb;     // 4 per H/halogen bond: A, B, H, type (1 hydrogen bond, 2 halogen bond)
   const double* vhb; // 2 per H/halogen bond: ca, cb
   Tables<double> d;
@@ -108,16 +135,16 @@ struct Dev {
   const double* tbox;
   int tbox_beads;
   double* vir;
-  int distinct;  // 1: every term's atoms are pairwise distinct
   int nterm[kKinds];  // terms per kind
   // mixed form, bond stretch gradient as a double-FP32 polynomial (see
   // bond_mixed): per bond kBondSer (hi, lo) pairs: 1/r0^2, r0^2, (use flag,
-  // 0), the kBondPoly coefficients
+  // 0), the kBondPoly coefficients, value by value as the tables
   const float2* bser;
-  // mixed form, NCI pairs with their constants folded (pair_mixed_v): per pair
-  // kVPair floats R0^6, R0^8, eps2 C6, eps2 C6 sr42, eps2 zab,
-  // alpha log2(e), qq, alpha, each rounded once from FP64
-  const float* fpair;
+  // mixed form, NCI pairs in batches of 32 in which no atom appears twice: atoms,
+  // class (kNoPair: none), eps2 C6, qq; and per class R0^6, R0^8, sr42, eps2 zab, alpha
+  // log2(e), alpha (which depend on the elements and the category alone)
+  const uint4* fpair;
+  const float4* pclass;
 };
 
 constexpr int kBondPoly = 24;             // polynomial of degree 23
@@ -180,101 +207,29 @@ struct Contrib {
   F g[4][3];
 };
 
-// Gradient accumulator of one bead in shared memory: FP64 in the plain form,
-// compensated FP32 (sum and compensation arrays) in the mixed form.
-template <class F>
-struct Grad;
-template <>
-struct Grad<double> {
-  double* g;
-  __device__ inline void add(int i, double v) { g[i] += v; }
-  __device__ inline double get(int i) const { return g[i]; }
-};
-template <>
-struct Grad<float> {
-  float2* sk;  // (sum, compensation) per coordinate: one 8-byte access each
-  float* pr;   // NCI pair contributions, a plain FP32 sum: they are ~1 % of
-               // the valence forces, so their own rounding stays below the
-               // compensated sum's, and keeping them apart leaves that sum
-               // free of many small additions
-  __device__ inline void add(int i, float v) {
-    float2 c = sk[i];
-    const float t = c.x + v;
-    c.y += (fabsf(c.x) >= fabsf(v)) ? ((c.x - t) + v) : ((v - t) + c.x);
-    c.x = t;
-    sk[i] = c;
-  }
-  __device__ inline double get(int i) const { return ((double)sk[i].x + (double)sk[i].y) + (double)pr[i]; }
-};
-
-// Adds a term's gradient for its NA atoms (compile-time count).  Mixed form
-// with distinct atoms (checked on the host, `Dev::distinct`): all loads are
-// issued before the stores, so the shared-memory round trips overlap.  The
-// FP64 form is bound by the FP64 pipe, not by these round trips, and keeps
-// the sequential adds (fewer live registers).
-template <int NA>
-__device__ inline void scatter(const Contrib<double>& c, Grad<double>& G, bool) {
-#pragma unroll
-  for (int m = 0; m < NA; ++m)
-#pragma unroll
-    for (int d = 0; d < 3; ++d) G.add(3 * c.a[m] + d, c.g[m][d]);
-}
-// bond of the mixed form: (hi, lo) parts in g[0..1] and g[2..3]
-__device__ inline void scatter_bond(const Contrib<float>& c, Grad<float>& G) {
+// A mixed-form pair's gradient onto its atoms: a plain FP32 sum (pair forces are
+// ~1 % of the valence forces, so its rounding stays below the compensated sum's).
+__device__ inline void scatter_pair(const Contrib<float>& c, float* pr) {
+  float a[2][3];
 #pragma unroll
   for (int m = 0; m < 2; ++m)
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      G.add(3 * c.a[m] + d, c.g[m][d]);
-      G.add(3 * c.a[m] + d, c.g[m + 2][d]);
-    }
-}
-template <int NA>
-__device__ inline void scatter_pair(const Contrib<float>& c, Grad<float>& G) {
-  float a[NA][3];
+    for (int d = 0; d < 3; ++d) a[m][d] = pr[3 * c.a[m] + d];
 #pragma unroll
-  for (int m = 0; m < NA; ++m)
+  for (int m = 0; m < 2; ++m)
 #pragma unroll
-    for (int d = 0; d < 3; ++d) a[m][d] = G.pr[3 * c.a[m] + d];
-#pragma unroll
-  for (int m = 0; m < NA; ++m)
-#pragma unroll
-    for (int d = 0; d < 3; ++d) G.pr[3 * c.a[m] + d] = a[m][d] + c.g[m][d];
-}
-template <int NA>
-__device__ inline void scatter(const Contrib<float>& c, Grad<float>& G, bool distinct) {
-  if (distinct) {
-    float2 a[NA][3];
-#pragma unroll
-    for (int m = 0; m < NA; ++m)
-#pragma unroll
-      for (int d = 0; d < 3; ++d) a[m][d] = G.sk[3 * c.a[m] + d];
-#pragma unroll
-    for (int m = 0; m < NA; ++m)
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const float v = c.g[m][d], s0 = a[m][d].x, t = s0 + v;
-        const float k = a[m][d].y + ((fabsf(s0) >= fabsf(v)) ? ((s0 - t) + v) : ((v - t) + s0));
-        G.sk[3 * c.a[m] + d] = make_float2(t, k);
-      }
-  } else {
-#pragma unroll
-    for (int m = 0; m < NA; ++m)
-#pragma unroll
-      for (int d = 0; d < 3; ++d) G.add(3 * c.a[m] + d, c.g[m][d]);
-  }
+    for (int d = 0; d < 3; ++d) pr[3 * c.a[m] + d] = a[m][d] + c.g[m][d];
 }
 
-// abdamp (src/abdamp.f90:36-51); the cutoff prefactor is the REAL(4) product 3.0*3.5710642
-__device__ inline void abdamp(float radi, float radj, float r2, float& damp, float& ddamp) {
-  const float s = radi + radj;
-  const float x = r2 / ((3.0f * 3.5710642f) * (s * s));
-  const float rr = x * x;
+// abdamp (src/abdamp.f90:36-51), irc = 1 / rcut
+__device__ inline void abdamp(float irc, float r2, float& damp, float& ddamp) {
+  const float x = r2 * irc, rr = x * x;
   damp = __frcp_rn(1.0f + rr);  // = 1/(1 + rr), correctly rounded
-  ddamp = -4.0f * rr * (damp * damp) / r2;
+  ddamp = -4.0f * irc * x * (damp * damp);
 }
 
-// A bead's coordinates: FP64, and (mixed form) the FP32 split x = hi + lo.
+// A bead's coordinates: FP64 (mixed form: in global memory, for the H/halogen bonds),
+// and (mixed form) the FP32 split x = hi + lo.
 struct BeadPos {
   const double* x;
   const float2* hl;  // (hi, lo) per coordinate (mixed form only)
@@ -366,8 +321,10 @@ __device__ inline void disp<float>(const BeadPos& X, int a, int b, float* v) {
 // as its (hi, lo) pair.  Beyond that range, and for the energy, the FP32
 // formula above (the FP64 pipe would cost more than the whole FP32 term).
 __device__ inline float bond_mixed(const Dev& D, const BeadPos& x, int m, Contrib<float>& c) {
-  const int i = D.bond[2 * m], j = D.bond[2 * m + 1];
-  const float2* ser = D.bser + (size_t)kBondSer * m;
+  const unsigned at = __ldg(D.bond + m);
+  const int i = lo16(at), j = hi16(at), st = D.st[0];
+  const float2* ser = D.bser + m;  // value c at [c st]
+  const float* v = D.f.bond + m;
   // displacement as double-FP32 from the (hi, lo) coordinates
   FF dv[3];
 #pragma unroll
@@ -384,13 +341,13 @@ __device__ inline float bond_mixed(const Dev& D, const BeadPos& x, int m, Contri
   FF r2f = ff_mul(dv[0], dv[0]);
   r2f = ff_add(r2f, ff_mul(dv[1], dv[1]));
   r2f = ff_add(r2f, ff_mul(dv[2], dv[2]));
-  const FF r0sq = ff_of(__ldg(ser + 1));
+  const FF r0sq = ff_of(__ldg(ser + st));
   const float r2 = r2f.hi;
   const float r = sqrtf(r2);
-  const float r0 = D.f.vbond[3 * m];
+  const float r0 = __ldg(v);
   const FF d2 = ff_add(r2f, FF{-r0sq.hi, -r0sq.lo});
   const float dr = (d2.hi + d2.lo) / (r + r0);  // r - r0
-  const float kij = D.f.vbond[3 * m + 1], aai = D.f.vbond[3 * m + 2];
+  const float kij = __ldg(v + st), aai = __ldg(v + 2 * st);
   const float lg = -0.5f * aai * log1pf(dr / r0);
   const float omu = -expm1f(lg);  // 1 - u
   const float u = 1.0f - omu;
@@ -399,12 +356,12 @@ __device__ inline float bond_mixed(const Dev& D, const BeadPos& x, int m, Contri
   c.a[0] = i;
   c.a[1] = j;
   const FF t = ff_add(ff_mul(r2f, ff_of(__ldg(ser))), FF{-1.0f, 0.0f});
-  if (__ldg(ser + 2).x != 0.0f && fabsf(t.hi) <= (float)kBondSerMaxT) {
+  if (__ldg(ser + 2 * st).x != 0.0f && fabsf(t.hi) <= (float)kBondSerMaxT) {
     // 1 / kBondSerMaxT = 20/9 as a double-FP32 constant
     const FF xs = ff_mul(t, FF{2.22222232818603515625f, -1.0596381372e-07f});
-    FF h = ff_of(__ldg(ser + 3 + kBondPoly - 1));
+    FF h = ff_of(__ldg(ser + (3 + kBondPoly - 1) * st));
 #pragma unroll
-    for (int k = kBondPoly - 2; k >= 0; --k) h = ff_add(ff_mul(h, xs), ff_of(__ldg(ser + 3 + k)));
+    for (int k = kBondPoly - 2; k >= 0; --k) h = ff_add(ff_mul(h, xs), ff_of(__ldg(ser + (3 + k) * st)));
     const FF f = ff_mul(t, h);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -430,10 +387,11 @@ __device__ inline float bond_mixed(const Dev& D, const BeadPos& x, int m, Contri
 // Angle bend with abdamp damping (src/ff_eg.f90:167-299), mixed form.
 __device__ inline float angle_mixed(const Dev& D, const BeadPos& x, int m, Contrib<float>& c) {
   using F = float;
-  const Tables<float>& T = D.f;
-  const int j = D.angl[3 * m], i = D.angl[3 * m + 1], k = D.angl[3 * m + 2];
-  const auto* v = &T.vangl[kVAngl * m];
-  const F c0 = v[0], kijk = v[1], cc0 = v[2];
+  const uint2 at = __ldg(D.angl + m);
+  const int i = lo16(at.x), j = hi16(at.x), k = (int)at.y, st = D.st[1];
+  const float* v = D.f.angl + m;
+  const F c0 = __ldg(v), kijk = __ldg(v + st), cc0 = __ldg(v + 2 * st);
+  const bool linear = __ldg(v + 3 * st) != 0.f;
   F vab[3], vcb[3], vp[3];
   disp<F>(x, i, j, vab);
   disp<F>(x, k, j, vcb);
@@ -448,13 +406,13 @@ __device__ inline float angle_mixed(const Dev& D, const BeadPos& x, int m, Contr
   // harmonic-cosine form as sqrt((1 - c)(1 + c)), free of cancellation away
   // from c = +-1 (where the linear form is used)
   F theta = F(0);
-  if (v[3] != F(0)) theta = acosf(cosa);
+  if (linear) theta = acosf(cosa);
   F dampij, damp2ij, dampjk, damp2jk;
-  abdamp(T.rad[i], T.rad[j], rab2, dampij, damp2ij);
-  abdamp(T.rad[k], T.rad[j], rcb2, dampjk, damp2jk);
+  abdamp(__ldg(v + 4 * st), rab2, dampij, damp2ij);
+  abdamp(__ldg(v + 5 * st), rcb2, dampjk, damp2jk);
   const F damp = dampij * dampjk;
   F ea, deddt;
-  if (v[3] != F(0)) {  // linear reference angle: harmonic in theta
+  if (linear) {  // linear reference angle: harmonic in theta
     const F dt = theta - c0;
     ea = kijk * (dt * dt);
     deddt = F(2) * kijk * dt;
@@ -514,13 +472,13 @@ __device__ inline F tors_virial(const F* vab, const F* vcb, const F* vdc, const 
 // inversions (tors type 2, src/ff_eg.f90:441-618), mixed form.
 __device__ inline float torsion_mixed(const Dev& D, const BeadPos& x, int m, Contrib<float>& c, float* vir = nullptr) {
   using F = float;
-  const Tables<float>& T = D.f;
   const F pi = (F)3.1415926535897932384626433832795029;
   const F pi2 = (F)6.28318530717958623199592693708837;
-  const int i = D.tors[6 * m], j = D.tors[6 * m + 1], k = D.tors[6 * m + 2], l = D.tors[6 * m + 3];
-  const int nt = D.tors[6 * m + 4], type = D.tors[6 * m + 5];
-  const auto* vt = &T.vtors[14 * m];
-  const F phi0 = vt[0];
+  const uint4 at = __ldg(D.tors + m);
+  const int i = lo16(at.x), j = hi16(at.x), k = lo16(at.y), l = hi16(at.y), nt = (int)(at.z & 255u), type = (int)(at.z >> 8);
+  const int st = D.st[2];
+  auto vt = [&](int c) { return __ldg(D.f.tors + c * st + m); };
+  const F phi0 = vt(0);
   F vab[3], vcb[3], vdc[3], dda[3], ddb[3], ddc[3], ddd[3];
   F et, dij, dampij, dampjk, dampX, d2ij, d2jk, d2X;
   c.na = 4;
@@ -532,9 +490,9 @@ __device__ inline float torsion_mixed(const Dev& D, const BeadPos& x, int m, Con
     disp<F>(x, i, j, vab);
     disp<F>(x, j, k, vcb);
     disp<F>(x, k, l, vdc);
-    abdamp(T.rad[i], T.rad[j], dot3(vab, vab), dampij, d2ij);
-    abdamp(T.rad[k], T.rad[j], dot3(vcb, vcb), dampjk, d2jk);
-    abdamp(T.rad[k], T.rad[l], dot3(vdc, vdc), dampX, d2X);
+    abdamp(vt(14), dot3(vab, vab), dampij, d2ij);
+    abdamp(vt(15), dot3(vcb, vcb), dampjk, d2jk);
+    abdamp(vt(16), dot3(vdc, vdc), dampX, d2X);
     // dphidr (src/dphidr.f90): ra = r_j - r_i, rb = r_k - r_j, rc = r_l - r_k
     const F ra[3] = {-vab[0], -vab[1], -vab[2]}, rb[3] = {-vcb[0], -vcb[1], -vcb[2]};
     const F rc[3] = {-vdc[0], -vdc[1], -vdc[2]};
@@ -574,7 +532,7 @@ __device__ inline float torsion_mixed(const Dev& D, const BeadPos& x, int m, Con
     const F ef = erff(phipi);
     const F expo = expf(-(phipi * phipi)) * 0.564189583547756286948f;  // 1/sqrt(pi)
     for (int it = 0; it < nt; ++it) {
-      const F rn = vt[2 + 3 * it], ph = vt[3 + 3 * it], vn = vt[4 + 3 * it];
+      const F rn = vt(2 + 3 * it), ph = vt(3 + 3 * it), vn = vt(4 + 3 * it);
       const F c1 = rn * (phi - phi0) + ph;
       const F c2 = rn * (phi + phi0 - pi2) + ph;
       F x1cos, x2cos, x1sin, x2sin;
@@ -585,9 +543,9 @@ __device__ inline float torsion_mixed(const Dev& D, const BeadPos& x, int m, Con
       dij = dij - expo * e1 - F(0.5) * (F(1) - ef) * vn * x1sin * rn + expo * e2 -
             (F(0.5) + F(0.5) * ef) * vn * x2sin * rn;
     }
-    et = et * vt[1];
+    et = et * vt(1);
     const F damp = dampjk * dampij * dampX;
-    dij = dij * vt[1] * damp;
+    dij = dij * vt(1) * damp;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const F t1 = et * d2ij * dampjk * dampX * vab[d];
@@ -605,9 +563,9 @@ __device__ inline float torsion_mixed(const Dev& D, const BeadPos& x, int m, Con
   disp<F>(x, j, i, vab);
   disp<F>(x, j, k, vcb);
   disp<F>(x, j, l, vdc);
-  abdamp(T.rad[i], T.rad[j], dot3(vab, vab), dampij, d2ij);
-  abdamp(T.rad[k], T.rad[j], dot3(vcb, vcb), dampjk, d2jk);
-  abdamp(T.rad[j], T.rad[l], dot3(vdc, vdc), dampX, d2X);
+  abdamp(vt(14), dot3(vab, vab), dampij, d2ij);
+  abdamp(vt(15), dot3(vcb, vcb), dampjk, d2jk);
+  abdamp(vt(16), dot3(vdc, vdc), dampX, d2X);
   const F re[3] = {-vab[0], -vab[1], -vab[2]};  // r_i - r_j
   const F rd[3] = {-vcb[0], -vcb[1], -vcb[2]};  // r_k - r_j
   F rv[3];
@@ -647,13 +605,13 @@ __device__ inline float torsion_mixed(const Dev& D, const BeadPos& x, int m, Con
     // which the large inversion barriers of planar centres (tens of Eh)
     // turn into force errors of 1e-6
     const float h = 0.5f * (om - phi0), sh = sinf(h);
-    if (vt[2] > 1e-6f) {
-      et = 2.f * sh * sh * vt[1];
-      dij = sinf(om - phi0) * vt[1] * damp;
+    if (vt(2) > 1e-6f) {
+      et = 2.f * sh * sh * vt(1);
+      dij = sinf(om - phi0) * vt(1) * damp;
     } else {
       const float dd = -2.f * sinf(0.5f * (om + phi0)) * sh;  // cos(om) - cos(phi0)
-      et = vt[1] * (dd * dd);
-      dij = -2.f * vt[1] * sinf(om) * dd * damp;
+      et = vt(1) * (dd * dd);
+      dij = -2.f * vt(1) * sinf(om) * dd * damp;
     }
   }
 #pragma unroll
@@ -668,22 +626,6 @@ __device__ inline float torsion_mixed(const Dev& D, const BeadPos& x, int m, Con
   }
   if (vir) *vir = tors_virial(vab, vcb, vdc, c);
   return et * damp;
-}
-
-// kVPair parameters of one pair with 16-byte loads (rows are 32 / 64 bytes).
-__device__ inline void load_pair_params(const float* p, float* v) {
-  const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-  v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-__device__ inline void load_pair_params(const double* p, double* v) {
-  const double2* q = reinterpret_cast<const double2*>(p);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const double2 t = __ldg(q + k);
-    v[2 * k] = t.x;
-    v[2 * k + 1] = t.y;
-  }
 }
 
 }  // namespace qmdff
@@ -713,31 +655,32 @@ __device__ inline float ex2_approx(float x) {
 }
 
 // One NCI pair in the mixed form: the formulas of pair_plain with the
-// per-pair constants folded into the table Dev::fpair (R0^6 and R0^8 of the
-// BJ damping, eps2 into the C6 / C8 and repulsion prefactors, alpha log2(e)
-// for a base-2 exponential).  The pair forces are ~1 % of the valence
+// constants folded (R0^6 and R0^8 of the BJ damping, eps2 into the C6 and
+// repulsion prefactors, alpha log2(e) for a base-2 exponential).  The pair forces are ~1 % of the valence
 // forces, so hardware approximations stay far below the form's error budget.
-__device__ inline float pair_mixed_v(const Dev& D, const BeadPos& x, int i1, int i2, const float (&v)[kVPair],
-                                     Contrib<float>& c, float* vir = nullptr) {
+__device__ inline float pair_mixed(const Dev& D, const BeadPos& x, uint4 pr, Contrib<float>& c, float* vir) {
+  const int i1 = lo16(pr.x), i2 = hi16(pr.x);
+  const float4 ca = __ldg(D.pclass + 2 * pr.y), cb = __ldg(D.pclass + 2 * pr.y + 1);
+  const float c6 = __uint_as_float(pr.z), qq = __uint_as_float(pr.w);
   float vab[3];
   disp<float>(x, i1, i2, vab);
   const float r2 = dot3(vab, vab);
   const float oner = rsqrt_approx(r2), r = r2 * oner, ir2 = oner * oner;
   const float r4 = r2 * r2, r6 = r4 * r2;
-  const float it6 = rcp_approx(r6 + v[0]), it8 = rcp_approx(r6 * r2 + v[1]);
-  const float d6 = v[2] * it6, d8 = v[3] * it8;
+  const float it6 = rcp_approx(r6 + ca.x), it8 = rcp_approx(r6 * r2 + ca.y);
+  const float d6 = c6 * it6, d8 = c6 * ca.z * it8;
   const bool vdw = !x.pbc || !(r > D.fvdw_cut);
   float e = vdw ? -(d6 + d8) : 0.0f;
   float drij = vdw ? 6.0f * d6 * (r4 * it6) + 8.0f * d8 * (r6 * it8) : 0.0f;
   if (vdw && r < 25.0f) {
-    const float t = v[4] * ex2_approx(-v[5] * r) * oner;
+    const float t = ca.w * ex2_approx(-cb.x * r) * oner;
     e += t;
-    drij = fmaf(-t * ir2, fmaf(v[7], r, 1.0f), drij);
+    drij = fmaf(-t * ir2, fmaf(cb.y, r, 1.0f), drij);
   }
   if (!(r > D.fcoul_cut)) {
     float e0;
-    if (D.zahn) e0 = v[6] * ((q_erfc<float>(D.fzahn_a * r) * oner) - D.fzahn_par * (r - D.fcoul_cut));
-    else e0 = v[6] * oner;
+    if (D.zahn) e0 = qq * ((q_erfc<float>(D.fzahn_a * r) * oner) - D.fzahn_par * (r - D.fcoul_cut));
+    else e0 = qq * oner;
     e += e0;
     drij = fmaf(-e0, ir2, drij);
   }
@@ -935,8 +878,6 @@ __device__ inline double term(const Dev& D, const BeadPos& x, int m, Contrib<dou
   else return hb_term<double>(D, D.d, x, m, c);
 }
 
-// All batches of one term kind (NA atoms per term): each lane evaluates its
-// slot's term, then the warp scatters colour by colour.
 // The virial trace of one term as the reference accumulates `vir_ten` for
 // NpT: bonds (src/ff_eg.f90:133-150) rbond.g_i, rbond = r_i - r_j; angles
 // (:270-281) vab.g_i + vcb.g_k about the centre j; torsions (:317-320,
@@ -951,7 +892,7 @@ __device__ inline double term(const Dev& D, const BeadPos& x, int m, Contrib<dou
 // terms' own.  Mixed-form bonds carry g_i as (hi, lo) in g[0] and g[2].
 template <class F, int KIND>
 __device__ inline F term_virial(const Dev& D, const BeadPos& X, int m, const Contrib<F>& c) {
-  F u[3], v[3], w[3];
+  F u[3], v[3];
   if constexpr (KIND == 0) {
     disp<F>(X, c.a[0], c.a[1], u);
     F g[3];
@@ -962,21 +903,6 @@ __device__ inline F term_virial(const Dev& D, const BeadPos& X, int m, const Con
     disp<F>(X, c.a[0], c.a[1], u);
     disp<F>(X, c.a[2], c.a[1], v);
     return dot3(u, c.g[0]) + dot3(v, c.g[2]);
-  } else if constexpr (KIND == 2) {
-    const int i = c.a[0], j = c.a[1], k = c.a[2], l = c.a[3];
-    if (D.tors[6 * m + 5] != 2) {
-      disp<F>(X, i, j, u);
-      disp<F>(X, j, k, v);
-      disp<F>(X, k, l, w);
-    } else {
-      disp<F>(X, j, i, u);
-      disp<F>(X, j, k, v);
-      disp<F>(X, j, l, w);
-    }
-    F gkl[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) gkl[d] = c.g[2][d] + c.g[3][d];
-    return dot3(u, c.g[0]) + dot3(v, gkl) + dot3(w, c.g[3]);
   } else if constexpr (KIND == 3) {
     disp<F>(X, c.a[0], c.a[1], u);
     return dot3(u, c.g[0]);
@@ -993,113 +919,151 @@ __device__ inline F term_virial(const Dev& D, const BeadPos& X, int m, const Con
 // box), kNpt (each trajectory's box from Dev::tbox, and the virial).
 constexpr int kFree = 0, kBox = 1, kNpt = 2;
 
-// Warps per bead of the FP64 forms.  An FP64 instruction holds its scheduler's
-// pipe 64 cycles and four warps fill an SM's four, so a bead is spread over them:
-// a small batch then takes a quarter of the time, a large one as long as with a
-// warp per bead.  Each warp sums into its own gradient; the four are added in
-// order.  With the terms of qmdff_plain.cuh, whole calls: the adjoint of 16 x 16
-// beads of C20H42 over 20 steps 47.4 -> 12.2 ms, C13H28 100 x 48, four steps 4.82 ->
-// 2.29 ms.
-constexpr int kTeam = 4;
-
-// the first batch of number b0 or more that falls to the warp
-template <int W>
-__device__ __forceinline__ int team_first(int b0, int warp) {
-  return W == 1 ? b0 : b0 + ((warp - b0) & (W - 1));
+// Buffer value of a list entry.
+__device__ __forceinline__ double signed_value(const double* buf, unsigned e) {
+  const double v = buf[e & (kNegate - 1)];
+  return __hiloint2double(__double2hiint(v) ^ (int)((e & kNegate) << 16), __double2loint(v));
 }
 
-// W warps share a bead: this one takes the batches whose number is warp modulo W.
-template <bool MIXED, int KIND, int NA, int MODE, int W>
-__device__ inline void kind_batches(const Dev& D, const BeadPos& X,
-                                    Grad<typename std::conditional<MIXED, float, double>::type>& G,
-                                    typename std::conditional<MIXED, float, double>::type& es,
-                                    typename std::conditional<MIXED, float, double>::type& ec,
-                                    typename std::conditional<MIXED, float, double>::type& wv, int warp, int lane) {
-  using F = typename std::conditional<MIXED, float, double>::type;
-  const Schedule& S = D.sched[MIXED ? 1 : 0];
-  const int b0 = S.boff[KIND], b1 = b0 + S.nb[KIND];
-  const bool distinct = D.distinct != 0;
-  for (int b = team_first<W>(b0, warp); b < b1; b += W) {
-    const int m = S.slot[32 * b + lane];
-    const int col = S.color[32 * b + lane];
-    const int ncol = S.ncol[b];
-    Contrib<F> c;
-    if (m >= 0) {
-      F v, w = F(0);
-      if constexpr (MODE == kNpt && KIND == 2) v = term<KIND>(D, X, m, c, &w);  // the torsion's own vectors
-      else v = term<KIND>(D, X, m, c, (F*)nullptr);
-      if constexpr (MODE == kNpt) {
-        if constexpr (KIND != 2) w = term_virial<F, KIND>(D, X, m, c);
-        wv += w;
-      }
-      if constexpr (MIXED) {  // compensated FP32 lane sum
-        const F t = es + v;
-        ec += (fabs(es) >= fabs(v)) ? ((es - t) + v) : ((v - t) + es);
-        es = t;
-      } else {
-        es += v;
-      }
-    }
-    for (int k = 0; k < ncol; ++k) {
-      if (m >= 0 && col == k) {
-        if constexpr (MIXED && KIND == 3) scatter_pair<NA>(c, G);
-        else if constexpr (MIXED && KIND == 0) scatter_bond(c, G);
-        else scatter<NA>(c, G, distinct);
-      }
-      __syncwarp();
-    }
+// Warps per bead of the FP64 forms.  An FP64 instruction holds its scheduler's
+// pipe 64 cycles, so four warps could fill an SM's four pipes, and two per pipe hide
+// the loads and the barriers; a bead is spread over eight: a small batch then takes an
+// eighth of the time, a large one as long as with a warp per bead.  With the terms of qmdff_plain.cuh, whole calls: the adjoint of 16 x 16
+// beads of C20H42 over 20 steps 47.4 -> 11.3 ms, C13H28 100 x 48, four steps 4.82 ->
+// 1.82 ms.
+constexpr int kTeam = 8;
+
+// The segment's values of one term at its slot i.
+template <bool MIXED, int KIND, class G>
+__device__ __forceinline__ void put_term(G* buf, int i, const Contrib<G>& c) {
+  constexpr int C = segment_terms(MIXED, KIND), NA = KIND == 1 || KIND == 4 ? 3 : KIND == 2 ? 4 : 1;
+#pragma unroll
+  for (int a = 0; a < NA; ++a)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) buf[(3 * a + d) * C + i] = c.g[a][d];
+  if constexpr (MIXED && KIND == 0) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) buf[(3 + d) * C + i] = c.g[2][d];
   }
 }
 
-// Mixed-form NCI pairs: every batch is one matching (one colour), so each
-// lane scatters right after its term; the next batch's slot, atom pair and
-// parameters are loaded before the current batch's arithmetic, so the L1
-// latency of the term tables overlaps the work.
-template <int MODE>
-__device__ inline void pair_batches_mixed(const Dev& D, const BeadPos& X, Grad<float>& G, float& es, float& ec,
-                                          float& wv, int lane) {
+// Sums of a segment's gather, rounds r0, r0 + step, ...: list value x onto
+// coordinate a by add(a, list).
+template <class Sum>
+__device__ __forceinline__ void gather(const Schedule& S, int4 sg, int r0, int step, int lane, Sum sum) {
+  for (int r = sg.z + r0; r < sg.z + sg.w; r += step) {
+    const int2 rd = __ldg(S.round + r);
+    const int a = S.dst[32 * r + lane];
+    if (a != kNoDst) sum(a, S.ent + rd.x + lane, rd.y);
+  }
+}
+
+// All segments of one term kind, mixed form, by one warp: compensated sums.
+template <int KIND, int MODE>
+__device__ inline void kind_segments(const Dev& D, const BeadPos& X, float* buf, float2* sk, float& es, float& ec,
+                                     float& wv, int lane) {
   const Schedule& S = D.sched[1];
-  const int b0 = S.boff[3], nb = S.nb[3];
-  if (nb <= 0) return;
-  int m = S.slot[32 * b0 + lane];
-  int2 ij = m >= 0 ? __ldg(reinterpret_cast<const int2*>(D.pair) + m) : make_int2(0, 0);
-  float4 pa = m >= 0 ? __ldg(reinterpret_cast<const float4*>(&D.fpair[kVPair * m])) : make_float4(0, 0, 0, 0);
-  float4 pb = m >= 0 ? __ldg(reinterpret_cast<const float4*>(&D.fpair[kVPair * m]) + 1) : make_float4(0, 0, 0, 0);
-  for (int b = b0; b < b0 + nb; ++b) {
-    const int mc = m;
-    const int2 ijc = ij;
-    const float v[kVPair] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
-    if (b + 1 < b0 + nb) {
-      m = S.slot[32 * (b + 1) + lane];
-      if (m >= 0) {
-        ij = __ldg(reinterpret_cast<const int2*>(D.pair) + m);
-        pa = __ldg(reinterpret_cast<const float4*>(&D.fpair[kVPair * m]));
-        pb = __ldg(reinterpret_cast<const float4*>(&D.fpair[kVPair * m]) + 1);
+  for (int sgi = S.seg0[KIND]; sgi < S.seg1[KIND]; ++sgi) {
+    const int4 sg = __ldg(S.seg + sgi);
+    for (int i = lane; i < sg.y; i += 32) {
+      const int m = sg.x + i;
+      Contrib<float> c;
+      float w = 0.f;
+      float v;
+      if constexpr (MODE == kNpt && KIND == 2) v = term<KIND>(D, X, m, c, &w);  // the torsion's own vectors
+      else v = term<KIND>(D, X, m, c, (float*)nullptr);
+      if constexpr (MODE == kNpt) {
+        if constexpr (KIND != 2) w = term_virial<float, KIND>(D, X, m, c);
+        wv += w;
       }
+      const float t = es + v;
+      ec += (fabsf(es) >= fabsf(v)) ? ((es - t) + v) : ((v - t) + es);
+      es = t;
+      put_term<true, KIND>(buf, i, c);
     }
-    if (mc >= 0) {
+    __syncwarp();
+    gather(S, sg, 0, 1, lane, [&](int a, const unsigned short* l, int n) {
+      float2 k = sk[a];
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) {
+        const unsigned e = __ldg(l + 32 * j);
+        const float v = __uint_as_float(__float_as_uint(buf[e & (kNegate - 1)]) ^ ((e & kNegate) << 16));
+        const float t = k.x + v, z = t - k.x;
+        k.y += (k.x - (t - z)) + (v - z);
+        k.x = t;
+      }
+      sk[a] = k;
+    });
+    __syncwarp();
+  }
+}
+
+// ... FP64 form, by a team of warps.
+template <int KIND, int MODE>
+__device__ inline void kind_segments(const Dev& D, const BeadPos& X, double* buf, double* g, double& es, double& wv) {
+  const Schedule& S = D.sched[0];
+  for (int sgi = S.seg0[KIND]; sgi < S.seg1[KIND]; ++sgi) {
+    const int4 sg = __ldg(S.seg + sgi);
+    for (int i = threadIdx.x; i < sg.y; i += kTeam * 32) {
+      const int m = sg.x + i;
+      Contrib<double> c;
+      double w = 0.0;
+      if constexpr (MODE == kNpt && KIND == 2) es += term<KIND>(D, X, m, c, &w);
+      else es += term<KIND>(D, X, m, c, (double*)nullptr);
+      if constexpr (MODE == kNpt) {
+        if constexpr (KIND != 2) w = term_virial<double, KIND>(D, X, m, c);
+        wv += w;
+      }
+      put_term<false, KIND>(buf, i, c);
+    }
+    __syncthreads();
+    gather(S, sg, threadIdx.x >> 5, kTeam, threadIdx.x & 31, [&](int a, const unsigned short* l, int n) {
+      double v = g[a];
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) v += signed_value(buf, __ldg(l + 32 * j));
+      g[a] = v;
+    });
+    __syncthreads();
+  }
+}
+
+// Mixed-form NCI pairs: every batch is one matching, so each lane adds its pair's
+// gradient right after the term; the next batch's table row is loaded before
+// the current batch's arithmetic, so its latency overlaps the work.
+template <int MODE>
+__device__ inline void pair_batches_mixed(const Dev& D, const BeadPos& X, float* pr, float& es, float& ec,
+                                          float& wv, int lane) {
+  const int nb = D.sched[1].npair;
+  if (nb <= 0) return;
+  uint4 next = __ldg(D.fpair + lane);
+  for (int b = 0; b < nb; ++b) {
+    const uint4 row = next;
+    if (b + 1 < nb) next = __ldg(D.fpair + 32 * (b + 1) + lane);
+    if (row.y != kNoPair) {
       Contrib<float> c;
       float w = 0.0f;
-      const float e = pair_mixed_v(D, X, ijc.x, ijc.y, v, c, MODE == kNpt ? &w : nullptr);
+      const float e = pair_mixed(D, X, row, c, MODE == kNpt ? &w : nullptr);
       const float t = es + e;
       ec += (fabsf(es) >= fabsf(e)) ? ((es - t) + e) : ((e - t) + es);
       es = t;
       if constexpr (MODE == kNpt) wv += w;
-      scatter_pair<2>(c, G);
+      scatter_pair(c, pr);
     }
     __syncwarp();
   }
 }
 
-// Shared memory of a mixed-form warp (bytes): coordinates (3n doubles), the FP32
-// split (hi, lo) (3n float pairs) and the gradient ((sum, compensation) float
-// pairs and the 3n floats of the pair sum), in whole 16-byte units: the warps'
-// regions follow one another, and 84 n bytes are no multiple of a double for odd n.
+// Shared memory of a mixed-form warp (bytes): the coordinates' FP32 split (hi, lo)
+// (3n float pairs), the gradient ((sum, compensation) float pairs and
+// the 3n floats of the pair sum) and the buffer with its zero, in whole 16-byte
+// units: the warps' regions follow one another.
 __host__ __device__ inline size_t warp_smem_bytes(int n) {
-  return ((size_t)3 * n * (8 + 4 + 4 + 8 + 4) + 15) / 16 * 16;
+  return ((size_t)3 * n * (4 + 4 + 8 + 4) + (buffer_values(true) + 1) * 4 + 15) / 16 * 16;
 }
-// ... of an FP64 team: coordinates, kTeam gradients, the warps' energies and virials
-__host__ __device__ inline size_t team_smem_bytes(int n) { return ((size_t)3 * n * (1 + kTeam) + 2 * kTeam) * 8; }
+// ... of an FP64 team: coordinates, gradient, buffer and zero, the warps' energies and virials
+__host__ __device__ inline size_t team_smem_bytes(int n) {
+  return ((size_t)3 * n * 2 + buffer_values(false) + 1 + 2 * kTeam) * 8;
+}
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -1122,40 +1086,37 @@ __device__ inline const PBox* launch_box(const Dev& D, size_t bead, PBox& tb) {
 }
 
 // Energy (with E_zero) and gradient of one bead by one warp, mixed form.
-// ws: the warp's shared memory with the bead's FP64 coordinates in its first
-// 3n doubles; gout, gout2: the gradient destinations (gout2 = gout: one).  Returns the energy on every lane.
+// ws: the warp's shared memory; x: the bead's coordinates; gout, gout2: the gradient destinations (gout2 = gout: one).  Returns the energy on every lane.
 // MODE (kFree, kBox, kNpt): with kNpt the bead's trajectory box from D.tbox
 // and the virial trace into D.vir (rows bead and twin).
 template <int MODE = kFree>
-__device__ inline double warp_egrad(const Dev& D, double* ws, double* gout, double* gout2, int lane, size_t bead,
-                                    size_t twin) {
+__device__ inline double warp_egrad(const Dev& D, void* ws, const double* x, double* gout, double* gout2, int lane,
+                                    size_t bead, size_t twin) {
   const int n3 = 3 * D.n;
-  double* xs = ws;
-  float2* hl = (float2*)(ws + n3);
+  float2* hl = (float2*)ws;
   PBox tb;
-  const BeadPos X{xs, hl, nullptr, launch_box<MODE>(D, bead, tb)};
-  Grad<float> G;
+  const BeadPos X{x, hl, nullptr, launch_box<MODE>(D, bead, tb)};
+  float2* sk = hl + n3;
+  float* pr = (float*)(sk + n3);
+  float* buf = pr + n3;
   for (int a = lane; a < n3; a += 32) {
-    const double v = xs[a];
+    const double v = x[a];
     const float h = __double2float_rn(v);
     hl[a] = make_float2(h, __double2float_rn(v - (double)h));
+    sk[a] = make_float2(0.f, 0.f);
+    pr[a] = 0.f;
   }
-  G.sk = hl + n3;
-  G.pr = (float*)(G.sk + n3);
-  for (int a = lane; a < n3; a += 32) {
-    G.sk[a] = make_float2(0.f, 0.f);
-    G.pr[a] = 0.f;
-  }
+  if (lane == 0) buf[buffer_values(true)] = 0.f;
   __syncwarp();
   float es = 0.f, ec = 0.f;  // compensated lane sum of term energies
   float wv = 0.f;            // lane sum of the terms' virial traces (NpT)
-  kind_batches<true, 0, 2, MODE, 1>(D, X, G, es, ec, wv, 0, lane);
-  kind_batches<true, 1, 3, MODE, 1>(D, X, G, es, ec, wv, 0, lane);
-  kind_batches<true, 2, 4, MODE, 1>(D, X, G, es, ec, wv, 0, lane);
-  pair_batches_mixed<MODE>(D, X, G, es, ec, wv, lane);
-  kind_batches<true, 4, 3, MODE, 1>(D, X, G, es, ec, wv, 0, lane);
+  kind_segments<0, MODE>(D, X, buf, sk, es, ec, wv, lane);
+  kind_segments<1, MODE>(D, X, buf, sk, es, ec, wv, lane);
+  kind_segments<2, MODE>(D, X, buf, sk, es, ec, wv, lane);
+  pair_batches_mixed<MODE>(D, X, pr, es, ec, wv, lane);
+  kind_segments<4, MODE>(D, X, buf, sk, es, ec, wv, lane);
   for (int a = lane; a < n3; a += 32) {
-    const double v = G.get(a);
+    const double v = ((double)sk[a].x + (double)sk[a].y) + (double)pr[a];
     gout[a] = v;
     if (gout2 != gout) gout2[a] = v;
   }
@@ -1178,16 +1139,17 @@ __device__ inline double team_egrad(const Dev& D, double* ws, double* gout, doub
   PBox tb;
   const BeadPos X{ws, nullptr, nullptr, launch_box<MODE>(D, bead, tb)};
   double* g = ws + n3;
-  double* red = g + kTeam * n3;
-  Grad<double> G{g + warp * n3};
-  for (int a = tid; a < kTeam * n3; a += kTeam * 32) g[a] = 0.0;
+  double* buf = g + n3;
+  double* red = buf + buffer_values(false) + 1;
+  for (int a = tid; a < n3; a += kTeam * 32) g[a] = 0.0;
+  if (tid == 0) buf[buffer_values(false)] = 0.0;
   __syncthreads();
-  double es = 0.0, ec = 0.0, wv = 0.0;
-  kind_batches<false, 0, 2, MODE, kTeam>(D, X, G, es, ec, wv, warp, lane);
-  kind_batches<false, 1, 3, MODE, kTeam>(D, X, G, es, ec, wv, warp, lane);
-  kind_batches<false, 2, 4, MODE, kTeam>(D, X, G, es, ec, wv, warp, lane);
-  kind_batches<false, 3, 2, MODE, kTeam>(D, X, G, es, ec, wv, warp, lane);
-  kind_batches<false, 4, 3, MODE, kTeam>(D, X, G, es, ec, wv, warp, lane);
+  double es = 0.0, wv = 0.0;
+  kind_segments<0, MODE>(D, X, buf, g, es, wv);
+  kind_segments<1, MODE>(D, X, buf, g, es, wv);
+  kind_segments<2, MODE>(D, X, buf, g, es, wv);
+  kind_segments<3, MODE>(D, X, buf, g, es, wv);
+  kind_segments<4, MODE>(D, X, buf, g, es, wv);
   es = warp_sum(es);
   if constexpr (MODE == kNpt) wv = warp_sum(wv);
   if (lane == 0) {
@@ -1196,11 +1158,8 @@ __device__ inline double team_egrad(const Dev& D, double* ws, double* gout, doub
   }
   __syncthreads();
   for (int a = tid; a < n3; a += kTeam * 32) {
-    double v = g[a];
-#pragma unroll
-    for (int w = 1; w < kTeam; ++w) v += g[w * n3 + a];
-    gout[a] = v;
-    if (gout2 != gout) gout2[a] = v;
+    gout[a] = g[a];
+    if (gout2 != gout) gout2[a] = g[a];
   }
   double e = 0.0, w = 0.0;
 #pragma unroll
@@ -1221,48 +1180,48 @@ __device__ inline double team_egrad(const Dev& D, double* ws, double* gout, doub
 // NCI pairs).
 // ---------------------------------------------------------------------------
 
-// Gradient value and tangent (H w) of one bead in shared memory.
-struct GradDual {
-  double* g;
-  double* h;
-  __device__ inline void add(int i, const Dual& v) {
-    g[i] += v.v;
-    h[i] += v.d;
-  }
-};
-
-// The plain form's schedule (sched[0]) with dual coordinates, by a team of warps.
-template <int KIND, int NA>
-__device__ inline void kind_batches_dual(const Dev& D, const BeadPos& X, GradDual& G, Dual& es, int warp, int lane) {
+// All segments of one term kind with dual coordinates: values in buf, tangents behind.
+template <int KIND>
+__device__ inline void kind_segments_dual(const Dev& D, const BeadPos& X, double* buf, double* g, double* h, Dual& es) {
+  constexpr int B = buffer_values(false) + 1, C = segment_terms(false, KIND), NA = KIND == 1 ? 3 : KIND == 2 ? 4 : 1;
   const Schedule& S = D.sched[0];
-  const int b0 = S.boff[KIND], b1 = b0 + S.nb[KIND];
-  for (int b = team_first<kTeam>(b0, warp); b < b1; b += kTeam) {
-    const int m = S.slot[32 * b + lane];
-    const int col = S.color[32 * b + lane];
-    const int ncol = S.ncol[b];
-    Contrib<Dual> c;
-    if (m >= 0) {
+  for (int sgi = S.seg0[KIND]; sgi < S.seg1[KIND]; ++sgi) {
+    const int4 sg = __ldg(S.seg + sgi);
+    for (int i = threadIdx.x; i < sg.y; i += kTeam * 32) {
+      const int m = sg.x + i;
+      Contrib<Dual> c;
       if constexpr (KIND == 0) es += bond_plain<Dual>(D, D.d, X, m, c);
       else if constexpr (KIND == 1) es += angle_plain<Dual>(D, D.d, X, m, c);
       else if constexpr (KIND == 2) es += torsion_plain<Dual>(D, D.d, X, m, c);
       else es += pair_plain<Dual>(D, D.d, X, m, c);
+#pragma unroll
+      for (int a = 0; a < NA; ++a)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          buf[(3 * a + d) * C + i] = c.g[a][d].v;
+          buf[B + (3 * a + d) * C + i] = c.g[a][d].d;
+        }
     }
-    for (int k = 0; k < ncol; ++k) {
-      if (m >= 0 && col == k) {
-#pragma unroll
-        for (int a = 0; a < NA; ++a)
-#pragma unroll
-          for (int d = 0; d < 3; ++d) G.add(3 * c.a[a] + d, c.g[a][d]);
+    __syncthreads();
+    gather(S, sg, threadIdx.x >> 5, kTeam, threadIdx.x & 31, [&](int a, const unsigned short* l, int n) {
+      double v = g[a], t = h[a];
+#pragma unroll 4
+      for (int j = 0; j < n; ++j) {
+        const unsigned e = __ldg(l + 32 * j);
+        v += signed_value(buf, e);
+        t += signed_value(buf + B, e);
       }
-      __syncwarp();
-    }
+      g[a] = v;
+      h[a] = t;
+    });
+    __syncthreads();
   }
 }
 
-// Shared memory of team_hvp: x, w, kTeam gradients and H w (3n doubles each), the
-// warps' energies and derivatives.
+// Shared memory of team_hvp: x, w, gradient, H w (3n doubles each), the buffer and
+// zero for values and tangents, the warps' energies and derivatives.
 __host__ __device__ inline size_t team_hvp_smem_bytes(int n) {
-  return ((size_t)3 * n * (2 + 2 * kTeam) + 2 * kTeam) * 8;
+  return ((size_t)3 * n * 4 + 2 * (buffer_values(false) + 1) + 2 * kTeam) * 8;
 }
 
 // Energy (with E_zero), gradient and Hessian-vector product H w of one bead
@@ -1273,19 +1232,20 @@ __device__ inline double team_hvp(const Dev& D, double* ws, double* gout, double
   const int n3 = 3 * D.n, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   double* w = ws + n3;
   double* g = w + n3;
-  double* h = g + kTeam * n3;
-  double* red = h + kTeam * n3;
-  GradDual G{g + warp * n3, h + warp * n3};
-  for (int a = tid; a < 2 * kTeam * n3; a += kTeam * 32) g[a] = 0.0;
+  double* h = g + n3;
+  double* buf = h + n3;
+  double* red = buf + 2 * (buffer_values(false) + 1);
+  for (int a = tid; a < 2 * n3; a += kTeam * 32) g[a] = 0.0;
+  if (tid < 2) buf[tid * (buffer_values(false) + 1) + buffer_values(false)] = 0.0;
   __syncthreads();
   PBox tb;
   if (D.periodic) tb = D.box;
   const BeadPos X{ws, nullptr, w, D.periodic ? &tb : nullptr};
   Dual es(0.0);
-  kind_batches_dual<0, 2>(D, X, G, es, warp, lane);
-  kind_batches_dual<1, 3>(D, X, G, es, warp, lane);
-  kind_batches_dual<2, 4>(D, X, G, es, warp, lane);
-  kind_batches_dual<3, 2>(D, X, G, es, warp, lane);
+  kind_segments_dual<0>(D, X, buf, g, h, es);
+  kind_segments_dual<1>(D, X, buf, g, h, es);
+  kind_segments_dual<2>(D, X, buf, g, h, es);
+  kind_segments_dual<3>(D, X, buf, g, h, es);
   const double e1 = warp_sum(es.v), d1 = warp_sum(es.d);
   if (lane == 0) {
     red[warp] = e1;
@@ -1293,14 +1253,8 @@ __device__ inline double team_hvp(const Dev& D, double* ws, double* gout, double
   }
   __syncthreads();
   for (int a = tid; a < n3; a += kTeam * 32) {
-    double gv = g[a], hv = h[a];
-#pragma unroll
-    for (int k = 1; k < kTeam; ++k) {
-      gv += g[k * n3 + a];
-      hv += h[k * n3 + a];
-    }
-    if (gout) gout[a] = gv;
-    hout[a] = hv;
+    if (gout) gout[a] = g[a];
+    hout[a] = h[a];
   }
   double e = 0.0;
   dew = 0.0;
@@ -1313,9 +1267,9 @@ __device__ inline double team_hvp(const Dev& D, double* ws, double* gout, double
 }
 
 // Linear parameters of the force field (the loss gradients of the adjoint are
-// taken with respect to these): bond force constant k (vbond[1]), angle force
-// constant k (vangl[1]), torsion barrier V (vtors[1]) and the NCI pair's
-// Coulomb product qq (vpair[6]: eps1 q_i q_j, or q_i q_j in the Zahn form).
+// taken with respect to these): bond force constant k, angle force
+// constant k, torsion barrier V and the NCI pair's
+// Coulomb product qq ( eps1 q_i q_j, or q_i q_j in the Zahn form).
 // Every term is linear in its parameter, so d/dtheta_t (v . grad E) is v .
 // grad E_t evaluated with theta_t = 1; the tables U hold the parameters with
 // those entries set to 1 (and, for pairs, the eps2 ones to 0: Coulomb only).
@@ -1337,7 +1291,7 @@ __device__ inline void team_vjp_kind(const Dev& D, const Tables<double>& U, cons
     for (int a = 0; a < NA; ++a)
 #pragma unroll
       for (int d = 0; d < 3; ++d) s = fma(vs[3 * c.a[a] + d], c.g[a][d], s);
-    out[m] = alpha * s + beta * e;
+    out[KIND == 2 ? (int)__ldg(D.tors + m).w : m] = alpha * s + beta * e;
   }
 }
 __device__ inline void team_param_vjp(const Dev& D, const Tables<double>& U, const double* xs, const double* vs,

@@ -90,10 +90,9 @@ __device__ inline void p_erf(Dual x, Dual& ef, Dual& ex) {
   ex.d = -x.v * ef.d;
 }
 
-// abdamp (src/abdamp.f90:36-51); the cutoff prefactor is the REAL(4) product 3.0*3.5710642
+// abdamp (src/abdamp.f90:36-51), irc = 1 / rcut
 template <class F>
-__device__ inline void abdamp_plain(double radi, double radj, F r2, F& damp, F& ddamp) {
-  const double s = radi + radj, irc = fx::rcp((double)(3.0f * 3.5710642f) * (s * s));
+__device__ inline void abdamp_plain(double irc, F r2, F& damp, F& ddamp) {
   const F x = r2 * irc;
   damp = p_rcp(1.0 + x * x);
   ddamp = (-4.0 * irc) * (x * (damp * damp));
@@ -103,12 +102,13 @@ __device__ inline void abdamp_plain(double radi, double radj, F r2, F& damp, F& 
 // e = k (1 + (r0/r)^a - 2 (r0/r)^(a/2)).
 template <class F>
 __device__ inline F bond_plain(const Dev& D, const Tables<double>& T, const BeadPos& x, int m, Contrib<F>& c) {
-  const int i = D.bond[2 * m], j = D.bond[2 * m + 1];
+  const unsigned at = __ldg(D.bond + m);
+  const int i = lo16(at), j = hi16(at);
   F rb[3], r, ir;
   disp<F>(x, i, j, rb);
   p_root(dot3(rb, rb), r, ir);
-  const double* v = &T.vbond[3 * m];
-  const double rij = v[0], kij = v[1], aai = v[2];
+  const double* v = T.bond + m;
+  const double rij = __ldg(v), kij = __ldg(v + D.st[0]), aai = __ldg(v + 2 * D.st[0]);
   const F pa2 = p_pow(rij * ir, aai / 2), pa = pa2 * pa2;
   const F fac = (aai * kij) * (pa2 - pa) * (ir * ir);
   c.na = 2;
@@ -125,9 +125,10 @@ __device__ inline F bond_plain(const Dev& D, const Tables<double>& T, const Bead
 // Angle bend with abdamp damping (src/ff_eg.f90:167-299).
 template <class F>
 __device__ inline F angle_plain(const Dev& D, const Tables<double>& T, const BeadPos& x, int m, Contrib<F>& c) {
-  const int j = D.angl[3 * m], i = D.angl[3 * m + 1], k = D.angl[3 * m + 2];
-  const double* v = &T.vangl[kVAngl * m];
-  const double c0 = v[0], kijk = v[1], cc0 = v[2];
+  const uint2 at = __ldg(D.angl + m);
+  const int i = lo16(at.x), j = hi16(at.x), k = (int)at.y, st = D.st[1];
+  const double* v = T.angl + m;
+  const double c0 = __ldg(v), kijk = __ldg(v + st), cc0 = __ldg(v + 2 * st);
   F vab[3], vcb[3], vp[3], al, ial, bl, ibl;
   disp<F>(x, i, j, vab);
   disp<F>(x, k, j, vcb);
@@ -142,11 +143,11 @@ __device__ inline F angle_plain(const Dev& D, const Tables<double>& T, const Bea
   F cosa = (al > 0.0 && bl > 0.0) ? dot3(vab, vcb) * (ial * ibl) : F(0);
   cosa = fmin(F(1), fmax(F(-1), cosa));
   F dampij, damp2ij, dampjk, damp2jk;
-  abdamp_plain<F>(T.rad[i], T.rad[j], rab2, dampij, damp2ij);
-  abdamp_plain<F>(T.rad[k], T.rad[j], rcb2, dampjk, damp2jk);
+  abdamp_plain<F>(__ldg(v + 4 * st), rab2, dampij, damp2ij);
+  abdamp_plain<F>(__ldg(v + 5 * st), rcb2, dampjk, damp2jk);
   const F damp = dampij * dampjk;
   F ea, deddt, sth, is;
-  if (v[3] != 0.0) {  // linear reference angle: harmonic in theta
+  if (__ldg(v + 3 * st) != 0.0) {  // linear reference angle: harmonic in theta
     F theta;
     p_angle(cosa, theta, sth);
     const F dt = theta - c0;
@@ -183,10 +184,11 @@ __device__ inline F torsion_plain(const Dev& D, const Tables<double>& T, const B
                                   F* vir = nullptr) {
   const double pi = 3.1415926535897932384626433832795029;
   const double pi2 = 6.28318530717958623199592693708837;
-  const int i = D.tors[6 * m], j = D.tors[6 * m + 1], k = D.tors[6 * m + 2], l = D.tors[6 * m + 3];
-  const int nt = D.tors[6 * m + 4], type = D.tors[6 * m + 5];
-  const double* vt = &T.vtors[14 * m];
-  const double phi0 = vt[0];
+  const uint4 at = __ldg(D.tors + m);
+  const int i = lo16(at.x), j = hi16(at.x), k = lo16(at.y), l = hi16(at.y), nt = (int)(at.z & 255u), type = (int)(at.z >> 8);
+  const int st = D.st[2];
+  auto vt = [&](int c) { return __ldg(T.tors + c * st + m); };
+  const double phi0 = vt(0);
   F vab[3], vcb[3], vdc[3];
   F et, dij, dampij, dampjk, dampX, d2ij, d2jk, d2X;
   c.na = 4;
@@ -199,9 +201,9 @@ __device__ inline F torsion_plain(const Dev& D, const Tables<double>& T, const B
     disp<F>(x, j, k, vcb);
     disp<F>(x, k, l, vdc);
     const F rcb2 = dot3(vcb, vcb);
-    abdamp_plain<F>(T.rad[i], T.rad[j], dot3(vab, vab), dampij, d2ij);
-    abdamp_plain<F>(T.rad[k], T.rad[j], rcb2, dampjk, d2jk);
-    abdamp_plain<F>(T.rad[k], T.rad[l], dot3(vdc, vdc), dampX, d2X);
+    abdamp_plain<F>(vt(14), dot3(vab, vab), dampij, d2ij);
+    abdamp_plain<F>(vt(15), rcb2, dampjk, d2jk);
+    abdamp_plain<F>(vt(16), dot3(vdc, vdc), dampX, d2X);
     F na[3], nb[3], nan_, ina, nbn, inb, L, iL, phi, sinphi;
     cross(vab, vcb, na);
     cross(vcb, vdc, nb);
@@ -226,7 +228,7 @@ __device__ inline F torsion_plain(const Dev& D, const Tables<double>& T, const B
     et = F(0);
     dij = F(0);
     for (int it = 0; it < nt; ++it) {
-      const double rn = vt[2 + 3 * it], ph = vt[3 + 3 * it], vn = vt[4 + 3 * it];
+      const double rn = vt(2 + 3 * it), ph = vt(3 + 3 * it), vn = vt(4 + 3 * it);
       F s1, c1, s2, c2;
       p_sincos(rn * (phi - phi0) + ph, s1, c1);
       p_sincos(rn * (phi + (phi0 - pi2)) + ph, s2, c2);
@@ -234,9 +236,9 @@ __device__ inline F torsion_plain(const Dev& D, const Tables<double>& T, const B
       et = et + a * (1.0 + c1) + b * (1.0 + c2);
       dij = dij + expo * (vn * (c2 - c1)) - rn * (a * s1 + b * s2);
     }
-    et = et * vt[1];
+    et = et * vt(1);
     const F damp = dampjk * dampij * dampX;
-    dij = dij * (vt[1] * damp);
+    dij = dij * (vt(1) * damp);
     // dphi/dr of the unsigned angle, s = sign(na . rc), rb = -vcb and so on:
     //   dphi/dr_i = -s |rb| na / |na|^2,  dphi/dr_l = s |rb| nb / |nb|^2,
     //   dphi/dr_j = -dphi/dr_i + s (u + v),  dphi/dr_k = -dphi/dr_l - s (u + v),
@@ -269,9 +271,9 @@ __device__ inline F torsion_plain(const Dev& D, const Tables<double>& T, const B
   disp<F>(x, j, i, vab);
   disp<F>(x, j, k, vcb);
   disp<F>(x, j, l, vdc);
-  abdamp_plain<F>(T.rad[i], T.rad[j], dot3(vab, vab), dampij, d2ij);
-  abdamp_plain<F>(T.rad[k], T.rad[j], dot3(vcb, vcb), dampjk, d2jk);
-  abdamp_plain<F>(T.rad[j], T.rad[l], dot3(vdc, vdc), dampX, d2X);
+  abdamp_plain<F>(vt(14), dot3(vab, vab), dampij, d2ij);
+  abdamp_plain<F>(vt(15), dot3(vcb, vcb), dampjk, d2jk);
+  abdamp_plain<F>(vt(16), dot3(vdc, vdc), dampX, d2X);
   const F re[3] = {-vab[0], -vab[1], -vab[2]};  // r_i - r_j
   const F rd[3] = {-vcb[0], -vcb[1], -vcb[2]};  // r_k - r_j
   F rv[3];
@@ -308,17 +310,17 @@ __device__ inline F torsion_plain(const Dev& D, const Tables<double>& T, const B
     for (int d = 0; d < 3; ++d) dda[d] = ddb[d] = ddc[d] = ddd[d] = F(0);
   }
   const F damp = dampjk * dampij * dampX;
-  if (vt[2] > 1e-6) {
+  if (vt(2) > 1e-6) {
     F s1, c1;
     p_sincos((om - phi0) + pi, s1, c1);
-    et = (1.0 + c1) * vt[1];
-    dij = -s1 * (vt[1] * damp);
+    et = (1.0 + c1) * vt(1);
+    dij = -s1 * (vt(1) * damp);
   } else {
     double s0, c0;
     p_sincos(phi0, s0, c0);
     const F dd = cosom - c0;
-    et = vt[1] * (dd * dd);
-    dij = (-2.0 * vt[1]) * (sinom * dd * damp);
+    et = vt(1) * (dd * dd);
+    dij = (-2.0 * vt(1)) * (sinom * dd * damp);
   }
   const F k1 = et * d2ij * (dampjk * dampX), k2 = et * d2jk * (dampij * dampX), k3 = et * d2X * (dampij * dampjk);
 #pragma unroll
@@ -335,15 +337,16 @@ __device__ inline F torsion_plain(const Dev& D, const Tables<double>& T, const B
 
 // One NCI pair (src/ff_nonb.f90): BJ-damped C6/C8 dispersion and, for
 // r < 25 bohr, exponential repulsion, both times eps2 (:79-193); Coulomb
-// within coul_cut (:337-416), eps1 q_i q_j / r or the Zahn form.  The table row
-// holds R0^6, R0^8, eps2 C6, eps2 C6 sr42, eps2 zab, alpha, qq.
+// within coul_cut (:337-416), eps1 q_i q_j / r or the Zahn form.
 template <class F>
 __device__ inline F pair_plain(const Dev& D, const Tables<double>& T, const BeadPos& x, int kp, Contrib<F>& c) {
-  const int2 ij = __ldg(reinterpret_cast<const int2*>(D.pair) + kp);
+  const unsigned at = __ldg(D.pair + kp);
+  const int i1 = lo16(at), i2 = hi16(at);
   double v[kVPair];
-  load_pair_params(&T.vpair[kVPair * kp], v);
+#pragma unroll
+  for (int k = 0; k < kVPair; ++k) v[k] = __ldg(T.pair + k * D.st[3] + kp);
   F vab[3], r, oner;
-  disp<F>(x, ij.x, ij.y, vab);
+  disp<F>(x, i1, i2, vab);
   const F r2 = dot3(vab, vab);
   p_root(r2, r, oner);
   const F r4 = r2 * r2, r6 = r4 * r2, ir2 = oner * oner;
@@ -366,8 +369,8 @@ __device__ inline F pair_plain(const Dev& D, const Tables<double>& T, const Bead
     drij = drij - e0 * ir2;
   }
   c.na = 2;
-  c.a[0] = ij.x;
-  c.a[1] = ij.y;
+  c.a[0] = i1;
+  c.a[1] = i2;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     c.g[0][d] = vab[d] * drij;
