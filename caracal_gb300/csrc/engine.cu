@@ -2029,9 +2029,11 @@ int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* th
     return fail(CR_ERR_ARG, "the trial runs exceed the recrossing step capacity set by cr_engine_set_recross");
   CR_CUDA(cudaStreamSynchronize(e->stream));
   // every trial starts from the same state: q, p, f, epot, status, the
-  // chain velocities and the step counter are saved and put back after it
+  // chain velocities, the momentum parts and the step counter are saved and
+  // put back after it
   const size_t nq = (size_t)e->T * e->P * e->NC, T = (size_t)e->T;
-  const size_t nsave = 3 * nq + T + 4 * T;
+  const size_t nparts = e->d_parts ? 2 * T * e->prm.U * e->NC : 0;
+  const size_t nsave = 3 * nq + T + 4 * T + nparts;
   double* save = nullptr;
   int* save_st = nullptr;
   CR_CUDA(cudaMalloc(&save, nsave * sizeof(double)));
@@ -2040,12 +2042,12 @@ int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* th
     return fail(CR_ERR_CUDA, "cudaMalloc failed for the autotuner's state copy");
   }
   auto copy_state = [&](bool out) -> cudaError_t {
-    double* dst[5] = {save, save + nq, save + 2 * nq, save + 3 * nq, save + 3 * nq + T};
-    double* src[5] = {e->d_q, e->d_p, e->d_f, e->d_epot, e->d_vnh};
-    const size_t n[5] = {nq, nq, nq, T, 4 * T};
+    double* dst[6] = {save, save + nq, save + 2 * nq, save + 3 * nq, save + 3 * nq + T, save + 3 * nq + 5 * T};
+    double* src[6] = {e->d_q, e->d_p, e->d_f, e->d_epot, e->d_vnh, e->d_parts};
+    const size_t n[6] = {nq, nq, nq, T, 4 * T, nparts};
     cudaError_t err = cudaSuccess;
-    for (int k = 0; k < 5 && err == cudaSuccess; ++k)
-      err = cudaMemcpyAsync(out ? dst[k] : src[k], out ? src[k] : dst[k], n[k] * 8, cudaMemcpyDeviceToDevice, e->stream);
+    for (int k = 0; k < 6 && err == cudaSuccess; ++k)
+      if (n[k]) err = cudaMemcpyAsync(out ? dst[k] : src[k], out ? src[k] : dst[k], n[k] * 8, cudaMemcpyDeviceToDevice, e->stream);
     if (err == cudaSuccess)
       err = cudaMemcpyAsync(out ? save_st : e->d_status, out ? e->d_status : save_st, T * sizeof(int),
                             cudaMemcpyDeviceToDevice, e->stream);
