@@ -170,40 +170,45 @@ __global__ void __launch_bounds__(MIXED ? kQmdffThreads : kTeamThreads, MINB)
 // Energy, gradient and Hessian-vector product H w per bead (plain form, dual
 // coordinates), a block per bead; dew[b] = w . grad E.
 __global__ void __launch_bounds__(kTeamThreads)
-    qmdff_hvp_kernel(qmdff::Dev D, int nbeads, const double* q, const double* w, double* e, double* g, double* hw,
-                     double* dew) {
+    qmdff_hvp_kernel(qmdff::Dev D, int nbeads, BeadRows rows, const double* q, const double* w, double* e, double* g,
+                     double* hw, double* dew) {
   extern __shared__ double qsm[];
   const int n3 = 3 * D.n;
   for (int b = blockIdx.x; b < nbeads; b += gridDim.x) {
-    const double* qb = q + (size_t)b * n3;
-    const double* wb = w + (size_t)b * n3;
+    const size_t r = rows.row(b), r2 = rows.twin(b);
+    const double* qb = q + r * n3;
+    const double* wb = w + r * n3;
     for (int a = threadIdx.x; a < n3; a += kTeamThreads) {
       qsm[a] = qb[a];
       qsm[n3 + a] = wb[a];
     }
     double de = 0.0;
-    const double v = qmdff::team_hvp(D, qsm, g ? g + (size_t)b * n3 : nullptr, hw + (size_t)b * n3, de);
+    const double v = qmdff::team_hvp(D, qsm, g ? g + r * n3 : nullptr, g ? g + r2 * n3 : nullptr, hw + r * n3, hw + r2 * n3, de);
     if (threadIdx.x == 0) {
-      if (e) e[b] = v;
-      if (dew) dew[b] = de;
+      if (e) e[r] = e[r2] = v;
+      if (dew) dew[r] = dew[r2] = de;
     }
     __syncthreads();
   }
 }
 
 // Per bead b and linear parameter t: out[b][t] = alpha_b (v_b . grad E_t|unit)
-// + beta_b E_t|unit (alpha = 1, beta = 0 where the weights are NULL), a block per bead.
+// + beta_b E_t|unit (alpha = 1, beta = 0 where the weights are NULL), a block per bead;
+// out's row b: evaluation b0 + b, twice where it stands for two beads.
 __global__ void __launch_bounds__(kTeamThreads)
-    qmdff_vjp_kernel(qmdff::Dev D, qmdff::Tables<double> U, int nbeads, int nlin, const double* q, const double* v,
-                     const double* alpha, const double* beta, double* out) {
+    qmdff_vjp_kernel(qmdff::Dev D, qmdff::Tables<double> U, BeadRows rows, size_t b0, int nlin, const double* q,
+                     const double* v, const double* alpha, const double* beta, double* out) {
   extern __shared__ double qsm[];
-  const int n3 = 3 * D.n, b = blockIdx.x;
+  const int n3 = 3 * D.n;
+  const size_t b = rows.row(b0 + blockIdx.x);
+  const double m = rows.twin(b0 + blockIdx.x) != b ? 2.0 : 1.0;
   for (int a = threadIdx.x; a < n3; a += kTeamThreads) {
-    qsm[a] = q[(size_t)b * n3 + a];
-    qsm[n3 + a] = v[(size_t)b * n3 + a];
+    qsm[a] = q[b * n3 + a];
+    qsm[n3 + a] = v[b * n3 + a];
   }
   __syncthreads();
-  qmdff::team_param_vjp(D, U, qsm, qsm + n3, alpha ? alpha[b] : 1.0, beta ? beta[b] : 0.0, out + (size_t)b * nlin);
+  qmdff::team_param_vjp(D, U, qsm, qsm + n3, m * (alpha ? alpha[b] : 1.0), m * (beta ? beta[b] : 0.0),
+                        out + (size_t)blockIdx.x * nlin);
 }
 
 // acc[t] += scale * sum_b in[b][t]: 32 columns per block, eight rows at a time in
@@ -229,13 +234,13 @@ __global__ void __launch_bounds__(kSumCols * kSumRows) sum_rows_kernel(int nrows
 }  // namespace cr
 
 int qmdff_hvp_launch(const cr_qmdff* ff, const double* d_q, const double* d_w, int nbeads, double* d_e, double* d_g,
-                     double* d_hw, double* d_dew, cudaStream_t s) {
+                     double* d_hw, double* d_dew, cudaStream_t s, cr::BeadRows rows) {
   if (ff->nterm[4] > 0) return cr_set_error(CR_ERR_UNSUPPORTED, "second derivatives of H/halogen-bond terms are not built");
   const size_t smem = cr::qmdff::team_hvp_smem_bytes(ff->n);
   CR_TRY_CUDA(cudaFuncSetAttribute(cr::qmdff_hvp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (nbeads == 0) return CR_OK;
   const int grid = std::min(nbeads, 1 << 20);
-  cr::qmdff_hvp_kernel<<<grid, cr::kTeamThreads, smem, s>>>(ff->dev, nbeads, d_q, d_w, d_e, d_g, d_hw, d_dew);
+  cr::qmdff_hvp_kernel<<<grid, cr::kTeamThreads, smem, s>>>(ff->dev, nbeads, rows, d_q, d_w, d_e, d_g, d_hw, d_dew);
   CR_TRY_CUDA(cudaGetLastError());
   return CR_OK;
 }
@@ -244,18 +249,16 @@ int qmdff_nlin(const cr_qmdff* ff) { return ff->nterm[0] + ff->nterm[1] + ff->nt
 
 int qmdff_vjp_launch(const cr_qmdff* ff, const double* d_q, const double* d_v, int nbeads, const double* d_alpha,
                      const double* d_beta, double scale, double* d_scratch, int scratch_beads, double* d_acc,
-                     cudaStream_t s) {
+                     cudaStream_t s, cr::BeadRows rows) {
   if (ff->nterm[4] > 0) return cr_set_error(CR_ERR_UNSUPPORTED, "parameter gradients of H/halogen-bond terms are not built");
   const int nlin = qmdff_nlin(ff);
   const size_t smem = (size_t)2 * 3 * ff->n * sizeof(double);
   CR_TRY_CUDA(cudaFuncSetAttribute(cr::qmdff_vjp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (nlin == 0) return CR_OK;
-  const size_t n3 = (size_t)3 * ff->n;
   for (int b0 = 0; b0 < nbeads; b0 += scratch_beads) {
     const int nb = std::min(scratch_beads, nbeads - b0);
-    cr::qmdff_vjp_kernel<<<nb, cr::kTeamThreads, smem, s>>>(ff->dev, ff->unit, nb, nlin, d_q + b0 * n3, d_v + b0 * n3,
-                                                              d_alpha ? d_alpha + b0 : nullptr,
-                                                              d_beta ? d_beta + b0 : nullptr, d_scratch);
+    cr::qmdff_vjp_kernel<<<nb, cr::kTeamThreads, smem, s>>>(ff->dev, ff->unit, rows, (size_t)b0, nlin, d_q, d_v, d_alpha,
+                                                            d_beta, d_scratch);
     CR_TRY_CUDA(cudaGetLastError());
     cr::sum_rows_kernel<<<(nlin + cr::kSumCols - 1) / cr::kSumCols, dim3(cr::kSumCols, cr::kSumRows), 0, s>>>(nb, nlin, d_scratch, scale, d_acc);
     CR_TRY_CUDA(cudaGetLastError());
@@ -715,16 +718,13 @@ int cr_qmdff_create(const cr_qmdff_def* d, cr_qmdff** out) {
     up(bser, &D.bser);
   }
   // unit tables of the linear parameters (parameter gradients)
-  std::vector<double> ubond = vbond, uangl = vangl, utors = vtors, upair = vpair;
+  std::vector<double> ubond = vbond, uangl = vangl, utors = vtors;
   std::fill_n(ubond.begin() + st[0], st[0], 1.0);
   std::fill_n(uangl.begin() + st[1], st[1], 1.0);
   std::fill_n(utors.begin() + st[2], st[2], 1.0);
-  std::fill_n(upair.begin() + (size_t)2 * st[3], (size_t)3 * st[3], 0.0);
-  std::fill_n(upair.begin() + (size_t)6 * st[3], st[3], 1.0);
   up(ubond, &ff->unit.bond);
   up(uangl, &ff->unit.angl);
   up(utors, &ff->unit.tors);
-  up(upair, &ff->unit.pair);
   const int rc = arena.upload(ff);
   if (rc != CR_OK) {
     cr_qmdff_destroy(ff);

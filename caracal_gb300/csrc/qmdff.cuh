@@ -180,7 +180,6 @@ template <> __device__ inline float q_sqrt<float>(float x) { return sqrtf(x); }
 template <class F> __device__ inline F q_erfc(F x);
 template <> __device__ inline double q_erfc<double>(double x) { return erfc(x); }
 template <> __device__ inline float q_erfc<float>(float x) { return erfcf(x); }
-template <> __device__ inline Dual q_erfc<Dual>(Dual x) { return erfc(x); }
 
 // |x| < 1e-14 and |x| > 1e-14 as the reference tests its FP64 denominators;
 // for FP32 the same sets of values without a conversion (1e-14 is not a
@@ -320,7 +319,7 @@ __device__ inline void disp<float>(const BeadPos& X, int a, int b, float* v) {
 // comes exactly from the (hi, lo) coordinates and the gradient is scattered
 // as its (hi, lo) pair.  Beyond that range, and for the energy, the FP32
 // formula above (the FP64 pipe would cost more than the whole FP32 term).
-__device__ inline float bond_mixed(const Dev& D, const BeadPos& x, int m, Contrib<float>& c) {
+__device__ inline float bond_mixed(const Dev& D, const BeadPos& x, int m, Contrib<float>& c, float* vir) {
   const unsigned at = __ldg(D.bond + m);
   const int i = lo16(at), j = hi16(at), st = D.st[0];
   const float2* ser = D.bser + m;  // value c at [c st]
@@ -381,11 +380,12 @@ __device__ inline float bond_mixed(const Dev& D, const BeadPos& x, int m, Contri
       c.g[3][d] = 0.0f;
     }
   }
+  if (vir) *vir = dv[0].hi * (c.g[0][0] + c.g[2][0]) + dv[1].hi * (c.g[0][1] + c.g[2][1]) + dv[2].hi * (c.g[0][2] + c.g[2][2]);
   return kij * omu * omu;
 }
 
 // Angle bend with abdamp damping (src/ff_eg.f90:167-299), mixed form.
-__device__ inline float angle_mixed(const Dev& D, const BeadPos& x, int m, Contrib<float>& c) {
+__device__ inline float angle_mixed(const Dev& D, const BeadPos& x, int m, Contrib<float>& c, float* vir) {
   using F = float;
   const uint2 at = __ldg(D.angl + m);
   const int i = lo16(at.x), j = hi16(at.x), k = (int)at.y, st = D.st[1];
@@ -439,6 +439,7 @@ __device__ inline float angle_mixed(const Dev& D, const BeadPos& x, int m, Contr
     c.g[1][d] = -(da + dc) * damp - t1 - t2;
     c.g[2][d] = dc * damp + t2;
   }
+  if (vir) *vir = dot3(vab, c.g[0]) + dot3(vcb, c.g[2]);
   return ea * damp;
 }
 
@@ -861,20 +862,20 @@ __device__ __noinline__ F hb_term(const Dev& D, const Tables<F>&, const BeadPos&
 }
 
 // Energy of one term of kind KIND (0 bond, 1 angle, 2 torsion, 3 pair, 4 H/halogen
-// bond); vir: the torsions' virial trace.
+// bond); vir: its virial trace (but for H/halogen bonds: hb_virial), or NULL.
 template <int KIND>
 __device__ inline float term(const Dev& D, const BeadPos& x, int m, Contrib<float>& c, float* vir) {
-  if constexpr (KIND == 0) return bond_mixed(D, x, m, c);
-  else if constexpr (KIND == 1) return angle_mixed(D, x, m, c);
+  if constexpr (KIND == 0) return bond_mixed(D, x, m, c, vir);
+  else if constexpr (KIND == 1) return angle_mixed(D, x, m, c, vir);
   else if constexpr (KIND == 2) return torsion_mixed(D, x, m, c, vir);
   else return hb_term<float>(D, D.f, x, m, c);
 }
 template <int KIND>
 __device__ inline double term(const Dev& D, const BeadPos& x, int m, Contrib<double>& c, double* vir) {
-  if constexpr (KIND == 0) return bond_plain<double>(D, D.d, x, m, c);
-  else if constexpr (KIND == 1) return angle_plain<double>(D, D.d, x, m, c);
+  if constexpr (KIND == 0) return bond_plain<double>(D, D.d, x, m, c, vir);
+  else if constexpr (KIND == 1) return angle_plain<double>(D, D.d, x, m, c, vir);
   else if constexpr (KIND == 2) return torsion_plain<double>(D, D.d, x, m, c, vir);
-  else if constexpr (KIND == 3) return pair_plain<double>(D, D.d, x, m, c);
+  else if constexpr (KIND == 3) return pair_plain(D, D.d, x, m, c, vir);
   else return hb_term<double>(D, D.d, x, m, c);
 }
 
@@ -890,28 +891,13 @@ __device__ inline double term(const Dev& D, const BeadPos& x, int m, Contrib<dou
 // (src/eabxag.f90:86-87, 140-153) (r_A - r_X).g_A + (r_B - r_X).g_X, the
 // X atom's gradient with the B vector.  Vectors minimum-imaged as the
 // terms' own.  Mixed-form bonds carry g_i as (hi, lo) in g[0] and g[2].
-template <class F, int KIND>
-__device__ inline F term_virial(const Dev& D, const BeadPos& X, int m, const Contrib<F>& c) {
+template <class F>
+__device__ inline F hb_virial(const Dev& D, const BeadPos& X, int m, const Contrib<F>& c) {
   F u[3], v[3];
-  if constexpr (KIND == 0) {
-    disp<F>(X, c.a[0], c.a[1], u);
-    F g[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) g[d] = std::is_same<F, float>::value ? c.g[0][d] + c.g[2][d] : c.g[0][d];
-    return dot3(u, g);
-  } else if constexpr (KIND == 1) {
-    disp<F>(X, c.a[0], c.a[1], u);
-    disp<F>(X, c.a[2], c.a[1], v);
-    return dot3(u, c.g[0]) + dot3(v, c.g[2]);
-  } else if constexpr (KIND == 3) {
-    disp<F>(X, c.a[0], c.a[1], u);
-    return dot3(u, c.g[0]);
-  } else {
-    disp<F>(X, c.a[0], c.a[2], u);
-    disp<F>(X, c.a[1], c.a[2], v);
-    const bool halogen = D.hb[4 * m + 3] != 1;
-    return dot3(u, c.g[0]) + dot3(v, halogen ? c.g[2] : c.g[1]);
-  }
+  disp<F>(X, c.a[0], c.a[2], u);
+  disp<F>(X, c.a[1], c.a[2], v);
+  const bool halogen = D.hb[4 * m + 3] != 1;
+  return dot3(u, c.g[0]) + dot3(v, halogen ? c.g[2] : c.g[1]);
 }
 
 // Box modes of the force kernel, compile-time so the free molecule's kernel
@@ -970,10 +956,9 @@ __device__ inline void kind_segments(const Dev& D, const BeadPos& X, float* buf,
       Contrib<float> c;
       float w = 0.f;
       float v;
-      if constexpr (MODE == kNpt && KIND == 2) v = term<KIND>(D, X, m, c, &w);  // the torsion's own vectors
-      else v = term<KIND>(D, X, m, c, (float*)nullptr);
+      v = term<KIND>(D, X, m, c, MODE == kNpt ? &w : nullptr);
       if constexpr (MODE == kNpt) {
-        if constexpr (KIND != 2) w = term_virial<float, KIND>(D, X, m, c);
+        if constexpr (KIND == 4) w = hb_virial<float>(D, X, m, c);
         wv += w;
       }
       const float t = es + v;
@@ -1008,10 +993,9 @@ __device__ inline void kind_segments(const Dev& D, const BeadPos& X, double* buf
       const int m = sg.x + i;
       Contrib<double> c;
       double w = 0.0;
-      if constexpr (MODE == kNpt && KIND == 2) es += term<KIND>(D, X, m, c, &w);
-      else es += term<KIND>(D, X, m, c, (double*)nullptr);
+      es += term<KIND>(D, X, m, c, MODE == kNpt ? &w : nullptr);
       if constexpr (MODE == kNpt) {
-        if constexpr (KIND != 2) w = term_virial<double, KIND>(D, X, m, c);
+        if constexpr (KIND == 4) w = hb_virial<double>(D, X, m, c);
         wv += w;
       }
       put_term<false, KIND>(buf, i, c);
@@ -1193,7 +1177,7 @@ __device__ inline void kind_segments_dual(const Dev& D, const BeadPos& X, double
       if constexpr (KIND == 0) es += bond_plain<Dual>(D, D.d, X, m, c);
       else if constexpr (KIND == 1) es += angle_plain<Dual>(D, D.d, X, m, c);
       else if constexpr (KIND == 2) es += torsion_plain<Dual>(D, D.d, X, m, c);
-      else es += pair_plain<Dual>(D, D.d, X, m, c);
+      else es += pair_tangent(D, D.d, X, m, c);
 #pragma unroll
       for (int a = 0; a < NA; ++a)
 #pragma unroll
@@ -1226,9 +1210,10 @@ __host__ __device__ inline size_t team_hvp_smem_bytes(int n) {
 
 // Energy (with E_zero), gradient and Hessian-vector product H w of one bead
 // by a block of kTeam warps.  ws: the block's shared memory holding x (3n
-// doubles) then w (3n doubles; a barrier follows here).  dew receives the
-// directional derivative w . grad E.
-__device__ inline double team_hvp(const Dev& D, double* ws, double* gout, double* hout, double& dew) {
+// doubles) then w (3n doubles; a barrier follows here).  gout, gout2, hout, hout2: the
+// destinations (equal: one).  dew receives the directional derivative w . grad E.
+__device__ inline double team_hvp(const Dev& D, double* ws, double* gout, double* gout2, double* hout, double* hout2,
+                                  double& dew) {
   const int n3 = 3 * D.n, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   double* w = ws + n3;
   double* g = w + n3;
@@ -1253,8 +1238,8 @@ __device__ inline double team_hvp(const Dev& D, double* ws, double* gout, double
   }
   __syncthreads();
   for (int a = tid; a < n3; a += kTeam * 32) {
-    if (gout) gout[a] = g[a];
-    hout[a] = h[a];
+    if (gout) gout[a] = gout2[a] = g[a];
+    hout[a] = hout2[a] = h[a];
   }
   double e = 0.0;
   dew = 0.0;
@@ -1272,7 +1257,7 @@ __device__ inline double team_hvp(const Dev& D, double* ws, double* gout, double
 // Coulomb product qq ( eps1 q_i q_j, or q_i q_j in the Zahn form).
 // Every term is linear in its parameter, so d/dtheta_t (v . grad E) is v .
 // grad E_t evaluated with theta_t = 1; the tables U hold the parameters with
-// those entries set to 1 (and, for pairs, the eps2 ones to 0: Coulomb only).
+// those entries set to 1 (the pairs need none: their Coulomb term alone).
 // Per term, out receives alpha * (v . grad E_t|unit) + beta * E_t|unit; the block's
 // threads take the terms of each kind in turn.
 template <int KIND>
@@ -1284,14 +1269,31 @@ __device__ inline void team_vjp_kind(const Dev& D, const Tables<double>& U, cons
     double e;
     if constexpr (KIND == 0) e = bond_plain<double>(D, U, X, m, c);
     else if constexpr (KIND == 1) e = angle_plain<double>(D, U, X, m, c);
-    else if constexpr (KIND == 2) e = torsion_plain<double>(D, U, X, m, c);
-    else e = pair_plain<double>(D, U, X, m, c);
+    else e = torsion_plain<double>(D, U, X, m, c);
     double s = 0.0;
 #pragma unroll
     for (int a = 0; a < NA; ++a)
 #pragma unroll
       for (int d = 0; d < 3; ++d) s = fma(vs[3 * c.a[a] + d], c.g[a][d], s);
     out[KIND == 2 ? (int)__ldg(D.tors + m).w : m] = alpha * s + beta * e;
+  }
+}
+// ... of the pairs: the Coulomb energy alone depends on qq
+__device__ inline void team_vjp_pairs(const Dev& D, const BeadPos& X, const double* vs, double alpha, double beta,
+                                      double* out) {
+  for (int m = threadIdx.x; m < D.nterm[3]; m += blockDim.x) {
+    const unsigned at = __ldg(D.pair + m);
+    const int i1 = lo16(at), i2 = hi16(at);
+    double vab[3], r, oner, s = 0.0, e = 0.0;
+    disp<double>(X, i1, i2, vab);
+    p_root(dot3(vab, vab), r, oner);
+    if (!(r > D.coul_cut)) {
+      e = pair_coulomb(D, r, oner);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) s = fma(vab[d], vs[3 * i1 + d] - vs[3 * i2 + d], s);
+      s = s * (-e * (oner * oner));
+    }
+    out[m] = alpha * s + beta * e;
   }
 }
 __device__ inline void team_param_vjp(const Dev& D, const Tables<double>& U, const double* xs, const double* vs,
@@ -1305,7 +1307,7 @@ __device__ inline void team_param_vjp(const Dev& D, const Tables<double>& U, con
   out += D.nterm[1];
   team_vjp_kind<2>(D, U, X, vs, alpha, beta, out);
   out += D.nterm[2];
-  team_vjp_kind<3>(D, U, X, vs, alpha, beta, out);
+  team_vjp_pairs(D, X, vs, alpha, beta, out);
 }
 
 }  // namespace qmdff

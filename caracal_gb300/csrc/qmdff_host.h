@@ -40,13 +40,14 @@ int qmdff_launch(const cr_qmdff* ff, const double* d_q, int nbeads, double* d_e,
 // Plain-form derivatives for the adjoint (bonds, angles, torsions, NCI pairs):
 // energy, gradient and H w per bead (d_e, d_g, d_dew may be NULL) ...
 int qmdff_hvp_launch(const cr_qmdff* ff, const double* d_q, const double* d_w, int nbeads, double* d_e, double* d_g,
-                     double* d_hw, double* d_dew, cudaStream_t s);
+                     double* d_hw, double* d_dew, cudaStream_t s, cr::BeadRows rows = cr::all_rows());
 // ... and d_acc[t] += scale * sum_b (alpha_b v_b . grad E_t|unit + beta_b E_t|unit)
 // over the linear parameters t (bond k, angle k, torsion V, pair qq; count
-// qmdff_nlin); d_scratch holds scratch_beads * nlin doubles.
+// qmdff_nlin); d_scratch holds scratch_beads * nlin doubles.  rows: the rows that the
+// nbeads evaluations read and write (a row that has a twin stands for both).
 int qmdff_vjp_launch(const cr_qmdff* ff, const double* d_q, const double* d_v, int nbeads, const double* d_alpha,
                      const double* d_beta, double scale, double* d_scratch, int scratch_beads, double* d_acc,
-                     cudaStream_t s);
+                     cudaStream_t s, cr::BeadRows rows = cr::all_rows());
 int qmdff_nlin(const cr_qmdff* ff);
 
 // dE-EVB of two force fields (csrc/evb.cu): e, g <- EVB energy and gradient;

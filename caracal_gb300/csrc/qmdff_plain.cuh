@@ -98,10 +98,16 @@ __device__ inline void abdamp_plain(double irc, F r2, F& damp, F& ddamp) {
   ddamp = (-4.0 * irc) * (x * (damp * damp));
 }
 
+// Coulomb energy of a pair per charge product: 1 / r, or the Zahn form
+__device__ inline double pair_coulomb(const Dev& D, double r, double oner) {
+  return D.zahn ? (q_erfc<double>(D.zahn_a * r) * oner) - D.zahn_par * (r - D.coul_cut) : oner;
+}
+
 // Bond stretch, generalised Lennard-Jones (src/ff_eg.f90:87-163):
 // e = k (1 + (r0/r)^a - 2 (r0/r)^(a/2)).
 template <class F>
-__device__ inline F bond_plain(const Dev& D, const Tables<double>& T, const BeadPos& x, int m, Contrib<F>& c) {
+__device__ inline F bond_plain(const Dev& D, const Tables<double>& T, const BeadPos& x, int m, Contrib<F>& c,
+                               F* vir = nullptr) {
   const unsigned at = __ldg(D.bond + m);
   const int i = lo16(at), j = hi16(at);
   F rb[3], r, ir;
@@ -119,12 +125,14 @@ __device__ inline F bond_plain(const Dev& D, const Tables<double>& T, const Bead
     c.g[0][d] = fac * rb[d];
     c.g[1][d] = -c.g[0][d];
   }
+  if (vir) *vir = dot3(rb, c.g[0]);
   return kij * (1. + pa - 2. * pa2);
 }
 
 // Angle bend with abdamp damping (src/ff_eg.f90:167-299).
 template <class F>
-__device__ inline F angle_plain(const Dev& D, const Tables<double>& T, const BeadPos& x, int m, Contrib<F>& c) {
+__device__ inline F angle_plain(const Dev& D, const Tables<double>& T, const BeadPos& x, int m, Contrib<F>& c,
+                                F* vir = nullptr) {
   const uint2 at = __ldg(D.angl + m);
   const int i = lo16(at.x), j = hi16(at.x), k = (int)at.y, st = D.st[1];
   const double* v = T.angl + m;
@@ -174,6 +182,7 @@ __device__ inline F angle_plain(const Dev& D, const Tables<double>& T, const Bea
     c.g[2][d] = dedc[d] * wc + k2 * vcb[d];
     c.g[1][d] = -c.g[0][d] - c.g[2][d];
   }
+  if (vir) *vir = dot3(vab, c.g[0]) + dot3(vcb, c.g[2]);
   return ea * damp;
 }
 
@@ -338,33 +347,31 @@ __device__ inline F torsion_plain(const Dev& D, const Tables<double>& T, const B
 // One NCI pair (src/ff_nonb.f90): BJ-damped C6/C8 dispersion and, for
 // r < 25 bohr, exponential repulsion, both times eps2 (:79-193); Coulomb
 // within coul_cut (:337-416), eps1 q_i q_j / r or the Zahn form.
-template <class F>
-__device__ inline F pair_plain(const Dev& D, const Tables<double>& T, const BeadPos& x, int kp, Contrib<F>& c) {
+__device__ inline double pair_plain(const Dev& D, const Tables<double>& T, const BeadPos& x, int kp, Contrib<double>& c,
+                                    double* vir = nullptr) {
   const unsigned at = __ldg(D.pair + kp);
   const int i1 = lo16(at), i2 = hi16(at);
   double v[kVPair];
 #pragma unroll
   for (int k = 0; k < kVPair; ++k) v[k] = __ldg(T.pair + k * D.st[3] + kp);
-  F vab[3], r, oner;
-  disp<F>(x, i1, i2, vab);
-  const F r2 = dot3(vab, vab);
+  double vab[3], r, oner;
+  disp<double>(x, i1, i2, vab);
+  const double r2 = dot3(vab, vab);
   p_root(r2, r, oner);
-  const F r4 = r2 * r2, r6 = r4 * r2, ir2 = oner * oner;
-  const F i6 = p_rcp(r6 + v[0]), i8 = p_rcp(r6 * r2 + v[1]);
-  const F d6 = v[2] * i6, d8 = v[3] * i8;
+  const double r4 = r2 * r2, r6 = r4 * r2, ir2 = oner * oner;
+  const double i6 = p_rcp(r6 + v[0]), i8 = p_rcp(r6 * r2 + v[1]);
+  const double d6 = v[2] * i6, d8 = v[3] * i8;
   // periodic: dispersion and repulsion only within vdw_cut (src/ff_nonb.f90:107)
   const bool vdw = !x.pbc || !(r > D.vdw_cut);
-  F e = vdw ? -(d6 + d8) : F(0);
-  F drij = vdw ? r4 * (6.0 * (d6 * i6) + 8.0 * (d8 * i8) * r2) : F(0);
+  double e = vdw ? -(d6 + d8) : 0.0;
+  double drij = vdw ? r4 * (6.0 * (d6 * i6) + 8.0 * (d8 * i8) * r2) : 0.0;
   if (vdw && r < 25.0) {
-    const F ar = v[5] * r, t = v[4] * p_exp(-ar) * oner;
+    const double ar = v[5] * r, t = v[4] * p_exp(-ar) * oner;
     e = e + t;
     drij = drij - t * ir2 * (ar + 1.0);
   }
   if (!(r > D.coul_cut)) {
-    F e0;
-    if (D.zahn) e0 = v[6] * ((q_erfc<F>(D.zahn_a * r) * oner) - D.zahn_par * (r - D.coul_cut));
-    else e0 = v[6] * oner;
+    const double e0 = v[6] * pair_coulomb(D, r, oner);
     e = e + e0;
     drij = drij - e0 * ir2;
   }
@@ -376,7 +383,66 @@ __device__ inline F pair_plain(const Dev& D, const Tables<double>& T, const Bead
     c.g[0][d] = vab[d] * drij;
     c.g[1][d] = -c.g[0][d];
   }
+  if (vir) *vir = r2 * drij;
   return e;
+}
+
+// The same with the tangent w, by hand: the gradient is drij v, its tangent drij w +
+// drij' (2 v.w) v with drij' = d drij / d r^2.  Some 60 FP64 additions and
+// multiplications, where dual arithmetic takes over 100.
+__device__ inline Dual pair_tangent(const Dev& D, const Tables<double>& T, const BeadPos& x, int kp, Contrib<Dual>& c) {
+  const unsigned at = __ldg(D.pair + kp);
+  const int i1 = lo16(at), i2 = hi16(at);
+  double v[kVPair];
+#pragma unroll
+  for (int k = 0; k < kVPair; ++k) v[k] = __ldg(T.pair + k * D.st[3] + kp);
+  double vab[3], w[3], r, oner;
+  disp<double>(x, i1, i2, vab);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) w[d] = x.w[3 * i1 + d] - x.w[3 * i2 + d];
+  const double r2 = dot3(vab, vab), vw = dot3(vab, w);
+  p_root(r2, r, oner);
+  const double r4 = r2 * r2, r6 = r4 * r2, r8 = r6 * r2, ir2 = oner * oner;
+  const double i6 = p_rcp(r6 + v[0]), i8 = p_rcp(r8 + v[1]);
+  const double d6 = v[2] * i6, d8 = v[3] * i8;
+  const bool vdw = !x.pbc || !(r > D.vdw_cut);
+  double e = 0.0, drij = 0.0, dd = 0.0;  // dd: r^2 drij'
+  if (vdw) {
+    const double f6 = 6.0 * (d6 * i6) * r4, f8 = 8.0 * (d8 * i8) * r6;
+    e = -(d6 + d8);
+    drij = f6 + f8;
+    dd = f6 * fma(-6.0 * r6, i6, 2.0) + f8 * fma(-8.0 * r8, i8, 3.0);
+    if (r < 25.0) {
+      const double ar = v[5] * r, t = v[4] * p_exp(-ar) * oner, u = t * ir2;
+      e = e + t;
+      drij = fma(-u, ar + 1.0, drij);
+      dd = fma(0.5 * u, fma(ar, ar + 3.0, 3.0), dd);
+    }
+  }
+  double de = drij * vw;
+  if (!(r > D.coul_cut)) {
+    // the reference's gradient of the Zahn form is that of e0 as if it were ~ 1/r
+    const double e0 = v[6] * pair_coulomb(D, r, oner), f = e0 * ir2;
+    double e1 = -0.5 * f;  // d e0 / d r^2
+    if (D.zahn) {
+      const double zr = D.zahn_a * r;
+      e1 = -0.5 * oner * v[6] * (oner * (2.0 * D.zahn_a * kInvSqrtPi * p_exp(-zr * zr) + oner * q_erfc<double>(zr)) + D.zahn_par);
+    }
+    e = e + e0;
+    de = fma(2.0 * e1, vw, de);
+    drij = drij - f;
+    dd = dd + f - e1;
+  }
+  const double s = 2.0 * vw * ir2 * dd;
+  c.na = 2;
+  c.a[0] = i1;
+  c.a[1] = i2;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    c.g[0][d] = Dual(vab[d] * drij, fma(s, vab[d], drij * w[d]));
+    c.g[1][d] = -c.g[0][d];
+  }
+  return Dual(e, de);
 }
 
 }  // namespace qmdff
