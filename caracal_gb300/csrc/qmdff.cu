@@ -270,17 +270,19 @@ namespace {
 
 using QmdffKernel = void (*)(cr::qmdff::Dev, int, cr::BeadRows, const double*, double*, double*);
 constexpr int kVariants = 3;
-// [precision][variant]: blocks per SM 1 / 2 / 3 (FP64), 4 / 5 / 6 (mixed)
+// [precision][variant]: blocks per SM 1 / 2 / 3 (FP64), 5 / 7 / 8 (mixed:
+// its stalls are on shared memory and L1, which warps hide better than registers:
+// C20H42 1024 x 64, per step 1434 us with 6 blocks, 1282 with 7, 1256 with 8)
 const QmdffKernel kKernels[2][kVariants] = {
     {cr::qmdff_egrad_kernel<false, 1>, cr::qmdff_egrad_kernel<false, 2>, cr::qmdff_egrad_kernel<false, 3>},
-    {cr::qmdff_egrad_kernel<true, 4>, cr::qmdff_egrad_kernel<true, 5>, cr::qmdff_egrad_kernel<true, 6>}};
+    {cr::qmdff_egrad_kernel<true, 5>, cr::qmdff_egrad_kernel<true, 7>, cr::qmdff_egrad_kernel<true, 8>}};
 constexpr int kDefaultVariant = 1;
 // the force field's periodic box, and NpT (per-trajectory boxes and the
 // virial): one variant per form each
 const QmdffKernel kBoxKernels[2] = {cr::qmdff_egrad_kernel<false, 2, cr::qmdff::kBox>,
-                                    cr::qmdff_egrad_kernel<true, 5, cr::qmdff::kBox>};
+                                    cr::qmdff_egrad_kernel<true, 7, cr::qmdff::kBox>};
 const QmdffKernel kNptKernels[2] = {cr::qmdff_egrad_kernel<false, 2, cr::qmdff::kNpt>,
-                                    cr::qmdff_egrad_kernel<true, 5, cr::qmdff::kNpt>};
+                                    cr::qmdff_egrad_kernel<true, 7, cr::qmdff::kNpt>};
 constexpr int kTuneMinBeads = 2048;  // smaller batches keep the default
 
 // Threads, blocks and dynamic shared memory of the force kernel's forms.
