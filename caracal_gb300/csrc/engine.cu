@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kFluxThreads) child_flux_kernel(int T, int P, 
 // kappa(t) numerator and denominator: num[s] = sum_t w[t] [xi_t > 0 after step s+1],
 // and *denom = sum_t w[t] [wpos].  32 steps per block (a row of side is read
 // together), kKappaRows partial sums over the trajectories added in order
-// (deterministic).  One thread per step took 693 us for 4096 x 40 (the kernels alone).
+// (deterministic).  One thread per step took 693 us for 4096 x 40 
 constexpr int kKappaRows = 32;
 __global__ void __launch_bounds__(32 * kKappaRows) kappa_kernel(int T, int nsteps, int stride, const unsigned char* side,
                                                                 const double* w, const int* wpos, double* num,
@@ -206,6 +206,7 @@ struct cr_engine {
   int tpb = 1;  // threads per bead of the persistent step kernel
   int gpb = 1;  // trajectories per block of that kernel
   int threads = 32;  // threads that its blocks launch
+  int min_threads = 0;  // of a block that has one trajectory (choose_launch)
   size_t smem = 0;
   int istep = 0;
   int launches = 0;
@@ -674,7 +675,7 @@ int split_group_launches(cr_engine* e, const cr::SplitParams& s, int t0, int tn,
   if (e->npt) {  // pressure and Berendsen scaling (src/verlet.f90:1111-1151)
     const cr::NptStep np{e->d_box + 3 * (size_t)t0, e->d_press + 2 * (size_t)t0, e->d_vir + (size_t)t0 * e->P,
                          e->npt_pressure, e->npt_rate};
-    cr::split_berendsen_kernel<<<tn, 128, 0, st>>>(s, np);
+    cr::split_berendsen_kernel<<<tn, cr::kFinishBlock, 0, st>>>(s, np);
     CR_CUDA(cudaGetLastError());
     ++n;
   }
@@ -684,7 +685,7 @@ int split_group_launches(cr_engine* e, const cr::SplitParams& s, int t0, int tn,
     const int S = cr::finish_slices(s.U * e->N);
     cr::split_moments_kernel<<<dim3(S, tn), cr::kMomentThreads, 0, st>>>(s);
     CR_CUDA(cudaGetLastError());
-    cr::split_solve_kernel<<<(tn + 127) / 128, 128, 0, st>>>(s, S);
+    cr::split_solve_kernel<<<(tn + 7) / 8, 32, 0, st>>>(s, S);
     CR_CUDA(cudaGetLastError());
     n += 2;
     if (s.transrot) {
@@ -800,7 +801,7 @@ bool apply_shape(cr_engine* e, int groups, int tpb) {
   while (gpb > 1 && !fits(gpb)) --gpb;
   if (!fits(gpb)) return false;
   const size_t smem = cr::step_smem_bytes(d, U, e->NC, gpb);
-  const int threads = (gpb * U * subs + 31) / 32 * 32;
+  const int threads = (std::max(gpb * U * subs, gpb == 1 ? e->min_threads : 0) + 31) / 32 * 32;
   e->block = groups * e->G * tpb;
   e->tpb = tpb;
   e->grid = (e->T + groups - 1) / groups;
@@ -836,6 +837,15 @@ void choose_launch(cr_engine* e) {
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const cr::PesRuns* r = cr::pes_runs(e->cfg.pes);
   const bool mixed = e->cfg.precision == CR_PREC_MIXED;
+  // one trajectory per block, and blocks that all fit the GPU at once with more
+  // threads than the surface takes: then threads for the tasks of the other stages (one
+  // per bead and coordinate; 64 x 16 H3 with PILE mixed 24.1 -> 21.8 us per step)
+  e->min_threads = 0;
+  for (int n = (std::min(e->NC * e->prm.U, cr::kStepThreads) + 31) / 32 * 32; r && n > 32 && !e->min_threads; n -= 32) {
+    int res = 0;
+    if (r->resident(mixed, n, cr::step_smem_bytes(cr::prop_dims(e->P), e->prm.U, e->NC, 1), &res) != cudaSuccess) break;
+    if (e->T <= res * sms) e->min_threads = n;
+  }
   if (e->T <= 4 * sms)
     for (int tpb = r ? r->max_tpb : 1; tpb >= 1; tpb /= 2)
       if (e->G * tpb <= 256 && apply_shape(e, 1, tpb)) return;
@@ -1182,12 +1192,16 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
     s.nv = pd.nv;
     s.su = pd.su;
     s.sv = pd.sv;
-    std::vector<double> mass2 = e->mass;  // [N] masses, then [N] twice the masses
+    std::vector<double> mass2 = e->mass;  // the masses, then twice the masses
     for (int i = 0; i < N; ++i) mass2.push_back(2.0 * e->mass[(size_t)i]);
-    if (cudaMalloc(&e->d_mass, (size_t)2 * N * 8) != cudaSuccess || cudaMalloc(&e->d_inv_mass, (size_t)N * 8) != cudaSuccess ||
+    std::vector<cr::Limbs> wfix;
+    s.wexp = cr::fixed_exponent(mass2);
+    cr::fixed_limbs(mass2, s.wexp, wfix);
+    if (cudaMalloc(&e->d_mass, (size_t)3 * N * 8) != cudaSuccess || cudaMalloc(&e->d_inv_mass, (size_t)N * 8) != cudaSuccess ||
         cudaMalloc(&e->d_sigma, (size_t)N * 8) != cudaSuccess || cudaMalloc(&e->d_istep, sizeof(int)) != cudaSuccess)
       return cleanup_fail(fail(CR_ERR_CUDA, "device allocation of the split tables failed"));
-    if (cudaMemcpy(e->d_mass, mass2.data(), (size_t)2 * N * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
+    if (cudaMemcpy(e->d_mass, mass2.data(), (size_t)N * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(e->d_mass + N, wfix.data(), (size_t)2 * N * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(e->d_inv_mass, inv.data(), (size_t)N * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(e->d_sigma, sig.data(), (size_t)N * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(e->d_istep, 0, sizeof(int)) != cudaSuccess)
@@ -1220,10 +1234,10 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
     s.seed = cfg->seed;
     s.traj0 = cfg->traj0;
     s.half_dt = 0.5 * cfg->dt;
-    s.totmass = totmass;
-    s.wsum = tm;
+    s.itm = 1.0 / totmass;
+    s.kap = (2.0 - tm / totmass) / totmass;
     s.mass = e->d_mass;
-    s.mass2 = e->d_mass + N;
+    s.wfix = reinterpret_cast<const int*>(e->d_mass + N);
     s.inv_mass = e->d_inv_mass;
     s.sigma = e->d_sigma;
     s.ke = e->d_ke;
@@ -1268,7 +1282,7 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
   s.dt = cfg->dt;
   s.half_dt = 0.5 * cfg->dt;
   s.beta = cfg->beta;
-  s.totmass = totmass;
+  s.itm = 1.0 / totmass;
   for (int i = 0; i < cr::kMaxAtoms; ++i) {
     double m = i < N ? e->mass[i] : 1.0;
     s.mass[i] = m;
@@ -1279,7 +1293,7 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
   s.vnh = e->d_vnh;
   s.pd = pd;
   s.inv_P = 1.0 / e->P;
-  s.wsum = tm;
+  s.kap = (2.0 - tm / totmass) / totmass;
   s.nm_mode = cfg->nm_mode;
   s.circ = e->d_circ;
   s.ke = e->d_maps;

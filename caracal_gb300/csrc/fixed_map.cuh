@@ -52,6 +52,11 @@ struct FixedSum {
     cr += (int64_t)x.hi * k.lo;
     cr += (int64_t)x.lo * k.hi;
   }
+  __device__ __forceinline__ void sub(Limbs x, Limbs k) {
+    hh -= (int64_t)x.hi * k.hi;
+    cr -= (int64_t)x.hi * k.lo;
+    cr -= (int64_t)x.lo * k.hi;
+  }
   __device__ __forceinline__ int64_t value() const { return hh + ((cr + (1 << (kLimbBits - 1))) >> kLimbBits); }
 };
 

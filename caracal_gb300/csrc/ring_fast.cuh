@@ -163,7 +163,6 @@ __device__ __forceinline__ bool row(Get get, Put put, bool isp, bool active, dou
     x[l] = up >= 0 ? x[l] << (up < 63 ? up : 0) : x[l] >> 1;
     if (l > 0 && l < M) x[l] <<= 1;
   }
-  Dct1<M>::run(x, X);
   // z = A X + msc B O with the partner's modes O
   const bool obad = __shfl_xor_sync(0xffffffffu, (int)bad, 1) != 0;
   const int eo = __shfl_xor_sync(0xffffffffu, ex, 1);
@@ -173,14 +172,20 @@ __device__ __forceinline__ bool row(Get get, Put put, bool isp, bool active, dou
   const int E = max(ev, eu);
   const int64_t* A = T.tab;
   const int64_t* B = T.tab + (isp ? 2 : 1) * (M + 1);
+  // both transforms by the same code: a warp passes through it once or twice only,
+  // and fetching it is a good part of the time
+#pragma unroll 1
+  for (int pass = 0;; ++pass) {
+    Dct1<M>::run(x, X);
+    if (pass == 1) break;
 #pragma unroll
-  for (int k = 0; k <= M; ++k) {
-    const int64_t o = __shfl_xor_sync(0xffffffffu, X[k], 1);
-    const int64_t v = mul_s64(X[k] << 1, __ldg((const long long*)A + k));
-    const int64_t u = mul_q64(mul_s64(o << 1, __ldg((const long long*)B + k)), mq);
-    x[k] = shr(v, E - ev) + shr(u, E - eu);
+    for (int k = 0; k <= M; ++k) {
+      const int64_t o = __shfl_xor_sync(0xffffffffu, X[k], 1);
+      const int64_t v = mul_s64(X[k] << 1, __ldg((const long long*)A + k));
+      const int64_t u = mul_q64(mul_s64(o << 1, __ldg((const long long*)B + k)), mq);
+      x[k] = shr(v, E - ev) + shr(u, E - eu);
+    }
   }
-  Dct1<M>::run(x, X);
   if (!active) return true;
   bool fine = !(bad || obad);
 #pragma unroll

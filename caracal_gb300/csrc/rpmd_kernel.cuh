@@ -227,8 +227,7 @@ struct StepParams {
   double dt;
   double half_dt;
   double beta;
-  double totmass;  // Caracal's transrot total mass (P^2 sum m)
-  double wsum;     // P sum m
+  double itm, kap; // transrot: 1/M and 2/M - W/M^2 of Caracal's total mass M = P^2 sum m and W = P sum m
   double mass[kMaxAtoms];
   double inv_mass[kMaxAtoms];
   double sigma[kMaxAtoms];    // sqrt(m P / beta): Andersen / PILE noise scale
@@ -274,103 +273,6 @@ struct StepParams {
 
 // Non-finite test on the exponent bits (integer pipe, no FP64 compare).
 __device__ inline bool nonfinite_bits(double x) { return (__double2hiint(x) & 0x7ff00000) == 0x7ff00000; }
-
-// Gauss-Jordan inverse with full pivoting of a 3x3 matrix (the algorithm of
-// Caracal's invert, src/invert.f90:38-124).  Returns false if singular.
-__device__ inline bool invert3(double (&a)[3][3]) {
-  int ipiv[3] = {0, 0, 0}, indxr[3], indxc[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    double big = 0.0;
-    int irow = 0, icol = 0;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      if (ipiv[j] != 1) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          if (ipiv[k] == 0 && fabs(a[j][k]) >= big) {
-            big = fabs(a[j][k]);
-            irow = j;
-            icol = k;
-          }
-        }
-      }
-    }
-    ipiv[icol] += 1;
-    if (irow != icol) {
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        double t = a[irow][j];
-        a[irow][j] = a[icol][j];
-        a[icol][j] = t;
-      }
-    }
-    indxr[i] = irow;
-    indxc[i] = icol;
-    if (a[icol][icol] == 0.0) return false;
-    double ipivot = fx::rcp(a[icol][icol]);
-    a[icol][icol] = 1.0;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) a[icol][j] *= ipivot;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      if (j != icol) {
-        double t = a[j][icol];
-        a[j][icol] = 0.0;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) a[j][k] -= a[icol][k] * t;
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 2; i >= 0; --i) {
-    if (indxr[i] != indxc[i]) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        double t = a[k][indxr[i]];
-        a[k][indxr[i]] = a[k][indxc[i]];
-        a[k][indxc[i]] = t;
-      }
-    }
-  }
-  return true;
-}
-
-// transrot's move from the fifteen moment sums over beads and atoms (sum p;
-// sum w x; sum x cross p; sum w x x^T as xx, xy, xz, yy, yz, zz): p <- p - m (b +
-// va cross x) with b in mv[0..2], va in mv[3..5].  The second moments about
-// Caracal's rotation centre xt come from the raw ones by the parallel-axis
-// identity C = S - xt Sx^T - Sx xt^T + W xt xt^T, W = sum w.  false: singular.
-__device__ inline bool transrot_move(const double* tot, double tm, double W, bool two_atoms, double* mv) {
-  const double itm = fx::rcp(tm);
-  const double vt[3] = {tot[0] * itm, tot[1] * itm, tot[2] * itm};
-  const double xt[3] = {tot[3] * itm, tot[4] * itm, tot[5] * itm};
-  const double cxx = tot[9] - 2.0 * xt[0] * tot[3] + W * xt[0] * xt[0];
-  const double cxy = tot[10] - xt[0] * tot[4] - tot[3] * xt[1] + W * xt[0] * xt[1];
-  const double cxz = tot[11] - xt[0] * tot[5] - tot[3] * xt[2] + W * xt[0] * xt[2];
-  const double cyy = tot[12] - 2.0 * xt[1] * tot[4] + W * xt[1] * xt[1];
-  const double cyz = tot[13] - xt[1] * tot[5] - tot[4] * xt[2] + W * xt[1] * xt[2];
-  const double czz = tot[14] - 2.0 * xt[2] * tot[5] + W * xt[2] * xt[2];
-  const double mang[3] = {tot[6] - (xt[1] * vt[2] - xt[2] * vt[1]) * tm,
-                          tot[7] - (xt[2] * vt[0] - xt[0] * vt[2]) * tm,
-                          tot[8] - (xt[0] * vt[1] - xt[1] * vt[0]) * tm};
-  double ten[3][3] = {{cyy + czz, -cxy, -cxz}, {-cxy, cxx + czz, -cyz}, {-cxz, -cyz, cxx + cyy}};
-  if (two_atoms) {
-    ten[0][0] += 0.000001;
-    ten[1][1] += 0.000001;
-    ten[2][2] += 0.000001;
-  }
-  if (!invert3(ten)) return false;
-  double va[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) va[a] = ten[a][0] * mang[0] + ten[a][1] * mang[1] + ten[a][2] * mang[2];
-  mv[0] = vt[0] - (va[1] * xt[2] - va[2] * xt[1]);
-  mv[1] = vt[1] - (va[2] * xt[0] - va[0] * xt[2]);
-  mv[2] = vt[2] - (va[0] * xt[1] - va[1] * xt[0]);
-#pragma unroll
-  for (int a = 0; a < 3; ++a) mv[3 + a] = va[a];
-  return true;
-}
 
 __device__ __forceinline__ Limbs ldg_limbs(const Limbs* p) {
   const int2 v = __ldg(reinterpret_cast<const int2*>(p));
@@ -532,29 +434,54 @@ __device__ inline double atom_moment(const Limbs* q, const Limbs* p, const int* 
 }
 
 // transrot's move from the moment sums over beads and atoms (sum p; sum m x; x
-// cross p; sum m x x^T as xx, xy, xz, yy, yz, zz), lane d = 0, 1, 2 of a quad
-// taking component d: p <- p - m (b + va cross x).  With S = sum m x, M
-// Caracal's total mass and W = sum m, the centre S/M gives the centred moments
-// S_ab - (2/M - W/M^2) S_a S_b and the angular momentum L - S x (sum p) / M; the
-// inertia system is solved by cofactors.  false: singular.
-__device__ inline bool transrot_quad(const double* tot, int lane, double tm, double W, double& bb, double& va) {
+// cross p; sum m x x^T as xx, xy, xz, yy, yz, zz), lanes 0, 1, 2 of a quad forming
+// component d each: p <- p - m (b + va cross x).  With S = sum m x, M Caracal's
+// total mass and W = sum m, the centre S/M gives the centred moments S_ab -
+// kap S_a S_b, kap = 2/M - W/M^2, and the angular momentum L - S x (sum p) / M.  The inertia
+// tensor is symmetric and positive, so pivots are taken on the diagonal (the
+// reference inverts it with full pivoting): for a nearly linear molecule the last
+// pivot is small, and what it divides turns the molecule about its own axis.
+// tot(k): moment sum k; two_atoms: the reference's 1e-6 on the diagonal.  false:
+// singular.
+template <class Tot>
+__device__ inline bool transrot_quad(Tot tot, int lane, double itm, double kap, bool two_atoms, double& bb, double& va) {
   const int d = lane < 3 ? lane : 0, e = d == 2 ? 0 : d + 1, f = d == 0 ? 2 : d - 1;
-  const double itm = fx::rcp(tm), kap = fma(-W * itm, itm, 2.0 * itm);
-  const double Sd = tot[3 + d], Se = tot[3 + e], Sf = tot[3 + f];
+  const double Sd = tot(3 + d), Se = tot(3 + e), Sf = tot(3 + f);
   // centred second moments: dd and the product of the other two axes
   const int dd = d == 0 ? 9 : d == 1 ? 12 : 14, ef = d == 0 ? 13 : d == 1 ? 11 : 10;
-  const double cdd = fma(-kap * Sd, Sd, tot[dd]), cef = fma(-kap * Se, Sf, tot[ef]);
-  const double L = fma(-itm, fma(Se, tot[f], -Sf * tot[e]), tot[6 + d]);
+  const double cdd = fma(-kap * Sd, Sd, tot(dd)), cef = fma(-kap * Se, Sf, tot(ef));
+  const double L = fma(-itm, fma(Se, tot(f), -Sf * tot(e)), tot(6 + d));
   auto at = [](double x, int src) { return __shfl_sync(0xffffffffu, x, src, 4); };
-  // row d of the tensor: tdd, and t between the other two axes
-  const double tdd = at(cdd, e) + at(cdd, f), tef = -cef;
-  const double tee = at(tdd, e), tff = at(tdd, f), tde = at(tef, f), tdf = at(tef, e);
-  const double Cdd = fma(tee, tff, -tef * tef), Cde = fma(tdf, tef, -tde * tff), Cdf = at(Cde, f);
-  const double det = at(fma(tdd, Cdd, fma(tde, Cde, tdf * Cdf)), 0);
-  va = fma(Cdd, L, fma(Cde, at(L, e), Cdf * at(L, f))) * fx::rcp(det);
-  const double ve = at(va, e), vf = at(va, f);
-  bb = fma(-ve, Sf, fma(vf, Se, tot[d])) * itm;
-  return det != 0.0;
+  const double tdd = at(cdd, e) + at(cdd, f) + (two_atoms ? 0.000001 : 0.0);
+  // first pivot: the largest of the diagonal (non-negative: the bits order them)
+  auto bits = [](double x) { return __double_as_longlong(fabs(x)); };
+  const double t0 = at(tdd, 0), t1 = at(tdd, 1), t2 = at(tdd, 2);
+  const int p = bits(t0) >= bits(t1) ? (bits(t0) >= bits(t2) ? 0 : 2) : (bits(t1) >= bits(t2) ? 1 : 2);
+  const int q = p == 2 ? 0 : p + 1, r = p == 0 ? 2 : p - 1;
+  const double tpp = at(tdd, p), tqq = at(tdd, q), trr = at(tdd, r);
+  const double tpq = -at(cef, r), tpr = -at(cef, q), tqr = -at(cef, p);
+  const double Lp = at(L, p), Lq = at(L, q), Lr = at(L, r);
+  const double ip = fx::rcp(tpp), a = tpq * ip, b = tpr * ip;
+  const double sqq = fma(-a, tpq, tqq), srr = fma(-b, tpr, trr), sqr = fma(-a, tpr, tqr);
+  const double yq = fma(-a, Lp, Lq), yr = fma(-b, Lp, Lr);
+  const bool swap = bits(srr) > bits(sqq);
+  const double s1 = swap ? srr : sqq, s2 = swap ? sqq : srr, y1 = swap ? yr : yq, y2 = swap ? yq : yr;
+  const double i1 = fx::rcp(s1), c = sqr * i1;
+  const double s3 = fma(-c, sqr, s2), v2 = fma(-c, y1, y2) * fx::rcp(s3), v1 = fma(-sqr, v2, y1) * i1;
+  const double vq = swap ? v2 : v1, vr = swap ? v1 : v2;
+  const double vp = fma(-tpr, vr, fma(-tpq, vq, Lp)) * ip;
+  auto comp = [&](int x) { return x == p ? vp : x == q ? vq : vr; };
+  va = comp(d);
+  bb = fma(-comp(e), Sf, fma(comp(f), Se, tot(d))) * itm;
+  return tpp != 0.0 && s1 != 0.0 && s3 != 0.0;
+}
+
+// x[k] of an array in registers
+__device__ __forceinline__ double pick(const double (&x)[16], int k) {
+  double r = x[0];
+#pragma unroll
+  for (int j = 1; j < 16; ++j) r = k == j ? x[j] : r;
+  return r;
 }
 
 // Dynamic shared memory: the propagator's limbs (3 nr (nu + nv)), then for the
@@ -1038,7 +965,8 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
         const bool real = gg < ng;
         double* mv = smove + 8 * (real ? gg : x0);
         double bb, va;
-        const bool ok = transrot_quad(ssum + 16 * (real ? gg : x0), tid & 3, prm.totmass, prm.wsum, bb, va);
+        const double* tot = ssum + 16 * (real ? gg : x0);
+        const bool ok = transrot_quad([&](int k) { return tot[k]; }, tid & 3, prm.itm, prm.kap, N <= 2, bb, va);
         if (real && (tid & 3) < 3) {
           mv[tid & 3] = bb;
           mv[3 + (tid & 3)] = va;

@@ -40,10 +40,11 @@ struct SplitParams {
   int su, sv;     // padded smem row strides of u and v
   int thermostat, andersen_step, transrot;
   uint32_t seed, traj0;
-  double half_dt, totmass;
-  double wsum;             // sum of the masses over beads and atoms (P sum m)
+  double half_dt;
+  double itm, kap;         // transrot's masses (StepParams)
   const double* mass;      // [N]
-  const double* mass2;     // [N] twice the masses
+  const int* wfix;         // [2 N] the masses, then twice the masses, as limbs under wexp (split_moments_kernel)
+  int wexp;                // value 2^(wexp - 56)
   const double* inv_mass;  // [N]
   const double* sigma;     // [N] sqrt(m P / beta)
   const double* ke;        // [3][nr][nu]: K1, K2, K3 (unit mass), even-mode part (or full rows)
@@ -545,15 +546,15 @@ __global__ void split_parent_init_kernel(SplitParams s) {
 //                         (slice 0), the NaN bits; fixed-order block sums.  Rows l
 //                         and P - l of q are equal after the drift, so an item
 //                         covers both with the sum of their momenta
-//   split_solve_kernel    one thread per trajectory: the S partials summed in
+//   split_solve_kernel    four lanes per trajectory: the S partials summed in
 //                         order, epot, status, and the 3x3 system for the
-//                         angular velocity (Gauss-Jordan, full pivoting)
+//                         angular velocity (transrot_quad)
 //   split_apply_kernel    every item: p <- m (v - vt - va x (x - xt)),
 //                         evaluated as p - m (b + va x x), b = vt - va x xt
 // The second moments about Caracal's rotation centre xt come from the raw
 // ones by the parallel-axis identity C = S - xt Sx^T - Sx xt^T + W xt xt^T,
 // W = sum w.  Traffic: half of q and p read twice, p written once; 1024 x 64 C20H42
-// 115, 12 and 71 us.
+// 65, 6 and 71 us.
 constexpr int kMomentThreads = 256;
 constexpr int kApplyItems = 4 * kMomentThreads;  // items of one block of split_apply_kernel
 constexpr int kFinishSums = 16;   // 15 moments + sum of bead energies
@@ -565,54 +566,33 @@ __host__ __device__ inline int finish_slices(int items) {
   return s < 1 ? 1 : (s > 16 ? 16 : s);
 }
 
-// Not NaN or infinite: exponent bits below all-ones (integer pipe only).
-__device__ inline bool finite_bits(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
-
-// Moment sums of one (bead, atom) item of mass w and momentum p.  On this GPU the
-// FP64 pipe bounds the finish, so the sums use w v = p (momentum) and w x once: 21
-// FP64 operations per item.
-__device__ inline void finish_accumulate(double w, const double (&q)[3], const double (&p)[3],
-                                         double (&acc)[kFinishSums], int& status) {
-  const double wq[3] = {w * q[0], w * q[1], w * q[2]};
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    if (!finite_bits(q[d])) status |= CR_TRAJ_NONFINITE;
-    acc[d] += p[d];
-    acc[3 + d] += wq[d];
-  }
-  acc[6] = fma(q[1], p[2], fma(-q[2], p[1], acc[6]));
-  acc[7] = fma(q[2], p[0], fma(-q[0], p[2], acc[7]));
-  acc[8] = fma(q[0], p[1], fma(-q[1], p[0], acc[8]));
-  acc[9] = fma(wq[0], q[0], acc[9]);
-  acc[10] = fma(wq[0], q[1], acc[10]);
-  acc[11] = fma(wq[0], q[2], acc[11]);
-  acc[12] = fma(wq[1], q[1], acc[12]);
-  acc[13] = fma(wq[1], q[2], acc[13]);
-  acc[14] = fma(wq[2], q[2], acc[14]);
-}
-
 // Warp sum of 16 values per lane as a reduce-scatter butterfly: at each of
 // the first four levels a lane keeps half of its values and adds the
-// partner's copy of that half (8 + 4 + 2 + 1 FP64 adds instead of 16 x 5),
+// partner's copy of that half (8 + 4 + 2 + 1 adds instead of 16 x 5),
 // then one exchange finishes.  Lane l returns the warp sum of value l >> 1.
-// Fixed order: deterministic.
-__device__ inline double warp_sum16(double (&v)[16], int lane) {
+__device__ inline int64_t warp_sum16(int64_t (&v)[16], int lane) {
 #pragma unroll
   for (int level = 0; level < 4; ++level) {
     const int half = 8 >> level;  // values kept per lane after this level
     const bool up = (lane >> (4 - level)) & 1;
 #pragma unroll
     for (int j = 0; j < half; ++j) {
-      const double keep = up ? v[half + j] : v[j];
-      const double give = up ? v[j] : v[half + j];
+      const int64_t keep = up ? v[half + j] : v[j];
+      const int64_t give = up ? v[j] : v[half + j];
       v[j] = keep + __shfl_xor_sync(0xffffffffu, give, 16 >> level);
     }
   }
   return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-__global__ void __launch_bounds__(kMomentThreads) split_moments_kernel(SplitParams s) {
-  constexpr int kWarps = kMomentThreads / 32;
+// Moment sums.  In FP64 the 24 operations of an item held the FP64 pipe for 94 of
+// 115 us (1024 x 64 C20H42; now 65 us); so a warp takes kWarpItems items per lane at
+// a time, brings their q and p under one exponent each as 55-bit integers, and
+// forms the products by limbs (fixed_map.cuh): rounded at 2^-55 of the largest
+// product, 64 items at a time, and summed exactly before one conversion to FP64.
+constexpr int kWarpItems = 2;
+__global__ void __launch_bounds__(kMomentThreads, 3) split_moments_kernel(const __grid_constant__ SplitParams s) {
+  constexpr int kWarps = kMomentThreads / 32, kGuard = 1;
   __shared__ double wpart[kWarps][kFinishSums];
   __shared__ int wstat[kWarps];
   const int S = gridDim.x, g = blockIdx.x, t = blockIdx.y, P = s.P, N = s.N;
@@ -620,30 +600,90 @@ __global__ void __launch_bounds__(kMomentThreads) split_moments_kernel(SplitPara
   const size_t tb = (size_t)t * P * s.NC;
   const int items = s.U * N;
   const int lo = (int)((long long)items * g / S), hi = (int)((long long)items * (g + 1) / S);
-  double acc[kFinishSums];
+  double total = 0.0;  // of value lane >> 1
+  bool bad = false;
+  for (int i0 = lo + warp * 32 * kWarpItems; i0 < hi; i0 += kMomentThreads * kWarpItems) {
+    double q[kWarpItems][3], p[kWarpItems][3], pt[kWarpItems][3];
+    int atom[kWarpItems];  // [k]: + N where the item stands for two rows
+    int eq = 0, ep = 0;
 #pragma unroll
-  for (int j = 0; j < kFinishSums; ++j) acc[j] = 0.0;
-  int status = 0;
-  for (int i = lo + threadIdx.x; i < hi; i += kMomentThreads) {
-    const int l = i / N, a = i - l * N, k = twin_row(s, l);
-    double q[3], p[3];
+    for (int k = 0; k < kWarpItems; ++k) {
+      const int i = i0 + 32 * k + lane;
+      atom[k] = -1;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      q[d] = s.q[tb + 3 * (size_t)i + d];
-      p[d] = s.p[tb + 3 * (size_t)i + d];
-      if (k != l) p[d] += s.p[tb + 3 * (size_t)(k * N + a) + d];
+      for (int d = 0; d < 3; ++d) q[k][d] = p[k][d] = pt[k][d] = 0.0;
+      if (i < hi) {
+        const int l = i / N, a = i - l * N, kt = twin_row(s, l);
+        atom[k] = a + (kt != l ? N : 0);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          q[k][d] = s.q[tb + 3 * (size_t)i + d];
+          p[k][d] = s.p[tb + 3 * (size_t)i + d];
+          if (kt != l) pt[k][d] = s.p[tb + 3 * (size_t)(kt * N + a) + d];
+        }
+      }
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        eq = max(eq, exponent_field(q[k][d]));
+        ep = max(ep, max(exponent_field(p[k][d]), exponent_field(pt[k][d])));
+      }
     }
-    finish_accumulate(k != l ? s.mass2[a] : s.mass[a], q, p, acc, status);
+    eq = __reduce_max_sync(0xffffffffu, eq);
+    ep = __reduce_max_sync(0xffffffffu, ep);
+    bad = bad || eq == kFixedNan;
+    int64_t sp[3] = {0, 0, 0}, sq[3] = {0, 0, 0};
+    FixedSum L[3], C[6];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) L[d] = FixedSum{0, 0};
+#pragma unroll
+    for (int d = 0; d < 6; ++d) C[d] = FixedSum{0, 0};
+#pragma unroll
+    for (int k = 0; k < kWarpItems; ++k) {
+      const int a = atom[k] < 0 ? 0 : atom[k];  // an empty item is zero in every value
+      // the mass (twice it for two rows): mass * 2^-em below 1 as 56 bits
+      const Limbs w{s.wfix[2 * a], s.wfix[2 * a + 1]};
+      Limbs x[3], wx[3], y[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const int64_t fq = to_fixed(q[k][d], eq, kGuard);
+        const int64_t fp = to_fixed(p[k][d], ep, kGuard + 1) + to_fixed(pt[k][d], ep, kGuard + 1);
+        x[d] = to_limbs(fq);
+        y[d] = to_limbs(fp);
+        FixedSum m{0, 0};
+        m.add(x[d], w);
+        const int64_t fw = m.value();
+        wx[d] = to_limbs(fw);
+        sp[d] += fp;
+        sq[d] += fw;
+      }
+      L[0].add(x[1], y[2]);
+      L[0].sub(x[2], y[1]);
+      L[1].add(x[2], y[0]);
+      L[1].sub(x[0], y[2]);
+      L[2].add(x[0], y[1]);
+      L[2].sub(x[1], y[0]);
+      C[0].add(wx[0], x[0]);
+      C[1].add(wx[0], x[1]);
+      C[2].add(wx[0], x[2]);
+      C[3].add(wx[1], x[1]);
+      C[4].add(wx[1], x[2]);
+      C[5].add(wx[2], x[2]);
+    }
+    int64_t v[16] = {sp[0], sp[1], sp[2], sq[0], sq[1], sq[2], L[0].value(), L[1].value(), L[2].value(),
+                     C[0].value(), C[1].value(), C[2].value(), C[3].value(), C[4].value(), C[5].value(), 0};
+    const int64_t sum = warp_sum16(v, lane);
+    // units: p 2^(ep - 1078 + guard + 1), q 2^(eq - 1078 + guard), m q the mass's exponent more
+    const int up = ep - 1077 + kGuard, uq = eq - 1078 + kGuard, j = lane >> 1, two = 2 * kLimbBits;
+    const int ex = j < 3 ? up : j < 6 ? uq + s.wexp : j < 9 ? uq + up + two : 2 * uq + s.wexp + two;
+    double r = from_fixed(sum, ex);
+    if (eq == kFixedNan || ep == kFixedNan) r = __longlong_as_double(0x7ff8000000000000ll);
+    total += r;
   }
-  if (g == 0)
-    for (int j = threadIdx.x; j < P; j += kMomentThreads) acc[15] += s.V[(size_t)t * P + j];
-  const double ws = warp_sum16(acc, lane);
-  status = __reduce_or_sync(0xffffffffu, status);
-  if ((lane & 1) == 0) wpart[warp][lane >> 1] = ws;
-  if (lane == 0) wstat[warp] = status;
+  if ((lane & 1) == 0) wpart[warp][lane >> 1] = total;
+  if (lane == 0) wstat[warp] = bad ? CR_TRAJ_NONFINITE : 0;
   __syncthreads();
   const size_t slot = (size_t)t * S + g;
-  if (threadIdx.x < kFinishSums) {
+  if (threadIdx.x < kFinishSums - 1) {
     double v = 0.0;
     for (int w = 0; w < kWarps; ++w) v += wpart[w][threadIdx.x];
     s.fsum[slot * kFinishSums + threadIdx.x] = v;
@@ -652,32 +692,47 @@ __global__ void __launch_bounds__(kMomentThreads) split_moments_kernel(SplitPara
     for (int w = 0; w < kWarps; ++w) st |= wstat[w];
     s.fstat[slot] = st;
   }
+  // the bead energies, by slice 0's second warp, in order over 32 partial sums
+  if (warp == 1) {
+    double e = 0.0;
+    if (g == 0)
+      for (int j = lane; j < P; j += 32) e += s.V[(size_t)t * P + j];
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    if (lane == 0) s.fsum[slot * kFinishSums + kFinishSums - 1] = e;
+  }
 }
 
-__global__ void split_solve_kernel(SplitParams s, int S) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= s.T) return;
-  double tot[kFinishSums];
+__global__ void split_solve_kernel(const __grid_constant__ SplitParams s, int S) {
+  const int x = blockIdx.x * 8 + threadIdx.x / 4, lane = threadIdx.x & 3;
+  const bool real = x < s.T;
+  const int t = real ? x : s.T - 1;  // a quad's shuffles need whole warps
+  // the partial sums, a quarter per lane, then all of them on every lane
+  double part[4] = {0.0, 0.0, 0.0, 0.0}, tot[kFinishSums];
   int status = 0;
-#pragma unroll
-  for (int j = 0; j < kFinishSums; ++j) tot[j] = 0.0;
   for (int g = 0; g < S; ++g) {
     const size_t slot = (size_t)t * S + g;
 #pragma unroll
-    for (int j = 0; j < kFinishSums; ++j) tot[j] += s.fsum[slot * kFinishSums + j];
+    for (int j = 0; j < 4; ++j) part[j] += s.fsum[slot * kFinishSums + 4 * lane + j];
     status |= s.fstat[slot];
   }
+#pragma unroll
+  for (int j = 0; j < kFinishSums; ++j) tot[j] = __shfl_sync(0xffffffffu, part[j & 3], j >> 2, 4);
+  double* mv = s.fmove + (size_t)t * kMoveDoubles;
+  if (s.transrot) {
+    double bb, va;
+    const bool ok = transrot_quad([&](int k) { return pick(tot, k); }, lane, s.itm, s.kap, s.N <= 2, bb, va);
+    if (real && lane < 3) {
+      mv[lane] = bb;
+      mv[3 + lane] = va;
+    }
+    if (real && lane == 0) mv[9] = ok ? 0.0 : 1.0;
+    if (!ok) status |= CR_TRAJ_SINGULAR_INERTIA;
+  }
+  if (!real || lane != 0) return;
   const bool shake_fail = s.constrain && s.shake_fail[t];
   if (shake_fail) status |= CR_TRAJ_SHAKE_FAILED;
   s.epot[t] = tot[15] + (shake_fail ? 100000.0 : 0.0);
-  double* mv = s.fmove + (size_t)t * kMoveDoubles;
-  if (s.transrot) {
-    mv[9] = 0.0;
-    if (!transrot_move(tot, s.totmass, s.wsum, s.N <= 2, mv)) {
-      status |= CR_TRAJ_SINGULAR_INERTIA;
-      mv[9] = 1.0;
-    }
-  }
   if (status) s.status[t] |= status;
 }
 
@@ -744,25 +799,37 @@ struct NptStep {
   double pressure;    // target, a.u.
   double rate;        // dt compress / taupres
 };
-__global__ void split_berendsen_kernel(SplitParams s, NptStep n) {
-  const int t = blockIdx.x;
-  const int P = s.P, nq = P * s.NC;
+__global__ void __launch_bounds__(kFinishBlock) split_berendsen_kernel(const __grid_constant__ SplitParams s, NptStep n) {
+  const int t = blockIdx.x, P = s.P, NC = s.NC;
   __shared__ double scale;
-  if (threadIdx.x == 0) {
-    double w = 0.0;
-    for (int b = 0; b < P; ++b) w += n.vir[(size_t)t * P + b];
-    double* L = n.box + 3 * (size_t)t;
-    const double factor = 1.0 / (L[0] * L[1] * L[2]);
-    const double pr = (factor * (0.0 - w)) / 3.0;
-    const double sc = pow(1.0 + n.rate * (pr - n.pressure), 1.0 / 3.0);
-    for (int k = 0; k < 3; ++k) L[k] = L[k] * sc;
-    n.press[2 * (size_t)t] = pr;
-    n.press[2 * (size_t)t + 1] += pr;  // press_avg (src/verlet.f90:1171-1173)
-    scale = sc;
+  if (threadIdx.x < 32) {
+    double w = 0.0;  // 32 partial sums, added as a tree
+    for (int b = threadIdx.x; b < P; b += 32) w += n.vir[(size_t)t * P + b];
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    if (threadIdx.x == 0) {
+      double* L = n.box + 3 * (size_t)t;
+      const double factor = 1.0 / (L[0] * L[1] * L[2]);
+      const double pr = (factor * (0.0 - w)) / 3.0;
+      const double sc = pow(1.0 + n.rate * (pr - n.pressure), 1.0 / 3.0);
+      for (int k = 0; k < 3; ++k) L[k] = L[k] * sc;
+      n.press[2 * (size_t)t] = pr;
+      n.press[2 * (size_t)t + 1] += pr;  // press_avg (src/verlet.f90:1171-1173)
+      scale = sc;
+    }
   }
   __syncthreads();
-  double* q = s.q + (size_t)t * nq;
-  for (int i = threadIdx.x; i < nq; i += blockDim.x) q[i] = q[i] * scale;
+  // rows l and P - l of q are equal after the drift
+  const double sc = scale;
+  double* q = s.q + (size_t)t * P * NC;
+  const int nq = s.U * NC;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < nq; i += kFinishBlock) {
+    const int l = i / NC, k = twin_row(s, l);
+    const double x = q[i] * sc;
+    q[i] = x;
+    if (k != l) q[i + (k - l) * NC] = x;
+  }
 }
 
 __global__ void split_advance_kernel(int* istep) { *istep += 1; }
