@@ -128,41 +128,36 @@ struct Dct1<2> {
 __device__ constexpr int log2i(int x) { return x <= 1 ? 0 : 1 + log2i(x / 2); }
 __device__ __forceinline__ int64_t shr(int64_t x, int n) { return x >> (n < 63 ? n : 63); }
 
-// One coordinate row, filled in by get, of q (isp 0) or p (isp 1) to put(0, .) ..
-// put(M, .); msc is 1/m for q, m for p.  Every lane of the warp takes part (active:
-// its row is real).  Returns whether the new row is finite.
-template <int M, class Get, class Put>
-__device__ __forceinline__ bool row(Get get, Put put, bool isp, bool active, double msc, const FastRing& T) {
+// One coordinate row x[0 .. M] of q (isp 0) or p (isp 1) in shared memory, in place;
+// msc is 1/m for q, m for p.  Every lane of the warp takes part; lanes that are not
+// active point at an active lane's row and write nothing.  Returns whether the new
+// row is finite; put(l, y) receives it.
+//
+// A warp passes through this once or twice only, so what it fetches as code
+// bounds it: unrolled as a whole (9000 instructions for M = 32) it waited for
+// instructions half of the time.  So only the transforms, which need their
+// arrays in registers, are straight code, once for both passes, and everything
+// element by element loops over the row in shared memory.
+template <int M, class Put>
+__device__ __forceinline__ bool row(double* buf, Put put, bool isp, bool active, double msc, const FastRing& T) {
   constexpr int kGuard = log2i(M) - 2, kBits = 56 - kGuard, kNone = -100000;
-  int64_t x[M + 1], X[M + 1];
-  double first = 0.0;
+  long long* fix = reinterpret_cast<long long*>(buf);
+  const double first = isp ? 0.0 : buf[0];
   int e = 0;
-  {
-    double v[M + 1];
-#pragma unroll
-    for (int l = 0; l <= M; ++l) v[l] = 0.0;
-    if (active) get(v);
-#pragma unroll
-    for (int l = 0; l <= M; ++l) e = max(e, exponent_field(v[l]));
-#pragma unroll
-    for (int l = 0; l <= M; ++l) x[l] = to_fixed(v[l], e, kGuard);
-    if (!isp) first = v[0];
-  }
+#pragma unroll 4
+  for (int l = 0; l <= M; ++l) e = max(e, exponent_field(buf[l]));
   const bool bad = e == kFixedNan;
   uint64_t mag = 0;
-  const int64_t x0 = isp ? 0 : x[0];
-#pragma unroll
+  const int64_t x0 = isp ? 0 : to_fixed(buf[0], e, kGuard);
+#pragma unroll 4
   for (int l = 0; l <= M; ++l) {
-    x[l] -= x0;
-    mag |= (uint64_t)(x[l] < 0 ? -x[l] : x[l]);
+    const int64_t x = to_fixed(buf[l], e, kGuard) - x0;
+    mag |= (uint64_t)(x < 0 ? -x : x);
+    if (active) fix[l] = x;
   }
   const int up = fx::clz64(mag) - (64 - kBits);  // -1 .. : left shift to kBits bits
   const int ex = mag == 0 ? kNone : e - 1078 + kGuard - up;
-#pragma unroll
-  for (int l = 0; l <= M; ++l) {
-    x[l] = up >= 0 ? x[l] << (up < 63 ? up : 0) : x[l] >> 1;
-    if (l > 0 && l < M) x[l] <<= 1;
-  }
+  const int left = up < 0 ? 0 : up < 63 ? up : 0, right = up < 0 ? 1 : 0;
   // z = A X + msc B O with the partner's modes O
   const bool obad = __shfl_xor_sync(0xffffffffu, (int)bad, 1) != 0;
   const int eo = __shfl_xor_sync(0xffffffffu, ex, 1);
@@ -170,30 +165,43 @@ __device__ __forceinline__ bool row(Get get, Put put, bool isp, bool active, dou
   const uint64_t mq = fx::signif(mb);
   const int ev = ex + 1, eu = eo == kNone ? kNone : eo + (isp ? T.ec : T.eb) + (fx::expo(mb) - 1023) + 2;
   const int E = max(ev, eu);
-  const int64_t* A = T.tab;
-  const int64_t* B = T.tab + (isp ? 2 : 1) * (M + 1);
-  // both transforms by the same code: a warp passes through it once or twice only,
-  // and fetching it is a good part of the time
+  const long long* A = (const long long*)T.tab;
+  const long long* B = A + (isp ? 2 : 1) * (M + 1);
+  // x_l normalised, twice it between the ends
+#pragma unroll 4
+  for (int l = 0; l <= M; ++l) {
+    const long long x = (fix[l] << left) >> right << (l > 0 && l < M ? 1 : 0);
+    if (active) fix[l] = x;
+  }
 #pragma unroll 1
   for (int pass = 0;; ++pass) {
+    int64_t x[M + 1], X[M + 1];
+#pragma unroll
+    for (int l = 0; l <= M; ++l) x[l] = fix[l];
     Dct1<M>::run(x, X);
-    if (pass == 1) break;
+    if (active) {
 #pragma unroll
-    for (int k = 0; k <= M; ++k) {
-      const int64_t o = __shfl_xor_sync(0xffffffffu, X[k], 1);
-      const int64_t v = mul_s64(X[k] << 1, __ldg((const long long*)A + k));
-      const int64_t u = mul_q64(mul_s64(o << 1, __ldg((const long long*)B + k)), mq);
-      x[k] = shr(v, E - ev) + shr(u, E - eu);
+      for (int l = 0; l <= M; ++l) fix[l] = X[l];
     }
-  }
-  if (!active) return true;
-  bool fine = !(bad || obad);
-#pragma unroll
-  for (int l = 0; l <= M; ++l) {
-    double y = from_fixed(X[l], E - log2i(M)) + first;
-    if (bad || obad) y = __longlong_as_double(0x7ff8000000000000ll);
-    fine = fine && exponent_field(y) != 0x7ff;
-    put(l, y);
+    if (pass == 1) break;
+#pragma unroll 4
+    for (int k = 0; k <= M; ++k) {
+      const int64_t own = fix[k], o = __shfl_xor_sync(0xffffffffu, own, 1);
+      const int64_t v = mul_s64(own << 1, __ldg(A + k));
+      const int64_t u = mul_q64(mul_s64(o << 1, __ldg(B + k)), mq);
+      if (active) fix[k] = shr(v, E - ev) + shr(u, E - eu);
+    }
+    }
+  bool fine = true;
+  if (active) {
+    fine = !(bad || obad);
+#pragma unroll 4
+    for (int l = 0; l <= M; ++l) {
+      double y = from_fixed(fix[l], E - log2i(M)) + first;
+      if (bad || obad) y = __longlong_as_double(0x7ff8000000000000ll);
+      fine = fine && exponent_field(y) != 0x7ff;
+      put(l, y);
+    }
   }
   return fine;
 }

@@ -505,13 +505,9 @@ __device__ __noinline__ void ring_rows(const StepParams& prm, double* sq, double
     const int x = x0 + (threadIdx.x & 31), y = x >> 1;
     const bool active = x < 2 * rows, isp = x & 1;
     const int i = active ? (y % NC) / 3 : 0;
-    double* r = (isp ? sp : sq) + (active ? y : 0) * (M + 1);
-    const bool fine = ring::row<M>(
-        [=](double (&v)[M + 1]) {
-#pragma unroll
-          for (int l = 0; l <= M; ++l) v[l] = r[l];
-        },
-        [=](int l, double v) { r[l] = v; }, isp, active, isp ? prm.mass[i] : prm.inv_mass[i], prm.fast);
+    double* r = (isp ? sp : sq) + (active ? y : x0 >> 1) * (M + 1);
+    const bool fine = ring::row<M>(r, [=](int l, double v) { r[l] = v; }, isp, active, isp ? prm.mass[i] : prm.inv_mass[i],
+                                   prm.fast);
     if (!fine) atomicOr(&sstat[y / NC], CR_TRAJ_NONFINITE);
   }
 }

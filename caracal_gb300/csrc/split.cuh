@@ -328,49 +328,50 @@ __device__ __forceinline__ bool same_bits(double a, double b) {
 // rows l and P - l (which mostly are equal: then nothing is added).  Block: 4 warps =
 // 64 coordinates; grid (ceil(NC / 64), T).  In FP64 the transforms were bound by
 // the FP64 pipe, some 900 instructions of 64 cycles per coordinate: 1024 x 64
-// C20H42 526 -> 281 us, where reading q, p, f and writing q, p takes 70.
+// C20H42 526 -> 203 us, where reading q, p, f and writing q, p takes 70.
+constexpr int kDriftThreads = 128;
 template <int M>
-__global__ void __launch_bounds__(128) split_drift_fast_kernel(const __grid_constant__ SplitParams s) {
+__global__ void __launch_bounds__(kDriftThreads) split_drift_fast_kernel(const __grid_constant__ SplitParams s) {
   constexpr int P = 2 * M;
+  __shared__ double rows[kDriftThreads * (M + 1)];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int NC = s.NC, t = blockIdx.y;
-  const int c = (blockIdx.x * 4 + warp) * 16 + (lane >> 1);
+  const int c0 = (blockIdx.x * 4 + warp) * 16, c = c0 + (lane >> 1);
+  if (c0 >= NC) return;
   const bool isp = lane & 1, active = c < NC;
-  const size_t tb = (size_t)t * P * NC + (active ? c : 0);
+  const size_t tb = (size_t)t * P * NC + (active ? c : c0);
   double* x = (isp ? s.p : s.q) + tb;
   const double* f = s.f + tb;
   const double hdt = isp ? s.half_dt : 0.0;
+  double* buf = rows + threadIdx.x * (M + 1);
   // kLoad rows at a time, so that their loads are in flight together
-  constexpr int kLoad = 11;
-  auto get = [&](double (&v)[M + 1]) {
+  constexpr int kLoad = M < 8 ? 5 : 11;
+#pragma unroll 1
+  for (int l0 = 0; l0 <= M; l0 += kLoad) {
+    double xa[kLoad], xb[kLoad], fa[kLoad], fb[kLoad];
 #pragma unroll
-    for (int l0 = 0; l0 <= M; l0 += kLoad) {
-      double xa[kLoad], xb[kLoad], fa[kLoad], fb[kLoad];
-#pragma unroll
-      for (int k = 0; k < kLoad; ++k) {
-        const int l = l0 + k;
-        if (l > M) continue;
-        const size_t a = (size_t)l * NC, b = (size_t)(l == 0 || l == M ? l : P - l) * NC;
-        xa[k] = x[a];
-        xb[k] = x[b];
-        fa[k] = isp ? f[a] : 0.0;
-        fb[k] = isp ? f[b] : 0.0;
-      }
-#pragma unroll
-      for (int k = 0; k < kLoad; ++k) {
-        const int l = l0 + k;
-        if (l > M) continue;
-        v[l] = fma(-hdt, fa[k], xa[k]);
-        if (!(same_bits(xa[k], xb[k]) && same_bits(fa[k], fb[k]))) v[l] = 0.5 * (v[l] + fma(-hdt, fb[k], xb[k]));
-      }
+    for (int k = 0; k < kLoad; ++k) {
+      const int l = min(l0 + k, M);
+      const size_t a = (size_t)l * NC, b = (size_t)(l == 0 || l == M ? l : P - l) * NC;
+      xa[k] = x[a];
+      xb[k] = x[b];
+      fa[k] = isp ? f[a] : 0.0;
+      fb[k] = isp ? f[b] : 0.0;
     }
-  };
+#pragma unroll
+    for (int k = 0; k < kLoad; ++k) {
+      const int l = l0 + k;
+      double v = fma(-hdt, fa[k], xa[k]);
+      if (!(same_bits(xa[k], xb[k]) && same_bits(fa[k], fb[k]))) v = 0.5 * (v + fma(-hdt, fb[k], xb[k]));
+      if (l <= M) buf[l] = v;
+    }
+  }
   auto put = [&](int l, double y) {
     x[(size_t)l * NC] = y;
     if (l > 0 && l < M) x[(size_t)(P - l) * NC] = y;
   };
   const int atom = active ? c / 3 : 0;
-  ring::row<M>(get, put, isp, active, isp ? s.mass[atom] : s.inv_mass[atom], s.fast);
+  ring::row<M>(buf, put, isp, active, isp ? s.mass[atom] : s.inv_mass[atom], s.fast);
 }
 
 // mode 0: 1/2 kick and thermostat; 1: 1/2 kick only; 2: thermostat only (the
