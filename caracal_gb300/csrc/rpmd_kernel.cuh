@@ -391,6 +391,14 @@ __device__ inline void umbrella_sample(const UmbrellaDev& u, size_t t, double xi
   }
 }
 
+// The largest exponent field of a row.
+__device__ __forceinline__ int row_exponent(const double* r, int U) {
+  int e = 0;
+#pragma unroll 4
+  for (int l = 0; l < U; ++l) e = max(e, exponent_field(r[l]));
+  return e;
+}
+
 // Bead sums of one atom's rows (row0 .. row0 + 2 of q and of p) in fixed point:
 // v = 0..2 p, 3..5 q, 6..11 q_a p_b for (a, b) = (y z), (z y), (z x), (x z), (x y),
 // (y x), 12..17 q_a q_b for xx, xy, xz, yy, yz, zz.  pair: interior beads count
@@ -651,11 +659,13 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
   constexpr int kEtaExp = 1025;
   auto pile_half = [&](uint32_t step, uint32_t tag, bool last) {
     Limbs* le = limbs + flat;
-    for (int x = tid; x < rows; x += nth) {
+    // the rows by the last threads, while the first draw (64 x 16 H3, both half
+    // steps: 15.1 -> 10.8 thousand cycles)
+    for (int x = nth - 1 - tid; x < rows; x += nth) {
       const double* r = sp + x * U;
-      int e = 0;
-      for (int k = 0; k < U; ++k) e = max(e, exponent_field(r[k]));
+      const int e = row_exponent(r, U);
       sexp[x] = e;
+#pragma unroll 3
       for (int k = 0; k < U; ++k) limbs[x * U + k] = to_limbs(to_fixed(r[k], e, prm.pguard + 1));
     }
     for (int x = tid; x < nb * NQ; x += nth) {
@@ -749,21 +759,20 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
       else ring_rows<32, NC>(prm, sq, sp, rows, sstat);
     } else {
       // fold: rows of q, then of p, into limbs: x_l + x_{M-l}, x_l - x_{M-l}
-      for (int x = tid; x < 2 * rows; x += nth) {
-        const double* r = x < rows ? sq + x * U : sp + (x - rows) * U;
-        Limbs* o = limbs + x * U;
-        int e = 0;
-        for (int k = 0; k < U; ++k) e = max(e, exponent_field(r[k]));
-        sexp[x] = e;
+      for (int x = tid; x < 2 * rows; x += nth) sexp[x] = row_exponent(x < rows ? sq + x * U : sp + (x - rows) * U, U);
+      __syncthreads();
+      const int nf = pd.split ? pd.nu : U;
+      for (int x = tid; x < 2 * rows * nf; x += nth) {
+        const int y = x / nf, l = x - y * nf, e = sexp[y];
+        const double* r = y < rows ? sq + y * U : sp + (y - rows) * U;
+        Limbs* o = limbs + y * U;
+        const int64_t a = to_fixed(r[l], e, prm.guard);
         if (pd.split) {
-          for (int l = 0; l < pd.nu; ++l) {
-            const int64_t a = to_fixed(r[l], e, prm.guard);
-            const int64_t c = 2 * l == pd.M ? 0 : to_fixed(r[pd.M - l], e, prm.guard);
-            o[l] = to_limbs(a + c);
-            if (l < pd.nv) o[pd.nu + l] = to_limbs(a - c);
-          }
+          const int64_t c = 2 * l == pd.M ? 0 : to_fixed(r[pd.M - l], e, prm.guard);
+          o[l] = to_limbs(a + c);
+          if (l < pd.nv) o[pd.nu + l] = to_limbs(a - c);
         } else {
-          for (int l = 0; l < U; ++l) o[l] = to_limbs(to_fixed(r[l], e, prm.guard));
+          o[l] = to_limbs(a);
         }
       }
       __syncthreads();
@@ -924,14 +933,10 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
       // q_a q_b in fixed point (in FP64 some 20 instructions per bead and atom, and the
       // solve on one lane: per step H3 64 x 16 PILE mixed 32.2 -> 24.8 us, OH + H2 1000 x 24
       // plain 61 -> 51 us)
-      for (int x = tid; x < 2 * rows; x += nth) {
-        const double* r = x < rows ? sq + x * U : sp + (x - rows) * U;
-        Limbs* o = limbs + x * U;
-        int e = 0;
-        for (int l = 0; l < U; ++l) e = max(e, exponent_field(r[l]));
-        sexp[x] = e;
-        for (int l = 0; l < U; ++l) o[l] = to_limbs(to_fixed(r[l], e, prm.pguard));
-      }
+      for (int x = tid; x < 2 * rows; x += nth) sexp[x] = row_exponent(x < rows ? sq + x * U : sp + (x - rows) * U, U);
+      __syncthreads();
+      for (int x = tid; x < 2 * flat; x += nth)
+        limbs[x] = to_limbs(to_fixed(x < flat ? sq[x] : sp[x - flat], sexp[x / U], prm.pguard));
       __syncthreads();
       for (int x = tid; x < ng * N * kMoments; x += nth) {
         const int y = x / kMoments, v = x - y * kMoments;  // y: trajectory and atom
@@ -979,7 +984,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
         const double* mv = smove + 8 * gg;
         if (mv[6] != 0.0) continue;
         const double qe = sq[x + (e - d) * U], qf = sq[x + (f - d) * U];
-        const double u = mv[d] + fma(mv[3 + e], qf, -mv[3 + f] * qe);
+        const double u = fma(mv[3 + e], qf, fma(-mv[3 + f], qe, mv[d]));
         sp[x] = fma(-prm.mass[c / 3], u, sp[x]);
       }
       __syncthreads();
