@@ -1322,6 +1322,8 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
       return cleanup_fail(fail(CR_ERR_CUDA, "upload of the ring tables failed"));
     s.fast_M = e->P / 2;
   }
+  const cr::PesRuns* runs = cr::pes_runs(cfg->pes);
+  s.quad = runs && runs->quad && (long long)e->T * s.U <= cr::kQuadBeads ? 1 : 0;
   choose_launch(e);
   *out = e;
   return CR_OK;

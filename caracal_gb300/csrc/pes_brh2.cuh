@@ -300,6 +300,7 @@ __device__ inline void egrad_bead(const double* q, double* V, double* g) {
 struct PesBrH2 {
   static constexpr int N = 3;
   static constexpr int kLanes = 1;  // per bead
+  static constexpr bool kQuad = false;
   template <class F>
   __device__ static inline void egrad(const double (&q)[9], double& V, double (&g)[9]) {
     brh2::egrad_bead(q, &V, g);

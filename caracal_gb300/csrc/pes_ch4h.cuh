@@ -86,6 +86,7 @@ __device__ inline void egrad(const Get& x, int i, double& V, const Put& put) {
 struct PesCH4H {
   static constexpr int N = 6;
   static constexpr int kLanes = 4;  // per bead
+  static constexpr bool kQuad = false;  // always four
   template <class F, class Get, class Put>
   __device__ static inline void egrad(const Get& x, int i, double& V, const Put& put) {
     ch4h::egrad<F>(x, i, V, put);

@@ -196,6 +196,7 @@ __device__ inline void egrad(const Get& x, int i, double& V, const Put& put) {
 struct PesCH4OH {
   static constexpr int N = 7;
   static constexpr int kLanes = 4;  // per bead
+  static constexpr bool kQuad = false;  // always four
   template <class F, class Get, class Put>
   __device__ static inline void egrad(const Get& x, int i, double& V, const Put& put) {
     ch4oh::egrad<F, ch4oh::ParCH4OH>(x, i, V, put);
@@ -208,6 +209,7 @@ struct PesCH4OH {
 struct PesGeH4OH {
   static constexpr int N = 7;
   static constexpr int kLanes = 4;
+  static constexpr bool kQuad = false;  // always four
   template <class F, class Get, class Put>
   __device__ static inline void egrad(const Get& x, int i, double& V, const Put& put) {
     ch4oh::egrad<F, ch4oh::ParGeH4OH>(x, i, V, put);

@@ -272,6 +272,7 @@ __device__ inline float pot_mixed(const float (&R)[6], const double (&Rd)[6], ff
 struct PesOH3 {
   static constexpr int N = 4;
   static constexpr int kLanes = 1;  // per bead
+  static constexpr bool kQuad = false;
   template <class F>
   __device__ static inline void egrad(const double (&q)[12], double& V, double (&g)[12]) {
     constexpr int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {1, 2, 3, 2, 3, 3};  // R_k = |q_pb - q_pa|

@@ -14,9 +14,16 @@ namespace cr {
 
 struct StepParams;
 
+// Most evaluated beads of a batch whose surface takes four lanes per bead where it has
+// both forms: one warp of quads per scheduler (152 SMs).  H3 x 16 plain, per step:
+// 300 trajectories (2700 beads) 27 us by quads, about 47 by single threads at any
+// number up to 1100; 1000 trajectories (9000 beads) 53 to 62 by quads.
+constexpr int kQuadBeads = 32 * 152;
+
 struct PesRuns {
   int max_tpb;  // most threads per bead of the step kernel on the surface
   int lanes;    // threads that evaluate a bead together (PES::kLanes)
+  bool quad;    // has the form by four lanes too (PES::kQuad)
   // rpmd_run_kernel<surface, mixed><<<grid, block, smem, st>>>(prm, istep, nsteps)
   cudaError_t (*run)(const StepParams& prm, bool mixed, int grid, int block, size_t smem, cudaStream_t st, int istep,
                      int nsteps);

@@ -26,14 +26,24 @@ struct RunsOf {
     return mixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, rpmd_run_kernel<PES, true, BM>, block, smem)
                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, rpmd_run_kernel<PES, false, BP>, block, smem);
   }
+  template <int L>
+  static void egrad_lanes(bool mixed, int nbeads, BeadRows rows, const double* q, double* V, double* g, cudaStream_t st) {
+    const int bs = 128 / L, nb = (nbeads + bs - 1) / bs;
+    if (mixed) egrad_kernel<PES, true, L><<<nb, 128, 0, st>>>(nbeads, rows, q, V, g);
+    else egrad_kernel<PES, false, L><<<nb, 128, 0, st>>>(nbeads, rows, q, V, g);
+  }
   static cudaError_t egrad(bool mixed, int nbeads, BeadRows rows, const double* q, double* V, double* g, cudaStream_t st) {
-    const int bs = 128 / PES::kLanes, nb = (nbeads + bs - 1) / bs;
     if (nbeads <= 0) return cudaSuccess;
-    if (mixed) egrad_kernel<PES, true><<<nb, 128, 0, st>>>(nbeads, rows, q, V, g);
-    else egrad_kernel<PES, false><<<nb, 128, 0, st>>>(nbeads, rows, q, V, g);
+    if constexpr (PES::kQuad) {
+      if (nbeads <= kQuadBeads) {
+        egrad_lanes<4>(mixed, nbeads, rows, q, V, g, st);
+        return cudaGetLastError();
+      }
+    }
+    egrad_lanes<PES::kLanes>(mixed, nbeads, rows, q, V, g, st);
     return cudaGetLastError();
   }
-  static constexpr PesRuns table() { return PesRuns{MAXTPB, PES::kLanes, &run, &set_smem, &resident, &egrad}; }
+  static constexpr PesRuns table() { return PesRuns{MAXTPB, PES::kLanes, PES::kQuad, &run, &set_smem, &resident, &egrad}; }
 };
 
 }  // namespace cr

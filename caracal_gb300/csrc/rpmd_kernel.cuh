@@ -36,6 +36,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "bead_rows.cuh"
 #include "cr_common.cuh"
 #include "fixed_map.cuh"
@@ -219,6 +221,7 @@ struct StepParams {
   int pair;        // 1: bead j stands for j and P - j too
   int gpb;         // trajectories per block
   int subs;        // threads per carried bead
+  int quad;        // the surface by four lanes per bead where it has that form (PES::kQuad)
   int thermostat;  // CR_THERMO_*
   int andersen_step;
   int transrot;
@@ -839,33 +842,44 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
     __syncthreads();
 
     // per-bead forces (src/verlet.f90:772-777)
-    if constexpr (PES::kLanes > 1) {
-      // kLanes lanes per bead, whole warps; a last partial pass repeats its
-      // first bead without storing
-      constexpr int L = PES::kLanes;
+    // by L lanes per bead, whole warps; a last partial pass repeats its first bead
+    // without storing it
+    auto by_lanes = [&](auto lanes, auto eval) {
+      constexpr int L = decltype(lanes)::value;
       for (int b0 = 0; b0 < nb; b0 += nth / L) {
         const int y = b0 + tid / L;
         if (b0 + (tid & ~31) / L >= nb) break;  // none of the warp's
         const bool store = y < nb;
         const int yb = store ? y : b0, yg = yb / U, off = yg * NC * U + (yb - yg * U);
         double v;
-        auto get = [&](int c) { return sq[off + c * U]; };
-        auto put = [&](int c, double x) {
-          if (store) sf[off + c * U] = x;
-        };
-        if (MIXED) PES::template egrad<float>(get, tid % L, v, put);
-        else PES::template egrad<double>(get, tid % L, v, put);
+        eval([&](int c) { return sq[off + c * U]; }, tid % L, v,
+             [&](int c, double x) {
+               if (store) sf[off + c * U] = x;
+             });
         if (store && tid % L == 0) svb[yb] = v;
       }
-    } else if (bead) {
-      double q[NC], gr[NC], v;
+    };
+    using F = typename std::conditional<MIXED, float, double>::type;
+    if constexpr (PES::kLanes > 1) {
+      by_lanes(std::integral_constant<int, PES::kLanes>{},
+               [](auto get, int lane, double& v, auto put) { PES::template egrad<F>(get, lane, v, put); });
+    } else {
+      bool quads = false;
+      if constexpr (PES::kQuad) quads = prm.quad;
+      if constexpr (PES::kQuad) {
+        if (quads)
+          by_lanes(std::integral_constant<int, 4>{},
+                   [](auto get, int lane, double& v, auto put) { PES::template quad<F>(get, lane, v, put); });
+      }
+      if (!quads && bead) {
+        double q[NC], gr[NC], v;
 #pragma unroll
-      for (int c = 0; c < NC; ++c) q[c] = sq[(g * NC + c) * U + j];
-      if (MIXED) PES::template egrad<float>(q, v, gr);
-      else PES::template egrad<double>(q, v, gr);
-      svb[b] = v;
+        for (int c = 0; c < NC; ++c) q[c] = sq[(g * NC + c) * U + j];
+        PES::template egrad<F>(q, v, gr);
+        svb[b] = v;
 #pragma unroll
-      for (int c = 0; c < NC; ++c) sf[(g * NC + c) * U + j] = gr[c];
+        for (int c = 0; c < NC; ++c) sf[(g * NC + c) * U + j] = gr[c];
+      }
     }
 
     // umbrella windows (src/verlet.f90:1043-1046): the bias at the centroid on
@@ -1023,10 +1037,12 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
   }
 }
 
-// PES::kLanes threads per evaluated bead: V and dV/dq.
-template <class PES, bool MIXED>
+// V and dV/dq, L threads per evaluated bead: PES::kLanes, or 4 where the surface has
+// that form too (PES::kQuad).
+template <class PES, bool MIXED, int L>
 __global__ void egrad_kernel(int nbeads_total, BeadRows rows, const double* q, double* V, double* g) {
-  constexpr int NC = 3 * PES::N, L = PES::kLanes;
+  constexpr int NC = 3 * PES::N;
+  using F = typename std::conditional<MIXED, float, double>::type;
   const int x = blockIdx.x * blockDim.x + threadIdx.x, e = x / L;
   if (L == 1 && e >= nbeads_total) return;
   const bool store = e < nbeads_total;  // a quad's shuffles need whole warps
@@ -1040,14 +1056,13 @@ __global__ void egrad_kernel(int nbeads_total, BeadRows rows, const double* q, d
       g[r * NC + c] = y;
       if (r2 != r) g[r2 * NC + c] = y;
     };
-    if (MIXED) PES::template egrad<float>(get, x % L, v, put);
-    else PES::template egrad<double>(get, x % L, v, put);
+    if constexpr (PES::kLanes > 1) PES::template egrad<F>(get, x % L, v, put);
+    else PES::template quad<F>(get, x % L, v, put);
   } else {
     double qq[NC], gg[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) qq[c] = q[r * NC + c];
-    if (MIXED) PES::template egrad<float>(qq, v, gg);
-    else PES::template egrad<double>(qq, v, gg);
+    PES::template egrad<F>(qq, v, gg);
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
       g[r * NC + c] = gg[c];
