@@ -483,8 +483,12 @@ def run_ours(args):
         # keep the sampler alive over at least a few samples
         if ms_mx < 500:
             extra = max(1, int(500 / max(ms_mx, 1e-3)))
+            # from the same state each time: thousands of steps further on, the mixed
+            # GeH4 + OH surface meets geometries outside its domain
+            state = eng_mx.get_state()[:3]
             for _ in range(min(extra, 50)):
                 eng_mx.run(K)
+                eng_mx.set_state(*state)
     clocks = clk.summary()
     bead_steps = wl.ntraj * wl.nbeads * K
     value = ws * bead_steps / (ms_mx * 1e-3)

@@ -1,5 +1,5 @@
 // Persistent RPMD step kernel: many trajectories, all steps of a run in one
-// launch, every bead's q, p, f held in registers across steps.
+// launch, every bead's q, p, f held in shared memory across steps.
 //
 // Drop-in for the per-step work of Caracal's `verlet` (src/verlet.f90:65-1308)
 // on the gas-phase path: 1/2 kick, free ring-polymer propagation in Caracal's
@@ -17,13 +17,15 @@
 // what a thermostat adds to the antisymmetric part of p -- which the next
 // drift removes -- is kept only where the run ends on it.
 //
-// Thread layout: a block holds several trajectories; thread b serves bead
-// b mod U of trajectory b / U for the surface, and every other stage is a set
-// of tasks (coordinate rows, row pairs, sums) shared by all threads of the
-// block through shared memory, where q, p and the gradient stay during the
-// run.  The state out of the registers leaves them to the surface.
+// Thread layout: a block holds one or several trajectories.  The surface takes
+// four lanes per bead, in passes over the block's beads (XH4; H3 in small batches),
+// or one thread per bead (thread b: bead b mod U of trajectory b / U), and every
+// other stage is a set of tasks (coordinate rows, row pairs, elements, sums) shared
+// by all threads of the block through shared memory, where q, p and the gradient
+// stay during the run.  The state out of the registers leaves them to the surface.
 //
-// The linear maps run on the integer pipe (fixed_map.cuh).  For even P
+// The linear maps run on the integer pipe (fixed_map.cuh; 32 and 64 beads:
+// ring_fast.cuh).  For even P
 // (M = P/2), C[M-r][k] = (-1)^k C[r][k], so with K = Ke + Ko split by mode
 // parity, K[r] = Ke[r] + Ko[r] and K[M-r] = Ke[r] - Ko[r]; Ke is even and Ko
 // odd under l -> M-l: one pass over x_l + x_{M-l} and x_l - x_{M-l} gives rows
@@ -527,11 +529,11 @@ __device__ __noinline__ void ring_rows(const StepParams& prm, double* sq, double
 // (the registers follow: 255 for 2, 168 for 3, 128 for 4).
 constexpr int kStepThreads = 128;
 
-// Threads per bead (TPB = 1, 2, 4).  subs threads share a carried bead: the
-// task stages spread over all gpb U subs threads of the block, the surface is
-// evaluated by the first gpb U.  Worth it where the batch is too small to fill
-// the GPU and the integrator weighs as much as the surface (H3, OH + H2).  The
-// sums do not depend on the block's shape or on subs.
+// subs threads share a carried bead: the task stages spread over all threads of
+// the block, a surface of one thread per bead is evaluated by the first gpb U.
+// Worth it where the batch is too small to fill the GPU and the integrator weighs
+// as much as the surface (H3, OH + H2).  The sums do not depend on the block's
+// shape or on subs.
 template <class PES, bool MIXED, int MINB>
 __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __grid_constant__ StepParams prm, int istep_arg, int nsteps) {
   const int istep0 = prm.istep_dev ? *prm.istep_dev : istep_arg;

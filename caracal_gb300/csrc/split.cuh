@@ -748,8 +748,8 @@ __global__ void __launch_bounds__(kMomentThreads) split_apply_kernel(SplitParams
     const int l = i / N, a = i - l * N, k = twin_row(s, l);
     const double* qq = q + 3 * (size_t)i;
     const double w = s.mass[a];
-    const double u[3] = {mv[0] + fma(mv[4], qq[2], -mv[5] * qq[1]), mv[1] + fma(mv[5], qq[0], -mv[3] * qq[2]),
-                         mv[2] + fma(mv[3], qq[1], -mv[4] * qq[0])};
+    const double u[3] = {fma(mv[4], qq[2], fma(-mv[5], qq[1], mv[0])), fma(mv[5], qq[0], fma(-mv[3], qq[2], mv[1])),
+                         fma(mv[3], qq[1], fma(-mv[4], qq[0], mv[2]))};
     double* pa = p + 3 * (size_t)i;
     double* pb = p + 3 * (size_t)(k * N + a);
 #pragma unroll

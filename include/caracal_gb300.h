@@ -312,8 +312,8 @@ int cr_qmdff_param_vjp(cr_qmdff* ff, const double* xyz, const double* v, int nbe
 int cr_qmdff_egrad_device(cr_qmdff* ff, const double* d_xyz, int nbeads, double* d_e, double* d_g,
                           int precision, void* stream);
 /* Term batches of the mixed form's warp schedule (batches[5]: bonds, angles,
- * torsions, NCI pairs, H/halogen bonds) and the colours they need
- * (diagnostics; the plain form uses full 32-term batches). */
+ * torsions, NCI pairs, H/halogen bonds) and their sum (diagnostics: each
+ * batch is one pass of a warp; its gradients need no further rounds). */
 int cr_qmdff_schedule_info(const cr_qmdff* ff, int* batches, int* colors);
 /* No counterpart in Caracal.  The force kernel comes in three occupancy
  * variants per form; the first launch of >= 2048 beads outside a stream
@@ -567,23 +567,23 @@ int cr_engine_get_npt(cr_engine* e, double* box_bohr, double* pressure_au, doubl
 
 /* Launch shape of the persistent step kernel (analytic surfaces; the graph
  * path of force fields has none and returns CR_ERR_UNSUPPORTED).  A
- * trajectory's beads sit on G = next_pow2(nbeads) threads, each served by
- * threads_per_bead (1, 2 or 4; 4 is built for H3 and OH + H2, 1 for CH4 + H
- * and CH4 + OH) threads that split the bead's atoms between them for the
- * integrator's per-coordinate work; threads_per_block (a multiple of
- * G x threads_per_bead, <= 256) sets how many trajectories share a block.
- * threads_per_block = 0 restores the built-in choice (one thread per bead,
- * 32 threads per block for a batch of at most 128 threads per SM, else 128).
+ * trajectory counts as G = next_pow2(nbeads) times threads_per_bead threads (1,
+ * 2 or 4; 4 is built for H3 and OH + H2, 1 for the others), threads_per_block
+ * (a multiple of that, <= 256) sets how many trajectories share a block.  The
+ * kernel itself runs at most 128 threads per block on the distinct beads and
+ * reduces a shape that would take more; the results do not depend on the
+ * shape.  threads_per_block = 0 restores the built-in choice (one trajectory per
+ * block for a batch of at most four per SM, else by a cost model).
  * No counterpart in the reference, which steps one trajectory at a time on
  * the host. */
 int cr_engine_set_launch(cr_engine* e, int threads_per_block, int threads_per_bead);
 int cr_engine_get_launch(cr_engine* e, int* threads_per_block, int* blocks, int* threads_per_bead);
 /* Autotuner: times nsteps steps at each launch shape (threads per bead 1, 2,
- * 4 as built; G x threads_per_bead, 32, 64, 128, 256 threads per block, those
- * that fit), each from the same saved state, which is then put back (q, p,
- * f, epot, status, chain velocities, step counter); keeps the fastest and
- * returns it with its time per step.  The noise is a function of the step
- * index, so the trials leave no trace in the run. */
+ * 4 as built; from one trajectory per block up to what fits 128 threads),
+ * each from the same saved state, which is then put back (q, p, f, epot,
+ * status, chain velocities, a thermostat's momentum parts, step counter);
+ * keeps the fastest and returns it with its time per step.  The noise is a
+ * function of the step index, so the trials leave no trace in the run. */
 int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* threads_per_bead,
                        float* ms_per_step);
 
