@@ -614,7 +614,7 @@ def run_ours(args):
     if wl.pes == "qmdff":
         gff = wl.extra["gpu_ff"]
         line["autotune"] = {"qmdff_egrad_kernel": {"fp64": gff.tuning("fp64"), "mixed": gff.tuning("mixed"),
-                                                   "variants": "min blocks/SM 2,3,4 (fp64); 4,5,6 (mixed)"}}
+                                                   "variants": "min blocks/SM 1,2,3 (fp64, 256 threads); 5,7,8 (mixed, 128 threads)"}}
     mp = measured_peaks()
     if mp:
         line["measured_peaks_file"] = {k: mp.get(k) for k in ("hbm_gbs", "bf16_tflops", "gpu_name")}

@@ -739,8 +739,10 @@ __global__ void split_solve_kernel(const __grid_constant__ SplitParams s, int S)
 
 __global__ void __launch_bounds__(kMomentThreads) split_apply_kernel(SplitParams s) {
   const int N = s.N, items = s.U * N, t = blockIdx.x;
-  const double* mv = s.fmove + (size_t)t * kMoveDoubles;
-  if (mv[9] != 0.0) return;
+  double mv[6];  // in registers: the stores to p below could be to fmove for all the compiler knows
+#pragma unroll
+  for (int k = 0; k < 6; ++k) mv[k] = s.fmove[(size_t)t * kMoveDoubles + k];
+  if (s.fmove[(size_t)t * kMoveDoubles + 9] != 0.0) return;
   const double* q = s.q + (size_t)t * s.P * s.NC;
   double* p = s.p + (size_t)t * s.P * s.NC;
   const int lo = blockIdx.y * kApplyItems, hi = min(lo + kApplyItems, items);
@@ -752,11 +754,17 @@ __global__ void __launch_bounds__(kMomentThreads) split_apply_kernel(SplitParams
                          fma(mv[3], qq[1], fma(-mv[4], qq[0], mv[2]))};
     double* pa = p + 3 * (size_t)i;
     double* pb = p + 3 * (size_t)(k * N + a);
+    double x[3], y[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const double x = pa[d], y = pb[d], r = fma(-w, u[d], x);
+      x[d] = pa[d];
+      y[d] = pb[d];
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double r = fma(-w, u[d], x[d]);
       pa[d] = r;
-      if (k != l) pb[d] = same_bits(x, y) ? r : fma(-w, u[d], y);
+      if (k != l) pb[d] = same_bits(x[d], y[d]) ? r : fma(-w, u[d], y[d]);
     }
   }
 }
