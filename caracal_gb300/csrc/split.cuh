@@ -555,7 +555,7 @@ __global__ void split_parent_init_kernel(SplitParams s) {
 // The second moments about Caracal's rotation centre xt come from the raw
 // ones by the parallel-axis identity C = S - xt Sx^T - Sx xt^T + W xt xt^T,
 // W = sum w.  Traffic: half of q and p read twice, p written once; 1024 x 64 C20H42
-// 65, 6 and 71 us.
+// 65, 6 and 64 us.
 constexpr int kMomentThreads = 256;
 constexpr int kApplyItems = 4 * kMomentThreads;  // items of one block of split_apply_kernel
 constexpr int kFinishSums = 16;   // 15 moments + sum of bead energies
