@@ -1890,6 +1890,37 @@ int cr_engine_set_parent(cr_engine* e, const cr_recross* rc) {
   return CR_OK;
 }
 
+// R with R^T R = J M^-1 J^T for xi's three vectors (rows of J: forming bond,
+// breaking bond, second reactant - first), upper triangle row by row.  In a
+// triatomic the three depend on one another and the last pivot is zero.
+static void xi_metric_factor(const cr_engine* e, const cr::XiDev& x, double* R) {
+  double J[3][cr::kMaxAtoms] = {};
+  J[0][x.form0] += 1.0;
+  J[0][x.form1] -= 1.0;
+  J[1][x.brk0] += 1.0;
+  J[1][x.brk1] -= 1.0;
+  for (int i = 0; i < x.nreac2; ++i) J[2][x.reac2[i]] += x.w2[i];
+  for (int i = 0; i < x.nreac1; ++i) J[2][x.reac1[i]] -= x.w1[i];
+  for (int k = 0; k < 3; ++k)
+    for (int i = 0; i < e->N; ++i) J[k][i] *= std::sqrt(e->prm.inv_mass[i]);
+  double full[3][3] = {};
+  for (int k = 0; k < 3; ++k) {  // orthogonalise the columns of (J M^-1/2)^T in turn
+    double rr = 0.0;
+    for (int i = 0; i < e->N; ++i) rr += J[k][i] * J[k][i];
+    full[k][k] = std::sqrt(rr);
+    if (!(rr > 0.0)) continue;
+    for (int i = 0; i < e->N; ++i) J[k][i] /= full[k][k];
+    for (int l = k + 1; l < 3; ++l) {
+      double dot = 0.0;
+      for (int i = 0; i < e->N; ++i) dot += J[k][i] * J[l][i];
+      full[k][l] = dot;
+      for (int i = 0; i < e->N; ++i) J[l][i] -= dot * J[k][i];
+    }
+  }
+  for (int k = 0, n = 0; k < 3; ++k)
+    for (int l = k; l < 3; ++l) R[n++] = full[k][l];
+}
+
 int cr_engine_set_umbrella(cr_engine* e, const cr_recross* rc, const double* centers, const double* kforce,
                            int nbins, double lo, double hi) {
   if (!e || !rc || !centers || !kforce) return fail(CR_ERR_ARG, "NULL argument");
@@ -1916,6 +1947,7 @@ int cr_engine_set_umbrella(cr_engine* e, const cr_recross* rc, const double* cen
   u.center = e->d_umb;
   u.kforce = e->d_umb + T;
   u.beta = e->cfg.beta;
+  xi_metric_factor(e, x, u.R);
   u.sampling = e->d_umb_flag;
   u.xsum = e->d_umb + 2 * T;
   u.xsum2 = e->d_umb + 3 * T;

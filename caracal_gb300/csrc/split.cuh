@@ -890,7 +890,7 @@ __global__ void split_sum_beads_kernel(int T, int P, const double* V, double* ep
 template <int N>
 __global__ void split_umbrella_kernel(SplitParams s) {
   constexpr int NC = 3 * N;
-  __shared__ double cq[NC], dxi[NC], bias[NC];
+  __shared__ double cq[NC], bias[NC];
   const int t = blockIdx.x, P = s.P;
   const size_t tb = (size_t)t * P * NC;
   for (int c = threadIdx.x; c < NC; c += blockDim.x) {
@@ -899,9 +899,9 @@ __global__ void split_umbrella_kernel(SplitParams s) {
     cq[c] = acc / P;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const double xi = umbrella_bias<N>(s.xi, cq, s.mass, s.inv_mass, s.umb.center[t], s.umb.kforce[t], s.umb.beta, dxi, bias);
-    if (*s.umb.sampling) umbrella_sample(s.umb, (size_t)t, xi);
+  if (threadIdx.x < 4) {
+    const double xi = umbrella_bias<N>(s.xi, s.umb, cq, s.umb.center[t], s.umb.kforce[t], threadIdx.x, bias);
+    if (threadIdx.x == 0 && *s.umb.sampling) umbrella_sample(s.umb, (size_t)t, xi);
   }
   __syncthreads();
   for (int idx = threadIdx.x; idx < P * NC; idx += blockDim.x) s.f[tb + idx] += bias[idx % NC];

@@ -7,7 +7,7 @@ import pytest
 
 from caracal_gb300 import RPMDEngine
 from caracal_gb300.pmf import umbrella_integration
-from caracal_gb300.workloads import ch4h_config, ch4h_recross_definition
+from caracal_gb300.workloads import ch4h_config, ch4h_recross_definition, h3_collinear, h3_config
 from conftest import rel_err
 from oracle import oracle as orc
 from test_oracle_parent import _xd
@@ -81,3 +81,31 @@ def test_umbrella_windows_give_a_profile(require_gpu):
     assert np.corrcoef(av, centers)[0, 1] > 0.9
     coord, pmf = umbrella_integration(centers, k, av, va, wl.beta, 0.96, 1.04, 41, n)
     assert np.all(np.isfinite(pmf)) and pmf.min() >= 0.0   # shifted by the min over all bins (last one 0)
+
+
+@pytest.mark.parametrize("nbeads,T", [(1, 45), (5, 3), (16, 9)])
+def test_umbrella_quads_per_block(require_gpu, nbeads, T):
+    """Four lanes a trajectory: more quads than a block has threads, one block with a remainder, a
+    triatomic (the three vectors of xi depend on one another).  One step of which only the bias and the
+    surface enter p: rounding of both, 1e-12 of the largest element as above."""
+    wl = h3_config(ntraj=T, nbeads=nbeads)
+    ts = h3_collinear(0.93, 0.93)
+    rd = dict(reac1=[1, 2], reac2=[3], bond_form=(2, 3), bond_break=(1, 2), r_inf=16.0, xi_ideal=1.0,
+              form_ref=float(np.linalg.norm(ts[1] - ts[2])), break_ref=float(np.linalg.norm(ts[0] - ts[1])))
+    centers, kforce = np.linspace(0.7, 1.05, T), np.linspace(0.2, 0.6, T)
+    eng = RPMDEngine("h3", wl.mass, nbeads, T, wl.dt_au, beta=wl.beta, thermostat="none", transrot=False, seed=7)
+    cfg = orc.Config("h3", wl.mass, nbeads, wl.dt_au, wl.beta, thermostat="none", transrot=False, seed=7)
+    eng.init_positions(ts, 0.1)
+    eng.init_momenta()
+    eng.set_umbrella(centers=centers, kforce=kforce, nbins=0, lo=0.0, hi=0.0, **rd)
+    eng.compute_forces()
+    q = orc.init_positions(cfg, T, ts, 0.1)
+    p = orc.init_momenta(cfg, T)
+    f, _ = orc.init_forces(cfg, q)
+    eng.run(1)
+    got = eng.get_state()
+    eng.close()
+    want = orc.run_umbrella(cfg, _xd(rd), q, p, f, 1, centers, kforce)
+    assert not got[4].any()
+    for a, b in zip(got[:4], want[:4]):
+        assert rel_err(a, b) <= 1e-12
