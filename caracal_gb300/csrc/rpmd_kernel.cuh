@@ -362,6 +362,27 @@ __device__ inline void umbrella_sample(const UmbrellaDev& u, size_t t, double xi
   }
 }
 
+// The windows' bias in a step: centroids into cen, the bias behind them, added to
+// every carried bead's gradient.  Out of line: code that few runs take stays out of
+// the step's loop.
+template <int N, class Sum>
+__device__ __noinline__ void umbrella_step(const XiDev& x, const UmbrellaDev& w, Sum bead_sum, const double* sq, double* sf,
+                                           double* cen, int t_first, int ng, int U, double inv_P) {
+  constexpr int NC = 3 * N;
+  const int tid = threadIdx.x, nth = blockDim.x, rows = ng * NC;
+  double* bias = cen + rows;
+  for (int y = tid; y < rows; y += nth) cen[y] = bead_sum(sq + y * U) * inv_P;
+  __syncthreads();
+#pragma unroll 1
+  for (int y = tid; y < 4 * ng; y += nth) {
+    const int g = y >> 2, t = t_first + g;
+    const double xi = umbrella_bias<N>(x, w, cen + g * NC, w.center[t], w.kforce[t], y & 3, bias + g * NC);
+    if ((y & 3) == 0 && *w.sampling) umbrella_sample(w, (size_t)t, xi);
+  }
+  __syncthreads();
+  for (int y = tid; y < rows * U; y += nth) sf[y] += bias[y / U];
+}
+
 // The largest exponent field of a row.
 __device__ __forceinline__ int row_exponent(const double* r, int U) {
   int e = 0;
@@ -852,19 +873,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
 
     // umbrella windows (src/verlet.f90:1043-1046): the bias at the centroid on
     // every bead's gradient
-    if (prm.umb_on) {
-      double* bias = area + rows;
-      for (int x = tid; x < rows; x += nth) area[x] = bead_sum(sq + x * U) * prm.inv_P;
-      __syncthreads();
-      for (int x = tid; x < 4 * ng; x += nth) {
-        const int g = x >> 2, tt = t_first + g;
-        const double xi = umbrella_bias<N>(prm.xi, prm.umb, area + g * NC, prm.umb.center[tt], prm.umb.kforce[tt], x & 3,
-                                           bias + g * NC);
-        if ((x & 3) == 0 && *prm.umb.sampling) umbrella_sample(prm.umb, (size_t)tt, xi);
-      }
-      __syncthreads();
-      for (int x = tid; x < flat; x += nth) sf[x] += bias[x / U];
-    }
+    if (prm.umb_on) umbrella_step<N>(prm.xi, prm.umb, bead_sum, sq, sf, area, t_first, ng, U, prm.inv_P);
 
     // reaction coordinate of the centroid (umbrella mode 1 of a child step,
     // src/verlet.f90:1049-1050 -> src/umbrella.f90:115-117)
