@@ -57,3 +57,24 @@ def test_run_beyond_capacity_is_rejected(require_gpu):
     eng.set_recross(max_steps=5, **ch4h_recross_definition(wl.q0))
     eng.init_children(np.repeat(wl.q0[None], 4, axis=0))
     assert eng.run(6, check=False) != 0
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_sides_do_not_depend_on_trajectories_per_block(require_gpu, precision):
+    """A warp records the sides of eight children: blocks of one child, of a remainder, of more children
+    than one warp takes.  The step's sums do not depend on the block, so the kappa sums agree exactly."""
+    T, P, n = 41, 4, 12
+    wl = ch4h_config(ntraj=T + 1, nbeads=P)
+    out = []
+    for threads in (4, 28, 48, 100):
+        eng = RPMDEngine("ch4h", wl.mass, P, T + 1, wl.dt_au, beta=wl.beta, thermostat="none", transrot=False,
+                         precision=precision, seed=wl.seed)
+        eng.set_launch(threads)
+        eng.set_recross(max_steps=n, **ch4h_recross_definition(wl.q0))
+        eng.init_children(np.repeat(wl.q0[None], P, axis=0))
+        eng.run(n)
+        out.append((eng.launch()[1],) + tuple(np.array(x) for x in eng.kappa(n)))
+        eng.close()
+    assert len({o[0] for o in out}) > 1
+    for o in out[1:]:
+        assert np.array_equal(o[1], out[0][1]) and o[2] == out[0][2] and np.array_equal(o[3], out[0][3])
