@@ -181,11 +181,9 @@ template <class F> __device__ inline F q_erfc(F x);
 template <> __device__ inline double q_erfc<double>(double x) { return erfc(x); }
 template <> __device__ inline float q_erfc<float>(float x) { return erfcf(x); }
 
-// |x| < 1e-14 and |x| > 1e-14 as the reference tests its FP64 denominators;
-// for FP32 the same sets of values without a conversion (1e-14 is not a
-// float: |x| < 1e-14 holds exactly for |x| <= 1e-14f).
-template <class F> __device__ inline bool below_1em14(F x) { return fabs((double)ad::val(x)) < 1e-14; }
-template <> __device__ inline bool below_1em14<float>(float x) { return fabsf(x) <= 1e-14f; }
+// |x| > 1e-14 as the reference tests its FP64 denominators; for FP32 the same set of
+// values without a conversion (1e-14 is not a float: |x| > 1e-14 holds exactly for
+// |x| > 1e-14f, the float below it).
 template <class F> __device__ inline bool above_1em14(F x) { return fabs((double)ad::val(x)) > 1e-14; }
 template <> __device__ inline bool above_1em14<float>(float x) { return fabsf(x) > 1e-14f; }
 

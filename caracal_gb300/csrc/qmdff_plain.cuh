@@ -219,18 +219,27 @@ __device__ inline F torsion_plain(const Dev& D, const Tables<double>& T, const B
     p_root(dot3(na, na), nan_, ina);
     p_root(dot3(nb, nb), nbn, inb);
     p_root(rcb2, L, iL);
-    // the normals are normalised where longer than 1e-14
+    // the normals are normalised where longer than 1e-14 (valijkl); where one is not
+    // (three atoms in line) the angle is the arc cosine of the product so formed, and its
+    // derivative is left out
+    const bool bent = nan_ > 1e-14 && nbn > 1e-14;
     F s = dot3(na, nb);
     if (nan_ > 1e-14) s = s * ina;
     if (nbn > 1e-14) s = s * inb;
-    // |na x nb| = |rb| |na . rc|
     const F tr = dot3(na, vdc);
-    sinphi = (L * (ina * inb)) * fabs(tr);
-    if (::fabs(::fabs(ad::val(s)) - 1.0) < 1e-14) {
-      s = ad::val(s) >= 0 ? F(1.0) : F(-1.0);
-      sinphi = F(0);
+    sinphi = F(0);
+    if (bent) {
+      // |na x nb| = |rb| |na . rc|
+      sinphi = (L * (ina * inb)) * fabs(tr);
+      if (::fabs(::fabs(ad::val(s)) - 1.0) < 1e-14) {
+        s = ad::val(s) >= 0 ? F(1.0) : F(-1.0);
+        sinphi = F(0);
+      }
+      phi = p_angle_of(s, sinphi);
+    } else {
+      F sine;
+      p_angle(s, phi, sine);
     }
-    phi = p_angle_of(s, sinphi);
     F ef, expo;
     p_erf(phi - pi, ef, expo);
     const F h1 = 0.5 - 0.5 * ef, h2 = 0.5 + 0.5 * ef;
@@ -252,9 +261,10 @@ __device__ inline F torsion_plain(const Dev& D, const Tables<double>& T, const B
     //   dphi/dr_i = -s |rb| na / |na|^2,  dphi/dr_l = s |rb| nb / |nb|^2,
     //   dphi/dr_j = -dphi/dr_i + s (u + v),  dphi/dr_k = -dphi/dr_l - s (u + v),
     //   u = (ra.rb) na / (|na|^2 |rb|),  v = (rc.rb) nb / (|nb|^2 |rb|);
-    // none where the reference's denominator |na| |nb| sin(phi) is below 1e-14
+    // none where the reference's denominator |na| |nb| sin(phi) is below 1e-14 (nor
+    // where it is no number: the reciprocals are infinite then)
     F wa = F(0), wb = F(0), wu = F(0), wv = F(0);
-    if (!below_1em14(nan_ * nbn * sinphi)) {
+    if (bent && nan_ * nbn * sinphi >= 1e-14) {
       const F ia2 = ina * ina, ib2 = inb * inb;
       const F w = tr < 0.0 ? dij : -dij;
       const F wl = w * L, wi = w * iL;
