@@ -27,6 +27,12 @@ struct BeadRows {
   }
 };
 
+// Evaluation that a thread belongs to where L threads take one together: the thread
+// count passes 2^31 before an int count of evaluations does.
+__host__ __device__ inline size_t evaluation_of(unsigned block, unsigned block_threads, unsigned thread, int L) {
+  return ((size_t)block * block_threads + thread) / (size_t)L;
+}
+
 // Every row.
 inline BeadRows all_rows() { return BeadRows{1, 1}; }
 // The distinct beads of a trajectory of P beads after a drift in nm_mode 0.

@@ -28,7 +28,7 @@ struct RunsOf {
   }
   template <int L>
   static void egrad_lanes(bool mixed, int nbeads, BeadRows rows, const double* q, double* V, double* g, cudaStream_t st) {
-    const int bs = 128 / L, nb = (nbeads + bs - 1) / bs;
+    const int bs = 128 / L, nb = nbeads / bs + (nbeads % bs != 0);
     if (mixed) egrad_kernel<PES, true, L><<<nb, 128, 0, st>>>(nbeads, rows, q, V, g);
     else egrad_kernel<PES, false, L><<<nb, 128, 0, st>>>(nbeads, rows, q, V, g);
   }

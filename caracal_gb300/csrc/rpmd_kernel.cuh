@@ -1028,10 +1028,11 @@ template <class PES, bool MIXED, int L>
 __global__ void egrad_kernel(int nbeads_total, BeadRows rows, const double* q, double* V, double* g) {
   constexpr int NC = 3 * PES::N;
   using F = typename std::conditional<MIXED, float, double>::type;
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, e = x / L;
-  if (L == 1 && e >= nbeads_total) return;
-  const bool store = e < nbeads_total;  // a quad's shuffles need whole warps
-  const int b = store ? e : nbeads_total - 1;
+  const size_t n = (size_t)nbeads_total, e = evaluation_of(blockIdx.x, blockDim.x, threadIdx.x, L);
+  const int lane = threadIdx.x % L;  // (blocks hold whole evaluations)
+  if (L == 1 && e >= n) return;
+  const bool store = e < n;  // a quad's shuffles need whole warps
+  const size_t b = store ? e : n - 1;
   const size_t r = rows.row(b), r2 = rows.twin(b);
   double v;
   if constexpr (L > 1) {
@@ -1041,8 +1042,8 @@ __global__ void egrad_kernel(int nbeads_total, BeadRows rows, const double* q, d
       g[r * NC + c] = y;
       if (r2 != r) g[r2 * NC + c] = y;
     };
-    if constexpr (PES::kLanes > 1) PES::template egrad<F>(get, x % L, v, put);
-    else PES::template quad<F>(get, x % L, v, put);
+    if constexpr (PES::kLanes > 1) PES::template egrad<F>(get, lane, v, put);
+    else PES::template quad<F>(get, lane, v, put);
   } else {
     double qq[NC], gg[NC];
 #pragma unroll
@@ -1054,7 +1055,7 @@ __global__ void egrad_kernel(int nbeads_total, BeadRows rows, const double* q, d
       if (r2 != r) g[r2 * NC + c] = gg[c];
     }
   }
-  if (store && x % L == 0) {
+  if (store && lane == 0) {
     V[r] = v;
     if (r2 != r) V[r2] = v;
   }
