@@ -465,7 +465,7 @@ int launch_run(cr_engine* e, int nsteps, bool dev_step = false) {
   if (!r) return fail(CR_ERR_UNSUPPORTED, "PES not built");
   const bool mixed = e->cfg.precision == CR_PREC_MIXED;
   if (!dev_step) {
-    CR_CUDA(r->set_smem(mixed, e->smem));
+    CR_CUDA(r->allow_smem(mixed));
     CR_CUDA(r->run(e->prm, mixed, (e->T + e->gpb - 1) / e->gpb, e->threads, e->smem, e->stream, e->istep, nsteps));
     return CR_OK;
   }
@@ -507,7 +507,7 @@ int launch_group(cr_engine* e, int t0, int tn, cudaStream_t st) {
 int set_run_smem(cr_engine* e) {
   const cr::PesRuns* r = cr::pes_runs(e->cfg.pes);
   if (!r) return fail(CR_ERR_UNSUPPORTED, "PES not built");
-  CR_CUDA(r->set_smem(e->cfg.precision == CR_PREC_MIXED, e->smem));
+  CR_CUDA(r->allow_smem(e->cfg.precision == CR_PREC_MIXED));
   return CR_OK;
 }
 
@@ -797,7 +797,7 @@ bool apply_shape(cr_engine* e, int groups, int tpb) {
   // trajectories (the results do not depend on either)
   int subs = tpb, gpb = std::min(groups, e->T);
   while (subs > 1 && U * subs > cr::kStepThreads) subs /= 2;
-  auto fits = [&](int n) { return n * U * subs <= cr::kStepThreads && cr::step_smem_bytes(d, U, e->NC, n) <= 220 * 1024; };
+  auto fits = [&](int n) { return n * U * subs <= cr::kStepThreads && cr::step_smem_bytes(d, U, e->NC, n) <= (size_t)cr::kStepSmemMax; };
   while (gpb > 1 && !fits(gpb)) --gpb;
   if (!fits(gpb)) return false;
   const size_t smem = cr::step_smem_bytes(d, U, e->NC, gpb);

@@ -27,8 +27,8 @@ struct PesRuns {
   // rpmd_run_kernel<surface, mixed><<<grid, block, smem, st>>>(prm, istep, nsteps)
   cudaError_t (*run)(const StepParams& prm, bool mixed, int grid, int block, size_t smem, cudaStream_t st, int istep,
                      int nsteps);
-  // dynamic shared-memory limit of that kernel (set outside a stream capture)
-  cudaError_t (*set_smem)(bool mixed, size_t smem);
+  // raises that kernel's limit on dynamic shared memory (outside a stream capture)
+  cudaError_t (*allow_smem)(bool mixed);
   // blocks of that many threads and bytes that an SM holds
   cudaError_t (*resident)(bool mixed, int block, size_t smem, int* blocks);
   // egrad_kernel<surface, mixed>: V and dV/dq of nbeads evaluations at the rows of `rows`

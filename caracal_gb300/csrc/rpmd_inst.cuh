@@ -16,12 +16,14 @@ struct RunsOf {
     else rpmd_run_kernel<PES, false, BP><<<grid, block, smem, st>>>(prm, istep, nsteps);
     return cudaGetLastError();
   }
-  static cudaError_t set_smem(bool mixed, size_t smem) {
-    return mixed ? cudaFuncSetAttribute(rpmd_run_kernel<PES, true, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                 : cudaFuncSetAttribute(rpmd_run_kernel<PES, false, BP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // The limit belongs to the kernel, whichever engine asks, so it is always the most
+  // that any launch shape takes: an engine's creation lowers no other's.
+  static cudaError_t allow_smem(bool mixed) {
+    return mixed ? cudaFuncSetAttribute(rpmd_run_kernel<PES, true, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmemMax)
+                 : cudaFuncSetAttribute(rpmd_run_kernel<PES, false, BP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStepSmemMax);
   }
   static cudaError_t resident(bool mixed, int block, size_t smem, int* blocks) {
-    cudaError_t err = set_smem(mixed, smem);
+    cudaError_t err = allow_smem(mixed);
     if (err != cudaSuccess) return err;
     return mixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, rpmd_run_kernel<PES, true, BM>, block, smem)
                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, rpmd_run_kernel<PES, false, BP>, block, smem);
@@ -43,7 +45,7 @@ struct RunsOf {
     egrad_lanes<PES::kLanes>(mixed, nbeads, rows, q, V, g, st);
     return cudaGetLastError();
   }
-  static constexpr PesRuns table() { return PesRuns{MAXTPB, PES::kLanes, PES::kQuad, &run, &set_smem, &resident, &egrad}; }
+  static constexpr PesRuns table() { return PesRuns{MAXTPB, PES::kLanes, PES::kQuad, &run, &allow_smem, &resident, &egrad}; }
 };
 
 }  // namespace cr

@@ -497,6 +497,9 @@ __host__ __device__ inline size_t step_smem_bytes(const PropDims& d, int U, int 
   return (size_t)3 * d.nr * (d.nu + d.nv) * 8 + step_group_bytes(U, NC) * groups;
 }
 
+// Most dynamic shared memory of a block (of the 227 KB that it may take).
+constexpr int kStepSmemMax = 220 * 1024;
+
 // The free ring polymer of the block's rows by fast transforms: lanes 2 y and
 // 2 y + 1 take row y of q and of p.
 template <int M, int NC>
