@@ -783,47 +783,79 @@ int dispatch_forces(cr_engine* e) {
   return launch_forces(e);
 }
 
+// Threads per bead and trajectories per block that the kernel runs of `groups`
+// trajectories per block with tpb threads per carried bead (U distinct beads): where
+// the block would be too large, fewer threads per bead, then fewer trajectories (the
+// results do not depend on either).  0: not one trajectory fits.
+int fitting_groups(const cr_engine* e, int groups, int tpb, int* subs) {
+  const cr::PropDims d = cr::prop_dims(e->P);
+  const int U = e->prm.U;
+  *subs = tpb;
+  while (*subs > 1 && U * *subs > cr::kStepThreads) *subs /= 2;
+  auto fits = [&](int n) {
+    return n * U * *subs <= cr::kStepThreads && cr::step_smem_bytes(d, U, e->NC, n) <= (size_t)cr::kStepSmemMax;
+  };
+  int n = std::min(groups, e->T);
+  while (n > 1 && !fits(n)) --n;
+  return fits(n) ? n : 0;
+}
+
+// Most trajectories per block that the API's threads_per_block can name, a thread
+// for every bead of the group of G = next_pow2(P): at most 256 threads, its scratch
+// by the API's rule within 200 KB.
+int nominal_groups(const cr_engine* e, int tpb) {
+  const int GT = e->G * tpb;
+  const cr::PropDims d = cr::prop_dims(e->P);
+  int n = 256 / GT;
+  auto scratch = [&](int k) {
+    return 8 * ((size_t)3 * d.nr * (d.nu + d.nv) + 2 * (size_t)e->P +
+                k * ((size_t)2 * e->NC * e->G + (size_t)2 * e->NC * (d.su + d.sv) + (size_t)((GT + 31) / 32) * 32));
+  };
+  while (n > 0 && scratch(n) > 200 * 1024) --n;
+  return n;
+}
+
 // Launch shape of `groups` trajectories per block with tpb threads per carried
-// bead: U tpb threads per trajectory (U distinct beads), rounded up to a warp.
-// The nominal block size counts a thread for every bead of the group of
-// G = next_pow2(P), as the API does.  false if the surface has no such variant
-// or the block is too large for the kernel.
+// bead: U tpb threads per trajectory, rounded up to a warp.  false if the surface has no such variant or the block is too
+// large for the kernel.
 bool apply_shape(cr_engine* e, int groups, int tpb) {
   const cr::PesRuns* r = cr::pes_runs(e->cfg.pes);
   if (!r || (tpb != 1 && tpb != 2 && tpb != 4) || tpb > r->max_tpb) return false;
-  const cr::PropDims d = cr::prop_dims(e->P);
-  const int U = e->prm.U;
-  // where the block would be too large, fewer threads per bead, then fewer
-  // trajectories (the results do not depend on either)
-  int subs = tpb, gpb = std::min(groups, e->T);
-  while (subs > 1 && U * subs > cr::kStepThreads) subs /= 2;
-  auto fits = [&](int n) { return n * U * subs <= cr::kStepThreads && cr::step_smem_bytes(d, U, e->NC, n) <= (size_t)cr::kStepSmemMax; };
-  while (gpb > 1 && !fits(gpb)) --gpb;
-  if (!fits(gpb)) return false;
-  const size_t smem = cr::step_smem_bytes(d, U, e->NC, gpb);
-  const int threads = (std::max(gpb * U * subs, gpb == 1 ? e->min_threads : 0) + 31) / 32 * 32;
-  e->block = groups * e->G * tpb;
+  int subs;
+  const int U = e->prm.U, gpb = fitting_groups(e, groups, tpb, &subs);
+  if (gpb < 1) return false;
+  e->block = std::max(1, std::min(groups, nominal_groups(e, tpb))) * e->G * tpb;
   e->tpb = tpb;
-  e->grid = (e->T + groups - 1) / groups;
   e->gpb = gpb;
-  e->threads = threads;
-  e->smem = smem;
+  e->grid = (e->T + gpb - 1) / gpb;
+  e->threads = (std::max(gpb * U * subs, gpb == 1 ? e->min_threads : 0) + 31) / 32 * 32;
+  e->smem = cr::step_smem_bytes(cr::prop_dims(e->P), U, e->NC, gpb);
   e->prm.gpb = gpb;
   e->prm.subs = subs;
   return true;
 }
 
-// The same for the API's `block` threads per block: a multiple of G tpb, at
-// most 256, its scratch by the API's rule within 200 KB.
-bool set_launch_shape(cr_engine* e, int block, int tpb) {
+// Trajectories per block that the API's `block` threads name; 0: none.  The largest
+// block that it can name stands for the fullest one that the kernel runs, which may
+// take more trajectories (U is little more than half of G).
+int named_groups(const cr_engine* e, int block, int tpb) {
+  if (tpb != 1 && tpb != 2 && tpb != 4) return 0;
   const int GT = e->G * tpb;
-  if (GT < 1 || block < GT || block % GT || block > 256) return false;
-  const cr::PropDims d = cr::prop_dims(e->P);
-  const size_t nominal = 8 * ((size_t)3 * d.nr * (d.nu + d.nv) + 2 * (size_t)e->P +
-                              (block / GT) * ((size_t)2 * e->NC * e->G + (size_t)2 * e->NC * (d.su + d.sv) +
-                                              (size_t)((GT + 31) / 32) * 32));
-  if (nominal > 200 * 1024) return false;
-  return apply_shape(e, block / GT, tpb);
+  if (block < GT || block % GT) return 0;
+  const int groups = block / GT, most = nominal_groups(e, tpb);
+  if (groups > most) return 0;
+  return groups == most && most > 1 ? std::max(groups, cr::kStepThreads) : groups;
+}
+// Whether set_launch can ask for that many: the built-in choice and the autotuner keep
+// to such shapes, so that what they report can be set.
+bool has_name(const cr_engine* e, int groups, int tpb) {
+  const int named = nominal_groups(e, tpb);
+  int subs;
+  return (groups == 1 && named > 0) || groups < named || (named > 1 && groups == fitting_groups(e, cr::kStepThreads, tpb, &subs));
+}
+bool set_launch_shape(cr_engine* e, int block, int tpb) {
+  const int groups = named_groups(e, block, tpb);
+  return groups > 0 && apply_shape(e, groups, tpb);
 }
 
 // Built-in launch shape.  A batch of at most a trajectory per scheduler is
@@ -852,7 +884,7 @@ void choose_launch(cr_engine* e) {
   double best = 0.0;
   int pick = 1;
   for (int groups = 1; groups * e->prm.U <= cr::kStepThreads; ++groups) {
-    if (!apply_shape(e, groups, 1) || e->gpb != std::min(groups, e->T)) continue;
+    if (!has_name(e, groups, 1) || !apply_shape(e, groups, 1) || e->gpb != std::min(groups, e->T)) continue;
     int res = 1;
     if (!r || r->resident(mixed, e->threads, e->smem, &res) != cudaSuccess || res < 1) res = 1;
     const int blocks = (e->T + groups - 1) / groups, per_sm = (blocks + sms - 1) / sms;
@@ -1778,7 +1810,7 @@ int cr_engine_last_kernel_ms(const cr_engine* e, float* ms) {
 int cr_engine_launch_info(const cr_engine* e, int* grid, int* block, int* smem_bytes, int* launches) {
   if (!e) return fail(CR_ERR_ARG, "NULL engine");
   if (grid) *grid = e->grid;
-  if (block) *block = e->block;
+  if (block) *block = persistent(e) ? e->threads : e->block;  // as launched
   if (smem_bytes) *smem_bytes = (int)e->smem;
   if (launches) *launches = e->launches;
   return CR_OK;
@@ -2101,13 +2133,18 @@ int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* th
                             cudaMemcpyDeviceToDevice, e->stream);
     return err;
   };
-  const int groups0 = e->block / (e->G * e->tpb), tpb0 = e->tpb, istep0 = e->istep;
-  int best = groups0, best_tpb = tpb0, rc = CR_OK;
+  const int block0 = e->block, tpb0 = e->tpb, istep0 = e->istep;
+  int best = e->gpb, best_tpb = tpb0, rc = CR_OK;
   float best_ms = 0.f;
   cudaError_t err = copy_state(true);
   for (int tpb = 1; tpb <= 4 && rc == CR_OK && err == cudaSuccess; tpb *= 2) {
-    for (int m = 1; m * e->prm.U * tpb <= cr::kStepThreads && rc == CR_OK && err == cudaSuccess; m += m < 8 ? 1 : m / 4) {
-      if (!apply_shape(e, m, tpb)) continue;
+    int subs;
+    const int most = fitting_groups(e, cr::kStepThreads, tpb, &subs);
+    if (subs != tpb) break;
+    // one, two, ... trajectories per block, in wider steps from eight on, and the most
+    for (int m = 1, next = 1; m > 0 && rc == CR_OK && err == cudaSuccess; m = next <= most ? next : m < most ? most : 0) {
+      next = m + (m < 8 ? 1 : m / 4);
+      if (!has_name(e, m, tpb) || !apply_shape(e, m, tpb)) continue;
       // one untimed step (first launch of this shape), then the timed run
       for (int rep = 0; rep < 2 && rc == CR_OK; ++rep) {
         if ((rc = engine_run_async(e, rep == 0 ? 1 : nsteps))) break;
@@ -2132,11 +2169,11 @@ int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* th
   cudaFree(save_st);
   e->istep = istep0;
   if (rc) {
-    apply_shape(e, groups0, tpb0);
+    set_launch_shape(e, block0, tpb0);
     return rc;
   }
   if (err != cudaSuccess) {
-    apply_shape(e, groups0, tpb0);
+    set_launch_shape(e, block0, tpb0);
     return fail(CR_ERR_CUDA, cudaGetErrorString(err));
   }
   apply_shape(e, best, best_tpb);

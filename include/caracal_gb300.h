@@ -476,7 +476,8 @@ int cr_engine_kappa(cr_engine* e, double* num, double* denom, double* weights, i
 int cr_engine_set_parent(cr_engine* e, const cr_recross* rc);
 
 /* Device time of the last cr_engine_run / step kernel (CUDA events on the
- * engine's stream), launches issued by it, and the launch shape chosen. */
+ * engine's stream), launches issued by it, and its blocks, their threads and dynamic
+ * shared memory. */
 int cr_engine_last_kernel_ms(const cr_engine* e, float* ms);
 int cr_engine_launch_info(const cr_engine* e, int* grid, int* block, int* smem_bytes, int* launches);
 /* Device pointers of the state arrays (owned by the engine). */
@@ -571,18 +572,22 @@ int cr_engine_get_npt(cr_engine* e, double* box_bohr, double* pressure_au, doubl
  * 2 or 4; 4 is built for H3 and OH + H2, 1 for the others), threads_per_block
  * (a multiple of that, <= 256) sets how many trajectories share a block.  The
  * kernel itself runs at most 128 threads per block on the distinct beads and
- * reduces a shape that would take more; the results do not depend on the
+ * reduces a shape that would take more; the largest block that can be asked for is the
+ * fullest one that it runs.  The results do not depend on the
  * shape.  threads_per_block = 0 restores the built-in choice (one trajectory per
  * block for a batch of at most four per SM, else by a cost model).
+ * cr_engine_get_launch names the shape in use in these terms (what it returns can be
+ * set again); blocks is the number launched, and cr_engine_launch_info has a block's
+ * own threads.
  * No counterpart in the reference, which steps one trajectory at a time on
  * the host. */
 int cr_engine_set_launch(cr_engine* e, int threads_per_block, int threads_per_bead);
 int cr_engine_get_launch(cr_engine* e, int* threads_per_block, int* blocks, int* threads_per_bead);
 /* Autotuner: times nsteps steps at each launch shape (threads per bead 1, 2,
- * 4 as built; from one trajectory per block up to what fits 128 threads),
+ * 4 as built; from one trajectory per block up to the fullest block),
  * each from the same saved state, which is then put back (q, p, f, epot,
  * status, chain velocities, a thermostat's momentum parts, step counter);
- * keeps the fastest and returns it with its time per step.  The noise is a
+ * keeps the fastest and returns it, as cr_engine_set_launch takes it, with its time per step.  The noise is a
  * function of the step index, so the trials leave no trace in the run. */
 int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* threads_per_bead,
                        float* ms_per_step);
