@@ -233,11 +233,26 @@ __global__ void __launch_bounds__(kSumCols * kSumRows) sum_rows_kernel(int nrows
 
 }  // namespace cr
 
+namespace {
+
+// A kernel's limit on dynamic shared memory is the process's, whichever force field
+// asks: always the most that a block may take, so that none lowers what another (in
+// another thread) is about to launch.
+template <class K>
+int allow_smem(K kernel, size_t bytes) {
+  constexpr int kMost = 227 * 1024;
+  if (bytes > (size_t)kMost) return cr_set_error(CR_ERR_CUDA, cudaGetErrorString(cudaErrorInvalidValue));
+  CR_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+  return CR_OK;
+}
+
+}  // namespace
+
 int qmdff_hvp_launch(const cr_qmdff* ff, const double* d_q, const double* d_w, int nbeads, double* d_e, double* d_g,
                      double* d_hw, double* d_dew, cudaStream_t s, cr::BeadRows rows) {
   if (ff->nterm[4] > 0) return cr_set_error(CR_ERR_UNSUPPORTED, "second derivatives of H/halogen-bond terms are not built");
   const size_t smem = cr::qmdff::team_hvp_smem_bytes(ff->n);
-  CR_TRY_CUDA(cudaFuncSetAttribute(cr::qmdff_hvp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (const int rc = allow_smem(cr::qmdff_hvp_kernel, smem)) return rc;
   if (nbeads == 0) return CR_OK;
   const int grid = std::min(nbeads, 1 << 20);
   cr::qmdff_hvp_kernel<<<grid, cr::kTeamThreads, smem, s>>>(ff->dev, nbeads, rows, d_q, d_w, d_e, d_g, d_hw, d_dew);
@@ -253,7 +268,7 @@ int qmdff_vjp_launch(const cr_qmdff* ff, const double* d_q, const double* d_v, i
   if (ff->nterm[4] > 0) return cr_set_error(CR_ERR_UNSUPPORTED, "parameter gradients of H/halogen-bond terms are not built");
   const int nlin = qmdff_nlin(ff);
   const size_t smem = (size_t)2 * 3 * ff->n * sizeof(double);
-  CR_TRY_CUDA(cudaFuncSetAttribute(cr::qmdff_vjp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (const int rc = allow_smem(cr::qmdff_vjp_kernel, smem)) return rc;
   if (nlin == 0) return CR_OK;
   for (int b0 = 0; b0 < nbeads; b0 += scratch_beads) {
     const int nb = std::min(scratch_beads, nbeads - b0);
@@ -294,6 +309,13 @@ size_t egrad_smem(int prec, int n) {
   return prec == 1 ? (size_t)kQmdffWarps * cr::qmdff::warp_smem_bytes(n) : cr::qmdff::team_smem_bytes(n);
 }
 
+int allow_egrad_smem(int prec, size_t smem) {
+  if (smem <= 48 * 1024) return CR_OK;
+  int rc = allow_smem(kBoxKernels[prec], smem);
+  for (int v = 0; v < kVariants && rc == CR_OK; ++v) rc = allow_smem(kKernels[prec][v], smem);
+  return rc;
+}
+
 int launch_dev(const cr::qmdff::Dev& D, int prec, int v, cr::BeadRows rows, const double* d_q, int nbeads, double* d_e, double* d_g,
                cudaStream_t s) {
   const size_t smem = egrad_smem(prec, D.n);
@@ -318,7 +340,7 @@ int launch_npt(const cr_qmdff* ff, int prec, const QmdffNpt& npt, cr::BeadRows r
   D.vir = npt.vir;
   const size_t smem = egrad_smem(prec, D.n);
   if (smem > 48 * 1024)
-    CR_TRY_CUDA(cudaFuncSetAttribute(kNptKernels[prec], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (const int rc = allow_smem(kNptKernels[prec], smem)) return rc;
   if (nbeads <= 0) return CR_OK;
   const int grid = egrad_grid(prec, nbeads);
   kNptKernels[prec]<<<grid, egrad_threads(prec), smem, s>>>(D, nbeads, rows, d_q, d_e, d_g);
@@ -335,11 +357,7 @@ int qmdff_launch_kinds(const cr_qmdff* ff, unsigned mask, bool ezero, const doub
   if (precision != CR_PREC_MIXED && precision != CR_PREC_FP64) return cr_set_error(CR_ERR_ARG, "unknown precision");
   const int prec = precision == CR_PREC_MIXED ? 1 : 0;
   const size_t smem = egrad_smem(prec, ff->n);
-  if (smem > 48 * 1024) {
-    for (int v = 0; v < kVariants; ++v)
-      CR_TRY_CUDA(cudaFuncSetAttribute(kKernels[prec][v], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CR_TRY_CUDA(cudaFuncSetAttribute(kBoxKernels[prec], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  }
+  if (const int rc = allow_egrad_smem(prec, smem)) return rc;
   if (nbeads <= 0) return CR_OK;
   cr::qmdff::Dev D = ff->dev;
   for (int p = 0; p < 2; ++p)
@@ -408,11 +426,7 @@ int qmdff_launch(const cr_qmdff* ff_c, const double* d_q, int nbeads, double* d_
   const size_t smem = egrad_smem(prec, ff->n);
   // the attribute is set even for nbeads = 0, so a caller can prepare the
   // kernels before a stream capture
-  if (smem > 48 * 1024) {
-    for (int v = 0; v < kVariants; ++v)
-      CR_TRY_CUDA(cudaFuncSetAttribute(kKernels[prec][v], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CR_TRY_CUDA(cudaFuncSetAttribute(kBoxKernels[prec], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  }
+  if (const int rc = allow_egrad_smem(prec, smem)) return rc;
   if (nbeads <= 0) return CR_OK;
   int choice = ff->variant[prec];
   if (choice < 0) {
