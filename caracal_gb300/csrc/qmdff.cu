@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(MIXED ? kQmdffThreads : kTeamThreads, MINB)
 }
 
 // Energy, gradient and Hessian-vector product H w per bead (plain form, dual
-// coordinates), a block per bead; dew[b] = w . grad E.
+// coordinates), a block per bead (hvp_threads); dew[b] = w . grad E.
 __global__ void __launch_bounds__(kTeamThreads)
     qmdff_hvp_kernel(qmdff::Dev D, int nbeads, BeadRows rows, const double* q, const double* w, double* e, double* g,
                      double* hw, double* dew) {
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(kTeamThreads)
     const size_t r = rows.row(b), r2 = rows.twin(b);
     const double* qb = q + r * n3;
     const double* wb = w + r * n3;
-    for (int a = threadIdx.x; a < n3; a += kTeamThreads) {
+    for (int a = threadIdx.x; a < n3; a += blockDim.x) {
       qsm[a] = qb[a];
       qsm[n3 + a] = wb[a];
     }
@@ -246,6 +246,17 @@ int allow_smem(K kernel, size_t bytes) {
   return CR_OK;
 }
 
+// Threads of a bead's block in the Hessian product: warps for the terms of the
+// largest kind and for the coordinates, kTeam at most. With eight warps a molecule of a
+// few atoms leaves all but one or two at the barriers, and registers let an SM hold
+// one such block only: host calls, C2H6 65 536 beads 22.1 -> 7.4 ms, C4H10 8192
+// beads 3.05 -> 1.19 ms, C6H14 (four warps) and larger unchanged.
+int hvp_threads(const cr_qmdff* ff) {
+  int most = 3 * ff->n;
+  for (int k = 0; k < 4; ++k) most = std::max(most, ff->nterm[k]);
+  return 32 * std::min((most + 31) / 32, cr::qmdff::kTeam);
+}
+
 }  // namespace
 
 int qmdff_hvp_launch(const cr_qmdff* ff, const double* d_q, const double* d_w, int nbeads, double* d_e, double* d_g,
@@ -255,7 +266,7 @@ int qmdff_hvp_launch(const cr_qmdff* ff, const double* d_q, const double* d_w, i
   if (const int rc = allow_smem(cr::qmdff_hvp_kernel, smem)) return rc;
   if (nbeads == 0) return CR_OK;
   const int grid = std::min(nbeads, 1 << 20);
-  cr::qmdff_hvp_kernel<<<grid, cr::kTeamThreads, smem, s>>>(ff->dev, nbeads, rows, d_q, d_w, d_e, d_g, d_hw, d_dew);
+  cr::qmdff_hvp_kernel<<<grid, hvp_threads(ff), smem, s>>>(ff->dev, nbeads, rows, d_q, d_w, d_e, d_g, d_hw, d_dew);
   CR_TRY_CUDA(cudaGetLastError());
   return CR_OK;
 }

@@ -1201,7 +1201,7 @@ __device__ inline void kind_segments_dual(const Dev& D, const BeadPos& X, double
   const Schedule& S = D.sched[0];
   for (int sgi = S.seg0[KIND]; sgi < S.seg1[KIND]; ++sgi) {
     const int4 sg = __ldg(S.seg + sgi);
-    for (int i = threadIdx.x; i < sg.y; i += kTeam * 32) {
+    for (int i = threadIdx.x; i < sg.y; i += blockDim.x) {
       const int m = sg.x + i;
       Contrib<Dual> c;
       if constexpr (KIND == 0) es += bond_plain<Dual>(D, D.d, X, m, c);
@@ -1217,7 +1217,7 @@ __device__ inline void kind_segments_dual(const Dev& D, const BeadPos& X, double
         }
     }
     __syncthreads();
-    gather(S, sg, threadIdx.x >> 5, kTeam, threadIdx.x & 31, [&](int a, const unsigned short* l, int n) {
+    gather(S, sg, threadIdx.x >> 5, blockDim.x >> 5, threadIdx.x & 31, [&](int a, const unsigned short* l, int n) {
       double v = g[a], t = h[a];
 #pragma unroll 4
       for (int j = 0; j < n; ++j) {
@@ -1239,7 +1239,7 @@ __host__ __device__ inline size_t team_hvp_smem_bytes(int n) {
 }
 
 // Energy (with E_zero), gradient and Hessian-vector product H w of one bead
-// by a block of kTeam warps.  ws: the block's shared memory holding x (3n
+// by a block of up to kTeam warps.  ws: the block's shared memory holding x (3n
 // doubles) then w (3n doubles; a barrier follows here).  gout, gout2, hout, hout2: the
 // destinations (equal: one).  dew receives the directional derivative w . grad E.
 __device__ inline double team_hvp(const Dev& D, double* ws, double* gout, double* gout2, double* hout, double* hout2,
@@ -1250,7 +1250,7 @@ __device__ inline double team_hvp(const Dev& D, double* ws, double* gout, double
   double* h = g + n3;
   double* buf = h + n3;
   double* red = buf + 2 * (buffer_values(false) + 1);
-  for (int a = tid; a < 2 * n3; a += kTeam * 32) g[a] = 0.0;
+  for (int a = tid; a < 2 * n3; a += blockDim.x) g[a] = 0.0;
   if (tid < 2) buf[tid * (buffer_values(false) + 1) + buffer_values(false)] = 0.0;
   __syncthreads();
   PBox tb;
@@ -1267,14 +1267,13 @@ __device__ inline double team_hvp(const Dev& D, double* ws, double* gout, double
     red[kTeam + warp] = d1;
   }
   __syncthreads();
-  for (int a = tid; a < n3; a += kTeam * 32) {
+  for (int a = tid; a < n3; a += blockDim.x) {
     if (gout) gout[a] = gout2[a] = g[a];
     hout[a] = hout2[a] = h[a];
   }
   double e = 0.0;
   dew = 0.0;
-#pragma unroll
-  for (int k = 0; k < kTeam; ++k) {
+  for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
     e += red[k];
     dew += red[kTeam + k];
   }
