@@ -415,45 +415,60 @@ void build_pile(int P, double beta, double dt, double tau0, std::vector<double>&
 // The persistent kernel's linear maps as limbs under one exponent each:
 // the propagator blocks on folded rows x_l + x_{M-l}, x_l - x_{M-l} of the
 // distinct beads (odd P: on the rows themselves; a bead that stands for two
-// counts twice), and the PILE circulants between the carried beads.
-void persistent_maps(cr_engine* e, const cr::PropDims& pd, const std::vector<double>& ke, const std::vector<double>& ko,
-                     const std::vector<double>& pile, std::vector<cr::Limbs>& maps, size_t& off_ko, size_t& off_pile) {
+// counts twice), and the PILE maps between the carried beads; in nm_mode 1,
+// which carries all beads, the circulants themselves.  Offsets into `maps`.
+struct MapOffsets {
+  size_t ko = 0, pile = 0;
+};
+MapOffsets persistent_maps(cr_engine* e, const cr::PropDims& pd, const std::vector<double>& ke,
+                           const std::vector<double>& ko, const std::vector<double>& pile, const std::vector<double>& circ,
+                           std::vector<cr::Limbs>& maps) {
   cr::StepParams& s = e->prm;
   const int P = e->P, pair = e->cfg.nm_mode == 0 ? 1 : 0, U = pair ? P / 2 + 1 : P;
   s.pair = pair;
   s.U = U;
   s.guard = cr::fixed_guard(pd.nu);
   s.pguard = cr::fixed_guard(U);
-  std::vector<double> me(ke), mo(ko);
-  mo.resize((size_t)3 * pd.nr * pd.nv);
-  for (size_t x = 0; x < me.size(); ++x)
-    if (x % pd.nu != 0) me[x] *= 2.0;
-  for (size_t x = 0; x < mo.size(); ++x)
-    if (x % pd.nv != 0) mo[x] *= 2.0;
-  const size_t ne = (size_t)pd.nr * pd.nu, no = (size_t)pd.nr * pd.nv;
-  for (int w = 0; w < 3; ++w) {
-    std::vector<double> both(me.begin() + w * ne, me.begin() + (w + 1) * ne);
-    both.insert(both.end(), mo.begin() + w * no, mo.begin() + (w + 1) * no);
-    s.ek[w] = cr::fixed_exponent(both);
+  MapOffsets off;
+  // part w of a table of equal parts, under its own exponent
+  auto put = [&](const std::vector<double>& v, int w, size_t n, int ek) {
+    cr::fixed_limbs(std::vector<double>(v.begin() + w * n, v.begin() + (w + 1) * n), ek, maps);
+  };
+  auto exponent = [&](const std::vector<double>& v, int w, size_t n) {
+    return cr::fixed_exponent(std::vector<double>(v.begin() + w * n, v.begin() + (w + 1) * n));
+  };
+  const size_t np = (size_t)P;
+  if (!pair) {
+    for (int w = 0; w < 3; ++w) put(circ, w, np, s.ek[w] = exponent(circ, w, np));
+  } else {
+    std::vector<double> me(ke), mo(ko);
+    mo.resize((size_t)3 * pd.nr * pd.nv);
+    for (size_t x = 0; x < me.size(); ++x)
+      if (x % pd.nu != 0) me[x] *= 2.0;
+    for (size_t x = 0; x < mo.size(); ++x)
+      if (x % pd.nv != 0) mo[x] *= 2.0;
+    const size_t ne = (size_t)pd.nr * pd.nu, no = (size_t)pd.nr * pd.nv;
+    for (int w = 0; w < 3; ++w) put(me, w, ne, s.ek[w] = std::max(exponent(me, w, ne), exponent(mo, w, no)));
+    off.ko = maps.size();
+    for (int w = 0; w < 3; ++w) put(mo, w, no, s.ek[w]);
   }
-  for (int w = 0; w < 3; ++w)
-    cr::fixed_limbs(std::vector<double>(me.begin() + w * ne, me.begin() + (w + 1) * ne), s.ek[w], maps);
-  off_ko = maps.size();
-  for (int w = 0; w < 3; ++w)
-    cr::fixed_limbs(std::vector<double>(mo.begin() + w * no, mo.begin() + (w + 1) * no), s.ek[w], maps);
-  off_pile = maps.size();
-  if (e->cfg.thermostat != CR_THERMO_PILE) return;
+  off.pile = maps.size();
+  if (e->cfg.thermostat != CR_THERMO_PILE) return off;
   for (int w = 0; w < 2; ++w) {
+    if (!pair) {
+      put(pile, w, np, s.ep[w] = exponent(pile, w, np));
+      continue;
+    }
     std::vector<double> m((size_t)U * U);
     for (int l = 0; l < U; ++l)
       for (int j = 0; j < U; ++j) {
         double v = pile[(size_t)w * P + ((j - l) % P + P) % P];
-        if (pair && l > 0 && 2 * l != P) v += pile[(size_t)w * P + (j + l) % P];
+        if (l > 0 && 2 * l != P) v += pile[(size_t)w * P + (j + l) % P];
         m[(size_t)l * U + j] = v;
       }
-    s.ep[w] = cr::fixed_exponent(m);
-    cr::fixed_limbs(m, s.ep[w], maps);
+    put(m, 0, m.size(), s.ep[w] = cr::fixed_exponent(m));
   }
+  return off;
 }
 
 // Persistent run of nsteps steps.  dev_step: the first step index is read
@@ -1168,8 +1183,8 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
   else circ.assign((size_t)3 * e->P, 0.0);
   // the persistent kernel's maps on the carried beads, as limbs (fixed_map.cuh)
   std::vector<cr::Limbs> maps;
-  size_t map_ko = 0, map_pile = 0;
-  if (!e->split) persistent_maps(e, pd, ke, ko, pile, maps, map_ko, map_pile);
+  MapOffsets at;
+  if (!e->split) at = persistent_maps(e, pd, ke, ko, pile, circ, maps);
   if (!maps.empty() &&
       (cudaMalloc(&e->d_maps, maps.size() * sizeof(cr::Limbs)) != cudaSuccess ||
        cudaMemcpy(e->d_maps, maps.data(), maps.size() * sizeof(cr::Limbs), cudaMemcpyHostToDevice) != cudaSuccess))
@@ -1327,10 +1342,10 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
   s.inv_P = 1.0 / e->P;
   s.kap = (2.0 - tm / totmass) / totmass;
   s.nm_mode = cfg->nm_mode;
-  s.circ = e->d_circ;
+  s.circ = e->d_maps;
   s.ke = e->d_maps;
-  s.ko = e->d_maps + map_ko;
-  s.pile = e->d_maps + map_pile;
+  s.ko = e->d_maps + at.ko;
+  s.pile = e->d_maps + at.pile;
   s.pile_b = e->d_pile + e->P;
   s.q = e->d_q;
   s.p = e->d_p;

@@ -244,7 +244,7 @@ struct StepParams {
   int guard;           // guard bits of the folded rows (fixed_map.cuh)
   int fast_M;          // P / 2 where the free ring polymer takes the fast transforms (ring_fast.cuh), else 0
   FastRing fast;
-  const Limbs* pile;   // [2][U][U] friction and noise maps on the carried beads, [w][l][j]
+  const Limbs* pile;   // pairs: [2][U][U] friction and noise maps on the carried beads, [w][l][j]; else the circulants [2][P]
   int ep[2];
   int pguard;
   const double* pile_b;  // [P] noise circulant (the antisymmetric part at the end of a run)
@@ -274,7 +274,7 @@ struct StepParams {
   // nm_mode 1 (orthonormal normal modes): K1, K2, K3 are circulant, row j
   // holds circ[w][(j - l) mod P] (unit mass)
   int nm_mode;
-  const double* circ;  // [3][P]
+  const Limbs* circ;  // [3][P], under the exponents ek
 };
 
 // Non-finite test on the exponent bits (integer pipe, no FP64 compare).
@@ -677,11 +677,23 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
     for (int x = tid; x < flat; x += nth) {
       const int r = x / U, k = x - r * U;
       FixedSum a{0, 0}, e{0, 0};
-      const Limbs* ka = prm.pile + k;
-      const Limbs* kb = ka + U * U;
-      for (int l = 0; l < U; ++l) {
-        a.add(limbs[r * U + l], ldg_limbs(ka + l * U));
-        e.add(le[r * U + l], ldg_limbs(kb + l * U));
+      const Limbs* lp = limbs + r * U;
+      const Limbs* ln = le + r * U;
+      if (prm.pair) {
+        const Limbs* ka = prm.pile + k;
+        const Limbs* kb = ka + U * U;
+        for (int l = 0; l < U; ++l) {
+          a.add(lp[l], ldg_limbs(ka + l * U));
+          e.add(ln[l], ldg_limbs(kb + l * U));
+        }
+      } else {
+        int m = k;  // (k - l) mod P
+#pragma unroll 4
+        for (int l = 0; l < U; ++l) {
+          a.add(lp[l], ldg_limbs(prm.pile + m));
+          e.add(ln[l], ldg_limbs(prm.pile + P + m));
+          m = (m == 0) ? P - 1 : m - 1;
+        }
       }
       const int c = r % NC;
       double v = from_fixed(a.value(), prm.ep[0] + sexp[r] - 1077 + prm.pguard);
@@ -725,29 +737,37 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
     // free ring polymer (src/verlet.f90:377-463): Caracal's cosine modes, or
     // orthonormal normal modes where nm_mode is set
     if (prm.nm_mode) {
-      for (int x = tid; x < flat; x += nth) {
-        const int r = x / U, k = x - r * U, c = r % NC;
-        const double* xp = sp + r * U;
-        const double* xq = sq + r * U;
-        double a1p = 0.0, a1q = 0.0, a2q = 0.0, a3p = 0.0;
-        int m = k;  // (k - l) mod P
-        for (int l = 0; l < P; ++l) {
-          const double c1 = __ldg(prm.circ + m), c2 = __ldg(prm.circ + P + m), c3 = __ldg(prm.circ + 2 * P + m);
-          a1p = fma(c1, xp[l], a1p);
-          a1q = fma(c1, xq[l], a1q);
-          a2q = fma(c2, xq[l], a2q);
-          a3p = fma(c3, xp[l], a3p);
-          m = (m == 0) ? P - 1 : m - 1;
-        }
-        area[x] = fma(prm.mass[c / 3], a2q, a1p);
-        area[flat + x] = fma(prm.inv_mass[c / 3], a3p, a1q);
-      }
+      // circulants, on the rows as limbs: the 4 P^2 products per coordinate held the
+      // FP64 pipe (H3 per step: 1 x 128 PILE mixed 684 -> 269 us with the noise's circulants
+      // below, 200 x 128 without a thermostat plain 362 -> 181)
+      for (int x = tid; x < 2 * rows; x += nth) sexp[x] = row_exponent(x < rows ? sq + x * U : sp + (x - rows) * U, U);
+      __syncthreads();
+      for (int x = tid; x < 2 * flat; x += nth)
+        limbs[x] = to_limbs(to_fixed(x < flat ? sq[x] : sp[x - flat], sexp[x / U], prm.pguard));
       __syncthreads();
       for (int x = tid; x < flat; x += nth) {
-        const double qn = area[flat + x];
-        sp[x] = area[x];
-        sq[x] = qn;
-        if (nonfinite_bits(qn)) atomicOr(&sstat[x / (NC * U)], CR_TRAJ_NONFINITE);
+        const int r = x / U, k = x - r * U, c = r % NC;
+        const Limbs* lq = limbs + r * U;
+        const Limbs* lp = lq + flat;
+        FixedSum a1q{0, 0}, a1p{0, 0}, a2q{0, 0}, a3p{0, 0};
+        int m = k;  // (k - l) mod P
+#pragma unroll 4
+        for (int l = 0; l < P; ++l) {
+          const Limbs vq = lq[l], vp = lp[l], w1 = ldg_limbs(prm.circ + m);
+          a1q.add(vq, w1);
+          a1p.add(vp, w1);
+          a2q.add(vq, ldg_limbs(prm.circ + P + m));
+          a3p.add(vp, ldg_limbs(prm.circ + 2 * P + m));
+          m = (m == 0) ? P - 1 : m - 1;
+        }
+        const int sq_e = sexp[r] - 1078 + prm.pguard, sp_e = sexp[rows + r] - 1078 + prm.pguard;
+        const bool bad = sexp[r] == kFixedNan || sexp[rows + r] == kFixedNan;
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+        const double pn = fma(prm.mass[c / 3], from_fixed(a2q.value(), prm.ek[1] + sq_e), from_fixed(a1p.value(), prm.ek[0] + sp_e));
+        const double qn = fma(prm.inv_mass[c / 3], from_fixed(a3p.value(), prm.ek[2] + sp_e), from_fixed(a1q.value(), prm.ek[0] + sq_e));
+        sp[x] = bad ? nan : pn;
+        sq[x] = bad ? nan : qn;
+        if (bad || nonfinite_bits(qn)) atomicOr(&sstat[r / NC], CR_TRAJ_NONFINITE);
       }
     } else if (prm.fast_M) {
       if (prm.fast_M == 16) ring_rows<16, NC>(prm, sq, sp, rows, sstat);
