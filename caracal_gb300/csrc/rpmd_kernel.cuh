@@ -476,6 +476,92 @@ __device__ inline bool transrot_quad(Tot tot, int lane, double itm, double kap, 
   return tpp != 0.0 && s1 != 0.0 && s3 != 0.0;
 }
 
+// transrot of one trajectory by one thread, for ring polymers of few carried beads
+// (rows q, p of NC x U in shared memory, bead j > 0 of odd P standing for two): the
+// reference's sums over atoms and beads about its centre (src/transrot.f90:36-237),
+// in FP64, the inertia tensor solved with pivots on the diagonal as in transrot_quad.
+// With one bead that is some 40 FP64 operations per atom and 100 for the solve, where
+// the moments by limbs take 18 tasks of a hundred instructions per atom whatever the
+// number of beads: H3 100 000 x 1 mixed 267 -> 111 us per step, plain 387 -> 232; with two,
+// 20 000 x 2 mixed 95 -> 65. false: singular.
+constexpr int kFewBeads = 2;
+template <int N>
+__device__ inline bool transrot_thread(const double* q, double* p, int U, int P, int pair, const double* mass, double itm) {
+  auto count = [&](int j) { return pair && j > 0 && 2 * j != P ? 2.0 : 1.0; };
+  double sp[3] = {0.0, 0.0, 0.0}, sq[3] = {0.0, 0.0, 0.0}, L[3] = {0.0, 0.0, 0.0};
+  for (int j = 0; j < U; ++j) {
+    const double k = count(j);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      double x[3], y[3];
+      const double w = k * mass[i];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        x[d] = q[(3 * i + d) * U + j];
+        y[d] = k * p[(3 * i + d) * U + j];
+        sp[d] += y[d];
+        sq[d] = fma(w, x[d], sq[d]);
+      }
+      L[0] += fma(x[1], y[2], -x[2] * y[1]);
+      L[1] += fma(x[2], y[0], -x[0] * y[2]);
+      L[2] += fma(x[0], y[1], -x[1] * y[0]);
+    }
+  }
+  const double xt[3] = {sq[0] * itm, sq[1] * itm, sq[2] * itm}, vt[3] = {sp[0] * itm, sp[1] * itm, sp[2] * itm};
+  L[0] -= fma(xt[1], sp[2], -xt[2] * sp[1]);
+  L[1] -= fma(xt[2], sp[0], -xt[0] * sp[2]);
+  L[2] -= fma(xt[0], sp[1], -xt[1] * sp[0]);
+  double c[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // xx, yy, zz, yz, zx, xy
+  for (int j = 0; j < U; ++j) {
+    const double k = count(j);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      double x[3], wx[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        x[d] = q[(3 * i + d) * U + j] - xt[d];
+        wx[d] = k * mass[i] * x[d];
+        c[d] = fma(wx[d], x[d], c[d]);
+      }
+      c[3] = fma(wx[1], x[2], c[3]);
+      c[4] = fma(wx[2], x[0], c[4]);
+      c[5] = fma(wx[0], x[1], c[5]);
+    }
+  }
+  const double e = N <= 2 ? 0.000001 : 0.0;
+  const double t0 = c[1] + c[2] + e, t1 = c[2] + c[0] + e, t2 = c[0] + c[1] + e;
+  // axes p, q, r in cyclic order with the largest diagonal element first
+  const int a = fabs(t0) >= fabs(t1) ? (fabs(t0) >= fabs(t2) ? 0 : 2) : (fabs(t1) >= fabs(t2) ? 1 : 2);
+  auto from = [&](int k, double u, double v, double w) { return k == 0 ? u : k == 1 ? v : w; };
+  const int b = a == 2 ? 0 : a + 1, f = a == 0 ? 2 : a - 1;
+  const double tpp = from(a, t0, t1, t2), tqq = from(b, t0, t1, t2), trr = from(f, t0, t1, t2);
+  const double tqr = -from(a, c[3], c[4], c[5]), tpr = -from(b, c[3], c[4], c[5]), tpq = -from(f, c[3], c[4], c[5]);
+  const double Lp = from(a, L[0], L[1], L[2]), Lq = from(b, L[0], L[1], L[2]), Lr = from(f, L[0], L[1], L[2]);
+  const double ip = fx::rcp(tpp), m1 = tpq * ip, m2 = tpr * ip;
+  const double sqq = fma(-m1, tpq, tqq), srr = fma(-m2, tpr, trr), sqr = fma(-m1, tpr, tqr);
+  const double yq = fma(-m1, Lp, Lq), yr = fma(-m2, Lp, Lr);
+  const bool swap = fabs(srr) > fabs(sqq);
+  const double s1 = swap ? srr : sqq, s2 = swap ? sqq : srr, y1 = swap ? yr : yq, y2 = swap ? yq : yr;
+  const double i1 = fx::rcp(s1), m3 = sqr * i1, s3 = fma(-m3, sqr, s2);
+  if (tpp == 0.0 || s1 == 0.0 || s3 == 0.0) return false;
+  const double v2 = fma(-m3, y1, y2) * fx::rcp(s3), v1 = fma(-sqr, v2, y1) * i1;
+  const double vq = swap ? v2 : v1, vr = swap ? v1 : v2, vp = fma(-tpr, vr, fma(-tpq, vq, Lp)) * ip;
+  // axis 0 is p, r or q as p is 0, 1 or 2, and so on round
+  const double va[3] = {from(a, vp, vr, vq), from(a, vq, vp, vr), from(a, vr, vq, vp)};
+  for (int j = 0; j < U; ++j)
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      double x[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) x[d] = q[(3 * i + d) * U + j] - xt[d];
+      const double u[3] = {fma(va[1], x[2], fma(-va[2], x[1], vt[0])), fma(va[2], x[0], fma(-va[0], x[2], vt[1])),
+                           fma(va[0], x[1], fma(-va[1], x[0], vt[2]))};
+#pragma unroll
+      for (int d = 0; d < 3; ++d) p[(3 * i + d) * U + j] = fma(-mass[i], u[d], p[(3 * i + d) * U + j]);
+    }
+  return true;
+}
+
 // x[k] of an array in registers
 __device__ __forceinline__ double pick(const double (&x)[16], int k) {
   double r = x[0];
@@ -950,7 +1036,12 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
 
     // transrot (src/transrot.f90:36-237): removed COM velocity and rotation
     // centre both carry Caracal's extra 1/P (total mass P^2 sum m)
-    if (prm.transrot) {
+    if (prm.transrot && U <= kFewBeads) {
+      for (int gg = tid; gg < ng; gg += nth)
+        if (!transrot_thread<N>(sq + gg * NC * U, sp + gg * NC * U, U, P, prm.pair, prm.mass, prm.itm))
+          atomicOr(&sstat[gg], CR_TRAJ_SINGULAR_INERTIA);
+      __syncthreads();
+    } else if (prm.transrot) {
       // rows of q and p as limbs; per atom the bead sums of p, q, q_a p_b and
       // q_a q_b in fixed point (in FP64 some 20 instructions per bead and atom, and the
       // solve on one lane: per step H3 64 x 16 PILE mixed 32.2 -> 24.8 us, OH + H2 1000 x 24
