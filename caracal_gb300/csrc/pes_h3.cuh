@@ -23,6 +23,7 @@
 
 #include "ff32.cuh"
 #include "fx64.cuh"
+#include "num.cuh"
 
 #define K4(x) (F)(x##f)
 #define K8(x) (F)(x)
@@ -30,17 +31,20 @@
 namespace cr {
 namespace h3 {
 
+// The surface is written for F = Num<double> or Num<float> (num.cuh): its two forms,
+// by one thread and by four lanes, then agree bit for bit, so that which one a batch
+// takes shows in nothing but the time.
 template <class F> __device__ inline F fexp(F x);
-template <> __device__ inline double fexp<double>(double x) { return fx::exp(x); }
-template <> __device__ inline float fexp<float>(float x) { return expf(x); }
+template <> __device__ inline Num<double> fexp<Num<double>>(Num<double> x) { return fx::exp(x.v); }
+template <> __device__ inline Num<float> fexp<Num<float>>(Num<float> x) { return expf(x.v); }
 template <class F> __device__ inline F fpow(F x, F y);
-template <> __device__ inline double fpow<double>(double x, double y) { return fx::pow(x, y); }
-template <> __device__ inline float fpow<float>(float x, float y) { return powf(x, y); }
-__device__ inline void froot(double x, double& r, double& ir) { fx::sqrt_rsqrt(x, r, ir); }
-__device__ inline void froot(float x, float& r, float& ir) { f_root(x, r, ir); }
+template <> __device__ inline Num<double> fpow<Num<double>>(Num<double> x, Num<double> y) { return fx::pow(x.v, y.v); }
+template <> __device__ inline Num<float> fpow<Num<float>>(Num<float> x, Num<float> y) { return powf(x.v, y.v); }
+__device__ inline void froot(Num<double> x, Num<double>& r, Num<double>& ir) { fx::sqrt_rsqrt(x.v, r.v, ir.v); }
+__device__ inline void froot(Num<float> x, Num<float>& r, Num<float>& ir) { f_root(x.v, r.v, ir.v); }
 template <class F> __device__ inline F frcp(F x);
-template <> __device__ inline double frcp<double>(double x) { return fx::rcp(x); }
-template <> __device__ inline float frcp<float>(float x) { return f_rcp(x); }
+template <> __device__ inline Num<double> frcp<Num<double>>(Num<double> x) { return fx::rcp(x.v); }
+template <> __device__ inline Num<float> frcp<Num<float>>(Num<float> x) { return f_rcp(x.v); }
 
 // Schwenke H2 singlet E(R) and dE/dR (VH2OPT95).
 // The polynomial alpha(R) of the Schwenke curve sums terms up to ~1e6 at
@@ -48,12 +52,13 @@ template <> __device__ inline float frcp<float>(float x) { return f_rcp(x); }
 // exp(alpha) by orders of magnitude: alpha and dalpha/dR are always evaluated
 // in FP64 from the FP64 distance Rd; the rest follows the compute type F.
 template <class F>
-__device__ inline void singlet(double Rd, double ird, F R, F& E, F& dE) {
+__device__ inline void singlet(Num<double> Rd, Num<double> ird, F R, F& E, F& dE) {
+  using D = Num<double>;
   const F R0 = K8(3.5284882), DD = K8(0.160979391);
   const F C6 = K8(6.499027), C8 = K8(124.3991), C10 = K8(3285.828);
   // polynomial part a1 + a2 R + ... + a16 R^15 and its derivative, Horner
   // form, FP64 (the a_i are the same widened REAL(4)/REAL(8) values)
-  const double b0 = (double)(0.03537359271649620f), b1 = (double)(2.013977588700072f),
+  const D b0 = (double)(0.03537359271649620f), b1 = (double)(2.013977588700072f),
                b2 = (double)(-2.827452449964767f), b3 = (double)(2.713257715593500f),
                b4 = (double)(-2.792039234205731f), b5 = (double)(2.166542078766724f),
                b6 = (double)(-1.272679684173909f), b7 = (double)(0.5630423099212294f),
@@ -62,20 +67,20 @@ __device__ inline void singlet(double Rd, double ird, F R, F& E, F& dE) {
                b12 = -1.227820520228028e-04, b13 = 8.638783190083473e-06,
                b14 = -4.036967926499151e-07, b15 = 1.123286608335365e-08,
                b16 = -1.406619156782167e-10;
-  double pa = b16, pd = 15.0 * b16;
-  pa = pa * Rd + b15; pd = pd * Rd + 14.0 * b15;
-  pa = pa * Rd + b14; pd = pd * Rd + 13.0 * b14;
-  pa = pa * Rd + b13; pd = pd * Rd + 12.0 * b13;
-  pa = pa * Rd + b12; pd = pd * Rd + 11.0 * b12;
-  pa = pa * Rd + b11; pd = pd * Rd + 10.0 * b11;
-  pa = pa * Rd + b10; pd = pd * Rd + 9.0 * b10;
-  pa = pa * Rd + b9;  pd = pd * Rd + 8.0 * b9;
-  pa = pa * Rd + b8;  pd = pd * Rd + 7.0 * b8;
-  pa = pa * Rd + b7;  pd = pd * Rd + 6.0 * b7;
-  pa = pa * Rd + b6;  pd = pd * Rd + 5.0 * b6;
-  pa = pa * Rd + b5;  pd = pd * Rd + 4.0 * b5;
-  pa = pa * Rd + b4;  pd = pd * Rd + 3.0 * b4;
-  pa = pa * Rd + b3;  pd = pd * Rd + 2.0 * b3;
+  D pa = b16, pd = D(15.0) * b16;
+  pa = pa * Rd + b15; pd = pd * Rd + D(14.0) * b15;
+  pa = pa * Rd + b14; pd = pd * Rd + D(13.0) * b14;
+  pa = pa * Rd + b13; pd = pd * Rd + D(12.0) * b13;
+  pa = pa * Rd + b12; pd = pd * Rd + D(11.0) * b12;
+  pa = pa * Rd + b11; pd = pd * Rd + D(10.0) * b11;
+  pa = pa * Rd + b10; pd = pd * Rd + D(9.0) * b10;
+  pa = pa * Rd + b9;  pd = pd * Rd + D(8.0) * b9;
+  pa = pa * Rd + b8;  pd = pd * Rd + D(7.0) * b8;
+  pa = pa * Rd + b7;  pd = pd * Rd + D(6.0) * b7;
+  pa = pa * Rd + b6;  pd = pd * Rd + D(5.0) * b6;
+  pa = pa * Rd + b5;  pd = pd * Rd + D(4.0) * b5;
+  pa = pa * Rd + b4;  pd = pd * Rd + D(3.0) * b4;
+  pa = pa * Rd + b3;  pd = pd * Rd + D(2.0) * b3;
   pa = pa * Rd + b2;  pd = pd * Rd + b2;
   pa = pa * Rd + b1;
   F alpha = (F)(b0 * ird + pa);
@@ -122,7 +127,7 @@ __device__ inline void triplet(F R, F ir, F e1, F de1, F& E3, F& dE3) {
 }
 
 template <class F>
-__device__ __forceinline__ F lane_of(F x, int src) { return __shfl_sync(0xffffffffu, x, src, 4); }
+__device__ __forceinline__ Num<F> lane_of(Num<F> x, int src) { return Num<F>(__shfl_sync(0xffffffffu, x.v, src, 4)); }
 template <class F>
 __device__ __forceinline__ F pick3(int i, F a, F b, F c) { return i == 0 ? a : i == 1 ? b : c; }
 
@@ -131,7 +136,7 @@ __device__ __forceinline__ F pick3(int i, F a, F b, F c) { return i == 0 ? a : i
 // of distance i (Rd, iRd: its own in element 0), the lanes' parity the coefficient
 // set of the bend terms; they hold some 60 % of the instructions.
 template <class F, bool QUAD>
-__device__ inline void pote(const F (&R)[3], const F (&ir)[3], const double (&Rd)[3], const double (&iRd)[3], int lane, F& V,
+__device__ inline void pote(const F (&R)[3], const F (&ir)[3], const Num<double> (&Rd)[3], const Num<double> (&iRd)[3], int lane, F& V,
                             F (&dV)[3]) {
   // ---- London term (H3LOND95)
   F Q[3], J[3], dQ[3], dJ[3];
@@ -447,59 +452,63 @@ struct PesH3 {
   static constexpr int N = 3;
   static constexpr int kLanes = 1;  // per bead; small batches: four (quad)
   static constexpr bool kQuad = true;
+  using D = Num<double>;
+  // the gradient component of an atom: the difference of its two bonds' shares
   template <class F>
+  __device__ static __forceinline__ double share(Num<F> x, Num<F> y) { return (double)(D(x) - D(y)); }
+
+  template <class T>
   __device__ static inline void egrad(const double (&q)[9], double& V, double (&g)[9]) {
+    using F = Num<T>;
     F d[3][3];  // d[0]=q2-q1 (AB), d[1]=q1-q3 (AC), d[2]=q3-q2 (BC)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      d[0][c] = (F)(q[3 + c] - q[c]);
-      d[1][c] = (F)(q[c] - q[6 + c]);
-      d[2][c] = (F)(q[6 + c] - q[3 + c]);
-    }
     F R[3], iR[3];
-    double Rd[3], iRd[3];
+    D Rd[3], iRd[3];
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       const int i0 = (b == 0) ? 3 : (b == 1) ? 0 : 6, i1 = (b == 0) ? 0 : (b == 1) ? 6 : 3;
-      const double x = q[i0] - q[i1], y = q[i0 + 1] - q[i1 + 1], z = q[i0 + 2] - q[i1 + 2];
-      fx::sqrt_rsqrt(x * x + y * y + z * z, Rd[b], iRd[b]);
-      R[b] = (F)Rd[b];
-      iR[b] = (F)iRd[b];
+      const D x[3] = {D(q[i0]) - D(q[i1]), D(q[i0 + 1]) - D(q[i1 + 1]), D(q[i0 + 2]) - D(q[i1 + 2])};
+      h3::froot(x[0] * x[0] + x[1] * x[1] + x[2] * x[2], Rd[b], iRd[b]);
+      R[b] = F(Rd[b]);
+      iR[b] = F(iRd[b]);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) d[b][c] = F(x[c]);
     }
     F v, dv[3];
     h3::pote<F, false>(R, iR, Rd, iRd, 0, v, dv);
     V = (double)v;
-    F u[3] = {dv[0] * iR[0], dv[1] * iR[1], dv[2] * iR[2]};
+    const F u[3] = {dv[0] * iR[0], dv[1] * iR[1], dv[2] * iR[2]};
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      g[c] = (double)(u[1] * d[1][c]) - (double)(u[0] * d[0][c]);
-      g[3 + c] = (double)(u[0] * d[0][c]) - (double)(u[2] * d[2][c]);
-      g[6 + c] = (double)(u[2] * d[2][c]) - (double)(u[1] * d[1][c]);
+      const F a = u[0] * d[0][c], b = u[1] * d[1][c], e = u[2] * d[2][c];
+      g[c] = share(b, a);
+      g[3 + c] = share(a, e);
+      g[6 + c] = share(e, b);
     }
   }
 
   // The same by four lanes of a warp (get(c): coordinate c, put(c, x): gradient
   // component c; lane: 0..3, lane 0's V counts): 64 x 16 with PILE mixed 20.4 -> 16.5
   // us per step, plain 51 -> 38.
-  template <class F, class Get, class Put>
+  template <class T, class Get, class Put>
   __device__ static inline void quad(Get get, int lane, double& V, Put put) {
+    using F = Num<T>;
     double q[9];
 #pragma unroll
     for (int c = 0; c < 9; ++c) q[c] = get(c);
     F d[3][3];  // d[0]=q2-q1 (AB), d[1]=q1-q3 (AC), d[2]=q3-q2 (BC)
-    double own[3];
+    D own[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const double x0 = q[3 + c] - q[c], x1 = q[c] - q[6 + c], x2 = q[6 + c] - q[3 + c];
-      d[0][c] = (F)x0;
-      d[1][c] = (F)x1;
-      d[2][c] = (F)x2;
+      const D x0 = D(q[3 + c]) - D(q[c]), x1 = D(q[c]) - D(q[6 + c]), x2 = D(q[6 + c]) - D(q[3 + c]);
+      d[0][c] = F(x0);
+      d[1][c] = F(x1);
+      d[2][c] = F(x2);
       own[c] = h3::pick3(lane, x0, x1, x2);
     }
     F R[3], iR[3];
-    double Rd[3], iRd[3];  // the lane's own distance
-    fx::sqrt_rsqrt(own[0] * own[0] + own[1] * own[1] + own[2] * own[2], Rd[0], iRd[0]);
-    const F Rl = (F)Rd[0], iRl = (F)iRd[0];
+    D Rd[3], iRd[3];  // the lane's own distance
+    h3::froot(own[0] * own[0] + own[1] * own[1] + own[2] * own[2], Rd[0], iRd[0]);
+    const F Rl = F(Rd[0]), iRl = F(iRd[0]);
 #pragma unroll
     for (int b = 0; b < 3; ++b) {
       R[b] = h3::lane_of(Rl, b);
@@ -514,13 +523,12 @@ struct PesH3 {
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const F a = u[0] * d[0][c], b = u[1] * d[1][c], e = u[2] * d[2][c];
-        put(3 * lane + c, (double)h3::pick3(lane, b, a, e) - (double)h3::pick3(lane, a, e, b));
+        put(3 * lane + c, share(h3::pick3(lane, b, a, e), h3::pick3(lane, a, e, b)));
       }
     }
   }
 };
 
 }  // namespace cr
-
 #undef K4
 #undef K8
