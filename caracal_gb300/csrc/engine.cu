@@ -216,7 +216,7 @@ struct cr_engine {
   double *d_q = nullptr, *d_p = nullptr, *d_f = nullptr, *d_epot = nullptr, *d_V = nullptr;
   double *d_pile = nullptr, *d_q0 = nullptr;
   cr::Limbs* d_maps = nullptr;  // StepParams::ke, ko and pile
-  double* d_parts = nullptr;    // StepParams::psym and panti
+  double* d_anti = nullptr;     // StepParams::anti
   int64_t* d_ring = nullptr;    // FastRing::tab
   double* d_circ = nullptr;  // [3][P] circulant propagator rows (nm_mode 1)
   int* d_status = nullptr;
@@ -468,6 +468,14 @@ MapOffsets persistent_maps(cr_engine* e, const cr::PropDims& pd, const std::vect
       }
     put(m, 0, m.size(), s.ep[w] = cr::fixed_exponent(m));
   }
+  if (pair && P > 2) {
+    const int h = (P - 1) / 2;
+    std::vector<double> m((size_t)h * U, 0.0);
+    for (int l = 1; l <= h; ++l)
+      for (int j = 1; j <= h; ++j)
+        m[(size_t)(l - 1) * U + j] = pile[np + ((j - l) % P + P) % P] - pile[np + (j + l) % P];
+    put(m, 0, m.size(), s.ep[2] = cr::fixed_exponent(m));
+  }
   return off;
 }
 
@@ -509,10 +517,7 @@ int launch_group(cr_engine* e, int t0, int tn, cudaStream_t st) {
   prm.epot += t0;
   prm.status += t0;
   prm.vnh += 4 * (size_t)t0;
-  if (prm.panti) {
-    prm.psym += (size_t)t0 * prm.U * e->NC;
-    prm.panti += (size_t)t0 * prm.U * e->NC;
-  }
+  if (prm.anti) prm.anti += (size_t)t0 * 2 * prm.U * e->NC;
   if (prm.side) prm.side += (size_t)t0 * prm.side_stride;
   CR_CUDA(r->run(prm, e->cfg.precision == CR_PREC_MIXED, (tn + e->gpb - 1) / e->gpb, e->threads, e->smem, st,
                  e->istep, 1));
@@ -808,7 +813,7 @@ int fitting_groups(const cr_engine* e, int groups, int tpb, int* subs) {
   *subs = tpb;
   while (*subs > 1 && U * *subs > cr::kStepThreads) *subs /= 2;
   auto fits = [&](int n) {
-    return n * U * *subs <= cr::kStepThreads && cr::step_smem_bytes(d, U, e->NC, n) <= (size_t)cr::kStepSmemMax;
+    return n * U * *subs <= cr::kStepThreads && cr::step_smem_bytes(d, U, e->NC, n, 0) <= (size_t)cr::kStepSmemMax;
   };
   int n = std::min(groups, e->T);
   while (n > 1 && !fits(n)) --n;
@@ -844,7 +849,20 @@ bool apply_shape(cr_engine* e, int groups, int tpb) {
   e->gpb = gpb;
   e->grid = (e->T + gpb - 1) / gpb;
   e->threads = (std::max(gpb * U * subs, gpb == 1 ? e->min_threads : 0) + 31) / 32 * 32;
-  e->smem = cr::step_smem_bytes(cr::prop_dims(e->P), U, e->NC, gpb);
+  // PILE's antisymmetric part, read and written twice per step, in shared memory where
+  // that costs no other block its place
+  e->smem = cr::step_smem_bytes(cr::prop_dims(e->P), U, e->NC, gpb, 0);
+  e->prm.anti_smem = 0;
+  if (e->prm.anti && e->cfg.thermostat == CR_THERMO_PILE) {
+    const bool mixed = e->cfg.precision == CR_PREC_MIXED;
+    const size_t more = cr::step_smem_bytes(cr::prop_dims(e->P), U, e->NC, gpb, 1);
+    int with = 0, without = 0;
+    if (more <= (size_t)cr::kStepSmemMax && r->resident(mixed, e->threads, more, &with) == cudaSuccess &&
+        r->resident(mixed, e->threads, e->smem, &without) == cudaSuccess && with == without) {
+      e->smem = more;
+      e->prm.anti_smem = 1;
+    }
+  }
   e->prm.gpb = gpb;
   e->prm.subs = subs;
   return true;
@@ -890,7 +908,7 @@ void choose_launch(cr_engine* e) {
   e->min_threads = 0;
   for (int n = (std::min(e->NC * e->prm.U, cr::kStepThreads) + 31) / 32 * 32; r && n > 32 && !e->min_threads; n -= 32) {
     int res = 0;
-    if (r->resident(mixed, n, cr::step_smem_bytes(cr::prop_dims(e->P), e->prm.U, e->NC, 1), &res) != cudaSuccess) break;
+    if (r->resident(mixed, n, cr::step_smem_bytes(cr::prop_dims(e->P), e->prm.U, e->NC, 1, 0), &res) != cudaSuccess) break;
     if (e->T <= res * sms) e->min_threads = n;
   }
   if (e->T <= 4 * sms)
@@ -1346,19 +1364,16 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
   s.ke = e->d_maps;
   s.ko = e->d_maps + at.ko;
   s.pile = e->d_maps + at.pile;
-  s.pile_b = e->d_pile + e->P;
   s.q = e->d_q;
   s.p = e->d_p;
   s.f = e->d_f;
   s.epot = e->d_epot;
   s.status = e->d_status;
   if (s.pair && e->P > 2 && (cfg->thermostat == CR_THERMO_ANDERSEN || cfg->thermostat == CR_THERMO_PILE)) {
-    const size_t n = (size_t)e->T * s.U * e->NC;
-    if (cudaMalloc(&e->d_parts, 2 * n * 8) != cudaSuccess ||
-        cudaMemsetAsync(e->d_parts, 0, 2 * n * 8, e->stream) != cudaSuccess)
-      return cleanup_fail(fail(CR_ERR_CUDA, "device allocation of the momentum parts failed"));
-    s.psym = e->d_parts;
-    s.panti = e->d_parts + n;
+    const size_t n = (size_t)e->T * 2 * s.U * e->NC;
+    if (cudaMalloc(&e->d_anti, n * 8) != cudaSuccess)
+      return cleanup_fail(fail(CR_ERR_CUDA, "device allocation of the momenta's antisymmetric part failed"));
+    s.anti = e->d_anti;
   }
   // fast transforms from 32 beads on: a row's transform is one chain of some
   // hundred products on one lane, which 16 beads do not repay (H3 64 x 16 PILE
@@ -1410,7 +1425,7 @@ int cr_engine_destroy(cr_engine* e) {
   cudaFree(e->d_q0);
   cudaFree(e->d_pile);
   cudaFree(e->d_maps);
-  cudaFree(e->d_parts);
+  cudaFree(e->d_anti);
   cudaFree(e->d_ring);
   cudaFree(e->d_side);
   cudaFree(e->d_w);
@@ -2124,11 +2139,9 @@ int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* th
     return fail(CR_ERR_ARG, "the trial runs exceed the recrossing step capacity set by cr_engine_set_recross");
   CR_CUDA(cudaStreamSynchronize(e->stream));
   // every trial starts from the same state: q, p, f, epot, status, the
-  // chain velocities, the momentum parts and the step counter are saved and
-  // put back after it
+  // chain velocities and the step counter are saved and put back after it
   const size_t nq = (size_t)e->T * e->P * e->NC, T = (size_t)e->T;
-  const size_t nparts = e->d_parts ? 2 * T * e->prm.U * e->NC : 0;
-  const size_t nsave = 3 * nq + T + 4 * T + nparts;
+  const size_t nsave = 3 * nq + T + 4 * T;
   double* save = nullptr;
   int* save_st = nullptr;
   CR_CUDA(cudaMalloc(&save, nsave * sizeof(double)));
@@ -2137,12 +2150,12 @@ int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* th
     return fail(CR_ERR_CUDA, "cudaMalloc failed for the autotuner's state copy");
   }
   auto copy_state = [&](bool out) -> cudaError_t {
-    double* dst[6] = {save, save + nq, save + 2 * nq, save + 3 * nq, save + 3 * nq + T, save + 3 * nq + 5 * T};
-    double* src[6] = {e->d_q, e->d_p, e->d_f, e->d_epot, e->d_vnh, e->d_parts};
-    const size_t n[6] = {nq, nq, nq, T, 4 * T, nparts};
+    double* dst[5] = {save, save + nq, save + 2 * nq, save + 3 * nq, save + 3 * nq + T};
+    double* src[5] = {e->d_q, e->d_p, e->d_f, e->d_epot, e->d_vnh};
+    const size_t n[5] = {nq, nq, nq, T, 4 * T};
     cudaError_t err = cudaSuccess;
-    for (int k = 0; k < 6 && err == cudaSuccess; ++k)
-      if (n[k]) err = cudaMemcpyAsync(out ? dst[k] : src[k], out ? src[k] : dst[k], n[k] * 8, cudaMemcpyDeviceToDevice, e->stream);
+    for (int k = 0; k < 5 && err == cudaSuccess; ++k)
+      err = cudaMemcpyAsync(out ? dst[k] : src[k], out ? src[k] : dst[k], n[k] * 8, cudaMemcpyDeviceToDevice, e->stream);
     if (err == cudaSuccess)
       err = cudaMemcpyAsync(out ? save_st : e->d_status, out ? e->d_status : save_st, T * sizeof(int),
                             cudaMemcpyDeviceToDevice, e->stream);

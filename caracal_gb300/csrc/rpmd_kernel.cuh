@@ -13,9 +13,12 @@
 // and it reads only the sums x_l + x_{P-l}.  From the first drift on, positions,
 // gradients and momenta of the two agree, so the kernel carries the U = P/2 + 1
 // distinct beads (all P where nm_mode 1 uses orthonormal modes): the starting
-// state enters as its symmetric part, sums over beads weigh the pairs twice, and
-// what a thermostat adds to the antisymmetric part of p -- which the next
-// drift removes -- is kept only where the run ends on it.
+// state enters as its symmetric part and sums over beads weigh the pairs twice.
+// What a thermostat's draw adds to the antisymmetric part of p the next drift
+// removes, but a state between steps has it: p = s +- a, rounded. Each draw
+// therefore goes on with the symmetric part of that state, (fl(s + a) + fl(s - a)) / 2,
+// whether the run ends there or not, so that a run in pieces, or from a state that was
+// saved and set again, is the run in one, bit for bit.
 //
 // Thread layout: a block holds one or several trajectories.  The surface takes
 // four lanes per bead, in passes over the block's beads (XH4; H3 in small batches),
@@ -244,17 +247,18 @@ struct StepParams {
   int guard;           // guard bits of the folded rows (fixed_map.cuh)
   int fast_M;          // P / 2 where the free ring polymer takes the fast transforms (ring_fast.cuh), else 0
   FastRing fast;
-  const Limbs* pile;   // pairs: [2][U][U] friction and noise maps on the carried beads, [w][l][j]; else the circulants [2][P]
-  int ep[2];
+  const Limbs* pile;   // pairs: [2][U][U] friction and noise maps on the carried beads, [w][l][j], and [h][U] the noise map
+                       // of the antisymmetric part on beads 1 .. h = (P - 1) / 2, [l - 1][j]; else the circulants [2][P]
+  int ep[3];           // their exponents
   int pguard;
-  const double* pile_b;  // [P] noise circulant (the antisymmetric part at the end of a run)
   NhcParams nhc;
   double* vnh;         // [T][4] Nose-Hoover chain velocities
   double* q;           // [T][P][N][3]
   double* p;
   double* f;
-  double* psym;        // [T][U][N][3] symmetric and antisymmetric part of p as the last run left
-  double* panti;       // them after a draw (NULL: no thermostat draws, or no pairs)
+  double* anti;        // scratch [T][2][N][3][U]: limbs of the deviates' antisymmetric part, and its share of p (NULL: no draws
+                       // or no pairs)
+  int anti_smem;       // 1: the same in the block's shared memory
   double* epot;        // [T]
   int* status;         // [T]
   // recrossing children: after each step, side[t*side_stride + istep-side_step0-1]
@@ -486,7 +490,7 @@ __device__ inline bool transrot_quad(Tot tot, int lane, double itm, double kap, 
 // 20 000 x 2 mixed 95 -> 65. false: singular.
 constexpr int kFewBeads = 2;
 template <int N>
-__device__ inline bool transrot_thread(const double* q, double* p, int U, int P, int pair, const double* mass, double itm) {
+__device__ __noinline__ bool transrot_thread(const double* q, double* p, int U, int P, int pair, const double* mass, double itm) {
   auto count = [&](int j) { return pair && j > 0 && 2 * j != P ? 2.0 : 1.0; };
   double sp[3] = {0.0, 0.0, 0.0}, sq[3] = {0.0, 0.0, 0.0}, L[3] = {0.0, 0.0, 0.0};
   for (int j = 0; j < U; ++j) {
@@ -573,14 +577,14 @@ __device__ __forceinline__ double pick(const double (&x)[16], int k) {
 // Dynamic shared memory: the propagator's limbs (3 nr (nu + nv)), then for the
 // gpb trajectories of the block, each array over all of them:
 //   q, p, f   [NC][U] doubles
-//   area      [2 NC][U]: limbs of the folded rows, PILE limbs, partial sums
+//   area      [2 NC][U]: limbs of the folded rows, PILE limbs, partial sums; anti: two more [NC][U] (StepParams::anti)
 //   energies  [U] doubles, transrot sums per atom [18 N] doubles, sums [16] doubles, move [8] doubles, chain velocities [4] doubles
 //   exponent of each row [2 NC] int, status int
-__host__ __device__ inline size_t step_group_bytes(int U, int NC) {
-  return (size_t)((5 * NC + 1) * U + 6 * NC + 16 + 8 + 4) * 8 + ((size_t)(2 * NC + 1) * 4 + 7) / 8 * 8;
+__host__ __device__ inline size_t step_group_bytes(int U, int NC, int anti) {
+  return (size_t)((5 * NC + (anti ? 2 * NC : 0) + 1) * U + 6 * NC + 16 + 8 + 4) * 8 + ((size_t)(2 * NC + 1) * 4 + 7) / 8 * 8;
 }
-__host__ __device__ inline size_t step_smem_bytes(const PropDims& d, int U, int NC, int groups) {
-  return (size_t)3 * d.nr * (d.nu + d.nv) * 8 + step_group_bytes(U, NC) * groups;
+__host__ __device__ inline size_t step_smem_bytes(const PropDims& d, int U, int NC, int groups, int anti) {
+  return (size_t)3 * d.nr * (d.nu + d.nv) * 8 + step_group_bytes(U, NC, anti) * groups;
 }
 
 // Most dynamic shared memory of a block (of the 227 KB that it may take).
@@ -601,6 +605,161 @@ __device__ __noinline__ void ring_rows(const StepParams& prm, double* sq, double
   }
 }
 
+// The free ring polymer in orthonormal normal modes (nm_mode 1): circulants, on the
+// rows as limbs. In FP64 the 4 P^2 products per coordinate held the pipe (H3 per step:
+// 1 x 128 PILE mixed 684 -> 269 us with the noise's circulants in pile_half, 200 x 128
+// without a thermostat plain 362 -> 181).
+template <int NC>
+__device__ __noinline__ void circulant_rows(const StepParams& prm, double* sq, double* sp, Limbs* limbs, int* sexp, int rows,
+                                            int* sstat) {
+  const int tid = threadIdx.x, nth = blockDim.x, U = prm.U, P = prm.P, flat = rows * U;
+  for (int x = tid; x < 2 * rows; x += nth) sexp[x] = row_exponent(x < rows ? sq + x * U : sp + (x - rows) * U, U);
+  __syncthreads();
+  for (int x = tid; x < 2 * flat; x += nth)
+    limbs[x] = to_limbs(to_fixed(x < flat ? sq[x] : sp[x - flat], sexp[x / U], prm.pguard));
+  __syncthreads();
+  for (int x = tid; x < flat; x += nth) {
+    const int r = x / U, k = x - r * U, c = r % NC;
+    const Limbs* lq = limbs + r * U;
+    const Limbs* lp = lq + flat;
+    FixedSum a1q{0, 0}, a1p{0, 0}, a2q{0, 0}, a3p{0, 0};
+    int m = k;  // (k - l) mod P
+#pragma unroll 4
+    for (int l = 0; l < P; ++l) {
+      const Limbs vq = lq[l], vp = lp[l], w1 = ldg_limbs(prm.circ + m);
+      a1q.add(vq, w1);
+      a1p.add(vp, w1);
+      a2q.add(vq, ldg_limbs(prm.circ + P + m));
+      a3p.add(vp, ldg_limbs(prm.circ + 2 * P + m));
+      m = (m == 0) ? P - 1 : m - 1;
+    }
+    const int sq_e = sexp[r] - 1078 + prm.pguard, sp_e = sexp[rows + r] - 1078 + prm.pguard;
+    const bool bad = sexp[r] == kFixedNan || sexp[rows + r] == kFixedNan;
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    const double pn = fma(prm.mass[c / 3], from_fixed(a2q.value(), prm.ek[1] + sq_e), from_fixed(a1p.value(), prm.ek[0] + sp_e));
+    const double qn = fma(prm.inv_mass[c / 3], from_fixed(a3p.value(), prm.ek[2] + sp_e), from_fixed(a1q.value(), prm.ek[0] + sq_e));
+    sp[x] = bad ? nan : pn;
+    sq[x] = bad ? nan : qn;
+    if (bad || nonfinite_bits(qn)) atomicOr(&sstat[r / NC], CR_TRAJ_NONFINITE);
+  }
+}
+
+// The deviates of bead k of trajectory t and of its twin kt for coordinates 4 i .. 4 i + 3.
+__device__ __forceinline__ void deviates(const StepParams& prm, int t, int k, int kt, int i, uint32_t step, uint32_t tag,
+                                         double (&za)[4], double (&zb)[4]) {
+  const uint32_t key = prm.traj0 + (uint32_t)t;
+  const uint4 r = philox4x32_10(make_uint4((uint32_t)i, (uint32_t)k, step, tag), prm.seed, key);
+  bm_pair(r.x, r.y, za[0], za[1]);
+  bm_pair(r.z, r.w, za[2], za[3]);
+  if (kt == k) {
+    for (int d = 0; d < 4; ++d) zb[d] = za[d];
+  } else {
+    const uint4 w = philox4x32_10(make_uint4((uint32_t)i, (uint32_t)kt, step, tag), prm.seed, key);
+    bm_pair(w.x, w.y, zb[0], zb[1]);
+    bm_pair(w.z, w.w, zb[2], zb[3]);
+  }
+}
+
+// Andersen's draw on the block's rows sp of p: the symmetric part, and the interior beads'
+// antisymmetric part into santi.
+template <int N>
+__device__ __noinline__ void andersen_rows(const StepParams& prm, double* sp, double* santi, int t_first, int ng, uint32_t step) {
+  constexpr int NC = 3 * N, NQ = (NC + 3) / 4;
+  const int U = prm.U, P = prm.P, nb = ng * U;
+  for (int x = threadIdx.x; x < nb * NQ; x += blockDim.x) {
+    const int i = x / nb, y = x - i * nb, gg = y / U, k = y - gg * U, kt = prm.pair && k > 0 && 2 * k != P ? P - k : k;
+    double za[4], zb[4];
+    deviates(prm, t_first + gg, k, kt, i, step, TAG_ANDERSEN, za, zb);
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+      const int c = 4 * i + d, z = (gg * NC + c) * U + k;
+      if (c >= NC) continue;
+      const double s = prm.sigma[c / 3];
+      sp[z] = kt == k ? za[d] * s : 0.5 * (za[d] + zb[d]) * s;
+      if (kt != k) santi[z] = 0.5 * (za[d] - zb[d]) * s;
+    }
+  }
+}
+
+// PILE half step on the block's rows sp of p: by the limbs of the rows and of the
+// deviates' symmetric part (|eta| < 8: one exponent for all), and with_anti of their
+// antisymmetric part, whose share of p (b * half the difference of two beads'
+// deviates, which the next drift removes) goes to the second half of anti. Out of line:
+// both half steps fetch the same code (64 x 16 H3 mixed 18.6 -> 16.9 us per step).
+template <int N>
+__device__ __noinline__ void pile_half(const StepParams& prm, double* sp, Limbs* limbs, int* sexp, double* anti, int t_first,
+                                       int ng, uint32_t step, uint32_t tag, bool with_anti) {
+  constexpr int NC = 3 * N, NQ = (NC + 3) / 4, kEtaExp = 1025;
+  const int tid = threadIdx.x, nth = blockDim.x, U = prm.U, P = prm.P, nb = ng * U, rows = ng * NC, flat = rows * U;
+  const int pair = prm.pair, guard = prm.pguard;
+  Limbs* le = limbs + flat;
+  Limbs* la = reinterpret_cast<Limbs*>(anti);
+  double* santi = anti + flat;
+  // the rows by the last threads, while the first draw (64 x 16 H3, both half
+  // steps: 15.1 -> 10.8 thousand cycles)
+  for (int x = nth - 1 - tid; x < rows; x += nth) {
+    const double* r = sp + x * U;
+    const int e = row_exponent(r, U);
+    sexp[x] = e;
+#pragma unroll 3
+    for (int k = 0; k < U; ++k) limbs[x * U + k] = to_limbs(to_fixed(r[k], e, guard + 1));
+  }
+  for (int x = tid; x < nb * NQ; x += nth) {
+    const int i = x / nb, y = x - i * nb, gg = y / U, k = y - gg * U;
+    double za[4], zb[4];
+    deviates(prm, t_first + gg, k, pair && k > 0 && 2 * k != P ? P - k : k, i, step, tag, za, zb);
+#pragma unroll
+    for (int d = 0; d < 4; ++d)
+      if (4 * i + d < NC) {
+        const int64_t a = to_fixed(za[d], kEtaExp, guard + 1), b = to_fixed(zb[d], kEtaExp, guard + 1);
+        const int z = (gg * NC + 4 * i + d) * U + k;
+        le[z] = to_limbs(a + b);
+        if (with_anti) la[z] = to_limbs(a - b);
+      }
+  }
+  __syncthreads();
+  // the carried beads' new momenta, then the interior beads' antisymmetric share
+  const int h = with_anti ? (P - 1) / 2 : 0;
+  for (int x = tid; x < flat + rows * h; x += nth) {
+    if (x < flat) {
+      const int r = x / U, k = x - r * U, c = r % NC;
+      const Limbs* lp = limbs + r * U;
+      const Limbs* ln = le + r * U;
+      FixedSum a{0, 0}, e{0, 0};
+      if (pair) {
+        const Limbs* ka = prm.pile + k;
+        const Limbs* kb = ka + U * U;
+#pragma unroll 2
+        for (int l = 0; l < U; ++l) {
+          a.add(lp[l], ldg_limbs(ka + l * U));
+          e.add(ln[l], ldg_limbs(kb + l * U));
+        }
+      } else {
+        int m = k;  // (k - l) mod P
+#pragma unroll 4
+        for (int l = 0; l < U; ++l) {
+          a.add(lp[l], ldg_limbs(prm.pile + m));
+          e.add(ln[l], ldg_limbs(prm.pile + P + m));
+          m = (m == 0) ? P - 1 : m - 1;
+        }
+      }
+      double v = from_fixed(a.value(), prm.ep[0] + sexp[r] - 1077 + guard);
+      if (sexp[r] == kFixedNan) v = __longlong_as_double(0x7ff8000000000000ll);
+      // half the sum of the two deviates: one bit of the exponent
+      sp[x] = fma(prm.sigma[c / 3], from_fixed(e.value(), prm.ep[1] + kEtaExp - 1078 + guard), v);
+    } else {
+      const int r = (x - flat) / h, k = x - flat - r * h + 1;
+      const Limbs* ln = la + r * U;
+      const Limbs* kc = prm.pile + 2 * U * U + k;
+      FixedSum a{0, 0};
+#pragma unroll 4
+      for (int l = 1; l <= h; ++l) a.add(ln[l], ldg_limbs(kc + (l - 1) * U));
+      santi[r * U + k] = prm.sigma[(r % NC) / 3] * from_fixed(a.value(), prm.ep[2] + kEtaExp - 1078 + guard);
+    }
+  }
+  __syncthreads();
+}
+
 // Most threads of a block of the step kernel; MINB blocks stay resident per SM
 // (the registers follow: 255 for 2, 168 for 3, 128 for 4).
 constexpr int kStepThreads = 128;
@@ -615,7 +774,6 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
   const int istep0 = prm.istep_dev ? *prm.istep_dev : istep_arg;
   constexpr int N = PES::N;
   constexpr int NC = 3 * N;
-  constexpr int NQ = (NC + 3) / 4;  // Philox blocks per bead
   extern __shared__ double smem[];
   const int P = prm.P, U = prm.U, gpb = prm.gpb;
   const int tid = threadIdx.x, nth = blockDim.x;
@@ -631,13 +789,16 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
   double* sf = sp + gpb * NC * U;
   double* area = sf + gpb * NC * U;
   Limbs* limbs = reinterpret_cast<Limbs*>(area);
-  double* svb = area + 2 * gpb * NC * U;  // bead energies
+  double* svb = area + (prm.anti_smem ? 4 : 2) * gpb * NC * U;  // bead energies
   double* smom = svb + gpb * U;
   double* ssum = smom + gpb * 6 * NC;
   double* smove = ssum + 16 * gpb;
   double* svnh = smove + 8 * gpb;
   int* sexp = reinterpret_cast<int*>(svnh + 4 * gpb);
   int* sstat = sexp + 2 * NC * gpb;
+  // rows of the antisymmetric part: the deviates' limbs, and what they add to p
+  double* anti = prm.anti_smem ? area + 2 * gpb * NC * U : prm.anti + (size_t)t_first * 2 * NC * U;
+  double* santi = anti + flat;
 
   if (!prm.nm_mode) {
     for (int x = tid; x < nke; x += nth) s_ke[x] = prm.ke[x];
@@ -664,7 +825,6 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
     return r;
   };
   const size_t row_a = ((size_t)t * P + j) * NC, row_b = ((size_t)t * P + twin_of(j)) * NC;
-  const size_t row_u = ((size_t)t * U + j) * NC;
   double ek_anti = 0.0;  // kinetic share of the antisymmetric starting momenta
   if (bead) {
     for (int c = 0; c < NC; ++c) {
@@ -674,14 +834,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
         const double pb = prm.p[row_b + c], d = 0.5 * (p - pb);
         ek_anti = fma(d * d, prm.inv_mass[c / 3], ek_anti);
         q = 0.5 * (q + prm.q[row_b + c]);
-        // the symmetric part; where p is still what the last run left, exactly
-        // the one that it carried, so that a run in pieces is the run in one
-        double ps = 0.5 * (p + pb);
-        if (prm.panti) {
-          const double s = prm.psym[row_u + c], a = prm.panti[row_u + c];
-          if (p == s + a && pb == s - a) ps = s;
-        }
-        p = ps;
+        p = 0.5 * (p + pb);
         f = 0.5 * (f + prm.f[row_b + c]);
       }
       sq[x] = q;
@@ -693,7 +846,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
   const bool nhc = prm.thermostat == CR_THERMO_NHC, pile = prm.thermostat == CR_THERMO_PILE;
   if (nhc && tid < ng)
     for (int k = 0; k < 4; ++k) svnh[4 * tid + k] = prm.vnh[4 * (size_t)(t_first + tid) + k];
-  bool anti_left = false;  // the run ends with an antisymmetric part of p (prm.panti)
+  bool drawn = false;  // the last step left an antisymmetric part of p (santi)
   __syncthreads();
 
   // nhc (src/nhc.f90): sum of p.p/(2m)/P/P, the chain, one scale
@@ -719,102 +872,17 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
     __syncthreads();
   };
 
-  // the deviates of bead k and its twin for coordinates 4 i .. 4 i + 3
-  auto quad = [&](int gg, int k, int i, uint32_t step, uint32_t tag, double (&za)[4], double (&zb)[4]) {
-    const uint32_t key = prm.traj0 + (uint32_t)(t_first + gg);
-    const uint4 r = philox4x32_10(make_uint4((uint32_t)i, (uint32_t)k, step, tag), prm.seed, key);
-    bm_pair(r.x, r.y, za[0], za[1]);
-    bm_pair(r.z, r.w, za[2], za[3]);
-    const int kt = twin_of(k);
-    if (kt == k) {
-      for (int d = 0; d < 4; ++d) zb[d] = za[d];
-    } else {
-      const uint4 w = philox4x32_10(make_uint4((uint32_t)i, (uint32_t)kt, step, tag), prm.seed, key);
-      bm_pair(w.x, w.y, zb[0], zb[1]);
-      bm_pair(w.z, w.w, zb[2], zb[3]);
-    }
-  };
-
-  // PILE half step on p; the limbs of p's rows, then those of the deviates'
-  // symmetric part (|eta| < 8: one exponent for all)
-  constexpr int kEtaExp = 1025;
-  auto pile_half = [&](uint32_t step, uint32_t tag, bool last) {
-    Limbs* le = limbs + flat;
-    // the rows by the last threads, while the first draw (64 x 16 H3, both half
-    // steps: 15.1 -> 10.8 thousand cycles)
-    for (int x = nth - 1 - tid; x < rows; x += nth) {
-      const double* r = sp + x * U;
-      const int e = row_exponent(r, U);
-      sexp[x] = e;
-#pragma unroll 3
-      for (int k = 0; k < U; ++k) limbs[x * U + k] = to_limbs(to_fixed(r[k], e, prm.pguard + 1));
-    }
-    for (int x = tid; x < nb * NQ; x += nth) {
-      const int i = x / nb, y = x - i * nb, gg = y / U, k = y - gg * U;
-      double za[4], zb[4];
-      quad(gg, k, i, step, tag, za, zb);
-#pragma unroll
-      for (int d = 0; d < 4; ++d)
-        if (4 * i + d < NC)
-          le[(gg * NC + 4 * i + d) * U + k] = to_limbs(to_fixed(za[d], kEtaExp, prm.pguard + 1) +
-                                                       to_fixed(zb[d], kEtaExp, prm.pguard + 1));
-    }
-    __syncthreads();
-    for (int x = tid; x < flat; x += nth) {
-      const int r = x / U, k = x - r * U;
-      FixedSum a{0, 0}, e{0, 0};
-      const Limbs* lp = limbs + r * U;
-      const Limbs* ln = le + r * U;
-      if (prm.pair) {
-        const Limbs* ka = prm.pile + k;
-        const Limbs* kb = ka + U * U;
-        for (int l = 0; l < U; ++l) {
-          a.add(lp[l], ldg_limbs(ka + l * U));
-          e.add(ln[l], ldg_limbs(kb + l * U));
-        }
-      } else {
-        int m = k;  // (k - l) mod P
-#pragma unroll 4
-        for (int l = 0; l < U; ++l) {
-          a.add(lp[l], ldg_limbs(prm.pile + m));
-          e.add(ln[l], ldg_limbs(prm.pile + P + m));
-          m = (m == 0) ? P - 1 : m - 1;
-        }
-      }
-      const int c = r % NC;
-      double v = from_fixed(a.value(), prm.ep[0] + sexp[r] - 1077 + prm.pguard);
-      if (sexp[r] == kFixedNan) v = __longlong_as_double(0x7ff8000000000000ll);
-      // half the sum of the two deviates: one bit of the exponent
-      sp[x] = fma(prm.sigma[c / 3], from_fixed(e.value(), prm.ep[1] + kEtaExp - 1078 + prm.pguard), v);
-    }
-    __syncthreads();
-    if (last && prm.panti) {
-      // b * (the deviates' antisymmetric part), which the next drift would remove
-      for (int x = tid; x < nb * NQ; x += nth) {
-        const int i = x / nb, y = x - i * nb, gg = y / U, k = y - gg * U;
-        double za[4], zb[4];
-        quad(gg, k, i, step, tag, za, zb);
-#pragma unroll
-        for (int d = 0; d < 4; ++d)
-          if (4 * i + d < NC) area[(gg * NC + 4 * i + d) * U + k] = 0.5 * (za[d] - zb[d]);
-      }
-      __syncthreads();
-      for (int x = tid; x < flat; x += nth) {
-        const int r = x / U, k = x - r * U, c = r % NC;
-        double acc = 0.0;
-        for (int l = 1; l <= (P - 1) / 2; ++l)
-          acc = fma(prm.pile_b[k >= l ? k - l : k - l + P] - prm.pile_b[k + l >= P ? k + l - P : k + l], area[r * U + l], acc);
-        prm.panti[((size_t)(t_first + r / NC) * U + k) * NC + c] = twin_of(k) == k ? 0.0 : prm.sigma[c / 3] * acc;
-      }
-      __syncthreads();
-    }
+  // the symmetric part of the state between two steps, of element x that carries p
+  auto between = [&](int x, double p) {
+    const int k = x % U;
+    return twin_of(k) == k ? p : 0.5 * ((p + santi[x]) + (p - santi[x]));
   };
 
   for (int n = 1; n <= nsteps; ++n) {
     const int istep = istep0 + n;
-    const bool last = n == nsteps;
+    drawn = false;
     if (nhc) nhc_half(n == 1 ? ek_anti : 0.0);  // src/verlet.f90:186-208
-    if (pile) pile_half((uint32_t)istep, TAG_PILE_A, false);
+    if (pile) pile_half<N>(prm, sp, limbs, sexp, anti, t_first, ng, (uint32_t)istep, TAG_PILE_A, false);
 
     // 1/2 kick (src/verlet.f90:216-218)
     for (int x = tid; x < flat; x += nth) sp[x] = fma(-prm.half_dt, sf[x], sp[x]);
@@ -823,38 +891,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
     // free ring polymer (src/verlet.f90:377-463): Caracal's cosine modes, or
     // orthonormal normal modes where nm_mode is set
     if (prm.nm_mode) {
-      // circulants, on the rows as limbs: the 4 P^2 products per coordinate held the
-      // FP64 pipe (H3 per step: 1 x 128 PILE mixed 684 -> 269 us with the noise's circulants
-      // below, 200 x 128 without a thermostat plain 362 -> 181)
-      for (int x = tid; x < 2 * rows; x += nth) sexp[x] = row_exponent(x < rows ? sq + x * U : sp + (x - rows) * U, U);
-      __syncthreads();
-      for (int x = tid; x < 2 * flat; x += nth)
-        limbs[x] = to_limbs(to_fixed(x < flat ? sq[x] : sp[x - flat], sexp[x / U], prm.pguard));
-      __syncthreads();
-      for (int x = tid; x < flat; x += nth) {
-        const int r = x / U, k = x - r * U, c = r % NC;
-        const Limbs* lq = limbs + r * U;
-        const Limbs* lp = lq + flat;
-        FixedSum a1q{0, 0}, a1p{0, 0}, a2q{0, 0}, a3p{0, 0};
-        int m = k;  // (k - l) mod P
-#pragma unroll 4
-        for (int l = 0; l < P; ++l) {
-          const Limbs vq = lq[l], vp = lp[l], w1 = ldg_limbs(prm.circ + m);
-          a1q.add(vq, w1);
-          a1p.add(vp, w1);
-          a2q.add(vq, ldg_limbs(prm.circ + P + m));
-          a3p.add(vp, ldg_limbs(prm.circ + 2 * P + m));
-          m = (m == 0) ? P - 1 : m - 1;
-        }
-        const int sq_e = sexp[r] - 1078 + prm.pguard, sp_e = sexp[rows + r] - 1078 + prm.pguard;
-        const bool bad = sexp[r] == kFixedNan || sexp[rows + r] == kFixedNan;
-        const double nan = __longlong_as_double(0x7ff8000000000000ll);
-        const double pn = fma(prm.mass[c / 3], from_fixed(a2q.value(), prm.ek[1] + sq_e), from_fixed(a1p.value(), prm.ek[0] + sp_e));
-        const double qn = fma(prm.inv_mass[c / 3], from_fixed(a3p.value(), prm.ek[2] + sp_e), from_fixed(a1q.value(), prm.ek[0] + sq_e));
-        sp[x] = bad ? nan : pn;
-        sq[x] = bad ? nan : qn;
-        if (bad || nonfinite_bits(qn)) atomicOr(&sstat[r / NC], CR_TRAJ_NONFINITE);
-      }
+      circulant_rows<NC>(prm, sq, sp, limbs, sexp, rows, sstat);
     } else if (prm.fast_M) {
       if (prm.fast_M == 16) ring_rows<16, NC>(prm, sq, sp, rows, sstat);
       else ring_rows<32, NC>(prm, sq, sp, rows, sstat);
@@ -1012,26 +1049,13 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
 
     // Andersen (src/verlet.f90:1159-1165): full resample every andersen_step
     if (prm.thermostat == CR_THERMO_ANDERSEN && (istep % prm.andersen_step) == 0) {
-      for (int x = tid; x < nb * NQ; x += nth) {
-        const int i = x / nb, y = x - i * nb, gg = y / U, k = y - gg * U, kt = twin_of(k);
-        double za[4], zb[4];
-        quad(gg, k, i, (uint32_t)istep, TAG_ANDERSEN, za, zb);
-#pragma unroll
-        for (int d = 0; d < 4; ++d) {
-          const int c = 4 * i + d;
-          if (c >= NC) continue;
-          const double s = prm.sigma[c / 3];
-          sp[(gg * NC + c) * U + k] = kt == k ? za[d] * s : 0.5 * (za[d] + zb[d]) * s;
-          if (last && prm.panti)
-            prm.panti[((size_t)(t_first + gg) * U + k) * NC + c] = kt == k ? 0.0 : 0.5 * (za[d] - zb[d]) * s;
-        }
-      }
-      anti_left = last && prm.panti;
+      andersen_rows<N>(prm, sp, santi, t_first, ng, (uint32_t)istep);
+      drawn = prm.anti != nullptr;
       __syncthreads();
     }
     if (pile) {
-      pile_half((uint32_t)istep, TAG_PILE_B, last);
-      anti_left = last && prm.panti;
+      drawn = prm.anti != nullptr;
+      pile_half<N>(prm, sp, limbs, sexp, anti, t_first, ng, (uint32_t)istep, TAG_PILE_B, drawn);
     }
 
     // transrot (src/transrot.f90:36-237): removed COM velocity and rotation
@@ -1095,11 +1119,16 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
         const int r = x / U, gg = r / NC, c = r - gg * NC, d = c % 3;
         const int e = d == 2 ? 0 : d + 1, f = d == 0 ? 2 : d - 1;
         const double* mv = smove + 8 * gg;
-        if (mv[6] != 0.0) continue;
         const double qe = sq[x + (e - d) * U], qf = sq[x + (f - d) * U];
         const double u = fma(mv[3 + e], qf, fma(-mv[3 + f], qe, mv[d]));
-        sp[x] = fma(-prm.mass[c / 3], u, sp[x]);
+        const double p = mv[6] != 0.0 ? sp[x] : fma(-prm.mass[c / 3], u, sp[x]);  // singular: left as it is
+        sp[x] = drawn && n < nsteps ? between(x, p) : p;
       }
+      __syncthreads();
+    }
+
+    if (drawn && n < nsteps && (!prm.transrot || U <= kFewBeads)) {
+      for (int x = tid; x < flat; x += nth) sp[x] = between(x, sp[x]);
       __syncthreads();
     }
   }
@@ -1112,11 +1141,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
       prm.q[row_a + c] = q;
       prm.f[row_a + c] = f;
       if (row_b != row_a) {
-        double a = 0.0;
-        if (anti_left) {
-          a = prm.panti[row_u + c];
-          prm.psym[row_u + c] = p;
-        }
+        const double a = drawn ? santi[x] : 0.0;
         prm.p[row_a + c] = p + a;
         prm.p[row_b + c] = p - a;
         prm.q[row_b + c] = q;
