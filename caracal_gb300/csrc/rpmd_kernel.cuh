@@ -46,6 +46,7 @@
 #include "bead_rows.cuh"
 #include "cr_common.cuh"
 #include "fixed_map.cuh"
+#include "num.cuh"
 #include "ring_fast.cuh"
 
 namespace cr {
@@ -482,90 +483,194 @@ __device__ inline bool transrot_quad(Tot tot, int lane, double itm, double kap, 
   return tpp != 0.0 && s1 != 0.0 && s3 != 0.0;
 }
 
-// transrot of one trajectory by one thread, for ring polymers of few carried beads
-// (rows q, p of NC x U in shared memory, bead j > 0 of odd P standing for two): the
-// reference's sums over atoms and beads about its centre (src/transrot.f90:36-237),
-// in FP64, the inertia tensor solved with pivots on the diagonal as in transrot_quad.
-// With one bead that is some 40 FP64 operations per atom and 100 for the solve, where
-// the moments by limbs take 18 tasks of a hundred instructions per atom whatever the
-// number of beads: H3 100 000 x 1 mixed 267 -> 111 us per step, plain 387 -> 232; with two,
-// 20 000 x 2 mixed 95 -> 65. false: singular.
-constexpr int kFewBeads = 2;
-template <int N>
-__device__ __noinline__ bool transrot_thread(const double* q, double* p, int U, int P, int pair, const double* mass, double itm) {
-  auto count = [&](int j) { return pair && j > 0 && 2 * j != P ? 2.0 : 1.0; };
-  double sp[3] = {0.0, 0.0, 0.0}, sq[3] = {0.0, 0.0, 0.0}, L[3] = {0.0, 0.0, 0.0};
-  for (int j = 0; j < U; ++j) {
-    const double k = count(j);
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      double x[3], y[3];
-      const double w = k * mass[i];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        x[d] = q[(3 * i + d) * U + j];
-        y[d] = k * p[(3 * i + d) * U + j];
-        sp[d] += y[d];
-        sq[d] = fma(w, x[d], sq[d]);
-      }
-      L[0] += fma(x[1], y[2], -x[2] * y[1]);
-      L[1] += fma(x[2], y[0], -x[0] * y[2]);
-      L[2] += fma(x[0], y[1], -x[1] * y[0]);
-    }
-  }
-  const double xt[3] = {sq[0] * itm, sq[1] * itm, sq[2] * itm}, vt[3] = {sp[0] * itm, sp[1] * itm, sp[2] * itm};
-  L[0] -= fma(xt[1], sp[2], -xt[2] * sp[1]);
-  L[1] -= fma(xt[2], sp[0], -xt[0] * sp[2]);
-  L[2] -= fma(xt[0], sp[1], -xt[1] * sp[0]);
-  double c[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // xx, yy, zz, yz, zx, xy
-  for (int j = 0; j < U; ++j) {
-    const double k = count(j);
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      double x[3], wx[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        x[d] = q[(3 * i + d) * U + j] - xt[d];
-        wx[d] = k * mass[i] * x[d];
-        c[d] = fma(wx[d], x[d], c[d]);
-      }
-      c[3] = fma(wx[1], x[2], c[3]);
-      c[4] = fma(wx[2], x[0], c[4]);
-      c[5] = fma(wx[0], x[1], c[5]);
-    }
-  }
-  const double e = N <= 2 ? 0.000001 : 0.0;
-  const double t0 = c[1] + c[2] + e, t1 = c[2] + c[0] + e, t2 = c[0] + c[1] + e;
-  // axes p, q, r in cyclic order with the largest diagonal element first
-  const int a = fabs(t0) >= fabs(t1) ? (fabs(t0) >= fabs(t2) ? 0 : 2) : (fabs(t1) >= fabs(t2) ? 1 : 2);
-  auto from = [&](int k, double u, double v, double w) { return k == 0 ? u : k == 1 ? v : w; };
-  const int b = a == 2 ? 0 : a + 1, f = a == 0 ? 2 : a - 1;
-  const double tpp = from(a, t0, t1, t2), tqq = from(b, t0, t1, t2), trr = from(f, t0, t1, t2);
-  const double tqr = -from(a, c[3], c[4], c[5]), tpr = -from(b, c[3], c[4], c[5]), tpq = -from(f, c[3], c[4], c[5]);
-  const double Lp = from(a, L[0], L[1], L[2]), Lq = from(b, L[0], L[1], L[2]), Lr = from(f, L[0], L[1], L[2]);
-  const double ip = fx::rcp(tpp), m1 = tpq * ip, m2 = tpr * ip;
-  const double sqq = fma(-m1, tpq, tqq), srr = fma(-m2, tpr, trr), sqr = fma(-m1, tpr, tqr);
-  const double yq = fma(-m1, Lp, Lq), yr = fma(-m2, Lp, Lr);
-  const bool swap = fabs(srr) > fabs(sqq);
+// The solve of transrot_quad by one thread, operation for operation: va = T^-1 L for the
+// tensor with centred moments c (xx, yy, zz, yz, zx, xy).  false: singular.
+__device__ inline bool transrot_solve(const double (&c)[6], const double (&L)[3], bool two_atoms, double (&va)[3]) {
+  const double small = two_atoms ? 0.000001 : 0.0;
+  const double t0 = c[1] + c[2] + small, t1 = c[2] + c[0] + small, t2 = c[0] + c[1] + small;
+  auto bits = [](double x) { return __double_as_longlong(fabs(x)); };
+  auto from = [](int k, double u, double v, double w) { return k == 0 ? u : k == 1 ? v : w; };
+  const int p = bits(t0) >= bits(t1) ? (bits(t0) >= bits(t2) ? 0 : 2) : (bits(t1) >= bits(t2) ? 1 : 2);
+  const int q = p == 2 ? 0 : p + 1, r = p == 0 ? 2 : p - 1;
+  const double tpp = from(p, t0, t1, t2), tqq = from(q, t0, t1, t2), trr = from(r, t0, t1, t2);
+  const double tqr = -from(p, c[3], c[4], c[5]), tpr = -from(q, c[3], c[4], c[5]), tpq = -from(r, c[3], c[4], c[5]);
+  const double Lp = from(p, L[0], L[1], L[2]), Lq = from(q, L[0], L[1], L[2]), Lr = from(r, L[0], L[1], L[2]);
+  const double ip = fx::rcp(tpp), a = tpq * ip, b = tpr * ip;
+  const double sqq = fma(-a, tpq, tqq), srr = fma(-b, tpr, trr), sqr = fma(-a, tpr, tqr);
+  const double yq = fma(-a, Lp, Lq), yr = fma(-b, Lp, Lr);
+  const bool swap = bits(srr) > bits(sqq);
   const double s1 = swap ? srr : sqq, s2 = swap ? sqq : srr, y1 = swap ? yr : yq, y2 = swap ? yq : yr;
-  const double i1 = fx::rcp(s1), m3 = sqr * i1, s3 = fma(-m3, sqr, s2);
-  if (tpp == 0.0 || s1 == 0.0 || s3 == 0.0) return false;
-  const double v2 = fma(-m3, y1, y2) * fx::rcp(s3), v1 = fma(-sqr, v2, y1) * i1;
+  const double i1 = fx::rcp(s1), m = sqr * i1, s3 = fma(-m, sqr, s2);
+  const double v2 = fma(-m, y1, y2) * fx::rcp(s3), v1 = fma(-sqr, v2, y1) * i1;
   const double vq = swap ? v2 : v1, vr = swap ? v1 : v2, vp = fma(-tpr, vr, fma(-tpq, vq, Lp)) * ip;
   // axis 0 is p, r or q as p is 0, 1 or 2, and so on round
-  const double va[3] = {from(a, vp, vr, vq), from(a, vq, vp, vr), from(a, vr, vq, vp)};
-  for (int j = 0; j < U; ++j)
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      double x[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) x[d] = q[(3 * i + d) * U + j] - xt[d];
-      const double u[3] = {fma(va[1], x[2], fma(-va[2], x[1], vt[0])), fma(va[2], x[0], fma(-va[0], x[2], vt[1])),
-                           fma(va[0], x[1], fma(-va[1], x[0], vt[2]))};
-#pragma unroll
-      for (int d = 0; d < 3; ++d) p[(3 * i + d) * U + j] = fma(-mass[i], u[d], p[(3 * i + d) * U + j]);
+  va[0] = from(p, vp, vr, vq);
+  va[1] = from(p, vq, vp, vr);
+  va[2] = from(p, vr, vq, vp);
+  return tpp != 0.0 && s1 != 0.0 && s3 != 0.0;
+}
+
+// transrot of ring polymers of one or two carried beads (rows q, p of NC x U in shared
+// memory, bead 1 of three standing for two): the reference's sums over atoms and beads
+// about its centre (src/transrot.f90:36-237) in FP64, by L = 4 lanes per trajectory, each
+// with the atoms i = lane, lane + 4, or by one thread that goes through the four lanes'
+// sums, with the same roundings (num.cuh). One thread per trajectory has the least
+// operations, some 40 per atom and 80 for the solve; four are faster where a block
+// has the threads to spare. The moments by limbs take 18 tasks of a hundred
+// instructions per atom whatever the number of beads, and with one bead about the origin
+// lose (R/r)^2 of the precision of a molecule at R. Per step, limbs and here: H3 100 000 x 1
+// mixed 267 and 116 us, plain 387 and 239; CH4 + H 60 000 x 1 mixed 256 and 168; H3 1 x 1 11.9 and 12.8.
+template <int N, int L>
+__device__ __noinline__ void transrot_few(const StepParams& prm, const double* sq, double* sp, int ng, int* sstat) {
+  using D = Num<double>;
+  constexpr int NC = 3 * N;
+  const int tid = threadIdx.x, nth = blockDim.x, U = prm.U, P = prm.P, lane = L == 4 ? tid & 3 : 0;
+  const bool twins = prm.pair && P == 3;  // bead 1 stands for beads 1 and 2
+  const D itm = prm.itm;
+  // of the four lanes' values, in one order
+  auto total = [&](auto part) {
+    if constexpr (L == 4) {
+      D x = part(lane);
+      x = x + D(__shfl_xor_sync(0xffffffffu, x.v, 1));
+      return x + D(__shfl_xor_sync(0xffffffffu, x.v, 2));
+    } else {
+      const D lo = N > 1 ? part(0) + part(1) : part(0);
+      return N > 3 ? lo + (part(2) + part(3)) : N > 2 ? lo + part(2) : lo;
     }
-  return true;
+  };
+  for (int x0 = 0; x0 < ng; x0 += nth / L) {
+    if (x0 + (tid & ~31) / L >= ng) break;  // a warp's shuffles want all of it
+    const int gg = x0 + tid / L;
+    const bool real = gg < ng;
+    const double* q = sq + (real ? gg : x0) * NC * U;
+    double* p = sp + (real ? gg : x0) * NC * U;
+    struct First {
+      D P[3], S[3], M[3];
+    } first[L == 4 ? 1 : 4];
+    auto sums = [&](int v, First& f) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) f.P[d] = f.S[d] = f.M[d] = D(0.0);
+#pragma unroll
+      for (int i = v; i < N; i += 4)
+        for (int j = 0; j < U; ++j) {
+          const D k = twins && j == 1 ? 2.0 : 1.0, w = k * D(prm.mass[i]);
+          D x[3], y[3];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            x[d] = q[(3 * i + d) * U + j];
+            y[d] = k * D(p[(3 * i + d) * U + j]);
+            f.P[d] = f.P[d] + y[d];
+            f.S[d] = w * x[d] + f.S[d];
+          }
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            const int e = d == 2 ? 0 : d + 1, g = d == 0 ? 2 : d - 1;
+            f.M[d] = x[e] * y[g] + f.M[d];
+            f.M[d] = f.M[d] - x[g] * y[e];
+          }
+        }
+    };
+    if constexpr (L == 4) {
+      sums(lane, first[0]);
+    } else {
+#pragma unroll
+      for (int v = 0; v < 4; ++v) sums(v, first[v]);
+    }
+    D Pt[3], xt[3], Lt[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      Pt[d] = total([&](int v) { return first[L == 4 ? 0 : v].P[d]; });
+      xt[d] = total([&](int v) { return first[L == 4 ? 0 : v].S[d]; }) * itm;
+      Lt[d] = total([&](int v) { return first[L == 4 ? 0 : v].M[d]; });
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int e = d == 2 ? 0 : d + 1, g = d == 0 ? 2 : d - 1;
+      Lt[d] = Lt[d] - xt[e] * Pt[g];
+      Lt[d] = xt[g] * Pt[e] + Lt[d];
+    }
+    struct Second {
+      D c[6];  // xx, yy, zz, yz, zx, xy
+    } second[L == 4 ? 1 : 4];
+    auto squares = [&](int v, Second& f) {
+#pragma unroll
+      for (int k = 0; k < 6; ++k) f.c[k] = D(0.0);
+#pragma unroll
+      for (int i = v; i < N; i += 4)
+        for (int j = 0; j < U; ++j) {
+          const D w = D(twins && j == 1 ? 2.0 : 1.0) * D(prm.mass[i]);
+          D x[3], wx[3];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            x[d] = D(q[(3 * i + d) * U + j]) - xt[d];
+            wx[d] = w * x[d];
+            f.c[d] = wx[d] * x[d] + f.c[d];
+          }
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            const int e = d == 2 ? 0 : d + 1, g = d == 0 ? 2 : d - 1;
+            f.c[3 + d] = wx[e] * x[g] + f.c[3 + d];
+          }
+        }
+    };
+    if constexpr (L == 4) {
+      squares(lane, second[0]);
+    } else {
+#pragma unroll
+      for (int v = 0; v < 4; ++v) squares(v, second[v]);
+    }
+    double c[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) c[k] = total([&](int v) { return second[L == 4 ? 0 : v].c[k]; }).v;
+    // the move vt + va x (x - xt)
+    D vt[3], va[3];
+    bool ok;
+    if constexpr (L == 4) {
+      // transrot_quad with the first moments taken out (kap = 0)
+      auto tot = [&](int k) {
+        double r = 0.0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) r = k == d ? Pt[d].v : k == 6 + d ? Lt[d].v : r;
+        // xx, xy, xz, yy, yz, zz
+        return k == 9 ? c[0] : k == 10 ? c[5] : k == 11 ? c[4] : k == 12 ? c[1] : k == 13 ? c[3] : k == 14 ? c[2] : r;
+      };
+      double b, w;
+      ok = transrot_quad(tot, lane, itm.v, 0.0, N <= 2, b, w);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        vt[d] = D(__shfl_sync(0xffffffffu, b, d, 4));
+        va[d] = D(__shfl_sync(0xffffffffu, w, d, 4));
+      }
+    } else {
+      const double Lv[3] = {Lt[0].v, Lt[1].v, Lt[2].v};
+      double w[3];
+      ok = transrot_solve(c, Lv, N <= 2, w);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        vt[d] = Pt[d] * itm;
+        va[d] = D(w[d]);
+      }
+    }
+    if (!real) continue;
+    if (!ok) {
+      if (lane == 0) atomicOr(&sstat[gg], CR_TRAJ_SINGULAR_INERTIA);
+      continue;
+    }
+    for (int v = lane; v < 4; v += L)
+#pragma unroll
+      for (int i = v; i < N; i += 4)
+        for (int j = 0; j < U; ++j) {
+          D x[3];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) x[d] = D(q[(3 * i + d) * U + j]) - xt[d];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            const int e = d == 2 ? 0 : d + 1, g = d == 0 ? 2 : d - 1;
+            const D u = va[e] * x[g] + (vt[d] - va[g] * x[e]);
+            p[(3 * i + d) * U + j] = (double)(D(p[(3 * i + d) * U + j]) - D(prm.mass[i]) * u);
+          }
+        }
+  }
 }
 
 // x[k] of an array in registers
@@ -1062,10 +1167,10 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
 
     // transrot (src/transrot.f90:36-237): removed COM velocity and rotation
     // centre both carry Caracal's extra 1/P (total mass P^2 sum m)
-    if (prm.transrot && U <= kFewBeads) {
-      for (int gg = tid; gg < ng; gg += nth)
-        if (!transrot_thread<N>(sq + gg * NC * U, sp + gg * NC * U, U, P, prm.pair, prm.mass, prm.itm))
-          atomicOr(&sstat[gg], CR_TRAJ_SINGULAR_INERTIA);
+    const bool few = PES::kLanes > 1 ? P == 1 : U <= 2;
+    if (prm.transrot && few) {
+      if (PES::kLanes > 1 || 4 * gpb <= nth) transrot_few<N, 4>(prm, sq, sp, ng, sstat);
+      else if constexpr (PES::kLanes == 1) transrot_few<N, 1>(prm, sq, sp, ng, sstat);
       __syncthreads();
     } else if (prm.transrot) {
       // rows of q and p as limbs; per atom the bead sums of p, q, q_a p_b and
@@ -1129,7 +1234,7 @@ __global__ void __launch_bounds__(kStepThreads, MINB) rpmd_run_kernel(const __gr
       __syncthreads();
     }
 
-    if (drawn && n < nsteps && (!prm.transrot || U <= kFewBeads)) {
+    if (drawn && n < nsteps && (!prm.transrot || few)) {
       for (int x = tid; x < flat; x += nth) sp[x] = between(x, sp[x]);
       __syncthreads();
     }

@@ -41,3 +41,25 @@ def test_few_beads(require_gpu, pes, ntraj, nbeads, away):
         errs = [rel_err(a, b) for a, b in ((qg, q), (pg, p), (fg, f), (eg, eo))]
         assert max(errs) <= 1e-12, errs
     e.close()
+
+
+@pytest.mark.parametrize("pes,per_bead", [("oh3", (1, 2, 4)), ("ch4h", (1,))])
+@pytest.mark.parametrize("nbeads", [1, 2, 3])
+def test_shapes_agree(require_gpu, pes, per_bead, nbeads):
+    """A trajectory by four lanes where the block has the threads, else by one: the same bits."""
+    wl, T, group = CONFIG[pes](), 150, 1 << (nbeads - 1).bit_length()
+    out = []
+    for tpb in per_bead:
+        for groups in (1, 7, 40, 64):
+            block = groups * group * tpb
+            if block > 256:
+                continue
+            e = RPMDEngine(pes, wl.mass, nbeads, T, wl.dt_au, beta=wl.beta, thermostat="andersen", andersen_step=3, seed=3)
+            e.init_positions(wl.q0, float(angstrom_to_bohr(0.02)))
+            e.init_momenta()
+            e.compute_forces()
+            e.set_launch(block, tpb)
+            e.run(10)
+            out.append(e.get_state())
+            e.close()
+    assert len(out) > 2 and all(np.array_equal(x, y) for o in out[1:] for x, y in zip(o, out[0]))
