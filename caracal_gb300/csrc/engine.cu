@@ -158,7 +158,8 @@ __global__ void __launch_bounds__(kFluxThreads) child_flux_kernel(int T, int P, 
 // kappa(t) numerator and denominator: num[s] = sum_t w[t] [xi_t > 0 after step s+1],
 // and *denom = sum_t w[t] [wpos].  32 steps per block (a row of side is read
 // together), kKappaRows partial sums over the trajectories added in order
-// (deterministic).  One thread per step took 693 us for 4096 x 40 
+// (deterministic).  One thread per step over all children took 693 us for 4096 of them and
+// 40 steps, this 95.
 constexpr int kKappaRows = 32;
 __global__ void __launch_bounds__(32 * kKappaRows) kappa_kernel(int T, int nsteps, int stride, const unsigned char* side,
                                                                 const double* w, const int* wpos, double* num,
@@ -895,7 +896,9 @@ bool set_launch_shape(cr_engine* e, int block, int tpb) {
 // latency-bound: one trajectory per block, with as many threads per bead as the
 // surface has.  A larger one takes the number of trajectories per block with
 // the least work per scheduler: SMs in whole blocks, resident blocks as
-// registers and shared memory allow, a wave costing its warps per scheduler.
+// registers and shared memory allow, a wave costing its warps per scheduler. The
+// model's constants were fitted to the four shapes named below; where they are off, it
+// costs time alone, and the autotuner measures.
 void choose_launch(cr_engine* e) {
   int sms = 152;
   int dev = 0;
@@ -1375,10 +1378,11 @@ static int engine_create(const cr_config* cfg, cr_qmdff* ff, cr_evb* evb, cr_wat
       return cleanup_fail(fail(CR_ERR_CUDA, "device allocation of the momenta's antisymmetric part failed"));
     s.anti = e->d_anti;
   }
-  // fast transforms from 32 beads on: a row's transform is one chain of some
+  // fast transforms for 32 and 64 beads: a row's transform is one chain of some
   // hundred products on one lane, which 16 beads do not repay (H3 64 x 16 PILE
   // mixed 36 us per step against 32 with the matrix products on all lanes; CH4 + H
-  // 4096 x 32 mixed 102 against 122, CH4 + OH 512 x 64 mixed 80 against 118)
+  // 4096 x 32 mixed 102 against 122, CH4 + OH 512 x 64 mixed 80 against 118), nor for
+  // 128, whose arrays of 2 x 65 64-bit values a lane's registers do not hold
   if (s.pair && (e->P == 32 || e->P == 64)) {
     if (!upload_fast_ring(e, cfg->beta, cfg->dt, s.fast))
       return cleanup_fail(fail(CR_ERR_CUDA, "upload of the ring tables failed"));

@@ -298,7 +298,9 @@ using QmdffKernel = void (*)(cr::qmdff::Dev, int, cr::BeadRows, const double*, d
 constexpr int kVariants = 3;
 // [precision][variant]: blocks per SM 1 / 2 / 3 (FP64), 5 / 7 / 8 (mixed:
 // its stalls are on shared memory and L1, which warps hide better than registers:
-// C20H42 1024 x 64, per step 1434 us with 6 blocks, 1282 with 7, 1256 with 8)
+// C20H42 1024 x 64, per step 1434 us with 6 blocks, 1282 with 7, 1256 with 8; molecules
+// whose shared memory allows fewer are no slower for the cap: against the kernels before,
+// 4 to 6 blocks, C100H202 512 beads 1.33 -> 0.87 ms, C200H402 256 beads 4.92 -> 2.91)
 const QmdffKernel kKernels[2][kVariants] = {
     {cr::qmdff_egrad_kernel<false, 1>, cr::qmdff_egrad_kernel<false, 2>, cr::qmdff_egrad_kernel<false, 3>},
     {cr::qmdff_egrad_kernel<true, 5>, cr::qmdff_egrad_kernel<true, 7>, cr::qmdff_egrad_kernel<true, 8>}};

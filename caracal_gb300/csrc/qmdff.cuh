@@ -1,9 +1,10 @@
-// QMDFF force field on the GB300: one warp per bead in the mixed form, four in FP64.
+// QMDFF force field on the GB300: one warp per bead in the mixed form, a block of eight
+// (kTeam) in FP64, of one to eight for Hessian products.
 //
 // Drop-in for Caracal's per-bead QMDFF gradient (src/gradient.f90:342-358:
 // ff_eg src/ff_eg.f90:41-629, ff_nonb src/ff_nonb.f90:34-889, E_zero shift),
-// non-periodic, one molecule.  A bead's coordinates and gradient live in the
-// warp's shared memory.  A lane evaluates a term and writes its gradient into a
+// non-periodic, one molecule.  A bead's coordinates and gradient live in
+// shared memory.  A lane evaluates a term and writes its gradient into a
 // buffer in shared memory; once a segment of terms is done, every coordinate
 // sums what the segment holds for it, along lists that the host prepared.  No
 // atomics, fixed accumulation order: results are deterministic run to run.
@@ -914,9 +915,10 @@ __device__ __forceinline__ double signed_value(const double* buf, unsigned e) {
 // Warps per bead of the FP64 forms.  An FP64 instruction holds its scheduler's
 // pipe 64 cycles, so four warps could fill an SM's four pipes, and two per pipe hide
 // the loads and the barriers; a bead is spread over eight: a small batch then takes an
-// eighth of the time, a large one as long as with a warp per bead.  With the terms of qmdff_plain.cuh, whole calls: the adjoint of 16 x 16
-// beads of C20H42 over 20 steps 47.4 -> 11.3 ms, C13H28 100 x 48, four steps 4.82 ->
-// 1.82 ms.
+// eighth of the time.  With the terms of qmdff_plain.cuh, against a warp per bead and
+// their former terms, whole calls: the adjoint of 16 x 16 beads of C20H42 over 20 steps 47.4 ->
+// 11.3 ms, C13H28 100 x 48, four steps 4.82 -> 1.82 ms; gradients of 65 536 beads of C2H6 4.96
+// -> 3.38 ms, 16 384 of C4H10 1.56 -> 0.92, 1024 of C50H102 3.23 -> 1.70.
 constexpr int kTeam = 8;
 
 // The segment's values of one term at its slot i.

@@ -9,7 +9,7 @@
 // multiplications instead of some 290.  Rounding errors over C20H42 geometries are
 // no larger than the reference formulas' in FP64 (bead spreads 0.02 to 0.1 bohr, of
 // the largest force: torsions 4e-16 against 5e-16).  Measured with the
-// four warps per bead: see kTeam.
+// eight warps per bead: see kTeam.
 #pragma once
 
 #include "dual.cuh"

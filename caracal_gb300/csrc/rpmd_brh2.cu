@@ -3,5 +3,5 @@
 #include "rpmd_inst.cuh"
 
 namespace cr {
-const PesRuns kRunsBrH2 = RunsOf<PesBrH2, 1, 2, 2>::table();
+const PesRuns kRunsBrH2 = RunsOf<PesBrH2, 1>::table();
 }  // namespace cr

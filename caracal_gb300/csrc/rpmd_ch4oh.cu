@@ -3,5 +3,5 @@
 #include "rpmd_inst.cuh"
 
 namespace cr {
-const PesRuns kRunsCH4OH = RunsOf<PesCH4OH, 1, 2, 2>::table();
+const PesRuns kRunsCH4OH = RunsOf<PesCH4OH, 1>::table();
 }  // namespace cr

@@ -3,5 +3,5 @@
 #include "rpmd_inst.cuh"
 
 namespace cr {
-const PesRuns kRunsGeH4OH = RunsOf<PesGeH4OH, 1, 2, 2>::table();
+const PesRuns kRunsGeH4OH = RunsOf<PesGeH4OH, 1>::table();
 }  // namespace cr

@@ -3,5 +3,5 @@
 #include "rpmd_inst.cuh"
 
 namespace cr {
-const PesRuns kRunsH3 = RunsOf<PesH3, 4, 2, 2>::table();
+const PesRuns kRunsH3 = RunsOf<PesH3, 4>::table();
 }  // namespace cr

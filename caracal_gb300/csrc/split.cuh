@@ -7,7 +7,9 @@
 //   (force kernel)       dV/dq and V of every bead
 //   split_kick_kernel    1/2 kick, Andersen resample or PILE half
 //   split_nhc_kernel     Nose-Hoover chain (NHC only)
-//   split_finish_kernel  NaN check, transrot, epot per trajectory
+//   split_berendsen_kernel  pressure and box scaling (NpT only)
+//   split_moments_kernel, split_solve_kernel, split_apply_kernel
+//                        NaN check, transrot, epot per trajectory
 //   split_advance_kernel step counter + 1
 // The order is Caracal's verlet (src/verlet.f90:216-218, 377-463, 772-777,
 // 1060-1062, 1159-1165, 1256-1306).  The step index lives on the device so a
@@ -75,7 +77,7 @@ struct SplitParams {
   // transrot / energy scratch of split_moments_kernel and split_solve_kernel
   double* fsum;            // [T][S][16] partial sums per slice
   int* fstat;              // [T][S] status bits per slice
-  double* fmove;           // [T][10] vt, xt, va, skip flag
+  double* fmove;           // [T][10] b, va, (3 unused), skip flag: kMoveDoubles
 };
 
 constexpr int kSplitBlock = 128;
@@ -559,7 +561,7 @@ __global__ void split_parent_init_kernel(SplitParams s) {
 constexpr int kMomentThreads = 256;
 constexpr int kApplyItems = 4 * kMomentThreads;  // items of one block of split_apply_kernel
 constexpr int kFinishSums = 16;   // 15 moments + sum of bead energies
-constexpr int kMoveDoubles = 10;  // b = vt - va x xt, va, (unused), skip flag per trajectory
+constexpr int kMoveDoubles = 10;  // b = vt - va x xt, va, (3 unused), skip flag per trajectory
 
 // slices per trajectory of split_moments_kernel: about 4 items per thread
 __host__ __device__ inline int finish_slices(int items) {
