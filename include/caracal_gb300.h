@@ -66,7 +66,8 @@ typedef struct cr_config {
   int transrot;       /* 1: remove COM translation/rotation each step (dynamic.x); 0: off (recrossing children) */
   int precision;      /* CR_PREC_* */
   unsigned int seed;  /* Gaussian stream key */
-  unsigned int traj0; /* global index of this engine's first trajectory (stream key) */
+  unsigned int traj0; /* global index of this engine's first trajectory (stream key); on the analytic surfaces a trajectory's
+                       * numbers are those of its state, seed and index, however many others share the engine */
   double dt;          /* time step, a.u. (Caracal: DELTAT[fs] / 2.41888428E-2 as REAL(4)) */
   double beta;        /* 1/(k_B T), a.u., k_B = 0.316679e-5 Eh/K */
   double pile_tau0;   /* PILE centroid time constant, a.u. */
@@ -405,7 +406,10 @@ int cr_engine_init_momenta(cr_engine* e, int zero);
 int cr_engine_compute_forces(cr_engine* e);
 
 /* Host <-> engine state, arrays (3, natoms, nbeads, ntraj).  f (dV/dq of the
- * current positions) may be NULL in set_state; it is then recomputed. */
+ * current positions) may be NULL in set_state; it is then recomputed.  A state that is set in an
+ * engine at the same step (the noise is a function of the step index) continues as
+ * the run that it was taken from, bit for bit (but for what an engine keeps besides:
+ * Nose-Hoover chains, NpT boxes, windows' statistics). */
 int cr_engine_set_state(cr_engine* e, const double* q, const double* p, const double* f);
 int cr_engine_get_state(cr_engine* e, double* q, double* p, double* f, double* epot, int* status);
 
