@@ -223,23 +223,16 @@ __device__ inline F torsion_plain(const Dev& D, const Tables<double>& T, const B
     // (three atoms in line) the angle is the arc cosine of the product so formed, and its
     // derivative is left out
     const bool bent = nan_ > 1e-14 && nbn > 1e-14;
-    F s = dot3(na, nb);
-    if (nan_ > 1e-14) s = s * ina;
-    if (nbn > 1e-14) s = s * inb;
+    const F ua = nan_ > 1e-14 ? ina : F(1), ub = nbn > 1e-14 ? inb : F(1);
+    F s = dot3(na, nb) * ua * ub;
+    // |na x nb| = |rb| |na . rc|; in line 1, with which p_angle_of takes the arc cosine
     const F tr = dot3(na, vdc);
-    sinphi = F(0);
-    if (bent) {
-      // |na x nb| = |rb| |na . rc|
-      sinphi = (L * (ina * inb)) * fabs(tr);
-      if (::fabs(::fabs(ad::val(s)) - 1.0) < 1e-14) {
-        s = ad::val(s) >= 0 ? F(1.0) : F(-1.0);
-        sinphi = F(0);
-      }
-      phi = p_angle_of(s, sinphi);
-    } else {
-      F sine;
-      p_angle(s, phi, sine);
+    sinphi = bent ? (L * (ua * ub)) * fabs(tr) : F(1);
+    if (bent && ::fabs(::fabs(ad::val(s)) - 1.0) < 1e-14) {
+      s = ad::val(s) >= 0 ? F(1.0) : F(-1.0);
+      sinphi = F(0);
     }
+    phi = p_angle_of(s, sinphi);
     F ef, expo;
     p_erf(phi - pi, ef, expo);
     const F h1 = 0.5 - 0.5 * ef, h2 = 0.5 + 0.5 * ef;
@@ -265,7 +258,7 @@ __device__ inline F torsion_plain(const Dev& D, const Tables<double>& T, const B
     // where it is no number: the reciprocals are infinite then)
     F wa = F(0), wb = F(0), wu = F(0), wv = F(0);
     if (bent && nan_ * nbn * sinphi >= 1e-14) {
-      const F ia2 = ina * ina, ib2 = inb * inb;
+      const F ia2 = ua * ua, ib2 = ub * ub;
       const F w = tr < 0.0 ? dij : -dij;
       const F wl = w * L, wi = w * iL;
       wa = wl * ia2;
