@@ -323,14 +323,19 @@ __device__ inline F bends(const Pairs* X, Bond<F>& G, int i) {
     F sum2 = F(0), sum4 = F(0), w[3] = {F(0), F(0), F(0)};
 #pragma unroll
     for (int k = 1; k < 4; ++k) {
-      const F arg = -(c[k] * sn);
+      F arg = -(c[k] * sn), sin2 = F(1) - arg * arg;
+      if constexpr (kPair) {
+        // a bond along the normal: FP32 may round past +-1, and sin^2 to 0
+        arg = fminf(1.f, fmaxf(-1.f, arg));
+        sin2 = fmaxf((1.f - arg) * (1.f + arg), 1.2e-7f);
+      }
       const F dl = (m_acos<F>(arg) - F(tau)) - (th[k] + tau_lo);
       const F d2 = dl * dl;
       sum2 += d2;
       sum4 += d2 * d2;
       const F coef = (sw * dl) * (F(2.0 * K::fch3) + F(4.0 * K::hch3) * d2);
       bth[k] = -(coef + of(coef, k));
-      const F ba = coef * m_rsqrt<F>(F(1) - arg * arg);  // -dV/d arg, arg = -n.u
+      const F ba = coef * m_rsqrt<F>(sin2);  // -dV/d arg, arg = -n.u
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
         w[d] += ba * un[k][d];
@@ -381,7 +386,7 @@ __device__ inline F bends(const Pairs* X, Bond<F>& G, int i) {
     for (int round = 0; round < 2; ++round) {
       const int k = round == 0 ? first : 3, src = (int)(threadIdx.x & 3) ^ k;
       const F thk = k == 1 ? th[1] : k == 2 ? th[2] : th[3];
-      F cs, dt;
+      F cs, dt, sin2;
       if constexpr (kPair) {
         // theta - tau as asin(sin(theta - tau)) from a float-pair cosine:
         // theta - th0 is a small difference of two ~1.9 rad angles, which
@@ -389,8 +394,11 @@ __device__ inline F bends(const Pairs* X, Bond<F>& G, int i) {
         const ff c = (X->tch[0] * from(X->tch[0], src) + X->tch[1] * from(X->tch[1], src) +
                       X->tch[2] * from(X->tch[2], src)) / (X->rch * from(X->rch, src));
         constexpr ff kCosTau = ff_const(-1.0 / 3.0), kSinTau = ff_const(0.94280904158206336587);
-        const ff y = ff_sqrt(ff_from(1.f) - c * c) * kCosTau - c * kSinTau;
+        const ff sq = ff_from(1.f) - c * c, y = ff_sqrt(sq) * kCosTau - c * kSinTau;
         cs = ff_float(c);
+        // two bonds in line (one of them broken, its stiffness about 0): the FP32
+        // 1 - cs^2 is 0 there, and 0 / 0 the force; the pair's has 2^-44
+        sin2 = fmaxf(sq.hi, 1e-12f);
         const float dtau = fabsf(y.hi) < 0.9f ? asinf(y.hi) + y.lo * m_rsqrt<float>(1.f - y.hi * y.hi)
                                               : acosf(cs) - F(tau);
         dt = dtau - thk;
@@ -399,8 +407,9 @@ __device__ inline F bends(const Pairs* X, Bond<F>& G, int i) {
                         k == 1 ? un[1][2] : k == 2 ? un[2][2] : un[3][2]};
         cs = dot3(G.u, v);
         dt = (m_acos<F>(cs) - F(tau)) - thk;
+        sin2 = F(1) - cs * cs;
       }
-      const F s = m_rsqrt<F>(F(1) - cs * cs);
+      const F s = m_rsqrt<F>(sin2);
       if (round == 0) {
         const F dt2 = from(dt, (int)(threadIdx.x & 3) ^ other), s2 = from(s, (int)(threadIdx.x & 3) ^ other);
         dth[1] = first == 1 ? dt : dt2;
