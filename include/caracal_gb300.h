@@ -590,7 +590,7 @@ int cr_engine_get_launch(cr_engine* e, int* threads_per_block, int* blocks, int*
 /* Autotuner: times nsteps steps at each launch shape (threads per bead 1, 2,
  * 4 as built; from one trajectory per block up to the fullest block),
  * each from the same saved state, which is then put back (q, p, f, epot,
- * status, chain velocities, a thermostat's momentum parts, step counter);
+ * status, chain velocities, step counter);
  * keeps the fastest and returns it, as cr_engine_set_launch takes it, with its time per step.  The noise is a
  * function of the step index, so the trials leave no trace in the run. */
 int cr_engine_autotune(cr_engine* e, int nsteps, int* threads_per_block, int* threads_per_bead,
